@@ -403,3 +403,67 @@ def test_bulk_staged_wait_runs_out_and_the_handle_recovers():
     _same(sim, fresh)
     sim.close()
     fresh.close()
+
+
+def _roomy(n, seed, mu, history, picard=False):
+    """packed_poly in a box that holds n grains."""
+    cfg, st, rad = packed_poly(n=n, seed=seed, mu=mu, history=history, picard=picard)
+    L = 0.5 * 0.95 * 5e-3 * np.ceil(n ** (1 / 3)) + 2e-3
+    ph = cfg.physics
+    for ax in "xyz":
+        setattr(cfg.domain, f"{ax}_min", -L)
+        setattr(cfg.domain, f"{ax}_max", L)
+        setattr(cfg, f"collision_grid_size_{ax}", int(2 * L / 7e-3))
+    ph.wall_x_min = ph.wall_y_min = ph.floor_z = -L
+    ph.wall_x_max = ph.wall_y_max = ph.ceiling_z = L
+    cfg.kernel_timing = False
+    return cfg, st, rad
+
+
+@pytest.mark.parametrize("n,history,picard", [(31, True, False), (33, False, False), (16383, True, False),
+                                              (16385, True, False), (20011, False, False),
+                                              (17001, True, True), (2049, True, True)])
+def test_contact_parallel_kernel_equals_search(n, history, picard):
+    """The contact-parallel kernel on both sides of its lanes-per-grain rule (four lanes
+    below 16,384 grains, one from there), with more contacts in a warp than one round
+    holds and with grains whose contacts a cell crossing re-ordered, against the searched
+    step bit for bit (both are sums in the canonical order, so no tolerance)."""
+    cfg, st, rad = _roomy(n, 50, 0.5, history, picard)
+    st = st.copy()
+    st[:, 3:] *= 10
+    sims = []
+    for skin in (0.0, 0.6e-3):
+        c = cfg.copy()
+        c.neighbor_skin = skin
+        sim = ParticleDynamics(c, state=st, radius=rad)
+        if skin:
+            sim.set_contact_kernel(256, 0)
+        sim.advance(30)
+        sims.append(sim)
+    _same(*sims)
+    assert sims[1].get_history()[0].sum() > 0 or not history
+    if n > 1000:
+        assert sims[1].list_resort_count() > 0
+
+
+@pytest.mark.parametrize("small", [30, 32, 33, 40, 47, 60])
+def test_contact_parallel_kernel_many_contacts_on_one_grain(small):
+    """A large grain touched by `small` others: up to 32 contacts are evaluated together,
+    more (or a list that overflows its 48 entries) by the grain's own lane."""
+    cfg, _, _ = packed_poly(n=8, seed=51, mu=0.5)
+    cfg.physics.gravity = 0.0
+    cfg.kernel_timing = False
+    for ax in "xyz":
+        setattr(cfg, f"collision_grid_size_{ax}", 4)
+    k = np.arange(small) + 0.5
+    z = 1 - 2 * k / small
+    phi = k * np.pi * (1 + 5 ** 0.5)
+    unit = np.stack([np.sqrt(1 - z * z) * np.cos(phi), np.sqrt(1 - z * z) * np.sin(phi), z], 1)
+    state = np.zeros((small + 1, 6), np.float32)
+    state[1:, :3] = unit * (10e-3 + 1.2e-3 - 1e-5)
+    state[1:, 3:] = np.random.default_rng(52).normal(0, 0.1, (small, 3))
+    radius = np.full(small + 1, 1.2e-3, np.float32)
+    radius[0] = 10e-3
+    ref, lst = _pair(cfg, state, radius, 40, 0.5e-3)
+    _same(ref, lst)
+    assert lst.tuning()["contact_variant"] == "warp-cooperative"

@@ -233,6 +233,13 @@ __device__ __forceinline__ void wall_forces(const DevParams& P, float3 pos, floa
     // the dashpot coefficient only where a wall is touched (most grains touch none)
     auto c_wall = [&]() { return damping(P, mi); };
     f.z = fmaf(-mi, P.gravity, f.z);
+    // A grain clear of all six walls adds six zeros (of either sign, to sums that such a
+    // zero leaves as they are): skipped. NaN takes the long way.
+    const float clear = fminf(
+        fminf(fminf((pos.x - P.wall_lo[0]) - ri, (P.wall_hi[0] - pos.x) - ri),
+              fminf((pos.y - P.wall_lo[1]) - ri, (P.wall_hi[1] - pos.y) - ri)),
+        fminf((pos.z - P.wall_lo[2]) - ri, (P.wall_hi[2] - pos.z) - ri));
+    if (clear > 0.f) return;
     const float p3[3] = {pos.x, pos.y, pos.z};
     const float v3[3] = {vel.x, vel.y, vel.z};
 #pragma unroll

@@ -298,50 +298,10 @@ __device__ __forceinline__ void prefetch_l1(const void* p) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
-// The contacts of a grain whose list entries a cell crossing re-ordered, in canonical
-// order: each pass takes the smallest visiting key above the last. (Inlined: an
+// The contacts (bitmask over list entries) of a grain that a cell crossing re-ordered, in
+// canonical order: each pass takes the smallest visiting key above the last. (Inlined: an
 // out-of-line call copies the parameter structs to local memory at kernel entry, which
 // was measured to cost more than the code it moves away.)
-template <bool HIST>
-__device__ __forceinline__ void list_contacts_sorted(const DevParams& P, const ListArgs& A, int s,
-                                                  int n, int cnt, float4 pi, float3 vel,
-                                                  float mi, float cut, int cx, int cy, int cz,
-                                                  float3& f, HistRow& h) {
-    const float ri = pi.w;
-    long long done = -1;
-    for (;;) {
-        long long best = 0x7fffffffffffffffll;
-        int bj = -1;
-        for (int e = 0; e < cnt; ++e) {
-            const int j = __ldg(&A.nbr[static_cast<int64_t>(e) * n + s]);
-            const float4 pj = __ldg(&A.pos[j]);
-            float3 d;
-            const float ns = pair_norm_sq(pi, pj, d);
-            if (ns > cut) continue;
-            const float dist = pair_dist(sqrtf(ns), ri, pj.w);
-            if (!(dist < 0.f)) continue;
-            const long long key =
-                static_cast<long long>(visit_key(P, cx, cy, cz, pj, __ldg(&A.ids[j])));
-            if (key > done && key < best) {
-                best = key;
-                bj = j;
-            }
-        }
-        if (bj < 0) break;
-        done = best;
-        const float4 pj = __ldg(&A.pos[bj]);
-        float3 d;
-        const float ns = pair_norm_sq(pi, pj, d);
-        const float norm = sqrtf(ns);
-        const float dist = pair_dist(norm, ri, pj.w);
-        const float4 vj = __ldg(&A.vel[bj]);
-        pair_force<HIST>(P, d, norm, dist, vel, mi, vj, static_cast<int>(best & 0xffffffffll),
-                         f, h, A.counters);
-    }
-}
-
-// The same for a grain whose contacts the scan found (bitmask over list entries): each
-// pass visits the contacts only, and takes the smallest visiting key above the last.
 template <bool HIST>
 __device__ __forceinline__ void list_contacts_sorted_mask(const DevParams& P, const ListArgs& A,
                                                        int s, int n, unsigned long long hits,
@@ -405,6 +365,78 @@ __device__ __forceinline__ void list_contacts_table(const DevParams& P, const Li
     }
 }
 
+// Whether a list entry at pj touches the grain at pi. The exact test takes a square root;
+// it decides only for pairs within 1e-5 of touching or closer: dist < 0 needs
+// |d| < r_i + r_j up to a few roundings of 2^-24, so a pair beyond that margin is no contact.
+__device__ __forceinline__ bool entry_hit(float4 pi, float4 pj) {
+    float3 d;
+    const float ns = pair_norm_sq(pi, pj, d);
+    const float rs = pi.w + pj.w;
+    return ns <= rs * rs * 1.00001f && pair_dist(sqrtf(ns), pi.w, pj.w) < 0.f;
+}
+
+// A slot of a frozen scene: its state copied through.
+template <bool HIST>
+__device__ __forceinline__ void list_copy_frozen(const ListArgs& A, int s, int scene, float4 pi,
+                                                 float4 vi, int id, bool order_out) {
+    A.pos_out[s] = pi;
+    A.vel_out[s] = vi;
+    if (order_out) {
+        A.ids_out[s] = id;
+        A.scene_out[s] = scene;
+    }
+    A.acc_out[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (HIST) A.hcnt_out[s] = 0;
+}
+
+// The integrator and the displacement measures of one grain under the force f, with
+// `out_count` springs written. order_out: write the slot's id (and scene) too.
+template <bool HIST, bool BATCH, bool PICARD>
+__device__ __forceinline__ void list_integrate(const DevParams& P, const ListArgs& A, int s,
+                                               int scene, float4 pi, float4 vi, int id, float3 f,
+                                               int out_count, float4 xb, bool exact,
+                                               bool order_out, uint32_t& disp_bits,
+                                               uint32_t& step_bits, uint32_t& res_bits) {
+    const float mi = vi.w;
+    const float3 pos = make_float3(pi.x, pi.y, pi.z);
+    if (HIST) A.hcnt_out[s] = out_count;
+    const float3 a = make_float3(f.x / mi, f.y / mi, f.z / mi);
+    float3 v1, x1;
+    if (!PICARD) {
+        v1 = make_float3(fmaf(P.dt, a.x, vi.x), fmaf(P.dt, a.y, vi.y), fmaf(P.dt, a.z, vi.z));
+        x1 = make_float3(fmaf(P.dt, v1.x, pos.x), fmaf(P.dt, v1.y, pos.y), fmaf(P.dt, v1.z, pos.z));
+    } else {
+        const float4 xn = A.xn[s], vn = A.vn[s];
+        v1 = make_float3(fmaf(P.dt, a.x, vn.x), fmaf(P.dt, a.y, vn.y), fmaf(P.dt, a.z, vn.z));
+        x1 = make_float3(fmaf(P.dt, v1.x, xn.x), fmaf(P.dt, v1.y, xn.y), fmaf(P.dt, v1.z, xn.z));
+        res_bits = max(res_bits, __float_as_uint(fabsf(x1.x - pos.x)));
+        res_bits = max(res_bits, __float_as_uint(fabsf(x1.y - pos.y)));
+        res_bits = max(res_bits, __float_as_uint(fabsf(x1.z - pos.z)));
+    }
+    A.pos_out[s] = make_float4(x1.x, x1.y, x1.z, pi.w);
+    A.vel_out[s] = make_float4(v1.x, v1.y, v1.z, mi);
+    if (order_out) {
+        A.ids_out[s] = id;
+        if (BATCH) A.scene_out[s] = scene;
+    }
+    A.acc_out[s] = make_float4(a.x, a.y, a.z, 0.f);
+    if (exact) disp_bits = max(disp_bits, disp_sq_bits(x1, xb));
+    if (!PICARD) step_bits = max(step_bits, disp_sq_bits(x1, pos));
+}
+
+// End of a Picard iteration's kernel: residual, validity and iteration counters.
+__device__ __forceinline__ void list_picard_report(const ListArgs& A, uint32_t res_bits, bool viol) {
+    // max of non-negative float bits (NaN above +inf, so it is kept)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) res_bits = max(res_bits, __shfl_xor_sync(0xffffffffu, res_bits, o));
+    if ((threadIdx.x & 31) == 0 && res_bits != 0u) atomicMax(A.res_slot, res_bits);
+    if (__any_sync(0xffffffffu, viol) && (threadIdx.x & 31) == 0) atomicOr(&A.list_ctrl[kLcViol], 1u);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *A.picard_used = A.iter + 1;
+        A.counters[kCntPicardIters] += 1ull;
+    }
+}
+
 // One grain of the list contact kernels, its per-slot values already loaded: contacts
 // from the list in canonical order (or the run table when the list overflowed), the
 // integrator, the displacement measures (maxima folded into disp_bits / step_bits /
@@ -429,14 +461,7 @@ __device__ __forceinline__ void list_grain(const DevParams& P0, const ListArgs& 
         }
     }
     if (BATCH && P.frozen) {
-        A.pos_out[s] = pi;
-        A.vel_out[s] = vi;
-        if (order_out) {
-            A.ids_out[s] = id;
-            A.scene_out[s] = scene;
-        }
-        A.acc_out[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (HIST) A.hcnt_out[s] = 0;
+        list_copy_frozen<HIST>(A, s, scene, pi, vi, id, order_out);
     } else {
         const float3 pos = make_float3(pi.x, pi.y, pi.z);
         const float3 vel = make_float3(vi.x, vi.y, vi.z);
@@ -476,10 +501,7 @@ __device__ __forceinline__ void list_grain(const DevParams& P0, const ListArgs& 
                     for (int u = 0; u < 4; ++u) pp[u] = __ldg(&A.pos[jj[u]]);
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        float3 d;
-                        const float ns = pair_norm_sq(pi, pp[u], d);
-                        const bool hit = e0 + u < cnt && !(ns > cut) &&
-                                         pair_dist(sqrtf(ns), ri, pp[u].w) < 0.f;
+                        const bool hit = e0 + u < cnt && entry_hit(pi, pp[u]);
                         hits |= hit ? (1ull << (e0 + u)) : 0ull;
                         // the contact's partner id and velocity are read after the scan
                         if (PREFETCH && hit) {
@@ -525,33 +547,8 @@ __device__ __forceinline__ void list_grain(const DevParams& P0, const ListArgs& 
                 list_contacts_table<HIST>(P, A, s, pi, vel, mi, cut, cx, cy, cz, f, h);
             }
         }
-        if (HIST) A.hcnt_out[s] = h.out_count;
-        const float3 a = make_float3(f.x / mi, f.y / mi, f.z / mi);
-        float3 v1, x1;
-        if (!PICARD) {
-            v1 = make_float3(fmaf(P.dt, a.x, vel.x), fmaf(P.dt, a.y, vel.y),
-                             fmaf(P.dt, a.z, vel.z));
-            x1 = make_float3(fmaf(P.dt, v1.x, pos.x), fmaf(P.dt, v1.y, pos.y),
-                             fmaf(P.dt, v1.z, pos.z));
-        } else {
-            const float4 xn = A.xn[s], vn = A.vn[s];
-            v1 = make_float3(fmaf(P.dt, a.x, vn.x), fmaf(P.dt, a.y, vn.y),
-                             fmaf(P.dt, a.z, vn.z));
-            x1 = make_float3(fmaf(P.dt, v1.x, xn.x), fmaf(P.dt, v1.y, xn.y),
-                             fmaf(P.dt, v1.z, xn.z));
-            res_bits = max(res_bits, __float_as_uint(fabsf(x1.x - pos.x)));
-            res_bits = max(res_bits, __float_as_uint(fabsf(x1.y - pos.y)));
-            res_bits = max(res_bits, __float_as_uint(fabsf(x1.z - pos.z)));
-        }
-        A.pos_out[s] = make_float4(x1.x, x1.y, x1.z, ri);
-        A.vel_out[s] = make_float4(v1.x, v1.y, v1.z, mi);
-        if (order_out) {
-            A.ids_out[s] = id;
-            if (BATCH) A.scene_out[s] = scene;
-        }
-        A.acc_out[s] = make_float4(a.x, a.y, a.z, 0.f);
-        if (exact) disp_bits = max(disp_bits, disp_sq_bits(x1, xb));
-        if (!PICARD) step_bits = max(step_bits, disp_sq_bits(x1, pos));
+        list_integrate<HIST, BATCH, PICARD>(P, A, s, scene, pi, vi, id, f, HIST ? h.out_count : 0,
+                                            xb, exact, order_out, disp_bits, step_bits, res_bits);
     }
 }
 
@@ -603,17 +600,7 @@ k_force_list(DevParams P0, ListArgs A) {
     }
     list_disp_report<PICARD>(A.list_ctrl, exact, disp_bits, step_bits);
     if (!PICARD) list_tail_decide(A);
-    if (PICARD) {
-        // max of non-negative float bits (NaN above +inf, so it is kept)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) res_bits = max(res_bits, __shfl_xor_sync(0xffffffffu, res_bits, o));
-        if ((threadIdx.x & 31) == 0 && res_bits != 0u) atomicMax(A.res_slot, res_bits);
-        if (__any_sync(0xffffffffu, viol) && (threadIdx.x & 31) == 0) atomicOr(&A.list_ctrl[kLcViol], 1u);
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            *A.picard_used = A.iter + 1;
-            A.counters[kCntPicardIters] += 1ull;
-        }
-    }
+    if (PICARD) list_picard_report(A, res_bits, viol);
 }
 
 // ---- bulk-staged list kernel -------------------------------------------------------
@@ -991,215 +978,316 @@ __global__ void k_list_picard_check(uint32_t* __restrict__ ctrl,
     if (use_cond) cudaGraphSetConditional(cond, redo ? 1u : 0u);
 }
 
-// Warp-cooperative variant: a contact's work (spring lookup, Coulomb cap, dashpot) is
-// spread over the lanes of the warp instead of running on its grain's lane alone, then
-// every grain accumulates its contacts' terms in order. The per-lane kernel above
-// spends most issue slots on one or two active lanes when contacts are sparse.
+// Contact-parallel list kernel: a warp finds the contacts of its grains, then its lanes
+// evaluate those contacts together, one each (distance, dashpot, spring lookup, Coulomb
+// cap), and every grain adds its own contacts' terms in order. A lane evaluating its
+// grain's contacts alone runs as many rounds of that long code as the busiest of its 32
+// grains has contacts, with about one lane in four active.
 //
-// Per warp: rounds over the list entries (e = 0, 1, ...) find the contacts of the 32
-// grains and queue them (partner slot, owner lane, owner's contact rank); a full queue
-// (kCoopCap) or the last round flushes it: the lanes compute the queued contacts' terms
-// (pair_terms, the springs written to their final rows), each grain's terms land in
-// its own run of the buffer, and each lane accumulates its run in order. Contacts are
-// found in list order, which is the canonical order unless a cell crossing changed it;
-// such a grain redoes its contacts in canonical order on its own lane at the end.
-constexpr int kCoopWarps = kBlock / 32;
-constexpr int kCoopCap = 64;
+// LPG lanes share one grain (a warp holds 32 / LPG grains): they scan its list side by
+// side, and the walls, the accumulation and the integrator run on the first of them.
+//
+// Per warp: the scan leaves each grain a bitmask of the list entries in contact; a prefix
+// sum over the grains numbers the warp's contacts; up to 32 at a time (whole grains) they
+// are queued in shared memory as (owner lane, entry) and evaluated, the new springs going
+// to their final rows and the terms to shared memory, from where each owner adds its run.
+// List order is the canonical order unless a cell crossing changed it: where a contact's
+// visiting key is below its predecessor's, the grain's contacts take their places by the
+// rank of their keys. (The per-lane kernels redo such a grain alone, a chain of about 30 us
+// for the busiest: a few hundred such grains in a million set the kernel's time.)
+//
+// The slots' own values come through shared memory by asynchronous copies issued one
+// group ahead, which hides their latency without holding registers.
+//
+// Bound by load latency and issue. Measured at 64 registers, 8 blocks per SM (80 and 6 for
+// Picard, whose grid is not one wave of equal work): 2^20 falling grains 41.3 us a step
+// (per-lane 42.3; without the copies 46); 1,000,003 packed grains (8 list entries, 0.4
+// springs each) 134 against 176; 200,003 packed, 8 Picard iterations 230 against 492.
+constexpr int kCoopBlock = 128;
+constexpr int kCoopWarps = kCoopBlock / 32;
 
-struct CoopWarp {
-    int qj[kCoopCap];
-    unsigned char qg[kCoopCap];
-    unsigned char qr[kCoopCap];
-    PairTerms terms[kCoopCap];
+struct __align__(16) CoopStage {
     float4 pos[32], vel[32];
-    int id[32], hin[32], outw[32], first[32], off[32], scene[32];
+    int id[32], cnt[32], hcnt[32], scene[32];
+};
+struct __align__(16) CoopWarp {
+    CoopStage stage[2];
+    float4 term[32][2];            // (nrm, fp), (t, cvn)
+    unsigned short queue[32];      // owner lane << 6 | list entry
 };
 
-template <bool HIST, bool BATCH>
-__device__ __forceinline__ void coop_flush(const DevParams& P0, const ListArgs& A, CoopWarp& W,
-                                           int q, int lane, int my_count, int& bstart,
-                                           bool reorder, float3& f) {
-    __syncwarp();
-    const int c = my_count - bstart;
-    int off = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, off, o);
-        if (lane >= o) off += y;
-    }
-    off -= c;
-    W.first[lane] = bstart;
-    W.off[lane] = off;
-    __syncwarp();
-    for (int i = lane; i < q; i += 32) {
-        const int j = W.qj[i];
-        const int g = W.qg[i];
-        const int r = W.qr[i];
-        const DevParams& P = BATCH ? A.scene_params[W.scene[g]] : P0;
-        const float4 pi = W.pos[g], vi = W.vel[g];
-        const float4 pj = __ldg(&A.pos[j]);
-        const float4 vj = __ldg(&A.vel[j]);
-        const int jd = __ldg(&A.ids[j]);
-        float3 d;
-        const float ns = pair_norm_sq(pi, pj, d);
-        const float norm = sqrtf(ns);
-        const float dist = pair_dist(norm, pi.w, pj.w);
-        const int gid = W.id[g];
-        float3 xi = HIST ? find_spring(A.hist_in + static_cast<int64_t>(gid) * kHistCap, W.hin[g], jd)
-                         : make_float3(0.f, 0.f, 0.f);
-        W.terms[W.off[g] + (r - W.first[g])] =
-            pair_terms<HIST>(P, d, norm, dist, make_float3(vi.x, vi.y, vi.z), vi.w, vj, xi);
-        if (HIST) {
-            const int slot = W.outw[g] + r;
-            if (slot < kHistCap)
-                A.hist_out[static_cast<int64_t>(gid) * kHistCap + slot] =
-                    make_float4(xi.x, xi.y, xi.z, __int_as_float(jd));
-        }
-    }
-    __syncwarp();
-    if (!reorder)
-        for (int k = 0; k < c; ++k) pair_accumulate<HIST>(f, W.terms[off + k]);
-    __syncwarp();
-    bstart = my_count;
+__device__ __forceinline__ void async_copy16(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void async_copy4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
-// One slot per lane of the warp-cooperative kernel (all lanes of the warp together).
-template <bool HIST, bool BATCH>
-__device__ __forceinline__ void coop_slot(const DevParams& P0, const ListArgs& A, CoopWarp& W, int s, bool exact,
-                                          bool order_out, uint32_t& disp_bits,
-                                          uint32_t& step_bits) {
-    const int lane = threadIdx.x & 31;
-    const int n = P0.n;
-    const bool active = s < n;
-    // per-slot loads, up front
-    const int scene = (BATCH && active) ? A.scene[s] : 0;
-    const float4 pi = active ? A.pos[s] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 vi = active ? A.vel[s] : make_float4(0.f, 0.f, 0.f, 1.f);
-    const int id = active ? A.ids[s] : 0;
-    const int cnt_raw = active ? A.nbr_cnt[s] : 0;
-    const float4 xb = (active && exact) ? A.xbuild[s] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const int hcnt_in = (HIST && active) ? A.hcnt_in[s] : 0;
+// This lane's share of the copies of one slot group into S: the lane that carries grain s
+// copies its values. One copy group per call, possibly empty.
+template <bool HIST, bool BATCH, int LPG>
+__device__ __forceinline__ void coop_stage(const ListArgs& A, CoopStage& S, int s, int n) {
+    const int lane = threadIdx.x & 31, g = lane / LPG;
+    if (lane % LPG == 0 && s < n) {
+        async_copy16(&S.pos[g], &A.pos[s]);
+        async_copy16(&S.vel[g], &A.vel[s]);
+        async_copy4(&S.cnt[g], &A.nbr_cnt[s]);
+        async_copy4(&S.id[g], &A.ids[s]);
+        if (HIST) async_copy4(&S.hcnt[g], &A.hcnt_in[s]);
+        if (BATCH) async_copy4(&S.scene[g], &A.scene[s]);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// One slot per group of LPG lanes (all lanes of the warp together; s may be >= n).
+template <bool HIST, bool BATCH, bool PICARD, int LPG>
+__device__ __forceinline__ void coop_slot(const DevParams& P0, const ListArgs& A, CoopWarp& W,
+                                          const CoopStage& S, int s, int n, bool exact,
+                                          bool order_out, uint32_t& disp_bits, uint32_t& step_bits,
+                                          uint32_t& res_bits, bool& viol) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane % LPG, g = lane / LPG;
+    const bool live = s < n;
+    int scene = 0, id = 0, cnt = 0, hcnt_in = 0;
+    float4 pi = make_float4(0.f, 0.f, 0.f, 0.f), vi = pi;
+    if (live) {
+        scene = BATCH ? S.scene[g] : 0;
+        pi = S.pos[g];
+        vi = S.vel[g];
+        id = S.id[g];
+        cnt = S.cnt[g];
+        hcnt_in = HIST ? S.hcnt[g] : 0;
+    }
     const DevParams& P = BATCH ? A.scene_params[scene] : P0;
-    const bool frozen = BATCH && active && P.frozen;
-    const bool work = active && !frozen;
-    const float3 pos = make_float3(pi.x, pi.y, pi.z);
+    const bool frozen = BATCH && live && P.frozen;
+    const bool own = live && sub == 0;      // the lane that carries the grain
+    if (PICARD && own) {
+        // the rhs of a Picard step pairs the last iterate's velocity with its forces
+        A.rhs_vel[s] = vi;
+        A.rhs_ids[s] = id;
+        if (A.iter > 0) {
+            const float4 xb = A.xbuild[s];
+            const float ex = pi.x - xb.x, ey = pi.y - xb.y, ez = pi.z - xb.z;
+            viol |= !(ex * ex + ey * ey + ez * ez < A.viol_thr);
+        }
+    }
     const float3 vel = make_float3(vi.x, vi.y, vi.z);
     const float ri = pi.w, mi = vi.w;
     float3 f = make_float3(0.f, 0.f, 0.f);
-    HistRow h;
-    h.in = A.hist_in + static_cast<int64_t>(id) * kHistCap;
-    h.in_count = hcnt_in;
-    h.out = A.hist_out + static_cast<int64_t>(id) * kHistCap;
-    h.out_count = 0;
-    if (work) wall_forces<HIST>(P, pos, vel, ri, mi, f, h, A.counters);
-    const float3 f_walls = f;
-    const int out_walls = HIST ? h.out_count : 0;
-    W.pos[lane] = pi;
-    W.vel[lane] = vi;
-    W.id[lane] = id;
-    W.hin[lane] = hcnt_in;
-    W.outw[lane] = out_walls;
-    W.scene[lane] = scene;
-    const float cut = contact_cutoff_sq(ri, P.rmax);
-    int cx = 0, cy = 0, cz = 0;
-    if (work) cell_coords(P, pi.x, pi.y, pi.z, cx, cy, cz);
-    const bool listed = work && cnt_raw <= kNbrCap;
-    const int cnt = listed ? cnt_raw : 0;
-    const int rounds = __reduce_max_sync(0xffffffffu, cnt);
-    int q = 0, my_count = 0, bstart = 0;
-    bool reorder = false;
-    unsigned long long last = 0ull;
-    for (int e = 0; e < rounds; ++e) {
-        bool hit = false;
-        int j = 0;
-        if (e < cnt) {
-            j = __ldg(&A.nbr[static_cast<int64_t>(e) * n + s]);
-            const float4 pj = __ldg(&A.pos[j]);
-            float3 d;
-            const float ns = pair_norm_sq(pi, pj, d);
-            if (!(ns > cut)) {
-                const float dist = pair_dist(sqrtf(ns), ri, pj.w);
-                if (dist < 0.f) {
-                    hit = true;
-                    const unsigned long long key = visit_key(P, cx, cy, cz, pj, __ldg(&A.ids[j]));
-                    if (key < last) reorder = true;
-                    last = key;
-                }
+    int out_walls = 0, out_count = 0;
+    const bool work = own && !frozen;
+    if (work) {
+        HistRow h;
+        if (HIST) {
+            h.in = A.hist_in + static_cast<int64_t>(id) * kHistCap;
+            h.in_count = hcnt_in;
+            h.out = A.hist_out + static_cast<int64_t>(id) * kHistCap;
+            h.out_count = 0;
+        }
+        wall_forces<HIST>(P, make_float3(pi.x, pi.y, pi.z), vel, ri, mi, f, h, A.counters);
+        if (HIST) out_walls = out_count = h.out_count;
+    }
+    if (frozen) cnt = 0;
+    if (__any_sync(kAll, cnt != 0)) {
+        // scan: this lane's entries, four entries' loads in flight at a time
+        unsigned long long hits = 0ull;
+        const int scan = cnt <= kNbrCap ? cnt : 0;
+        for (int e0 = sub; e0 < scan; e0 += 4 * LPG) {
+            int jj[4];
+            float4 pp[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int e = e0 + u * LPG;
+                jj[u] = e < scan ? __ldg(&A.nbr[static_cast<int64_t>(e) * n + s]) : s;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) pp[u] = __ldg(&A.pos[jj[u]]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int e = e0 + u * LPG;
+                if (e < scan && entry_hit(pi, pp[u])) hits |= 1ull << e;
             }
         }
-        const unsigned b = __ballot_sync(0xffffffffu, hit);
-        const int add = __popc(b);
-        if (q + add > kCoopCap) {
-            coop_flush<HIST, BATCH>(P0, A, W, q, lane, my_count, bstart, reorder, f);
-            q = 0;
+#pragma unroll
+        for (int o = 1; o < LPG; o <<= 1) hits |= __shfl_xor_sync(kAll, hits, o);
+        if (cnt > kNbrCap || __popcll(hits) > 32) {
+            // a list that overflowed (this step built the lists, so the run table is fresh),
+            // or more contacts than one round holds: the grain's own lane takes them all
+            if (work) {
+                HistRow h;
+                if (HIST) {
+                    h.in = A.hist_in + static_cast<int64_t>(id) * kHistCap;
+                    h.in_count = hcnt_in;
+                    h.out = A.hist_out + static_cast<int64_t>(id) * kHistCap;
+                }
+                h.out_count = out_count;
+                int cx, cy, cz;
+                cell_coords(P, pi.x, pi.y, pi.z, cx, cy, cz);
+                if (cnt > kNbrCap)
+                    list_contacts_table<HIST>(P, A, s, pi, vel, mi, contact_cutoff_sq(ri, P.rmax), cx,
+                                              cy, cz, f, h);
+                else
+                    list_contacts_sorted_mask<HIST>(P, A, s, n, hits, pi, vel, mi, cx, cy, cz, f, h);
+                out_count = h.out_count;
+            }
+            hits = 0ull;
         }
-        if (hit) {
-            const int at = q + __popc(b & ((1u << lane) - 1u));
-            W.qj[at] = j;
-            W.qg[at] = static_cast<unsigned char>(lane);
-            W.qr[at] = static_cast<unsigned char>(my_count);
-            ++my_count;
+        if (__any_sync(kAll, hits != 0ull)) {
+            // number the warp's contacts, grain by grain
+            const int c = __popcll(hits);
+            int upto = sub == 0 ? c : 0;
+#pragma unroll
+            for (int o = LPG; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(kAll, upto, o);
+                if (lane >= o) upto += y;
+            }
+            if (LPG > 1) upto = __shfl_sync(kAll, upto, lane - sub);
+            const int off = upto - c;
+            const int total = __shfl_sync(kAll, upto, 31);
+            unsigned long long left = sub == 0 ? hits : 0ull;
+            int at = off;
+            for (int base = 0, end; base < total; base = end) {
+                // up to 32 contacts, all of each grain's (none has more than 32 here)
+                end = static_cast<int>(__reduce_max_sync(kAll, static_cast<unsigned>(upto <= base + 32 ? upto : 0)));
+                for (; left && at < end; ++at) {
+                    W.queue[at - base] = static_cast<unsigned short>(
+                        (lane << 6) | (__ffsll(static_cast<long long>(left)) - 1));
+                    left &= left - 1ull;
+                }
+                __syncwarp();
+                const bool active = base + lane < end;
+                const int q = active ? W.queue[lane] : 0;
+                const int o = q >> 6, e = q & 63;
+                const int so = __shfl_sync(kAll, s, o);
+                const int oo = __shfl_sync(kAll, off, o);
+                const int first = HIST ? __shfl_sync(kAll, out_walls, o) : 0;
+                int r = base + lane - oo;   // the contact's place among its grain's
+                unsigned long long key = 0ull;
+                PairTerms t;
+                float3 xi = make_float3(0.f, 0.f, 0.f);
+                int io = 0, jd = 0;
+                if (active) {
+                    const int go = o / LPG;
+                    const DevParams& Q = BATCH ? A.scene_params[S.scene[go]] : P0;
+                    const int j = __ldg(&A.nbr[static_cast<int64_t>(e) * n + so]);
+                    const float4 po = S.pos[go], vo = S.vel[go];
+                    const float4 pj = __ldg(&A.pos[j]), vj = __ldg(&A.vel[j]);
+                    jd = __ldg(&A.ids[j]);
+                    if (HIST) {
+                        io = S.id[go];
+                        const int row = S.hcnt[go];
+                        if (row > 0) {
+                            // rows keep the visiting order, so a lasting contact is about
+                            // where it was
+                            HistRow h;
+                            h.in = A.hist_in + static_cast<int64_t>(io) * kHistCap;
+                            h.in_count = row;
+                            h.cursor = min(first + r, row - 1);
+                            xi = find_spring(h, jd);
+                        }
+                    }
+                    int cx, cy, cz;
+                    cell_coords(Q, po.x, po.y, po.z, cx, cy, cz);
+                    key = visit_key(Q, cx, cy, cz, pj, jd);
+                    float3 d;
+                    const float ns = pair_norm_sq(po, pj, d);
+                    const float norm = sqrtf(ns);
+                    const float dist = pair_dist(norm, po.w, pj.w);
+                    t = pair_terms<HIST>(Q, d, norm, dist, make_float3(vo.x, vo.y, vo.z), vo.w, vj, xi);
+                }
+                const unsigned long long up_key = __shfl_up_sync(kAll, key, 1);
+                const int up_owner = __shfl_up_sync(kAll, o, 1);
+                const unsigned bad = __reduce_or_sync(
+                    kAll, active && lane > 0 && up_owner == o && key < up_key ? 1u << o : 0u);
+                if (bad) {
+                    // a cell crossing re-ordered these grains' contacts: each takes the place
+                    // of its key's rank
+                    int rank = 0;
+                    const int owner = active ? o : -1;
+                    for (int k = 0; k < 32; ++k) {
+                        const unsigned long long key_k = __shfl_sync(kAll, key, k);
+                        const int owner_k = __shfl_sync(kAll, owner, k);
+                        if (owner_k == o && key_k < key) ++rank;
+                    }
+                    if ((bad >> o) & 1u) r = rank;
+                    if (lane == 0)
+                        atomicAdd(&A.counters[kCntListResort], static_cast<unsigned long long>(__popc(bad)));
+                }
+                if (active) {
+                    const int place = oo + r - base;
+                    W.term[place][0] = make_float4(t.nrm.x, t.nrm.y, t.nrm.z, t.fp);
+                    W.term[place][1] = make_float4(t.t.x, t.t.y, t.t.z, t.cvn);
+                    if (HIST && first + r < kHistCap)
+                        A.hist_out[static_cast<int64_t>(io) * kHistCap + first + r] =
+                            make_float4(xi.x, xi.y, xi.z, __int_as_float(jd));
+                }
+                __syncwarp();
+                if (sub == 0) {
+                    // a grain of this round has all its contacts in it
+                    const int e1 = upto <= end ? upto - base : 0;
+                    for (int k = max(off - base, 0); k < e1; ++k) {
+                        const float4 a = W.term[k][0], b = W.term[k][1];
+                        PairTerms u;
+                        u.nrm = make_float3(a.x, a.y, a.z);
+                        u.fp = a.w;
+                        u.t = make_float3(b.x, b.y, b.z);
+                        u.cvn = b.w;
+                        pair_accumulate<HIST>(f, u);
+                    }
+                }
+                __syncwarp();               // the queue and the terms are free again
+            }
+            if (HIST && work && c > 0) {
+                out_count = min(out_walls + c, kHistCap);
+                if (out_walls + c > kHistCap)
+                    atomicAdd(&A.counters[kCntHistOverflow],
+                              static_cast<unsigned long long>(out_walls + c - kHistCap));
+            }
         }
-        q += add;
     }
-    if (rounds > 0) coop_flush<HIST, BATCH>(P0, A, W, q, lane, my_count, bstart, reorder, f);
     if (work) {
-        if (!listed) {
-            // list overflow: this step built the lists, so the run table is fresh
-            h.out_count = out_walls;
-            list_contacts_table<HIST>(P, A, s, pi, vel, mi, cut, cx, cy, cz, f, h);
-        } else if (reorder) {
-            // a cell crossing re-ordered this grain's contacts: redo them in canonical order
-            f = f_walls;
-            h.out_count = out_walls;
-            list_contacts_sorted<HIST>(P, A, s, n, cnt, pi, vel, mi, cut, cx, cy, cz, f, h);
-        } else if (HIST) {
-            h.out_count = min(out_walls + my_count, kHistCap);
-            if (out_walls + my_count > kHistCap)
-                atomicAdd(&A.counters[kCntHistOverflow],
-                          static_cast<unsigned long long>(out_walls + my_count - kHistCap));
-        }
-        if (HIST) A.hcnt_out[s] = h.out_count;
-        const float3 a = make_float3(f.x / mi, f.y / mi, f.z / mi);
-        const float3 v1 = make_float3(fmaf(P.dt, a.x, vel.x), fmaf(P.dt, a.y, vel.y),
-                                      fmaf(P.dt, a.z, vel.z));
-        const float3 x1 = make_float3(fmaf(P.dt, v1.x, pos.x), fmaf(P.dt, v1.y, pos.y),
-                                      fmaf(P.dt, v1.z, pos.z));
-        A.pos_out[s] = make_float4(x1.x, x1.y, x1.z, ri);
-        A.vel_out[s] = make_float4(v1.x, v1.y, v1.z, mi);
-        if (order_out) {
-            A.ids_out[s] = id;
-            if (BATCH) A.scene_out[s] = scene;
-        }
-        A.acc_out[s] = make_float4(a.x, a.y, a.z, 0.f);
-        if (exact) disp_bits = max(disp_bits, disp_sq_bits(x1, xb));
-        step_bits = max(step_bits, disp_sq_bits(x1, pos));
-    } else if (frozen) {
-        A.pos_out[s] = pi;
-        A.vel_out[s] = vi;
-        if (order_out) {
-            A.ids_out[s] = id;
-            A.scene_out[s] = scene;
-        }
-        A.acc_out[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (HIST) A.hcnt_out[s] = 0;
+        // the slot's values are read again from the stage, not held in registers meanwhile
+        const float4 x = S.pos[g], v = S.vel[g];
+        const float4 xb = exact ? A.xbuild[s] : x;
+        list_integrate<HIST, BATCH, PICARD>(P, A, s, scene, x, v, S.id[g], f,
+                                            out_count, xb, exact, order_out, disp_bits,
+                                            step_bits, res_bits);
+    } else if (own) {
+        list_copy_frozen<HIST>(A, s, scene, pi, vi, id, order_out);
     }
 }
 
-// Grid-stride over warps of 32 slots (one wave for the fused build decision).
-template <bool HIST, bool BATCH>
-__global__ void __launch_bounds__(kBlock, 4)
+// Grid-stride over groups of slots; semi-implicit Euler in one wave, so that the fused
+// build decision waits once per resident block.
+template <bool HIST, bool BATCH, bool PICARD, int LPG>
+__global__ void __launch_bounds__(kCoopBlock, PICARD ? 6 : 8)
 k_force_list_coop(DevParams P0, ListArgs A) {
+    if (PICARD && skipped(A.skip)) return;
     __shared__ CoopWarp warps[kCoopWarps];
     CoopWarp& W = warps[threadIdx.x >> 5];
-    const bool exact = A.list_ctrl[kLcExact] != 0u;
-    const bool order_out = A.list_ctrl[kLcDecision] != 0u;  // first step after a build
-    uint32_t disp_bits = 0u, step_bits = 0u;
-    for (int base = blockIdx.x * blockDim.x; base < P0.n; base += gridDim.x * blockDim.x)
-        coop_slot<HIST, BATCH>(P0, A, W, base + threadIdx.x, exact, order_out, disp_bits,
-                               step_bits);
-    list_disp_report<false>(A.list_ctrl, exact, disp_bits, step_bits);
-    list_tail_decide(A);
+    const int n = P0.n;
+    const bool exact = PICARD || A.list_ctrl[kLcExact] != 0u;
+    const bool order_out = PICARD || A.list_ctrl[kLcDecision] != 0u;  // first step after a build
+    uint32_t disp_bits = 0u, step_bits = 0u, res_bits = 0u;
+    bool viol = false;
+    // the next group's values are on their way while this one is computed
+    constexpr int per = kCoopBlock / LPG;   // slots per block
+    const int stride = gridDim.x * per;
+    int s = blockIdx.x * per + static_cast<int>(threadIdx.x) / LPG;
+    coop_stage<HIST, BATCH, LPG>(A, W.stage[0], s, n);
+    int st = 0;
+    for (int base = blockIdx.x * per; base < n; base += stride, s += stride, st ^= 1) {
+        __syncwarp();                       // the other stage has been read
+        coop_stage<HIST, BATCH, LPG>(A, W.stage[st ^ 1], s + stride, n);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();                       // every lane's copies have arrived
+        coop_slot<HIST, BATCH, PICARD, LPG>(P0, A, W, W.stage[st], s, n, exact, order_out, disp_bits,
+                                            step_bits, res_bits, viol);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    list_disp_report<PICARD>(A.list_ctrl, exact, disp_bits, step_bits);
+    if (PICARD) list_picard_report(A, res_bits, viol);
+    else list_tail_decide(A);
 }
 
 __global__ void __launch_bounds__(kBlock)
@@ -1294,6 +1382,35 @@ void force_list_variant(const DevParams& P, const ListArgs& a, cudaStream_t st, 
     }
 }
 
+template <bool HIST, bool BATCH, bool PICARD, int LPG>
+void force_list_coop_launch(const DevParams& P, const ListArgs& a, cudaStream_t st) {
+    const int per = kCoopBlock / LPG;
+    const int nb = std::min((P.n + per - 1) / per,
+                            one_wave<k_force_list_coop<HIST, BATCH, PICARD, LPG>>(kCoopBlock));
+    k_force_list_coop<HIST, BATCH, PICARD, LPG><<<nb, kCoopBlock, 0, st>>>(P, a);
+}
+
+template <bool PICARD, int LPG>
+void force_list_coop_lanes(const DevParams& P, const ListArgs& a, cudaStream_t st) {
+    const bool batch = a.scene_params != nullptr;
+    if (P.history) {
+        if (batch) force_list_coop_launch<true, true, PICARD, LPG>(P, a, st);
+        else force_list_coop_launch<true, false, PICARD, LPG>(P, a, st);
+    } else {
+        if (batch) force_list_coop_launch<false, true, PICARD, LPG>(P, a, st);
+        else force_list_coop_launch<false, false, PICARD, LPG>(P, a, st);
+    }
+}
+
+template <bool PICARD>
+void force_list_coop(const DevParams& P, const ListArgs& a, cudaStream_t st) {
+    // Four lanes a grain where one each would leave most of the chip idle and the step is
+    // one warp's latency: 2^10 packed grains with springs 20.1 vs 21.4 us a step, 5,000 22.0
+    // vs 23.9, 10,000 24.3 vs 26.0, 20,000 25.5 vs 26.1, 40,000 30.4 vs 27.0.
+    if (P.n < 16384) force_list_coop_lanes<PICARD, 4>(P, a, st);
+    else force_list_coop_lanes<PICARD, 1>(P, a, st);
+}
+
 void launch_list_finalize(int n, const int* picard_used, const float4* xpos,
                           const float4* xvel, float4* pos, float4* vel, cudaStream_t st) {
     k_list_finalize<<<blocks_for(n), kBlock, 0, st>>>(n, picard_used, xpos, xvel, pos, vel);
@@ -1306,8 +1423,13 @@ void launch_list_picard_check(uint32_t* list_ctrl, unsigned long long* counters,
 
 void launch_force_list(const DevParams& P, const ListArgs& a, cudaStream_t st, int block,
                        int min_blocks, bool picard) {
+    if (min_blocks == 0) {
+        if (picard) force_list_coop<true>(P, a, st);
+        else force_list_coop<false>(P, a, st);
+        return;
+    }
     if (picard) {
-        // the per-lane kernel (the cooperative one has no Picard form)
+        // the per-lane kernel (the bulk-staged one has no Picard form)
         if (min_blocks == 4) force_list_variant<4, true>(P, a, st, block == 0 ? kBlock : block);
         else force_list_variant<5, true>(P, a, st, block);
         return;
@@ -1325,25 +1447,7 @@ void launch_force_list(const DevParams& P, const ListArgs& a, cudaStream_t st, i
         }
         return;
     }
-    if (min_blocks == 0) {
-        // warp-cooperative kernel: its shared queues are sized for kBlock threads; one
-        // wave, grid-stride
-        const int nb = blocks_for(P.n, kBlock);
-        const bool batch = a.scene_params != nullptr;
-        if (P.history) {
-            if (batch) {
-                k_force_list_coop<true, true><<<std::min(nb, one_wave<k_force_list_coop<true, true>>(kBlock)), kBlock, 0, st>>>(P, a);
-            } else {
-                k_force_list_coop<true, false><<<std::min(nb, one_wave<k_force_list_coop<true, false>>(kBlock)), kBlock, 0, st>>>(P, a);
-            }
-        } else {
-            if (batch) {
-                k_force_list_coop<false, true><<<std::min(nb, one_wave<k_force_list_coop<false, true>>(kBlock)), kBlock, 0, st>>>(P, a);
-            } else {
-                k_force_list_coop<false, false><<<std::min(nb, one_wave<k_force_list_coop<false, false>>(kBlock)), kBlock, 0, st>>>(P, a);
-            }
-        }
-    } else if (min_blocks == 4) {
+    if (min_blocks == 4) {
         force_list_variant<4, false>(P, a, st, block);
     } else {
         force_list_variant<5, false>(P, a, st, block);

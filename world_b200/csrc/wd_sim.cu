@@ -139,7 +139,7 @@ struct wd_sim {
     bool lists = false;
     int lpar = 0;
     int force_block = wd::kBlock;   // threads per block of the contact kernel
-    int force_minb = 1;             // list contact kernel variant (1: bulk-staged)
+    int force_minb = 0;             // list contact kernel variant (0: contact-parallel)
     // Picard with lists: scratch iterate buffers (and, for a redo's gather, ids / scenes)
     float4* xpos = nullptr;
     float4* xvel = nullptr;
@@ -740,7 +740,8 @@ cudaError_t enqueue_step_list_picard(wd_sim* s, int parity, cudaStream_t st, boo
         a.skip = wd::Skip{k == 0 ? nullptr : s->picard_res + (k - 1), P.picard_tol};
         a.rhs_vel = s->rhs_vel;
         a.rhs_ids = s->rhs_ids;
-        wd::launch_force_list(P, a, st, s->force_block, s->force_minb == 4 ? 4 : 5, true);
+        wd::launch_force_list(P, a, st, s->force_block,
+                              s->force_minb == 4 || s->force_minb == 0 ? s->force_minb : 5, true);
     }
     wd::launch_list_finalize(s->n, s->picard_used, s->xpos, s->xvel, s->posB, s->velB, st);
     if (!capture) {
@@ -2427,8 +2428,8 @@ int wd_autotune(wd_sim* sim, int32_t steps, const char* cache_path, float* skin_
         std::vector<float> skins = {0.f};
         for (float f : {0.05f, 0.1f, 0.15f, 0.2f, 0.3f, 0.4f}) skins.push_back(f * d);
         // (block, variant): variant 5 / 4 = per-lane list kernel with 48 / 64 registers,
-        // 0 = warp-cooperative list kernel, 1 / 2 = bulk-staged persistent list kernel
-        // with 48 / 64 registers (256 threads each)
+        // 0 = contact-parallel list kernel (its own block), 1 / 2 = bulk-staged persistent
+        // list kernel with 48 / 64 registers (256 threads)
         const int cands[][2] = {{128, 5}, {256, 5}, {128, 4}, {256, 4}, {256, 0}, {256, 1},
                                 {256, 2}};
         const int ncands = static_cast<int>(sizeof(cands) / sizeof(cands[0]));
@@ -2446,7 +2447,7 @@ int wd_autotune(wd_sim* sim, int32_t steps, const char* cache_path, float* skin_
                 const int bl = cands[cand][0];
                 const int mb = cands[cand][1];
                 if (sk == 0.f && mb != 5) continue;  // the searched kernel has one variant
-                if (sim->picard && mb <= 2) continue;  // Picard: the per-lane kernel only
+                if (sim->picard && (mb == 1 || mb == 2)) continue;  // no bulk-staged Picard form
                 rc = apply_skin(sim, sk);
                 if (rc == WD_OK) {
                     sim->force_block = bl;

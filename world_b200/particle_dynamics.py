@@ -364,7 +364,8 @@ class ParticleDynamics:
 
     def set_contact_kernel(self, block: int = 256, variant: int = 48) -> None:
         """Contact-kernel block size and list-kernel variant (48 / 64: per-lane with that
-        many registers, 0: warp-cooperative, 1 / 2: bulk-staged persistent with 48 / 64
+        many registers, 0: warp-cooperative, the default, which evaluates the contacts
+        of a warp's grains together, 1 / 2: bulk-staged persistent with 48 / 64
         registers, whose per-slot arrays arrive in shared memory by bulk copies); results
         do not depend on them."""
         check(lib.wd_set_contact_kernel(self._h, int(block), int(variant)))
