@@ -271,7 +271,12 @@ int wd_compute_max_acceleration(wd_sim* sim, float* max_accel);
  * grain is dropped here: the sorted search has no per-cell capacity. */
 int wd_grid_overflow_count(wd_sim* sim, int64_t* count);
 /* Switch the Verlet-list skin of a live handle (0: grid search every step). The
- * trajectory does not depend on it. */
+ * trajectory does not depend on it. A handle created with simulation.neighbor_skin 0 and
+ * never switched uses lists of the library's own where a run of three steps or more
+ * between state uploads pays for them: the same states, springs and counts to the bit
+ * (single scenes, semi-implicit Euler, cells at least one largest diameter wide, list
+ * buffers of at most a quarter of the free device memory); calling this (or the
+ * autotuner) ends that. */
 int wd_set_neighbor_skin(wd_sim* sim, float skin);
 /* Autotuner (extension): times `steps` steps for each neighbor skin in {0, 0.05,
  * 0.1, 0.15, 0.2, 0.3, 0.4} mean diameters, contact-kernel block size in {128, 256} and, with

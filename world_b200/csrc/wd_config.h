@@ -4,7 +4,9 @@
 // (src/sim_config.h:28-205, src/sim_config.cpp:54-195). New keys live in the existing
 // sections and default to the reference's behaviour when absent:
 //   simulation.history            false  -> viscous tangential friction (reference)
-//   simulation.neighbor_skin      0      -> neighbor search every step (reference); > 0:
+//   simulation.neighbor_skin      0      -> the results of a neighbor search every step
+//                                           (reference), with lists of the library's own
+//                                           where a run of steps pays for them; > 0:
 //                                           Verlet lists with this skin (m), rebuilt when
 //                                           a grain has moved 0.49 skin since the build
 //   physics.normal_stiffness      0      -> k_n = max_force / particle_radius

@@ -209,9 +209,9 @@ k_energy(DevParams P0, SceneTab T, const float4* __restrict__ pos, const float4*
 
 // Segmented sums, step 1: one block per 256-grain chunk of a scene's segment (chunks
 // are aligned to the segment start, so a scene reduces the same way alone or in a
-// batch). comps values per grain, component-major: v[c * n + slot].
+// batch). comps values per grain, value c of grain i at v[c * comp_step + i * grain_step].
 __global__ void __launch_bounds__(kBlock)
-k_segment_chunks(const double* __restrict__ v, int n, int comps, const int* __restrict__ seg,
+k_segment_chunks(const double* __restrict__ v, int64_t comp_step, int grain_step, int comps, const int* __restrict__ seg,
                  const int* __restrict__ chunk_base, int scenes, double* __restrict__ partials,
                  int total_chunks) {
     const int b = blockIdx.x;
@@ -224,7 +224,8 @@ k_segment_chunks(const double* __restrict__ v, int n, int comps, const int* __re
     const int first = seg[sc] + (b - chunk_base[sc]) * kBlock;
     const int i = first + static_cast<int>(threadIdx.x);
     for (int c = 0; c < comps; ++c) {
-        const double x = i < seg[sc + 1] ? v[static_cast<int64_t>(c) * n + i] : 0.0;
+        const double x =
+            i < seg[sc + 1] ? v[c * comp_step + static_cast<int64_t>(i) * grain_step] : 0.0;
         const double t = block_sum(x);
         if (threadIdx.x == 0) partials[static_cast<int64_t>(c) * total_chunks + b] = t;
     }
@@ -245,15 +246,19 @@ k_segment_finish(const double* __restrict__ partials, const int* __restrict__ ch
     }
 }
 
+// Momentum terms by grain id, so that the sums do not depend on the order of the slots
+// (which a step on lists leaves as the last build made it).
 __global__ void __launch_bounds__(kBlock)
-k_momentum(int n, const float4* __restrict__ vel, double* __restrict__ out) {
+k_momentum(int n, const float4* __restrict__ vel, const int* __restrict__ ids,
+           double* __restrict__ out) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const float4 v = vel[s];
     const double m = v.w;
-    out[s] = m * v.x;
-    out[static_cast<int64_t>(n) + s] = m * v.y;
-    out[2 * static_cast<int64_t>(n) + s] = m * v.z;
+    // one whole 32-byte sector per grain
+    double2* o = reinterpret_cast<double2*>(out + 4 * static_cast<int64_t>(ids[s]));
+    o[0] = make_double2(m * v.x, m * v.y);
+    o[1] = make_double2(m * v.z, 0.0);
 }
 
 // reference src/particle_dynamics.cu:328-344: sqrt(ax^2 + ay^2 + az^2), unfused.
@@ -314,9 +319,10 @@ void launch_force(const DevParams& P, const ForceArgs& a, bool picard, Skip skip
 int reduction_blocks(int n) { return blocks_for(n > 0 ? n : 1); }
 
 void launch_segment_sums(const double* values, int n, int comps, const Segments& g,
-                         double* partials, double* out, cudaStream_t st) {
-    k_segment_chunks<<<g.total_chunks, kBlock, 0, st>>>(values, n, comps, g.seg, g.chunk_base,
-                                                        g.scenes, partials, g.total_chunks);
+                         double* partials, double* out, cudaStream_t st, int grain_step) {
+    k_segment_chunks<<<g.total_chunks, kBlock, 0, st>>>(values, grain_step > 1 ? 1 : n, grain_step,
+                                                        comps, g.seg, g.chunk_base, g.scenes,
+                                                        partials, g.total_chunks);
     k_segment_finish<<<g.scenes, kBlock, 0, st>>>(partials, g.chunk_base, comps, g.total_chunks, out);
 }
 
@@ -336,10 +342,10 @@ void launch_energy(const DevParams& P, SceneTab T, const float4* pos, const floa
     launch_segment_sums(per_grain, P.n, 1, g, partials, out, st);
 }
 
-void launch_momentum(int n, const float4* vel, const Segments& g, double* per_grain,
-                     double* partials, double* out3, cudaStream_t st) {
-    k_momentum<<<reduction_blocks(n), kBlock, 0, st>>>(n, vel, per_grain);
-    launch_segment_sums(per_grain, n, 3, g, partials, out3, st);
+void launch_momentum(int n, const float4* vel, const int* ids, const Segments& g,
+                     double* per_grain, double* partials, double* out3, cudaStream_t st) {
+    k_momentum<<<reduction_blocks(n), kBlock, 0, st>>>(n, vel, ids, per_grain);
+    launch_segment_sums(per_grain, n, 3, g, partials, out3, st, 4);
 }
 
 void launch_max_accel(int n, const float4* acc, unsigned long long* counters,

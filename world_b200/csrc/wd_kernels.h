@@ -143,13 +143,17 @@ void launch_force(const DevParams& P, const ForceArgs& a, bool picard, Skip skip
 // tests). Picard builds earlier, at kPicardBuildAt, so that its iterates rarely leave.
 constexpr float kListValid = 0.49f;
 constexpr float kPicardBuildAt = 0.30f;
+// kLcCrowded / kLcSteps / kLcBuilds: the library's own lists under neighbor_skin 0 (a cell
+// may hold more than particles_per_cell grains before the next build; list steps and their
+// builds so far).
 // kLcStallTest / kLcWaitUs: the bulk-staged contact kernel's wait test. A nonzero
 // kLcStallTest makes each warp's first stage expect 16 bytes that no copy delivers (no
 // copy is issued for it), so its bounded wait runs out; kLcWaitUs is that wait's limit
 // in microseconds (0: one second).
 enum ListCtrl {
     kLcDisp = 0, kLcOverflow = 1, kLcForce = 2, kLcDecision = 3, kLcViol = 4, kLcRedo = 5,
-    kLcStep = 6, kLcExact = 7, kLcBound = 8, kLcStallTest = 10, kLcWaitUs = 11, kLcWords = 12
+    kLcStep = 6, kLcExact = 7, kLcBound = 8, kLcStallTest = 10, kLcWaitUs = 11, kLcCrowded = 12,
+    kLcSteps = 13, kLcBuilds = 14, kLcWords = 16
 };
 struct ListArgs {
     const float4* pos; const float4* vel; const int* ids;  // state of the step
@@ -171,6 +175,8 @@ struct ListArgs {
     // semi-implicit Euler: the build decision for the next step, made by the kernel's
     // last block (threshold on max |x - x_build|, block ticket, the build's IF node)
     float thr; unsigned* tail_count; int use_cond; cudaGraphConditionalHandle cond;
+    // the library's own lists: counters of the last build's gather, host-visible words
+    unsigned long long* pend; uint32_t* host_word;
 };
 // Device-side launches of the list build's graphs (wd_launch.cu, the one translation
 // unit built with relocatable device code for the device runtime): one thread
@@ -183,8 +189,13 @@ void launch_graph_if(const uint32_t* flag, cudaGraphExec_t graph, unsigned long 
 void launch_graph_pick(const int* flag, cudaGraphExec_t on_zero, cudaGraphExec_t on_one,
                        unsigned long long* counters, cudaStream_t st);
 void launch_list_decide(uint32_t* list_ctrl, float thr, bool always_exact,
-                        unsigned long long* counters,
-                        bool use_cond, cudaGraphConditionalHandle cond, cudaStream_t st);
+                        unsigned long long* counters, unsigned long long* pend, bool use_cond, cudaGraphConditionalHandle cond, cudaStream_t st);
+// The library's own lists under neighbor_skin 0: counts, per collision cell, the grains of
+// the build that can be in it while the lists hold (those within half a skin of its box), and
+// sets kLcCrowded where that exceeds particles_per_cell. xbuild: the positions of the build
+// before, whose cells are cleared.
+void launch_cell_load(const DevParams& P, const float4* pos, const float4* xbuild, uint32_t* load,
+                      uint32_t* list_ctrl, Skip skip, cudaStream_t st);
 // The sorted state a list build copies back into the step's buffers (one pass with the
 // listing: pos is read there anyway).
 struct ListCopy {
@@ -249,11 +260,13 @@ void launch_deposit_batch(int n, const float4* pos, const float4* vel, SceneTab 
                           int64_t total_nodes, uint32_t* bounds, unsigned long long* acc,
                           float* out, cudaStream_t st);
 
-// Reductions (per scene: out3[3 * scene + axis]).
+// Reductions (per scene: out3[3 * scene + axis]). values: component-major, or with
+// grain_step > 1 that many doubles per grain, its components first.
 void launch_segment_sums(const double* values, int n, int comps, const Segments& g,
-                         double* partials, double* out, cudaStream_t st);
-void launch_momentum(int n, const float4* vel, const Segments& g, double* per_grain,
-                     double* partials, double* out3, cudaStream_t st);
+                         double* partials, double* out, cudaStream_t st, int grain_step = 1);
+// per_grain: 4n doubles, 16-byte aligned.
+void launch_momentum(int n, const float4* vel, const int* ids, const Segments& g,
+                     double* per_grain, double* partials, double* out3, cudaStream_t st);
 void launch_max_accel(int n, const float4* acc, unsigned long long* counters,
                       cudaStream_t st);
 // is_stable: sets counters[kCntUnstable]; a batch also flags scene_unstable[scene].

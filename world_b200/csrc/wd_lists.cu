@@ -45,8 +45,15 @@ __device__ __forceinline__ bool skipped(const Skip& s) {
 // A NaN or infinite displacement makes B infinite: the step builds.
 // One thread. Volatile accesses: the fused form runs in the last block of a contact
 // kernel whose other blocks updated these words with atomics.
+// pend: non-null for the library's own lists under neighbor_skin 0, whose searched steps
+// count a (cell, search) incident whenever a cell holds more than particles_per_cell grains.
+// A build counts them of the state it sorts into pend; they are due when the next step
+// starts from that state, here at its end (`step`). Between builds there are none unless the
+// build found a cell that could fill up (kLcCrowded): then every step builds, and
+// host_word[2] tells the host to search instead.
 __device__ bool list_decide_core(uint32_t* ctrl_, float thr, int always_exact,
-                                 unsigned long long* counters) {
+                                 unsigned long long* counters, unsigned long long* pend,
+                                 uint32_t* host_word, bool at_step) {
     volatile uint32_t* ctrl = ctrl_;
     volatile double* bound = reinterpret_cast<volatile double*>(ctrl_ + kLcBound);
     const double grow = 1.0 + 1.0 / 65536.0;
@@ -54,29 +61,84 @@ __device__ bool list_decide_core(uint32_t* ctrl_, float thr, int always_exact,
     double b = ctrl[kLcExact] != 0u
                    ? sqrt(static_cast<double>(__uint_as_float(ctrl[kLcDisp]))) * grow
                    : *bound + step;
-    const bool build = ctrl[kLcForce] != 0u || ctrl[kLcOverflow] != 0u || !(b < thr);
+    bool build = ctrl[kLcForce] != 0u || ctrl[kLcOverflow] != 0u || !(b < thr);
+    if (pend != nullptr) {
+        const bool crowded = ctrl[kLcCrowded] != 0u;
+        if (at_step) {
+            counters[kCntGridOverflow] += pend[kCntGridOverflow];
+            ctrl[kLcSteps] = ctrl[kLcSteps] + 1u;
+            build |= crowded;
+            if (build) {
+                ctrl[kLcBuilds] = ctrl[kLcBuilds] + 1u;
+                volatile uint32_t* w = host_word;
+                w[0] = ctrl[kLcSteps];
+                w[1] = ctrl[kLcBuilds];
+                if (crowded) w[2] = 1u;
+            }
+        }
+        if (build) {
+            pend[kCntGridOverflow] = 0ull;
+            ctrl[kLcCrowded] = 0u;
+        }
+    }
     ctrl[kLcDecision] = build ? __float_as_uint(1.f) : 0u;
     if (build) {
         b = 0.0;
         ctrl[kLcOverflow] = 0u;
         ctrl[kLcForce] = 0u;
-        counters[kCntListBuilds] += 1ull;
+        if (pend == nullptr) counters[kCntListBuilds] += 1ull;
     }
     *bound = b;
     ctrl[kLcDisp] = 0u;
     ctrl[kLcStep] = 0u;
     const bool exact = always_exact || (!build && !(b + 2.0 * step < thr));
     ctrl[kLcExact] = exact ? 1u : 0u;
-    if (exact) counters[kCntListExact] += 1ull;
+    if (exact && pend == nullptr) counters[kCntListExact] += 1ull;
     return build;
 }
 
 __global__ void k_list_decide(uint32_t* __restrict__ ctrl, float thr, int always_exact,
-                              unsigned long long* __restrict__ counters, int use_cond,
+                              unsigned long long* __restrict__ counters,
+                              unsigned long long* __restrict__ pend, int use_cond,
                               cudaGraphConditionalHandle cond) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const bool build = list_decide_core(ctrl, thr, always_exact, counters);
+    const bool build = list_decide_core(ctrl, thr, always_exact, counters, pend, nullptr, false);
     if (use_cond) cudaGraphSetConditional(cond, build ? 1u : 0u);
+}
+
+// Cells that a grain at p can be in while it stays within half a skin of p (the lists hold
+// up to 0.49 skin; the rest covers the rounding of p -+ r and of the displacement bound).
+template <typename Visit>
+__device__ __forceinline__ void reachable_cells(const DevParams& P, float4 p, Visit visit) {
+    const float r = 0.5f * P.skin;
+    int a0, a1, b0, b1, c0, c1;
+    cell_coords(P, p.x - r, p.y - r, p.z - r, a0, b0, c0);
+    cell_coords(P, p.x + r, p.y + r, p.z + r, a1, b1, c1);
+    for (int x = a0; x <= a1; ++x)
+        for (int y = b0; y <= b1; ++y)
+            for (int z = c0; z <= c1; ++z) visit(P.cell_base + flat_cell(P, x, y, z));
+}
+
+__global__ void __launch_bounds__(kBlock)
+k_cell_clear(DevParams P, const float4* __restrict__ xbuild, uint32_t* __restrict__ load, Skip skip) {
+    if (skipped(skip)) return;
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < P.n) reachable_cells(P, xbuild[s], [&](uint32_t c) { load[c] = 0u; });
+}
+
+// One atomic per reachable cell: 1.3 a grain at this skin, spread over the grid (about 8 us
+// for 2^20 grains, of a build of about 300).
+__global__ void __launch_bounds__(kBlock)
+k_cell_load(DevParams P, const float4* __restrict__ pos, uint32_t* __restrict__ load,
+            uint32_t* __restrict__ ctrl, Skip skip) {
+    if (skipped(skip)) return;
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= P.n) return;
+    bool over = false;
+    reachable_cells(P, pos[s], [&](uint32_t c) {
+        over |= static_cast<int64_t>(atomicAdd(&load[c], 1u)) >= static_cast<int64_t>(P.ppc);
+    });
+    if (over) atomicOr(&ctrl[kLcCrowded], 1u);
 }
 
 // The decision fused into the tail of a semi-implicit Euler list kernel: the last block
@@ -93,7 +155,8 @@ __device__ __forceinline__ void list_tail_decide(const ListArgs& A) {
         const unsigned ticket = atomicAdd(A.tail_count, 1u);
         if (ticket == gridDim.x - 1) {
             __threadfence();
-            const bool build = list_decide_core(A.list_ctrl, A.thr, 0, A.counters);
+            const bool build =
+                list_decide_core(A.list_ctrl, A.thr, 0, A.counters, A.pend, A.host_word, true);
             *reinterpret_cast<volatile unsigned*>(A.tail_count) = 0u;
             if (A.use_cond) cudaGraphSetConditional(A.cond, build ? 1u : 0u);
         }
@@ -1302,10 +1365,16 @@ k_list_length(int n, const int* __restrict__ cnt, unsigned long long* __restrict
 }  // namespace
 
 void launch_list_decide(uint32_t* list_ctrl, float thr, bool always_exact,
-                        unsigned long long* counters,
-                        bool use_cond, cudaGraphConditionalHandle cond, cudaStream_t st) {
-    k_list_decide<<<1, 32, 0, st>>>(list_ctrl, thr, always_exact ? 1 : 0, counters,
+                        unsigned long long* counters, unsigned long long* pend, bool use_cond,
+                        cudaGraphConditionalHandle cond, cudaStream_t st) {
+    k_list_decide<<<1, 32, 0, st>>>(list_ctrl, thr, always_exact ? 1 : 0, counters, pend,
                                     use_cond ? 1 : 0, cond);
+}
+
+void launch_cell_load(const DevParams& P, const float4* pos, const float4* xbuild, uint32_t* load,
+                      uint32_t* list_ctrl, Skip skip, cudaStream_t st) {
+    k_cell_clear<<<blocks_for(P.n), kBlock, 0, st>>>(P, xbuild, load, skip);
+    k_cell_load<<<blocks_for(P.n), kBlock, 0, st>>>(P, pos, load, list_ctrl, skip);
 }
 
 void launch_list_build(const DevParams& P, SceneTab T, const float4* pos, const int2* table,

@@ -110,7 +110,7 @@ struct wd_sim {
     int* d_seg = nullptr;                 // S+1 segment starts (int)
     int* d_chunk_base = nullptr;          // S+1 reduction chunk offsets
     int total_chunks = 0;
-    double* grain_vals = nullptr;         // 3n per-grain values for reductions
+    double* grain_vals = nullptr;         // 4n per-grain values for reductions
     double* scene_sums = nullptr;         // 3S per-scene sums
     unsigned long long* scene_overflow = nullptr;  // S lifetime overflow counts (batch)
     int* scene_unstable = nullptr;        // S is_stable flags (batch)
@@ -157,6 +157,20 @@ struct wd_sim {
     unsigned* tail_count = nullptr;  // block ticket of the contact kernel's fused decision
     bool need_build = false;         // host-side change: rebuild before the next step
 
+    // Lists of the library's own choice under simulation.neighbor_skin 0 (see auto_mode):
+    // P.skin holds their skin, cfg.neighbor_skin stays 0 and `lists` is the mode of the
+    // step at hand.
+    bool auto_ok = false;                    // this handle may use them
+    unsigned long long* auto_pend = nullptr; // counters that a build's gather adds to
+    uint32_t* auto_load = nullptr;           // per cell: grains that can be in it before the next build
+    uint32_t* auto_word = nullptr;           // pinned: list steps, builds, a crowded cell seen
+    uint32_t* auto_word_dev = nullptr;
+    int64_t run_steps = 0, last_run = 0;     // steps since the last upload, and between the two before
+    int64_t auto_off = 0, auto_backoff = 512;// steps to search before lists are tried again
+    uint32_t auto_seen[2] = {0, 0};
+    bool list_work = false;                  // list steps or builds since the last synchronise
+    unsigned long long* pinned = nullptr;    // host copy of the counters, read after a synchronise
+
     // reverse pass: snapshots of the step state (checkpoints of a recorded window and
     // the states of the segment being replayed) and the adjoint buffers
     struct Snap {
@@ -183,7 +197,8 @@ struct wd_sim {
     };
     std::vector<TapeStep> adj_tape;
     unsigned long long* adj_ovf = nullptr;
-    // captured replay / walk-back graphs per (segment length, parity); -1: replay
+    // captured replay / walk-back graphs per segment length and parity (-1: replay) with
+    // the buffer parity
     std::map<std::pair<int, int>, cudaGraphExec_t> adj_graphs;
     int64_t adj_steps = 0;
     int adj_every = 0;
@@ -213,22 +228,27 @@ struct wd_sim {
     std::vector<float> radius, mass;
     std::vector<int32_t> material;
 
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
-    // list mode (semi-implicit Euler): the list build as device-launchable graphs per
-    // step parity -- the search head (keys, mover sort), then the mover path (merge) or
-    // the radix path, each followed by the gather and the listing; the contact kernel
-    // tail-launches the head when it decides a build, the mover kernel the rest
-    cudaGraphExec_t dev_head[2] = {nullptr, nullptr};
-    cudaGraphExec_t dev_mover[2] = {nullptr, nullptr};
-    cudaGraphExec_t dev_radix[2] = {nullptr, nullptr};
-    // searched semi-implicit Euler steps: the step graph holds the search head (keys,
-    // mover sort) and a kernel that tail-launches the rest of the step as one of two
-    // device-launchable graphs: the mover path (merge) or the radix path, each followed
-    // by the gather and the contact kernel
-    cudaGraphExec_t dev_step_mover[2] = {nullptr, nullptr};
-    cudaGraphExec_t dev_step_radix[2] = {nullptr, nullptr};
+    // Step graphs, captured when first needed, by what their nodes' pointers depend on: the
+    // mode (searched or on lists), which buffers are A (lpar) and the spring parity
+    // (hist_cur). Each keeps the device-launchable graphs that its kernels tail-launch:
+    //   on lists (semi-implicit Euler): the list build -- the search head (keys, mover
+    //     sort), then the mover path (merge) or the radix path, each followed by the
+    //     gather and the listing; the contact kernel's successor launches the head when a
+    //     build was decided, the mover kernel's the rest;
+    //   searched: the rest of the step after the search head, the mover path or the radix
+    //     path, each followed by the gather and the contact kernel.
+    struct StepGraph {
+        cudaGraphExec_t step = nullptr;
+        cudaGraphExec_t build_if = nullptr;   // on lists: the launcher of the build alone
+        cudaGraphExec_t head = nullptr, mover = nullptr, radix = nullptr;
+        // on lists: the build of the state in A, launched from the host (graphs of its own:
+        // one that the device may yet launch is not launched from the host)
+        cudaGraphExec_t now_head = nullptr, now_mover = nullptr, now_radix = nullptr;
+    };
+    StepGraph graphs[8];
+    bool built_now = false;   // a host-requested build has run before
+    StepGraph& graph_now() { return graphs[(lists ? 4 : 0) + 2 * lpar + hist_cur]; }
     bool graph_dirty = true;
-    int kernels_per_step = 0;
 
     // kernel_timing: lifetime ms [search, contact+integrate, integrate, deposit]
     float wct[4] = {0.f, 0.f, 0.f, 0.f};
@@ -248,16 +268,11 @@ void destroy_graphs(wd_sim* s) {
     // steps still in flight may yet tail-launch the device graphs: let them finish first
     if (s->stream) cudaStreamSynchronize(s->stream);
     clear_adj_graphs(s);
-    for (auto& g : s->graph) {
-        if (g) cudaGraphExecDestroy(g);
-        g = nullptr;
-    }
-    for (cudaGraphExec_t* set : {s->dev_head, s->dev_mover, s->dev_radix, s->dev_step_mover,
-                                 s->dev_step_radix}) {
-        for (int q = 0; q < 2; ++q) {
-            if (set[q]) cudaGraphExecDestroy(set[q]);
-            set[q] = nullptr;
-        }
+    for (auto& g : s->graphs) {
+        for (cudaGraphExec_t x : {g.step, g.build_if, g.head, g.mover, g.radix, g.now_head, g.now_mover,
+                                  g.now_radix})
+            if (x) cudaGraphExecDestroy(x);
+        g = wd_sim::StepGraph{};
     }
     s->graph_dirty = true;
 }
@@ -367,9 +382,11 @@ void free_sim(wd_sim* s) {
                     s->scene_overflow, s->scene_unstable, s->d_node_seg, s->d_node_chunk,
                     s->node_vals, s->chaos_partials, s->chaos_sums, s->grain_sums,
                     s->chaos_grid, s->nbr, s->nbr_cnt, s->xbuild, s->list_ctrl, s->list_len,
-                    s->tail_count, s->xpos, s->xvel, s->xids, s->xscene, s->rhs_vel, s->rhs_ids};
+                    s->tail_count, s->auto_pend, s->auto_load, s->xpos, s->xvel, s->xids, s->xscene, s->rhs_vel, s->rhs_ids};
     for (void* b : bufs)
         if (b) cudaFree(b);
+    if (s->auto_word) cudaFreeHost(s->auto_word);
+    if (s->pinned) cudaFreeHost(s->pinned);
     for (cudaEvent_t e : s->ev_pool) cudaEventDestroy(e);
     for (cudaEvent_t e : s->ev_pending) cudaEventDestroy(e);
     free_tape(s);
@@ -559,12 +576,12 @@ cudaError_t enqueue_step(wd_sim* s, int parity, cudaStream_t st, bool capture,
     fa.scene_out = s->sceneA;
     const wd::Skip none{nullptr, 0.f};
     if (!s->picard) {
-        if (capture && s->dev_step_mover[parity] != nullptr) {
+        if (capture && s->graph_now().mover != nullptr) {
             // the search head here, the rest of the step tail-launched from the device
             wd::launch_search_head(P, tab(s, s->sceneA), s->posA, s->idsA, s->sb, none, nullptr,
                                    0, false, 0, s->counters, st);
-            wd::launch_graph_pick(s->sb.ctrl + 1, s->dev_step_mover[parity],
-                                  s->dev_step_radix[parity], s->counters, st);
+            wd::launch_graph_pick(s->sb.ctrl + 1, s->graph_now().mover, s->graph_now().radix,
+                                  s->counters, st);
             return cudaGetLastError();
         }
         cudaError_t e = enqueue_search(s, none, nullptr, 0, capture, st);
@@ -614,8 +631,10 @@ void enqueue_list_build_tail(wd_sim* s, wd::Skip gate, cudaStream_t st) {
     wd::launch_gather(P, s->sb, s->posA, s->velA, s->posB, s->velB, s->idsB, nullptr, nullptr,
                       nullptr, nullptr, false, hist ? s->hcnt_slot : nullptr,
                       hist ? s->hcnt_g : nullptr, batch ? s->sceneA : nullptr,
-                      batch ? s->sceneB : nullptr, true, s->counters, s->scene_overflow,
-                      s->d_scene_P, gate, st);
+                      batch ? s->sceneB : nullptr, true, s->auto_ok ? s->auto_pend : s->counters,
+                      s->scene_overflow, s->d_scene_P, gate, st);
+    if (s->auto_ok)
+        wd::launch_cell_load(P, s->posB, s->xbuild, s->auto_load, s->list_ctrl, gate, st);
     wd::ListCopy cp{s->velB, s->idsB, hist ? s->hcnt_g : nullptr, batch ? s->sceneB : nullptr,
                     s->posA, s->velA, s->idsA, hist ? s->hcnt_slot : nullptr,
                     batch ? s->sceneA : nullptr};
@@ -663,14 +682,15 @@ cudaError_t capture_cond(cudaStream_t st, cudaGraphConditionalHandle* cond) {
 // thr: the build threshold on max |x - x_build| (m).
 cudaError_t enqueue_list_decide_build(wd_sim* s, float thr, cudaStream_t st, bool capture) {
     if (!capture) {
-        wd::launch_list_decide(s->list_ctrl, thr, s->picard, s->counters, false, 0, st);
+        wd::launch_list_decide(s->list_ctrl, thr, s->picard, s->counters,
+                               s->auto_ok ? s->auto_pend : nullptr, false, 0, st);
         enqueue_list_build(s, wd::Skip{s->list_ctrl + wd::kLcDecision, 0.5f}, st);
         return cudaGetLastError();
     }
     cudaGraphConditionalHandle cond;
     cudaError_t e = capture_cond(st, &cond);
     if (e != cudaSuccess) return e;
-    wd::launch_list_decide(s->list_ctrl, thr, s->picard, s->counters, true, cond, st);
+    wd::launch_list_decide(s->list_ctrl, thr, s->picard, s->counters, nullptr, true, cond, st);
     return capture_if_build(s, st, cond);
 }
 
@@ -831,75 +851,85 @@ cudaError_t capture_device_graph(wd_sim* s, cudaGraphExec_t* out, Body body) {
     return cudaGraphUpload(*out, s->aux_stream);
 }
 
-// The list build of the step graph of parity q as device graphs (see dev_head), on the
-// buffers that graph's build sees. On failure none is kept and the step graph holds
-// the build in a conditional node instead.
-cudaError_t capture_device_builds(wd_sim* s, int q) {
+void drop_device_graphs(wd_sim::StepGraph& g) {
+    for (cudaGraphExec_t* x : {&g.build_if, &g.head, &g.mover, &g.radix}) {
+        if (*x) cudaGraphExecDestroy(*x);
+        *x = nullptr;
+    }
+    cudaGetLastError();
+}
+
+// The list build of the state in A as three device graphs: the head, which launches one of
+// the other two.
+cudaError_t capture_build(wd_sim* s, cudaGraphExec_t* head, cudaGraphExec_t* mover,
+                          cudaGraphExec_t* radix) {
     const DevParams& P = s->P;
     const wd::Skip none{nullptr, 0.f};
-    BuildView view(s);
-    cudaError_t e = capture_device_graph(s, &s->dev_mover[q], [&](cudaStream_t st) {
+    cudaError_t e = capture_device_graph(s, mover, [&](cudaStream_t st) {
         wd::launch_search_merge(P, s->idsA, s->sb, none, st);
         enqueue_list_build_tail(s, none, st);
     });
     if (e == cudaSuccess)
-        e = capture_device_graph(s, &s->dev_radix[q], [&](cudaStream_t st) {
+        e = capture_device_graph(s, radix, [&](cudaStream_t st) {
             wd::launch_search_radix(P, s->idsA, s->sb, none, st);
             enqueue_list_build_tail(s, none, st);
         });
     if (e == cudaSuccess)
-        e = capture_device_graph(s, &s->dev_head[q], [&](cudaStream_t st) {
+        e = capture_device_graph(s, head, [&](cudaStream_t st) {
             wd::launch_search_head(P, tab(s, s->sceneA), s->posA, s->idsA, s->sb, none, nullptr,
                                    0, false, 0, s->counters, st);
             // the path the mover kernel picked (ctrl[1]: the radix sort)
-            wd::launch_graph_pick(s->sb.ctrl + 1, s->dev_mover[q], s->dev_radix[q], s->counters,
-                                  st);
+            wd::launch_graph_pick(s->sb.ctrl + 1, *mover, *radix, s->counters, st);
         });
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux_stream);
-    if (e != cudaSuccess) {
-        for (cudaGraphExec_t* x : {&s->dev_head[q], &s->dev_mover[q], &s->dev_radix[q]}) {
-            if (*x) cudaGraphExecDestroy(*x);
-            *x = nullptr;
-        }
-        cudaGetLastError();
-    }
     return e;
 }
 
-// The rest of a searched step of parity q as device graphs (see dev_step_mover). On
-// failure none is kept and the step graph holds the radix path in a conditional node.
-cudaError_t capture_device_search_steps(wd_sim* s, int q) {
-    const DevParams& P = s->P;
-    const wd::Skip none{nullptr, 0.f};
-    cudaError_t e = capture_device_graph(s, &s->dev_step_mover[q], [&](cudaStream_t st) {
-        wd::launch_search_merge(P, s->idsA, s->sb, none, st);
-        enqueue_step_tail(s, q, st, nullptr);
-    });
+// The list build after a list step from the current buffers (see StepGraph). On failure
+// none is kept and the step graph holds the build in a conditional node instead.
+cudaError_t capture_device_builds(wd_sim* s) {
+    wd_sim::StepGraph& g = s->graph_now();
+    BuildView view(s);
+    cudaError_t e = capture_build(s, &g.head, &g.mover, &g.radix);
     if (e == cudaSuccess)
-        e = capture_device_graph(s, &s->dev_step_radix[q], [&](cudaStream_t st) {
-            wd::launch_search_radix(P, s->idsA, s->sb, none, st);
-            enqueue_step_tail(s, q, st, nullptr);
+        e = capture_device_graph(s, &g.build_if, [&](cudaStream_t st) {
+            wd::launch_graph_if(s->list_ctrl + wd::kLcDecision, g.head, s->counters, st);
         });
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux_stream);
-    if (e != cudaSuccess) {
-        for (cudaGraphExec_t* x : {&s->dev_step_mover[q], &s->dev_step_radix[q]}) {
-            if (*x) cudaGraphExecDestroy(*x);
-            *x = nullptr;
-        }
-        cudaGetLastError();
-    }
+    if (e != cudaSuccess) drop_device_graphs(g);
+    return e;
+}
+
+// The rest of a searched step from the current buffers as device graphs. On failure none
+// is kept and the step graph holds the radix path in a conditional node.
+cudaError_t capture_device_search_steps(wd_sim* s, int parity) {
+    const DevParams& P = s->P;
+    const wd::Skip none{nullptr, 0.f};
+    wd_sim::StepGraph& g = s->graph_now();
+    cudaError_t e = capture_device_graph(s, &g.mover, [&](cudaStream_t st) {
+        wd::launch_search_merge(P, s->idsA, s->sb, none, st);
+        enqueue_step_tail(s, parity, st, nullptr);
+    });
+    if (e == cudaSuccess)
+        e = capture_device_graph(s, &g.radix, [&](cudaStream_t st) {
+            wd::launch_search_radix(P, s->idsA, s->sb, none, st);
+            enqueue_step_tail(s, parity, st, nullptr);
+        });
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux_stream);
+    if (e != cudaSuccess) drop_device_graphs(g);
     return e;
 }
 
 // One list-mode step: decide, build if needed, contacts + integration from A into B.
+// `launcher`: outside a capture, the graph that launches a decided build from the device
+// (NULL: the build's kernels directly, gated by the decision).
 cudaError_t enqueue_step_list(wd_sim* s, int parity, cudaStream_t st, bool capture,
-                              cudaEvent_t mid = nullptr) {
+                              cudaEvent_t mid = nullptr, cudaGraphExec_t launcher = nullptr) {
     if (s->picard) return enqueue_step_list_picard(s, parity, st, capture, mid);
     const DevParams& P = s->P;
     const bool hist = P.history != 0, batch = s->scenes > 1;
     // in a graph, the build is either tail-launched from the device (its graphs exist)
     // or an IF node that the contact kernel switches
-    const bool device_build = capture && s->dev_head[parity] != nullptr;
+    const bool device_build = capture && s->graph_now().head != nullptr;
     cudaGraphConditionalHandle cond = 0;
     if (capture && !device_build) {
         const cudaError_t e = capture_cond(st, &cond);
@@ -908,6 +938,8 @@ cudaError_t enqueue_step_list(wd_sim* s, int parity, cudaStream_t st, bool captu
     wd::ListArgs a{};
     a.thr = wd::kListValid * P.skin;
     a.tail_count = s->tail_count;
+    a.pend = s->auto_ok ? s->auto_pend : nullptr;
+    a.host_word = s->auto_word_dev;
     a.use_cond = capture && !device_build ? 1 : 0;
     a.cond = cond;
     a.pos = s->posA; a.vel = s->velA; a.ids = s->idsA; a.table = s->sb.table;
@@ -923,9 +955,10 @@ cudaError_t enqueue_step_list(wd_sim* s, int parity, cudaStream_t st, bool captu
     a.scene_out = s->sceneB;
     wd::launch_force_list(P, a, st, s->force_block, s->force_minb);
     if (mid) cudaEventRecord(mid, st);
+    if (!capture && launcher) return cudaGraphLaunch(launcher, st);
     if (device_build) {
         // the build the kernel's last block decided on (kLcDecision), from the device
-        wd::launch_graph_if(s->list_ctrl + wd::kLcDecision, s->dev_head[parity], s->counters, st);
+        wd::launch_graph_if(s->list_ctrl + wd::kLcDecision, s->graph_now().head, s->counters, st);
         return cudaGetLastError();
     }
     // the build the kernel's last block decided on, of the new state in B
@@ -946,7 +979,29 @@ cudaError_t enqueue_pending_build(wd_sim* s, cudaStream_t st) {
     if (!s->need_build) return cudaSuccess;
     s->need_build = false;
     if (s->picard) return cudaSuccess;  // the Picard step decides at its start
-    return enqueue_list_decide_build(s, wd::kListValid * s->P.skin, st, false);
+    const float thr = wd::kListValid * s->P.skin;
+    // From the second on, two launches: the decision and the head of the build's device
+    // graphs (directly, gated: about 18 launches, most of them idle; 2^20 grains 0.05 ms).
+    if (s->built_now && !s->graph_dirty && s->graphs[4 + 2 * s->lpar].now_head == nullptr) {
+        wd_sim::StepGraph& g = s->graphs[4 + 2 * s->lpar];
+        cudaError_t e = capture_build(s, &g.now_head, &g.now_mover, &g.now_radix);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux_stream);
+        if (e != cudaSuccess) {
+            for (cudaGraphExec_t* x : {&g.now_head, &g.now_mover, &g.now_radix}) {
+                if (*x) cudaGraphExecDestroy(*x);
+                *x = nullptr;
+            }
+            cudaGetLastError();
+        }
+    }
+    s->built_now = true;
+    if (!s->graph_dirty && s->graphs[4 + 2 * s->lpar].now_head) {
+        wd::launch_list_decide(s->list_ctrl, thr, false, s->counters,
+                               s->auto_ok ? s->auto_pend : nullptr, false, 0, st);
+        const cudaError_t e = cudaGetLastError();
+        return e != cudaSuccess ? e : cudaGraphLaunch(s->graphs[4 + 2 * s->lpar].now_head, st);
+    }
+    return enqueue_list_decide_build(s, thr, st, false);
 }
 
 cudaError_t enqueue_any_step(wd_sim* s, int parity, cudaStream_t st, bool capture,
@@ -955,35 +1010,32 @@ cudaError_t enqueue_any_step(wd_sim* s, int parity, cudaStream_t st, bool captur
                     : enqueue_step(s, parity, st, capture, mid);
 }
 
-int build_graphs(wd_sim* s) {
-    destroy_graphs(s);
-    const int count = (s->P.history || s->lists) ? 2 : 1;
-    for (int parity = 0; parity < count; ++parity) {
-        cudaGraph_t g = nullptr;
-        // list mode: capture the graph of parity q with the buffers it will see
-        const bool swapped = s->lists && s->lpar != parity;
-        if (swapped) swap_state(s);
-        // semi-implicit Euler on lists: the build as device-launched graphs (kept only
-        // when they instantiate; otherwise the step graph holds an IF node)
-        if (s->lists && !s->picard) capture_device_builds(s, parity);
-        if (!s->lists && !s->picard) capture_device_search_steps(s, parity);
-        WD_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-        const cudaError_t ce = enqueue_any_step(s, parity, s->stream, true);
-        const cudaError_t ee = cudaStreamEndCapture(s->stream, &g);
-        if (swapped) swap_state(s);
-        if (ce != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            WD_CUDA(ce);
-        }
-        WD_CUDA(ee);
-        size_t nodes = 0;
-        cudaGraphGetNodes(g, nullptr, &nodes);
-        s->kernels_per_step = static_cast<int>(nodes);
-        const cudaError_t e = cudaGraphInstantiate(&s->graph[parity], g, 0);
-        cudaGraphDestroy(g);
-        WD_CUDA(e);
-    }
+// The graph of the next step, captured if it is not there yet.
+int ensure_graph(wd_sim* s, bool launcher_only = false) {
+    if (s->graph_dirty) destroy_graphs(s);
     s->graph_dirty = false;
+    wd_sim::StepGraph& sg = s->graph_now();
+    if (sg.step) return WD_OK;
+    const int parity = s->P.history ? s->hist_cur : 0;
+    // semi-implicit Euler: the build, or the rest of a searched step, as device-launched
+    // graphs (kept only when they instantiate; otherwise the step graph holds an IF node)
+    if (!s->picard && !sg.head && !sg.mover) {
+        if (s->lists) capture_device_builds(s);
+        else capture_device_search_steps(s, parity);
+    }
+    if (launcher_only) return WD_OK;
+    cudaGraph_t g = nullptr;
+    WD_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+    const cudaError_t ce = enqueue_any_step(s, parity, s->stream, true);
+    const cudaError_t ee = cudaStreamEndCapture(s->stream, &g);
+    if (ce != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        WD_CUDA(ce);
+    }
+    WD_CUDA(ee);
+    const cudaError_t e = cudaGraphInstantiate(&sg.step, g, 0);
+    cudaGraphDestroy(g);
+    WD_CUDA(e);
     return WD_OK;
 }
 
@@ -1029,7 +1081,14 @@ int timed_step(wd_sim* s, int parity) {
     cudaEvent_t e0 = take_event(s), e1 = take_event(s), e2 = take_event(s);
     WD_CUDA(cudaEventRecord(e0, st));
     if (s->picard) WD_CUDA(cudaEventRecord(e1, st));
-    WD_CUDA(enqueue_any_step(s, parity, st, false, s->picard ? nullptr : e1));
+    if (s->lists && s->auto_ok) {
+        // the library's own lists: the contact kernel, then the launcher of its build
+        const int rc = ensure_graph(s, true);
+        if (rc) return rc;
+        WD_CUDA(enqueue_step_list(s, parity, st, false, e1, s->graph_now().build_if));
+    } else {
+        WD_CUDA(enqueue_any_step(s, parity, st, false, s->picard ? nullptr : e1));
+    }
     WD_CUDA(cudaEventRecord(e2, st));
     WD_CUDA(cudaGetLastError());
     s->ev_pending.push_back(e0);
@@ -1041,11 +1100,11 @@ int timed_step(wd_sim* s, int parity) {
 
 // The C state buffers: on-demand searches and the list build's gather scratch.
 cudaError_t alloc_c_buffers(wd_sim* s) {
-    if (s->posC) return cudaSuccess;
-    cudaError_t e = dalloc(&s->posC, s->n);
-    if (e == cudaSuccess) e = dalloc(&s->velC, s->n);
-    if (e == cudaSuccess) e = dalloc(&s->idsC, s->n);
-    if (e == cudaSuccess && s->scenes > 1) e = dalloc(&s->sceneC, s->n);
+    cudaError_t e = cudaSuccess;
+    if (!s->posC) e = dalloc(&s->posC, s->n);
+    if (e == cudaSuccess && !s->velC) e = dalloc(&s->velC, s->n);
+    if (e == cudaSuccess && !s->idsC) e = dalloc(&s->idsC, s->n);
+    if (e == cudaSuccess && s->scenes > 1 && !s->sceneC) e = dalloc(&s->sceneC, s->n);
     return e;
 }
 
@@ -1064,36 +1123,147 @@ int ondemand_search(wd_sim* s) {
 }
 
 int sync_stream(wd_sim* s) {
+    // list builds that did not launch, and stages of the bulk-staged contact kernel that
+    // never arrived, are counted on the device: the counters come along with the wait
+    const bool lists = s->list_work && s->pinned != nullptr;
+    s->list_work = false;
+    if (lists)
+        WD_CUDA(cudaMemcpyAsync(s->pinned, s->counters, sizeof(unsigned long long) * wd::kNumCounters,
+                                cudaMemcpyDeviceToHost, s->stream));
     WD_CUDA(cudaStreamSynchronize(s->stream));
     WD_CUDA(cudaGetLastError());
-    if (s->lists && !s->picard) {
+    if (!lists) return WD_OK;
+    if (!s->picard && s->pinned[wd::kCntLaunchFail]) {
         // a list build whose device-side graph launch failed did not run
-        unsigned long long failed = 0;
-        WD_CUDA(cudaMemcpy(&failed, s->counters + wd::kCntLaunchFail, sizeof(failed),
-                           cudaMemcpyDeviceToHost));
-        if (failed) {
-            WD_CUDA(cudaMemset(s->counters + wd::kCntLaunchFail, 0, sizeof(failed)));
-            WD_CUDA(request_list_build(s));
-            return fail(WD_ERR_CUDA, "list build: a device-side graph launch failed; the "
-                                     "steps since the last synchronisation are invalid");
-        }
+        WD_CUDA(cudaMemset(s->counters + wd::kCntLaunchFail, 0, sizeof(unsigned long long)));
+        WD_CUDA(request_list_build(s));
+        return fail(WD_ERR_CUDA, "list build: a device-side graph launch failed; the "
+                                 "steps since the last synchronisation are invalid");
     }
-    if (s->lists && (s->force_minb == 1 || s->force_minb == 2)) {
-        // the bulk-staged contact kernel flags stages that never arrived (bounded waits)
-        unsigned long long stalls = 0;
-        WD_CUDA(cudaMemcpy(&stalls, s->counters + wd::kCntStageTimeout, sizeof(stalls),
-                           cudaMemcpyDeviceToHost));
-        if (stalls) {
-            // reported once: the handle stays usable. The step stopped part-way, so even
-            // its slot order may be mixed (the first step after a build rewrites the
-            // ids); the next state upload starts from a fresh slot order.
-            WD_CUDA(cudaMemset(s->counters + wd::kCntStageTimeout, 0, sizeof(stalls)));
-            s->slots_invalid = true;
-            return fail(WD_ERR_CUDA, "contact kernel: a bulk copy into shared memory did not "
-                                     "complete within its wait limit; the state is invalid");
-        }
+    if (s->pinned[wd::kCntStageTimeout]) {
+        // reported once: the handle stays usable. The step stopped part-way, so even
+        // its slot order may be mixed (the first step after a build rewrites the
+        // ids); the next state upload starts from a fresh slot order.
+        WD_CUDA(cudaMemset(s->counters + wd::kCntStageTimeout, 0, sizeof(unsigned long long)));
+        s->slots_invalid = true;
+        return fail(WD_ERR_CUDA, "contact kernel: a bulk copy into shared memory did not "
+                                 "complete within its wait limit; the state is invalid");
     }
     return WD_OK;
+}
+
+// Skin of the library's own lists for a handle whose configuration has none, or 0 where
+// they are not used: batches and Picard; cells narrower than the largest contact distance
+// (a searched step sees the 27 cells only, so a wider list could hold other contacts);
+// boxes so large that float rounding of a position comes near the lists' 1% slack.
+float auto_skin(const wd_sim* s) {
+    if (s->cfg.neighbor_skin > 0.f || s->scenes != 1 || s->picard || !(s->P.rmax > 0.f)) return 0.f;
+    if (!(s->P.cell_min * (1.f - 1e-5f) >= 2.f * s->P.rmax)) return 0.f;
+    double mean = 0.0;
+    for (float r : s->radius) mean += r;
+    mean /= static_cast<double>(s->radius.size());
+    const double skin = 0.15 * 2.0 * mean;
+    double far = 0.0;
+    for (int a = 0; a < 3; ++a)
+        far = std::max({far, std::fabs(static_cast<double>(s->P.lo[a])), std::fabs(static_cast<double>(s->P.hi[a]))});
+    if (!(0.005 * skin > std::ldexp(far, -22))) return 0.f;
+    return static_cast<float>(skin);
+}
+
+cudaError_t alloc_list_buffers(wd_sim* s) {
+    const int n = s->n;
+    if (s->nbr) return cudaSuccess;
+    cudaError_t e = alloc_c_buffers(s);
+    if (e == cudaSuccess && !s->nbr_cnt) e = dalloc(&s->nbr_cnt, n);
+    if (e == cudaSuccess && !s->xbuild) e = dalloc(&s->xbuild, n);
+    if (e == cudaSuccess && !s->list_ctrl) e = dalloc(&s->list_ctrl, wd::kLcWords);
+    if (e == cudaSuccess && !s->list_len) e = dalloc(&s->list_len, 1);
+    if (e == cudaSuccess && !s->tail_count) e = dalloc(&s->tail_count, 1);
+    if (e == cudaSuccess && !s->pinned)
+        e = cudaMallocHost(reinterpret_cast<void**>(&s->pinned), sizeof(unsigned long long) * wd::kNumCounters);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->list_ctrl, 0, sizeof(uint32_t) * wd::kLcWords, s->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->tail_count, 0, sizeof(unsigned), s->stream);
+    if (e == cudaSuccess) e = dalloc(&s->nbr, static_cast<size_t>(n) * wd::kNbrCap);
+    return e;
+}
+
+// The buffers of the library's own lists, at creation (allocated between two steps they cost
+// 5 to 500 ms at 2^20 grains); not where they would take more than a quarter of the free
+// memory: such a handle searches.
+void auto_prepare(wd_sim* s) {
+    size_t free_b = 0, all = 0;
+    const size_t need = static_cast<size_t>(s->n) * (sizeof(int) * (wd::kNbrCap + 2) + 3 * sizeof(float4)) +
+                        s->num_cells * sizeof(uint32_t);
+    bool ok = cudaMemGetInfo(&free_b, &all) == cudaSuccess && need <= free_b / 4;
+    if (ok) {
+        cudaError_t e = alloc_list_buffers(s);
+        if (e == cudaSuccess && !s->auto_load) e = dalloc(&s->auto_load, s->num_cells);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(s->auto_load, 0, sizeof(uint32_t) * s->num_cells, s->stream);
+        if (e == cudaSuccess)
+            e = cudaHostAlloc(reinterpret_cast<void**>(&s->auto_word), 3 * sizeof(uint32_t), cudaHostAllocMapped);
+        if (e == cudaSuccess) {
+            std::memset(s->auto_word, 0, 3 * sizeof(uint32_t));
+            e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->auto_word_dev), s->auto_word, 0);
+        }
+        // the build positions are read before a first build has written them: any in-range
+        // cells are cleared then
+        if (e == cudaSuccess) e = cudaMemsetAsync(s->xbuild, 0, sizeof(float4) * s->n, s->stream);
+        unsigned long long* pend = nullptr;
+        if (e == cudaSuccess) e = dalloc(&pend, wd::kNumCounters);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(pend, 0, sizeof(unsigned long long) * wd::kNumCounters, s->stream);
+        s->auto_pend = pend;
+        ok = e == cudaSuccess;
+    }
+    if (!ok) cudaGetLastError();
+    s->auto_ok = ok;
+}
+
+// The mode of the next step of a handle that may use the library's own lists, with
+// `ahead` steps of this call to come. The lists give the searched step's results bit for
+// bit; what they cost is a build after every upload and one whenever a grain has moved
+// half a skin. So they are used for runs of kAutoRun steps and more between uploads (this
+// call's, or as long as the last such run), and not while more than one step in four
+// would build; the wait before they are tried again then doubles. Measured, upload and k
+// steps, searched against lists: 2^20 falling grains 75 + 157 k and 260 + 37 k us,
+// 100,003 packed 30 + 113 k and 100 + 31 k, the default cube 68 + 98 k and 175 + 10 k.
+constexpr int64_t kAutoRun = 3;
+
+cudaError_t auto_mode(wd_sim* s, int64_t ahead) {
+    if (s->auto_off > 0) --s->auto_off;
+    if (s->lists && (s->run_steps & 15) == 0 && s->auto_word) {
+        const volatile uint32_t* w = s->auto_word;
+        const uint32_t steps = w[0] - s->auto_seen[0], builds = w[1] - s->auto_seen[1];
+        if (w[2]) {
+            // a cell may hold more than particles_per_cell grains: every step has to be
+            // searched to count that
+            s->auto_ok = false;
+            s->lists = false;
+            s->graph_dirty = true;
+            return cudaSuccess;
+        }
+        if (steps >= 32) {
+            s->auto_seen[0] += steps;
+            s->auto_seen[1] += builds;
+            if (4 * builds > steps) {
+                s->auto_off = s->auto_backoff;
+                s->auto_backoff = std::min<int64_t>(2 * s->auto_backoff, 1 << 20);
+            } else {
+                s->auto_backoff = 512;
+            }
+        }
+    }
+    const bool lists = s->auto_off == 0 && (s->run_steps + ahead >= kAutoRun || s->last_run >= kAutoRun);
+    const bool enter = lists && !s->lists;
+    s->lists = lists;
+    return enter ? request_list_build(s) : cudaSuccess;
+}
+
+// A state upload ends a run of steps.
+void note_upload(wd_sim* s) {
+    if (s->run_steps > 0) s->last_run = s->run_steps;
+    s->run_steps = 0;
 }
 
 int alloc_sim(wd_sim* s) {
@@ -1174,7 +1344,7 @@ int alloc_sim(wd_sim* s) {
     WD_CUDA(cudaMemcpy(s->d_chunk_base, chunk.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice));
     WD_CUDA(dalloc(&s->partials, static_cast<size_t>(3) * s->total_chunks));
     WD_CUDA(dalloc(&s->scene_sums, static_cast<size_t>(3) * S));
-    WD_CUDA(dalloc(&s->grain_vals, static_cast<size_t>(3) * n));
+    WD_CUDA(dalloc(&s->grain_vals, static_cast<size_t>(4) * n));
     if (S > 1) {
         WD_CUDA(dalloc(&s->d_scene_P, S));
         WD_CUDA(cudaMemcpy(s->d_scene_P, s->scene_P.data(), sizeof(DevParams) * S, cudaMemcpyHostToDevice));
@@ -1185,14 +1355,8 @@ int alloc_sim(wd_sim* s) {
         WD_CUDA(dalloc(&s->scene_unstable, S));
     }
     if (s->lists) {
-        WD_CUDA(dalloc(&s->nbr, static_cast<size_t>(n) * wd::kNbrCap));
-        WD_CUDA(dalloc(&s->nbr_cnt, n));
-        WD_CUDA(dalloc(&s->xbuild, n));
-        WD_CUDA(dalloc(&s->list_ctrl, wd::kLcWords));
-        WD_CUDA(dalloc(&s->list_len, 1));
-        WD_CUDA(dalloc(&s->tail_count, 1));
-        WD_CUDA(cudaMemset(s->tail_count, 0, sizeof(unsigned)));
-        WD_CUDA(alloc_c_buffers(s));
+        WD_CUDA(alloc_list_buffers(s));
+        WD_CUDA(cudaStreamSynchronize(s->stream));
         uint32_t init[wd::kLcWords] = {};
         init[wd::kLcForce] = 1u;  // the first step builds
         WD_CUDA(cudaMemcpy(s->list_ctrl, init, sizeof(init), cudaMemcpyHostToDevice));
@@ -1361,7 +1525,17 @@ int create_scenes(const wd::Config* const* cfgs, int S, const int64_t* counts,
     for (int k = 0; k < S; ++k)
         std::memcpy(all_state.data() + 6 * s->scene_off[k], states[k],
                     sizeof(float) * 6 * static_cast<size_t>(counts[k]));
+    const float own = auto_skin(s);
+    if (own > 0.f) {
+        s->P.skin = own;
+        s->scene_P[0].skin = own;
+    }
     int rc = alloc_sim(s);
+    if (rc == WD_OK && own > 0.f) {
+        auto_prepare(s);
+        const cudaError_t e = cudaStreamSynchronize(s->stream);
+        if (e != cudaSuccess) rc = fail(WD_ERR_CUDA, cudaGetErrorString(e));
+    }
     if (rc == WD_OK) rc = upload_initial(s, all_state.data());
     if (rc != WD_OK) {
         const std::string msg = wd::last_error_cstr();
@@ -1538,17 +1712,20 @@ int wd_destroy(wd_sim* sim) {
 int wd_step(wd_sim* sim, int64_t nsteps) {
     if (!sim || nsteps < 0) return fail(WD_ERR_INVALID, "wd_step: bad argument");
     for (int64_t k = 0; k < nsteps; ++k) {
-        const int parity = sim->lists ? sim->lpar : (sim->P.history ? sim->hist_cur : 0);
-        if (sim->lists) WD_CUDA(enqueue_pending_build(sim, sim->stream));
+        const int parity = sim->P.history ? sim->hist_cur : 0;
+        if (sim->auto_ok) WD_CUDA(auto_mode(sim, nsteps - k));
+        ++sim->run_steps;
+        if (sim->lists) {
+            sim->list_work = true;
+            WD_CUDA(enqueue_pending_build(sim, sim->stream));
+        }
         if (sim->cfg.kernel_timing) {
             const int rc = timed_step(sim, parity);
             if (rc) return rc;
         } else {
-            if (sim->graph_dirty) {
-                const int rc = build_graphs(sim);
-                if (rc) return rc;
-            }
-            WD_CUDA(cudaGraphLaunch(sim->graph[parity], sim->stream));
+            const int rc = ensure_graph(sim);
+            if (rc) return rc;
+            WD_CUDA(cudaGraphLaunch(sim->graph_now().step, sim->stream));
         }
         if (sim->lists) swap_state(sim);
         if (sim->P.history) sim->hist_cur ^= 1;
@@ -1661,6 +1838,7 @@ int wd_set_state_device(wd_sim* sim, const float* d_state) {
     }
     wd::launch_state_from_aos(sim->n, d_state, sim->posA, sim->velA, sim->idsA, sim->stream);
     WD_CUDA(cudaGetLastError());
+    note_upload(sim);
     WD_CUDA(request_list_build(sim));
     return WD_OK;
 }
@@ -1774,6 +1952,7 @@ int wd_set_state_async(wd_sim* sim, const float* state) {
     wd::launch_state_from_aos(sim->n, sim->io_in[i], sim->posA, sim->velA, sim->idsA, sim->stream);
     WD_CUDA(cudaGetLastError());
     WD_CUDA(cudaEventRecord(sim->ev_in_free[i], sim->stream));
+    note_upload(sim);
     WD_CUDA(request_list_build(sim));
     return WD_OK;
 }
@@ -1962,7 +2141,7 @@ int wd_compute_total_energy(wd_sim* sim, double* energy) {
 
 int wd_compute_scene_momenta(wd_sim* sim, double* momenta) {
     if (!sim || !momenta) return fail(WD_ERR_INVALID, "wd_compute_scene_momenta: NULL argument");
-    wd::launch_momentum(sim->n, sim->velA, segments(sim), sim->grain_vals, sim->partials,
+    wd::launch_momentum(sim->n, sim->velA, sim->idsA, segments(sim), sim->grain_vals, sim->partials,
                         sim->scene_sums, sim->stream);
     WD_CUDA(cudaGetLastError());
     WD_CUDA(cudaMemcpyAsync(momenta, sim->scene_sums, 3 * sizeof(double) * sim->scenes,
@@ -2052,6 +2231,13 @@ int wd_set_kernel_timing(wd_sim* sim, int32_t enabled) {
     return WD_OK;
 }
 
+// Whether the step graphs of the current mode hand work to device-launched graphs.
+static bool device_graphs(const wd_sim* sim) {
+    for (int k = 0; k < 4; ++k)
+        if (sim->graphs[(sim->lists ? 4 : 0) + k].mover != nullptr) return true;
+    return false;
+}
+
 int wd_kernels_per_step(const wd_sim* sim_c, int64_t* kernels) {
     wd_sim* sim = const_cast<wd_sim*>(sim_c);
     if (!sim || !kernels) return fail(WD_ERR_INVALID, "wd_kernels_per_step: NULL argument");
@@ -2062,12 +2248,10 @@ int wd_kernels_per_step(const wd_sim* sim_c, int64_t* kernels) {
     // wd_list_stats' count (Picard: the decision, the iterations, the last iterate's
     // copy, the redo check)
     if (sim->lists && !sim->picard) {
-        const bool device = sim->dev_head[0] != nullptr || sim->dev_head[1] != nullptr;
-        *kernels = device ? 2 : 1;
+        *kernels = device_graphs(sim) ? 2 : 1;
     } else if (!sim->lists && !sim->picard) {
         // the searched step: with its tail launched from the device, the path-pick kernel
-        const bool device = sim->dev_step_mover[0] != nullptr || sim->dev_step_mover[1] != nullptr;
-        *kernels = device ? 6 : 5;
+        *kernels = device_graphs(sim) ? 6 : 5;
     } else {
         *kernels = sim->lists ? sim->picard_iters + 3 : static_cast<int64_t>(5) * sim->picard_iters;
     }
@@ -2142,18 +2326,8 @@ int wd_debug_candidates(wd_sim* sim, int64_t* offsets, int32_t* cand, uint8_t* c
 static int apply_skin(wd_sim* s, float skin) {
     if (skin < 0.f) return fail(WD_ERR_INVALID, "neighbor skin must be >= 0");
     const bool lists = skin > 0.f;
-    if (lists && !s->nbr) {
-        const int n = s->n;
-        WD_CUDA(dalloc(&s->nbr, static_cast<size_t>(n) * wd::kNbrCap));
-        WD_CUDA(dalloc(&s->nbr_cnt, n));
-        WD_CUDA(dalloc(&s->xbuild, n));
-        WD_CUDA(dalloc(&s->list_ctrl, wd::kLcWords));
-        WD_CUDA(dalloc(&s->list_len, 1));
-        WD_CUDA(dalloc(&s->tail_count, 1));
-        WD_CUDA(alloc_c_buffers(s));
-        WD_CUDA(cudaMemsetAsync(s->list_ctrl, 0, sizeof(uint32_t) * wd::kLcWords, s->stream));
-        WD_CUDA(cudaMemsetAsync(s->tail_count, 0, sizeof(unsigned), s->stream));
-    }
+    s->auto_ok = false;   // the caller's choice, 0 included
+    if (lists) WD_CUDA(alloc_list_buffers(s));
     if (lists && s->picard && !s->xpos) {
         const int n = s->n;
         WD_CUDA(dalloc(&s->xpos, n));
@@ -2166,7 +2340,6 @@ static int apply_skin(wd_sim* s, float skin) {
         WD_CUDA(cudaMemcpyAsync(s->rhs_ids, s->idsB, sizeof(int) * n, cudaMemcpyDeviceToDevice, s->stream));
         if (s->scenes > 1) WD_CUDA(dalloc(&s->xscene, n));
     }
-    if (lists && !s->lists) s->lpar = s->P.history ? s->hist_cur : s->lpar;
     s->lists = lists;
     s->cfg.neighbor_skin = skin;
     s->P.skin = skin;
@@ -2216,8 +2389,7 @@ int wd_list_stats(wd_sim* sim, int64_t* builds, int32_t* kernels_each, double* m
         // device-launched builds: the head (keys, mover sort, path pick) and the mover
         // path (merge, gather, listing); in a conditional node or direct launches: every
         // search kernel (the radix ones return at once when idle), gather and listing
-        const bool device = sim->dev_head[0] != nullptr || sim->dev_head[1] != nullptr;
-        *kernels_each = !sim->lists ? 0 : device ? 6 : 2 + (1 + 3 * sim->sb.passes) + 1 + 2;
+        *kernels_each = !(sim->cfg.neighbor_skin > 0.f) ? 0 : device_graphs(sim) ? 6 : 2 + (1 + 3 * sim->sb.passes) + 1 + 2;
     }
     if (builds) {
         int rc = read_counter(sim, wd::kCntListBuilds, builds);
@@ -2225,7 +2397,7 @@ int wd_list_stats(wd_sim* sim, int64_t* builds, int32_t* kernels_each, double* m
     }
     if (mean_length) {
         *mean_length = 0.0;
-        if (sim->lists) {
+        if (sim->cfg.neighbor_skin > 0.f) {
             WD_CUDA(cudaMemsetAsync(sim->list_len, 0, sizeof(unsigned long long), sim->stream));
             wd::launch_list_length(sim->n, sim->nbr_cnt, sim->list_len, sim->stream);
             WD_CUDA(cudaGetLastError());
@@ -2315,7 +2487,7 @@ cudaError_t adj_back_body(wd_sim* s, int len, int cur, cudaStream_t st) {
 // One replay (parity -1) or walk-back segment, from a graph captured once per
 // (length, parity) and kept until the step parameters or the tape change.
 cudaError_t run_adj_graph(wd_sim* s, int len, int parity) {
-    const auto key = std::make_pair(len, parity);
+    const auto key = std::make_pair(len, 2 * (parity + 1) + s->lpar);
     auto it = s->adj_graphs.find(key);
     if (it == s->adj_graphs.end()) {
         cudaGraph_t g = nullptr;
@@ -2518,9 +2690,10 @@ int wd_set_contact_params(wd_sim* sim, float mu, float restitution, float k_n) {
     sim->cfg.friction = mu;
     sim->cfg.restitution = restitution;
     sim->cfg.normal_stiffness = k_n;
-    const float rmax = sim->P.rmax;
+    const float rmax = sim->P.rmax, skin = sim->P.skin;
     sim->P = make_params(sim->cfg, sim->n, sim->dt);
     sim->P.rmax = rmax;
+    sim->P.skin = skin;   // the lists' skin, chosen by the library when the caller has none
     sim->scene_P[0] = sim->P;
     sim->scene_cfg[0] = sim->cfg;
     sim->graph_dirty = true;
@@ -2543,6 +2716,7 @@ int wd_adjoint_record(wd_sim* sim, int64_t steps, int32_t checkpoint_every) {
         WD_CUDA(alloc_snap(sim, sim->adj_ckpt.back()));
     }
     if (!sim->adj_end.pos) WD_CUDA(alloc_snap(sim, sim->adj_end));
+    sim->last_run = std::max(sim->last_run, steps);   // the run's length is known
     int64_t hist_over0 = 0;
     rc = read_counter(sim, wd::kCntHistOverflow, &hist_over0);
     if (rc) return rc;
