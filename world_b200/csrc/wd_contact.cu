@@ -147,15 +147,12 @@ __device__ __forceinline__ double block_sum(double v) {
 // 1/2 k_t |xi|^2 of stored contacts in history mode. Terms in FP32 as the
 // reference, the grain's sum in FP64, written per sorted position for the segmented
 // reduction below.
-template <bool HIST, bool BATCH>
-__global__ void __launch_bounds__(kBlock)
-k_energy(DevParams P0, SceneTab T, const float4* __restrict__ pos, const float4* __restrict__ vel,
-         const int* __restrict__ ids, const int2* __restrict__ table,
-         const float4* __restrict__ hist, const int* __restrict__ hcnt,
-         const int* __restrict__ src, double* __restrict__ out) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= P0.n) return;
-    const DevParams& P = scene_params<BATCH>(P0, T, s);
+template <bool HIST>
+__device__ __forceinline__ double energy_of(const DevParams& P, int s, const float4* __restrict__ pos,
+                                            const float4* __restrict__ vel, const int* __restrict__ ids,
+                                            const int2* __restrict__ table,
+                                            const float4* __restrict__ hist,
+                                            const int* __restrict__ hcnt, const int* __restrict__ src) {
     double e = 0.0;
     const float4 pi = pos[s], vi = vel[s];
     const int id = ids[s];
@@ -174,22 +171,30 @@ k_energy(DevParams P0, SceneTab T, const float4* __restrict__ pos, const float4*
     }
     int cx, cy, cz;
     cell_coords(P, pi.x, pi.y, pi.z, cx, cy, cz);
+    // a column's nine table entries in one go, candidates two at a time; the partner's id
+    // only for the few pairs that overlap (1,000,003 grains 84 us; with the id of every
+    // candidate read before its position 114)
+    auto visit = [&](int j, float4 pj) {
+        float3 d;
+        const float ns = pair_norm_sq(pi, pj, d);
+        if (!maybe_contact(ns, ri, pj.w) || j == s || ids[j] <= id) return;
+        e += static_cast<double>(contact_energy((ri + pj.w) - sqrtf(ns), cd, F, k));
+    };
     for (int dx = -1; dx <= 1; ++dx) {
         const int nx = cx + dx;
         if (nx < 0 || nx >= P.grid[0]) continue;
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int ny = cy + dy;
-            if (ny < 0 || ny >= P.grid[1]) continue;
-            int lo, hi;
-            column_range(P, table, nx, ny, cz, lo, hi);
-            for (int j = lo; j < hi; ++j) {
-                if (j == s || ids[j] <= id) continue;
-                const float4 pj = pos[j];
-                float3 d;
-                const float ns = pair_norm_sq(pi, pj, d);
-                if (!maybe_contact(ns, ri, pj.w)) continue;
-                e += static_cast<double>(contact_energy((ri + pj.w) - sqrtf(ns), cd, F, k));
+        int lo[3], hi[3];
+        row_ranges(P, table, nx, cy, cz, lo, hi);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            int j = lo[t];
+            // an empty row has lo = INT_MAX, hi = 0: the difference does not overflow
+            for (; hi[t] - j > 1; j += 2) {
+                const float4 p0 = __ldg(&pos[j]), p1 = __ldg(&pos[j + 1]);
+                visit(j, p0);
+                visit(j + 1, p1);
             }
+            if (j < hi[t]) visit(j, __ldg(&pos[j]));
         }
     }
     if (HIST) {
@@ -204,7 +209,24 @@ k_energy(DevParams P0, SceneTab T, const float4* __restrict__ pos, const float4*
             e += static_cast<double>(0.5f * P.k_t * xs);
         }
     }
-    out[s] = e;
+    return e;
+}
+
+// CHUNK: a single scene's chunks are this kernel's blocks, so each block leaves its chunk's
+// sum (the tree of k_segment_chunks) instead of its grains' values.
+template <bool HIST, bool BATCH, bool CHUNK>
+__global__ void __launch_bounds__(kBlock, 5)
+k_energy(DevParams P0, SceneTab T, const float4* __restrict__ pos, const float4* __restrict__ vel,
+         const int* __restrict__ ids, const int2* __restrict__ table,
+         const float4* __restrict__ hist, const int* __restrict__ hcnt,
+         const int* __restrict__ src, double* __restrict__ out) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (CHUNK) {
+        const double t = block_sum(s < P0.n ? energy_of<HIST>(P0, s, pos, vel, ids, table, hist, hcnt, src) : 0.0);
+        if (threadIdx.x == 0) out[blockIdx.x] = t;
+    } else if (s < P0.n) {
+        out[s] = energy_of<HIST>(scene_params<BATCH>(P0, T, s), s, pos, vel, ids, table, hist, hcnt, src);
+    }
 }
 
 // Segmented sums, step 1: one block per 256-grain chunk of a scene's segment (chunks
@@ -231,19 +253,27 @@ k_segment_chunks(const double* __restrict__ v, int64_t comp_step, int grain_step
     }
 }
 
-// Segmented sums, step 2: one block per scene sums its chunk partials in a fixed order.
+// Segmented sums, step 2: one block per scene and component sums its chunk partials in a
+// fixed order, eight loads in flight (one block alone waits for each: 11 us for the 3,907
+// partials of 1,000,003 grains, and that three times over for the momentum).
 __global__ void __launch_bounds__(kBlock)
 k_segment_finish(const double* __restrict__ partials, const int* __restrict__ chunk_base,
                  int comps, int total_chunks, double* __restrict__ out) {
-    const int sc = blockIdx.x;
+    const int sc = blockIdx.x, c = blockIdx.y;
     const int c0 = chunk_base[sc], c1 = chunk_base[sc + 1];
-    for (int c = 0; c < comps; ++c) {
-        double x = 0.0;
-        for (int i = c0 + static_cast<int>(threadIdx.x); i < c1; i += blockDim.x)
-            x += partials[static_cast<int64_t>(c) * total_chunks + i];
-        const double t = block_sum(x);
-        if (threadIdx.x == 0) out[sc * comps + c] = t;
+    const double* v = partials + static_cast<int64_t>(c) * total_chunks;
+    double x = 0.0;
+    int i = c0 + static_cast<int>(threadIdx.x);
+    for (; i + 7 * kBlock < c1; i += 8 * kBlock) {
+        double a[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) a[u] = __ldg(&v[i + u * kBlock]);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x += a[u];
     }
+    for (; i < c1; i += kBlock) x += __ldg(&v[i]);
+    const double t = block_sum(x);
+    if (threadIdx.x == 0) out[sc * comps + c] = t;
 }
 
 // Momentum terms by grain id, so that the sums do not depend on the order of the slots
@@ -323,7 +353,7 @@ void launch_segment_sums(const double* values, int n, int comps, const Segments&
     k_segment_chunks<<<g.total_chunks, kBlock, 0, st>>>(values, grain_step > 1 ? 1 : n, grain_step,
                                                         comps, g.seg, g.chunk_base, g.scenes,
                                                         partials, g.total_chunks);
-    k_segment_finish<<<g.scenes, kBlock, 0, st>>>(partials, g.chunk_base, comps, g.total_chunks, out);
+    k_segment_finish<<<dim3(g.scenes, comps), kBlock, 0, st>>>(partials, g.chunk_base, comps, g.total_chunks, out);
 }
 
 void launch_energy(const DevParams& P, SceneTab T, const float4* pos, const float4* vel,
@@ -331,15 +361,23 @@ void launch_energy(const DevParams& P, SceneTab T, const float4* pos, const floa
                    const int* src, const Segments& g, double* per_grain, double* partials,
                    double* out, cudaStream_t st) {
     const int nb = reduction_blocks(P.n);
-    const bool batch = T.params != nullptr;
+    const bool batch = T.params != nullptr, chunk = g.scenes == 1 && per_grain == nullptr;
+    double* to = chunk ? partials : per_grain;
+#define WD_ENERGY(H, B, C) k_energy<H, B, C><<<nb, kBlock, 0, st>>>(P, T, pos, vel, ids, table, hist, hcnt, src, to)
     if (P.history) {
-        if (batch) k_energy<true, true><<<nb, kBlock, 0, st>>>(P, T, pos, vel, ids, table, hist, hcnt, src, per_grain);
-        else k_energy<true, false><<<nb, kBlock, 0, st>>>(P, T, pos, vel, ids, table, hist, hcnt, src, per_grain);
+        if (batch) WD_ENERGY(true, true, false);
+        else if (chunk) WD_ENERGY(true, false, true);
+        else WD_ENERGY(true, false, false);
     } else {
-        if (batch) k_energy<false, true><<<nb, kBlock, 0, st>>>(P, T, pos, vel, ids, table, hist, hcnt, src, per_grain);
-        else k_energy<false, false><<<nb, kBlock, 0, st>>>(P, T, pos, vel, ids, table, hist, hcnt, src, per_grain);
+        if (batch) WD_ENERGY(false, true, false);
+        else if (chunk) WD_ENERGY(false, false, true);
+        else WD_ENERGY(false, false, false);
     }
-    launch_segment_sums(per_grain, P.n, 1, g, partials, out, st);
+#undef WD_ENERGY
+    if (chunk)
+        k_segment_finish<<<1, kBlock, 0, st>>>(partials, g.chunk_base, 1, g.total_chunks, out);
+    else
+        launch_segment_sums(per_grain, P.n, 1, g, partials, out, st);
 }
 
 void launch_momentum(int n, const float4* vel, const int* ids, const Segments& g,

@@ -8,8 +8,10 @@
 // integer with a power-of-two scale chosen per channel from a bound on the channel's
 // total, and accumulated with integer atomics: integer addition is associative, so
 // the field is bit-identical run to run and is the correctly rounded sum up to the
-// 2^-62-relative quantum. Grains are visited in cell order, so neighbouring lanes hit
-// the same nodes; identical nodes inside a warp are combined before the atomic.
+// 2^-62-relative quantum. Because every part adds the same integers, it may group them as
+// it likes; the accumulators are node-major (the four channels of a node share one
+// 32-byte sector) and k_deposit's lanes are laid over corners and channels (see there).
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 
@@ -42,232 +44,262 @@ struct DepositGeom {
     int size[3];
 };
 
-// Channel bounds: max |m| and max |m v_a| over grains (float bits; max of
-// non-negative floats is order-independent).
-__global__ void __launch_bounds__(kBlock)
-k_deposit_bounds(int n, const float4* __restrict__ vel, uint32_t* __restrict__ bounds) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t b[4] = {0u, 0u, 0u, 0u};
-    if (s < n) {
-        const float4 v = vel[s];
-        const float m = v.w;
-        if (m != 0.f) {
-            b[0] = __float_as_uint(fabsf(m));
-            b[1] = __float_as_uint(fabsf(m * v.x));
-            b[2] = __float_as_uint(fabsf(m * v.y));
-            b[3] = __float_as_uint(fabsf(m * v.z));
+// Where a deposit's grains come from: the simulation's slots (pos, vel with the mass in w),
+// slots of a batch (their scene's grid, scale and nodes), or the caller's AoS6 states.
+struct FromSlots {
+    const float4* pos;
+    const float4* vel;
+    DepositGeom g;
+    __device__ __forceinline__ float4 momentum(int s) const { return vel[s]; }   // vx vy vz m
+    __device__ __forceinline__ float3 place(int s) const {
+        const float4 p = pos[s];
+        return make_float3(p.x, p.y, p.z);
+    }
+    __device__ __forceinline__ int scene(int) const { return 0; }
+    __device__ __forceinline__ int count(int, int n) const { return n; }
+    __device__ __forceinline__ DepositGeom geom(int) const { return g; }
+    __device__ __forceinline__ int first_node(int) const { return 0; }
+};
+struct FromScenes {
+    const float4* pos;
+    const float4* vel;
+    SceneTab T;
+    __device__ __forceinline__ float4 momentum(int s) const { return vel[s]; }
+    __device__ __forceinline__ float3 place(int s) const {
+        const float4 p = pos[s];
+        return make_float3(p.x, p.y, p.z);
+    }
+    __device__ __forceinline__ int scene(int s) const { return T.scene[s]; }
+    __device__ __forceinline__ int count(int sc, int) const { return T.params[sc].n; }
+    __device__ __forceinline__ DepositGeom geom(int sc) const {
+        const DevParams& Q = T.params[sc];
+        DepositGeom g;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            g.lo[a] = Q.lo[a];
+            g.hi[a] = Q.hi[a];
+            g.size[a] = Q.dgrid[a];
         }
+        return g;
     }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        uint32_t x = b[c];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x = max(x, __shfl_xor_sync(0xffffffffu, x, o));
-        if ((threadIdx.x & 31) == 0 && x) atomicMax(&bounds[c], x);
+    __device__ __forceinline__ int first_node(int sc) const { return T.params[sc].node_base; }
+};
+struct FromAos {
+    const float* state;
+    const float* mass;
+    DepositGeom g;
+    __device__ __forceinline__ float4 momentum(int s) const {
+        const float* q = state + 6 * static_cast<int64_t>(s);
+        return make_float4(q[3], q[4], q[5], mass[s]);
     }
-}
+    __device__ __forceinline__ float3 place(int s) const {
+        const float* q = state + 6 * static_cast<int64_t>(s);
+        return make_float3(q[0], q[1], q[2]);
+    }
+    __device__ __forceinline__ int scene(int) const { return 0; }
+    __device__ __forceinline__ int count(int, int n) const { return n; }
+    __device__ __forceinline__ DepositGeom geom(int) const { return g; }
+    __device__ __forceinline__ int first_node(int) const { return 0; }
+};
 
-// Scale 2^(62-e) with n * bound < 2^e, so every partial sum stays below 2^62.
-__device__ __forceinline__ double channel_scale(int n, uint32_t bound_bits) {
-    const double b = static_cast<double>(__uint_as_float(bound_bits)) * static_cast<double>(n);
-    if (!(b > 0.0) || !isfinite(b)) return 1.0;
-    int e;
-    frexp(b, &e);
-    return ldexp(1.0, 62 - e);
-}
+// Channel bounds: max |m| and max |m v_a| over grains, per scene (float bits; max of
+// non-negative floats is order-independent). A grid of at most kBoundBlocks blocks: the
+// maxima meet at four words per scene, and an atomic per warp of 10^6 grains on each took
+// 84 us where one per block takes 7. Slots of a scene are consecutive, so a thread's
+// grains change scene rarely; it hands its maxima over when they do.
+constexpr int kBoundBlocks = 4 * 148;
 
-// Adds up q over each run of adjacent lanes that hold the same key: a segmented inclusive
-// scan by shuffles (one step per doubling of the longest run in the warp), after which the
-// last lane of each run holds the run's total. Returns true on that lane. Grains arrive in
-// cell order, so lanes that deposit on one node are mostly adjacent; a node that comes back
-// later in the warp forms a second run with its own atomic. The values are integers, so the
-// node totals do not depend on how the lanes are grouped.
-__device__ __forceinline__ bool run_totals(long long key, long long (&q)[4]) {
-    const int lane = threadIdx.x & 31;
-    const long long prev = __shfl_up_sync(0xffffffffu, key, 1);
-    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != key);
-    const bool last = lane == 31 || ((heads >> (lane + 1)) & 1u);
-    if (heads == 0xffffffffu) return true;
-    const int start = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-    const unsigned longest = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(lane - start + 1));
-    for (unsigned d = 1; d < longest; d <<= 1) {
+template <class Src>
+__global__ void __launch_bounds__(kBlock)
+k_deposit_bounds(int n, Src src, uint32_t* __restrict__ bounds) {
+    __shared__ uint32_t block_max[4];
+    __shared__ int block_scene;
+    const int per = (n + gridDim.x - 1) / gridDim.x;          // consecutive grains per block
+    const int first = blockIdx.x * per, last = min(n, first + per);
+    if (threadIdx.x < 4) block_max[threadIdx.x] = 0u;
+    if (threadIdx.x == 0) block_scene = first < last ? src.scene(first) : 0;
+    __syncthreads();
+    uint32_t b[4] = {0u, 0u, 0u, 0u};
+    int held = block_scene;
+    auto hand_over = [&]() {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const long long t = __shfl_up_sync(0xffffffffu, q[c], d);
-            if (lane - static_cast<int>(d) >= start) q[c] += t;
+            if (b[c]) atomicMax(&bounds[4 * held + c], b[c]);
+            b[c] = 0u;
+        }
+    };
+    for (int s = first + static_cast<int>(threadIdx.x); s < last; s += blockDim.x) {
+        const int sc = src.scene(s);
+        if (sc != held) {
+            hand_over();
+            held = sc;
+        }
+        const float4 v = src.momentum(s);
+        const float m = v.w;
+        if (m != 0.f) {
+            b[0] = max(b[0], __float_as_uint(fabsf(m)));
+            b[1] = max(b[1], __float_as_uint(fabsf(m * v.x)));
+            b[2] = max(b[2], __float_as_uint(fabsf(m * v.y)));
+            b[3] = max(b[3], __float_as_uint(fabsf(m * v.z)));
         }
     }
-    return last;
+    if (held != block_scene) hand_over();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const uint32_t x = __reduce_max_sync(0xffffffffu, b[c]);
+        if ((threadIdx.x & 31) == 0 && x) atomicMax(&block_max[c], x);
+    }
+    __syncthreads();
+    if (threadIdx.x < 4 && block_max[threadIdx.x])
+        atomicMax(&bounds[4 * block_scene + threadIdx.x], block_max[threadIdx.x]);
 }
 
-__global__ void __launch_bounds__(kBlock)
-k_deposit(int n, const float4* __restrict__ pos, const float4* __restrict__ vel,
-          DepositGeom g, const uint32_t* __restrict__ bounds,
-          unsigned long long* __restrict__ acc) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t nodes = static_cast<int64_t>(g.size[0]) * g.size[1] * g.size[2];
-    double scale[4];
+// Exponent k of the scale 2^k = 2^(62-e) with n * bound < 2^e, so that every partial sum
+// stays below 2^62 (bound * n is a normal double, whose exponent field gives e).
+__device__ __forceinline__ int scale_exponent(int n, uint32_t bound_bits) {
+    const double b = static_cast<double>(__uint_as_float(bound_bits)) * static_cast<double>(n);
+    if (!(b > 0.0) || !isfinite(b)) return 0;
+    return 62 - (((__double2hiint(b) >> 20) & 0x7ff) - 1022);
+}
+__device__ __forceinline__ float exp2_float(int k) { return __int_as_float((k + 127) << 23); }   // |k| < 127
+__device__ __forceinline__ double exp2_double(int k) { return __hiloint2double((k + 1023) << 20, 0); }
+
+// One warp per kDepositGroup consecutive grains, 32 at a time. Each lane works out one
+// grain's 32 contributions (8 corners, 4 channels) as integers and leaves them and the 8
+// node indices in shared memory; then lane l takes corner l / 4, channel l % 4 of every
+// grain in turn and adds up while its node stays the same, so that a node change costs one
+// atomic per lane. The lanes of a node's channels, and of the two nodes adjacent in z, fall
+// in one or two sectors of the node-major accumulators: 8 sector updates a grain where
+// channel planes took 32, and fewer where consecutive grains share nodes.
+// A contribution is float(m w) times a power of two, converted to int64: exact but for the
+// conversion's own rounding, as the double product was (where the scaled value is too small
+// for a normal float it rounds to zero in both). The power goes in two factors, since
+// 2^k, k up to 211, need not be a float.
+// Bound by the accumulators' sector updates. 1,000,003 grains onto 128^3 nodes in lattice
+// order (no two neighbours on a node, the worst case): 77 us, with channel planes and a
+// shuffle scan per corner 151; the finish 14 instead of 37, the bounds 8 instead of 84.
+constexpr int kDepositWarps = 4;
+constexpr int kDepositGroup = 128;
+
+template <class Src>
+__global__ void __launch_bounds__(32 * kDepositWarps)
+k_deposit(int n, Src src, const uint32_t* __restrict__ bounds, unsigned long long* __restrict__ acc) {
+    __shared__ long long val[kDepositWarps][32][33];
+    __shared__ int node[kDepositWarps][32][9];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t first = (static_cast<int64_t>(blockIdx.x) * kDepositWarps + w) * kDepositGroup;
+    const int corner = lane >> 2, channel = lane & 3;
+    long long sum = 0;
+    int cur = -1;
+    for (int64_t base = first; base < min(first + kDepositGroup, static_cast<int64_t>(n)); base += 32) {
+        const int s = static_cast<int>(base) + lane;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s < n) v = src.momentum(s);
+        const float m = v.w;
+        if (m != 0.f) {
+            const int sc = src.scene(s);
+            const DepositGeom g = src.geom(sc);
+            const int cnt = src.count(sc, n);
+            const float3 x = src.place(s);
+            float lo_f[4], hi_f[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) scale[c] = channel_scale(n, bounds[c]);
-    bool active = s < n;
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), v = x;
-    if (active) {
-        x = pos[s];
-        v = vel[s];
-        active = v.w != 0.f;
-    }
-    int ix[2] = {0, 0}, iy[2] = {0, 0}, iz[2] = {0, 0};
-    float wx[2] = {0.f, 0.f}, wy[2] = {0.f, 0.f}, wz[2] = {0.f, 0.f};
-    const float m = v.w;
-    const float mom[3] = {m * v.x, m * v.y, m * v.z};
-    if (active) {
-        axis_weights(x.x, g.lo[0], g.hi[0], g.size[0], ix[0], ix[1], wx[0], wx[1]);
-        axis_weights(x.y, g.lo[1], g.hi[1], g.size[1], iy[0], iy[1], wy[0], wy[1]);
-        axis_weights(x.z, g.lo[2], g.hi[2], g.size[2], iz[0], iz[1], wz[0], wz[1]);
-    }
-#pragma unroll
-    for (int cx = 0; cx < 2; ++cx)
-#pragma unroll
-        for (int cy = 0; cy < 2; ++cy)
-#pragma unroll
-            for (int cz = 0; cz < 2; ++cz) {
-                const float w = wx[cx] * wy[cy] * wz[cz];
-                const bool live = active && w != 0.f;
-                const long long node =
-                    live ? (static_cast<long long>(ix[cx]) * g.size[1] + iy[cy]) * g.size[2] + iz[cz]
-                         : -1ll;
-                long long q[4] = {0, 0, 0, 0};
-                if (live) {
-                    q[0] = __double2ll_rn(static_cast<double>(m * w) * scale[0]);
-#pragma unroll
-                    for (int a = 0; a < 3; ++a)
-                        q[a + 1] = __double2ll_rn(static_cast<double>(mom[a] * w) * scale[a + 1]);
-                }
-                // combine adjacent lanes that hit the same node, then one atomic per run
-                const bool tail = run_totals(node, q);
-                if (live && tail) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        if (q[c] != 0)
-                            atomicAdd(&acc[c * nodes + node], static_cast<unsigned long long>(q[c]));
-                }
+            for (int c = 0; c < 4; ++c) {
+                const int k = scale_exponent(cnt, bounds[4 * sc + c]);
+                const int k1 = min(k, 126);
+                lo_f[c] = exp2_float(k1);
+                hi_f[c] = exp2_float(k - k1);
             }
+            int ix[2], iy[2], iz[2];
+            float wx[2], wy[2], wz[2];
+            axis_weights(x.x, g.lo[0], g.hi[0], g.size[0], ix[0], ix[1], wx[0], wx[1]);
+            axis_weights(x.y, g.lo[1], g.hi[1], g.size[1], iy[0], iy[1], wy[0], wy[1]);
+            axis_weights(x.z, g.lo[2], g.hi[2], g.size[2], iz[0], iz[1], wz[0], wz[1]);
+            const float part[4] = {m, m * v.x, m * v.y, m * v.z};
+            const int nodes0 = src.first_node(sc);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int cx = k >> 2, cy = (k >> 1) & 1, cz = k & 1;
+                const float wt = wx[cx] * wy[cy] * wz[cz];
+                node[w][lane][k] = nodes0 + (ix[cx] * g.size[1] + iy[cy]) * g.size[2] + iz[cz];
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    val[w][lane][4 * k + c] =
+                        wt != 0.f ? __float2ll_rn(((part[c] * wt) * lo_f[c]) * hi_f[c]) : 0ll;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) node[w][lane][k] = -1;
+        }
+        __syncwarp();
+#pragma unroll 4
+        for (int q = 0; q < 32; ++q) {
+            const int nd = node[w][q][corner];
+            if (nd < 0) continue;                     // no mass: the whole warp skips it
+            if (nd != cur) {
+                if (sum != 0)
+                    atomicAdd(&acc[4 * static_cast<int64_t>(cur) + channel],
+                              static_cast<unsigned long long>(sum));
+                sum = 0;
+                cur = nd;
+            }
+            sum += val[w][q][lane];
+        }
+        __syncwarp();
+    }
+    if (sum != 0)
+        atomicAdd(&acc[4 * static_cast<int64_t>(cur) + channel], static_cast<unsigned long long>(sum));
+}
+
+// Node-major integers to the channel-major field, one node per thread.
+__device__ __forceinline__ void finish_node(const unsigned long long* __restrict__ acc, int64_t at,
+                                            int64_t nodes, int cnt, const uint32_t* __restrict__ bounds,
+                                            float* __restrict__ out) {
+    const ulonglong2* a = reinterpret_cast<const ulonglong2*>(acc + 4 * at);
+    const ulonglong2 p = a[0], q = a[1];
+    const unsigned long long v[4] = {p.x, p.y, q.x, q.y};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        // a NaN or infinite mass or momentum makes its whole channel NaN (the bound is the
+        // largest |value| by its bits, so it is not finite exactly when some value is not)
+        const bool fine = __uint_as_float(bounds[c]) <= FLT_MAX;
+        const double inv = exp2_double(-scale_exponent(cnt, bounds[c]));
+        out[c * nodes] = fine ? static_cast<float>(static_cast<double>(static_cast<long long>(v[c])) * inv)
+                              : __uint_as_float(0x7fc00000u);
+    }
 }
 
 __global__ void __launch_bounds__(kBlock)
-k_deposit_finish(int n, int64_t nodes, const uint32_t* __restrict__ bounds,
+k_deposit_finish(int n, int nodes, const uint32_t* __restrict__ bounds,
                  const unsigned long long* __restrict__ acc, float* __restrict__ out) {
-    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= 4 * nodes) return;
-    const int c = static_cast<int>(t / nodes);
-    // a NaN or infinite mass or momentum makes its whole channel NaN (the bound is the
-    // largest |value| by its bits, so it is not finite exactly when some value is not)
-    if (!(__uint_as_float(bounds[c]) <= FLT_MAX)) {
-        out[t] = __uint_as_float(0x7fc00000u);
-        return;
-    }
-    const double inv = 1.0 / channel_scale(n, bounds[c]);
-    out[t] = static_cast<float>(static_cast<double>(static_cast<long long>(acc[t])) * inv);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < nodes) finish_node(acc, t, nodes, n, bounds, out + t);
 }
 
 // Batched scenes: one field per scene, laid out scene after scene
-// ([scene][4][nodes of that scene]); each grain deposits with its own scene's grid and
-// the channel scale of its scene (bounds and grain count per scene), so a scene's
-// field is bit-identical to the one it gets alone.
+// ([scene][4][nodes of that scene]), each with its own scale.
 __global__ void __launch_bounds__(kBlock)
-k_deposit_bounds_batch(int n, const float4* __restrict__ vel, SceneTab T,
-                       uint32_t* __restrict__ bounds) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const float4 v = vel[s];
-    const float m = v.w;
-    if (m == 0.f) return;
-    uint32_t* b = bounds + 4 * T.scene[s];
-    atomicMax(&b[0], __float_as_uint(fabsf(m)));
-    atomicMax(&b[1], __float_as_uint(fabsf(m * v.x)));
-    atomicMax(&b[2], __float_as_uint(fabsf(m * v.y)));
-    atomicMax(&b[3], __float_as_uint(fabsf(m * v.z)));
-}
-
-__global__ void __launch_bounds__(kBlock)
-k_deposit_batch(int n, const float4* __restrict__ pos, const float4* __restrict__ vel, SceneTab T,
-                const uint32_t* __restrict__ bounds, unsigned long long* __restrict__ acc) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    bool active = s < n;
-    int sc = 0;
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), v = x;
-    if (active) {
-        sc = T.scene[s];
-        x = pos[s];
-        v = vel[s];
-        active = v.w != 0.f;
-    }
-    const DevParams& Q = T.params[sc];
-    const int64_t nodes = static_cast<int64_t>(Q.dgrid[0]) * Q.dgrid[1] * Q.dgrid[2];
-    unsigned long long* a = acc + 4 * static_cast<int64_t>(Q.node_base);
-    double scale[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) scale[c] = channel_scale(Q.n, bounds[4 * sc + c]);
-    int ix[2] = {0, 0}, iy[2] = {0, 0}, iz[2] = {0, 0};
-    float wx[2] = {0.f, 0.f}, wy[2] = {0.f, 0.f}, wz[2] = {0.f, 0.f};
-    const float m = v.w;
-    const float mom[3] = {m * v.x, m * v.y, m * v.z};
-    if (active) {
-        axis_weights(x.x, Q.lo[0], Q.hi[0], Q.dgrid[0], ix[0], ix[1], wx[0], wx[1]);
-        axis_weights(x.y, Q.lo[1], Q.hi[1], Q.dgrid[1], iy[0], iy[1], wy[0], wy[1]);
-        axis_weights(x.z, Q.lo[2], Q.hi[2], Q.dgrid[2], iz[0], iz[1], wz[0], wz[1]);
-    }
-#pragma unroll
-    for (int cx = 0; cx < 2; ++cx)
-#pragma unroll
-        for (int cy = 0; cy < 2; ++cy)
-#pragma unroll
-            for (int cz = 0; cz < 2; ++cz) {
-                const float w = wx[cx] * wy[cy] * wz[cz];
-                const bool live = active && w != 0.f;
-                const long long node =
-                    live ? (static_cast<long long>(ix[cx]) * Q.dgrid[1] + iy[cy]) * Q.dgrid[2] + iz[cz]
-                         : -1ll;
-                // lanes combine only within one scene: key the runs on (scene, node)
-                const long long key = live ? (static_cast<long long>(sc) << 40) | node : -1ll;
-                long long q[4] = {0, 0, 0, 0};
-                if (live) {
-                    q[0] = __double2ll_rn(static_cast<double>(m * w) * scale[0]);
-#pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                        q[k + 1] = __double2ll_rn(static_cast<double>(mom[k] * w) * scale[k + 1]);
-                }
-                // combine adjacent lanes that hit the same node, then one atomic per run
-                const bool tail = run_totals(key, q);
-                if (live && tail) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        if (q[c] != 0)
-                            atomicAdd(&a[c * nodes + node], static_cast<unsigned long long>(q[c]));
-                }
-            }
-}
-
-__global__ void __launch_bounds__(kBlock)
-k_deposit_finish_batch(const DevParams* __restrict__ params, int scenes, int64_t total,
+k_deposit_finish_batch(const DevParams* __restrict__ params, int scenes, int total,
                        const uint32_t* __restrict__ bounds,
                        const unsigned long long* __restrict__ acc, float* __restrict__ out) {
-    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
     int lo = 0, hi = scenes;
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (4 * static_cast<int64_t>(params[mid].node_base) <= t) lo = mid; else hi = mid;
+        if (params[mid].node_base <= t) lo = mid; else hi = mid;
     }
     const DevParams& Q = params[lo];
     const int64_t nodes = static_cast<int64_t>(Q.dgrid[0]) * Q.dgrid[1] * Q.dgrid[2];
-    const int c = static_cast<int>((t - 4 * static_cast<int64_t>(Q.node_base)) / nodes);
-    if (!(__uint_as_float(bounds[4 * lo + c]) <= FLT_MAX)) {   // non-finite input: NaN channel
-        out[t] = __uint_as_float(0x7fc00000u);
-        return;
-    }
-    const double inv = 1.0 / channel_scale(Q.n, bounds[4 * lo + c]);
-    out[t] = static_cast<float>(static_cast<double>(static_cast<long long>(acc[t])) * inv);
+    finish_node(acc, t, nodes, Q.n, bounds + 4 * lo,
+                out + 4 * static_cast<int64_t>(Q.node_base) + (t - Q.node_base));
+}
+
+template <class Src>
+void launch_sums(int n, const Src& src, uint32_t* bounds, unsigned long long* acc, cudaStream_t st) {
+    if (n <= 0) return;
+    k_deposit_bounds<<<std::min(blocks_for(n), kBoundBlocks), kBlock, 0, st>>>(n, src, bounds);
+    constexpr int per = kDepositWarps * kDepositGroup;
+    k_deposit<<<(n - 1) / per + 1, 32 * kDepositWarps, 0, st>>>(n, src, bounds, acc);
 }
 
 }  // namespace
@@ -284,12 +316,8 @@ void launch_deposit(int n, const float4* pos, const float4* vel, const float* lo
     const int64_t nodes = static_cast<int64_t>(dgrid[0]) * dgrid[1] * dgrid[2];
     cudaMemsetAsync(bounds, 0, 4 * sizeof(uint32_t), st);
     cudaMemsetAsync(acc, 0, 4 * nodes * sizeof(unsigned long long), st);
-    if (n > 0) {
-        k_deposit_bounds<<<blocks_for(n), kBlock, 0, st>>>(n, vel, bounds);
-        k_deposit<<<blocks_for(n), kBlock, 0, st>>>(n, pos, vel, g, bounds, acc);
-    }
-    k_deposit_finish<<<static_cast<int>((4 * nodes + kBlock - 1) / kBlock), kBlock, 0, st>>>(
-        n, nodes, bounds, acc, out);
+    launch_sums(n, FromSlots{pos, vel, g}, bounds, acc, st);
+    k_deposit_finish<<<blocks_for(nodes), kBlock, 0, st>>>(n, static_cast<int>(nodes), bounds, acc, out);
 }
 
 void launch_deposit_batch(int n, const float4* pos, const float4* vel, SceneTab T, int scenes,
@@ -297,12 +325,9 @@ void launch_deposit_batch(int n, const float4* pos, const float4* vel, SceneTab 
                           float* out, cudaStream_t st) {
     cudaMemsetAsync(bounds, 0, 4 * sizeof(uint32_t) * static_cast<size_t>(scenes), st);
     cudaMemsetAsync(acc, 0, 4 * total_nodes * sizeof(unsigned long long), st);
-    if (n > 0) {
-        k_deposit_bounds_batch<<<blocks_for(n), kBlock, 0, st>>>(n, vel, T, bounds);
-        k_deposit_batch<<<blocks_for(n), kBlock, 0, st>>>(n, pos, vel, T, bounds, acc);
-    }
-    k_deposit_finish_batch<<<static_cast<int>((4 * total_nodes + kBlock - 1) / kBlock), kBlock, 0,
-                             st>>>(T.params, scenes, 4 * total_nodes, bounds, acc, out);
+    launch_sums(n, FromScenes{pos, vel, T}, bounds, acc, st);
+    k_deposit_finish_batch<<<blocks_for(total_nodes), kBlock, 0, st>>>(
+        T.params, scenes, static_cast<int>(total_nodes), bounds, acc, out);
 }
 
 }  // namespace wd
@@ -324,88 +349,6 @@ constexpr long long kNoAllocNodes = WD_NOALLOC_MAX_NODES;
 // 4 channels of 64-bit accumulators, then 2 words holding the four 32-bit bounds.
 static __device__ __align__(256) unsigned long long g_deposit_scratch[4 * kNoAllocNodes + 2];
 
-
-__global__ void __launch_bounds__(wd::kBlock)
-k_deposit_bounds_aos(int n, const float* __restrict__ state, const float* __restrict__ mass,
-                     uint32_t* __restrict__ bounds) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t b[4] = {0u, 0u, 0u, 0u};
-    if (s < n) {
-        const float m = mass[s];
-        if (m != 0.f) {
-            const float* q = state + 6 * static_cast<int64_t>(s);
-            b[0] = __float_as_uint(fabsf(m));
-            b[1] = __float_as_uint(fabsf(m * q[3]));
-            b[2] = __float_as_uint(fabsf(m * q[4]));
-            b[3] = __float_as_uint(fabsf(m * q[5]));
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        uint32_t x = b[c];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x = max(x, __shfl_xor_sync(0xffffffffu, x, o));
-        if ((threadIdx.x & 31) == 0 && x) atomicMax(&bounds[c], x);
-    }
-}
-
-// Same contributions, scale and per-warp combining as k_deposit; integer sums make
-// the field independent of the order grains arrive in.
-__global__ void __launch_bounds__(wd::kBlock)
-k_deposit_aos(int n, const float* __restrict__ state, const float* __restrict__ mass,
-              wd::DepositGeom g, const uint32_t* __restrict__ bounds,
-              unsigned long long* __restrict__ acc) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t nodes = static_cast<int64_t>(g.size[0]) * g.size[1] * g.size[2];
-    double scale[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) scale[c] = wd::channel_scale(n, bounds[c]);
-    bool active = s < n;
-    float p[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    float m = 0.f;
-    if (active) {
-        const float* q = state + 6 * static_cast<int64_t>(s);
-#pragma unroll
-        for (int a = 0; a < 6; ++a) p[a] = q[a];
-        m = mass[s];
-        active = m != 0.f;
-    }
-    int ix[2] = {0, 0}, iy[2] = {0, 0}, iz[2] = {0, 0};
-    float wx[2] = {0.f, 0.f}, wy[2] = {0.f, 0.f}, wz[2] = {0.f, 0.f};
-    const float mom[3] = {m * p[3], m * p[4], m * p[5]};
-    if (active) {
-        wd::axis_weights(p[0], g.lo[0], g.hi[0], g.size[0], ix[0], ix[1], wx[0], wx[1]);
-        wd::axis_weights(p[1], g.lo[1], g.hi[1], g.size[1], iy[0], iy[1], wy[0], wy[1]);
-        wd::axis_weights(p[2], g.lo[2], g.hi[2], g.size[2], iz[0], iz[1], wz[0], wz[1]);
-    }
-#pragma unroll
-    for (int cx = 0; cx < 2; ++cx)
-#pragma unroll
-        for (int cy = 0; cy < 2; ++cy)
-#pragma unroll
-            for (int cz = 0; cz < 2; ++cz) {
-                const float w = wx[cx] * wy[cy] * wz[cz];
-                const bool live = active && w != 0.f;
-                const long long node =
-                    live ? (static_cast<long long>(ix[cx]) * g.size[1] + iy[cy]) * g.size[2] + iz[cz]
-                         : -1ll;
-                long long q[4] = {0, 0, 0, 0};
-                if (live) {
-                    q[0] = __double2ll_rn(static_cast<double>(m * w) * scale[0]);
-#pragma unroll
-                    for (int a = 0; a < 3; ++a)
-                        q[a + 1] = __double2ll_rn(static_cast<double>(mom[a] * w) * scale[a + 1]);
-                }
-                // combine adjacent lanes that hit the same node, then one atomic per run
-                const bool tail = wd::run_totals(node, q);
-                if (live && tail) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        if (q[c] != 0)
-                            atomicAdd(&acc[c * nodes + node], static_cast<unsigned long long>(q[c]));
-                }
-            }
-}
 
 // Device address of the scratch array in the current device's context. Looked up on
 // every call (a host-side table lookup, no allocation and no device work), so the
@@ -465,13 +408,12 @@ extern "C" int wd_deposit_grid_noalloc(const float* d_state, const float* d_mass
     if (e == cudaSuccess)
         e = cudaMemsetAsync(acc, 0, static_cast<size_t>(4 * nodes) * sizeof(unsigned long long), st);
     if (e == cudaSuccess && n > 0) {
-        const int ni = static_cast<int>(n);
-        k_deposit_bounds_aos<<<wd::blocks_for(ni), wd::kBlock, 0, st>>>(ni, d_state, d_mass, bounds);
-        k_deposit_aos<<<wd::blocks_for(ni), wd::kBlock, 0, st>>>(ni, d_state, d_mass, g, bounds, acc);
+        // the same contributions and scale as the simulation's own deposit
+        wd::launch_sums(static_cast<int>(n), wd::FromAos{d_state, d_mass, g}, bounds, acc, st);
     }
     if (e == cudaSuccess) {
-        wd::k_deposit_finish<<<static_cast<int>((4 * nodes + wd::kBlock - 1) / wd::kBlock), wd::kBlock, 0,
-                               st>>>(static_cast<int>(n), nodes, bounds, acc, d_grid);
+        wd::k_deposit_finish<<<wd::blocks_for(nodes), wd::kBlock, 0, st>>>(
+            static_cast<int>(n), static_cast<int>(nodes), bounds, acc, d_grid);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {

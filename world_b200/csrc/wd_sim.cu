@@ -33,6 +33,8 @@ namespace {
 
 using wd::DevParams;
 
+constexpr int kPinnedExtra = 64;   // 8-byte words for small results (see read_small)
+
 constexpr const char* kVersion = "world_b200 0.1.0 (sm_100a)";
 
 int fail(int code, const std::string& msg) {
@@ -169,7 +171,8 @@ struct wd_sim {
     int64_t auto_off = 0, auto_backoff = 512;// steps to search before lists are tried again
     uint32_t auto_seen[2] = {0, 0};
     bool list_work = false;                  // list steps or builds since the last synchronise
-    unsigned long long* pinned = nullptr;    // host copy of the counters, read after a synchronise
+    // host copies read after a synchronise: the counters, then kPinnedExtra words for results
+    unsigned long long* pinned = nullptr;
 
     // reverse pass: snapshots of the step state (checkpoints of a recorded window and
     // the states of the segment being replayed) and the adjoint buffers
@@ -247,6 +250,12 @@ struct wd_sim {
     };
     StepGraph graphs[8];
     bool built_now = false;   // a host-requested build has run before
+    // the on-demand search (energy, probes) per buffer parity
+    struct SearchGraph {
+        cudaGraphExec_t head = nullptr, mover = nullptr, radix = nullptr;
+        bool seen = false, failed = false;
+    };
+    SearchGraph search_graph[2];
     StepGraph& graph_now() { return graphs[(lists ? 4 : 0) + 2 * lpar + hist_cur]; }
     bool graph_dirty = true;
 
@@ -264,6 +273,12 @@ void clear_adj_graphs(wd_sim* s) {
     s->adj_graphs.clear();
 }
 
+void drop_search_graph(wd_sim::SearchGraph& g) {
+    for (cudaGraphExec_t x : {g.head, g.mover, g.radix})
+        if (x) cudaGraphExecDestroy(x);
+    g = wd_sim::SearchGraph{};
+}
+
 void destroy_graphs(wd_sim* s) {
     // steps still in flight may yet tail-launch the device graphs: let them finish first
     if (s->stream) cudaStreamSynchronize(s->stream);
@@ -274,6 +289,7 @@ void destroy_graphs(wd_sim* s) {
             if (x) cudaGraphExecDestroy(x);
         g = wd_sim::StepGraph{};
     }
+    for (auto& g : s->search_graph) drop_search_graph(g);
     s->graph_dirty = true;
 }
 
@@ -1108,16 +1124,58 @@ cudaError_t alloc_c_buffers(wd_sim* s) {
     return e;
 }
 
-// Search on the current state into the C buffers (energy, probes).
-int ondemand_search(wd_sim* s) {
+void enqueue_gather_c(wd_sim* s, cudaStream_t st) {
     const bool batch = s->scenes > 1;
-    WD_CUDA(alloc_c_buffers(s));
-    const wd::Skip none{nullptr, 0.f};
-    wd::launch_search(s->P, tab(s, s->sceneA), s->posA, s->idsA, s->sb, none, nullptr, 0,
-                      s->counters, s->stream);
     wd::launch_gather(s->P, s->sb, s->posA, s->velA, s->posC, s->velC, s->idsC, nullptr, nullptr,
                       nullptr, nullptr, false, nullptr, nullptr, batch ? s->sceneA : nullptr,
-                      batch ? s->sceneC : nullptr, false, s->counters, s->scene_overflow, s->d_scene_P, none, s->stream);
+                      batch ? s->sceneC : nullptr, false, s->counters, s->scene_overflow,
+                      s->d_scene_P, wd::Skip{nullptr, 0.f}, st);
+}
+
+// Search on the current state into the C buffers (energy, probes). From the second on (per
+// buffer parity) it is one launch of device graphs: the head, which launches the mover or
+// the radix path with the gather; directly it is 8 to 17 launches, the idle path's among
+// them.
+int ondemand_search(wd_sim* s) {
+    WD_CUDA(alloc_c_buffers(s));
+    const wd::Skip none{nullptr, 0.f};
+    if (s->graph_dirty) {
+        destroy_graphs(s);
+        s->graph_dirty = false;
+    }
+    wd_sim::SearchGraph& g = s->search_graph[s->lpar];
+    if (g.seen && !g.head && !g.failed) {
+        cudaError_t e = capture_device_graph(s, &g.mover, [&](cudaStream_t st) {
+            wd::launch_search_merge(s->P, s->idsA, s->sb, none, st);
+            enqueue_gather_c(s, st);
+        });
+        if (e == cudaSuccess)
+            e = capture_device_graph(s, &g.radix, [&](cudaStream_t st) {
+                wd::launch_search_radix(s->P, s->idsA, s->sb, none, st);
+                enqueue_gather_c(s, st);
+            });
+        if (e == cudaSuccess)
+            e = capture_device_graph(s, &g.head, [&](cudaStream_t st) {
+                wd::launch_search_head(s->P, tab(s, s->sceneA), s->posA, s->idsA, s->sb, none, nullptr,
+                                       0, false, 0, s->counters, st);
+                wd::launch_graph_pick(s->sb.ctrl + 1, g.mover, g.radix, s->counters, st);
+            });
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux_stream);
+        if (e != cudaSuccess) {
+            drop_search_graph(g);
+            g.failed = true;
+            cudaGetLastError();
+        }
+    }
+    g.seen = true;
+    if (g.head) {
+        s->list_work = true;   // a launch that fails on the device is looked for at the next wait
+        WD_CUDA(cudaGraphLaunch(g.head, s->stream));
+        return WD_OK;
+    }
+    wd::launch_search(s->P, tab(s, s->sceneA), s->posA, s->idsA, s->sb, none, nullptr, 0,
+                      s->counters, s->stream);
+    enqueue_gather_c(s, s->stream);
     WD_CUDA(cudaGetLastError());
     return WD_OK;
 }
@@ -1125,7 +1183,7 @@ int ondemand_search(wd_sim* s) {
 int sync_stream(wd_sim* s) {
     // list builds that did not launch, and stages of the bulk-staged contact kernel that
     // never arrived, are counted on the device: the counters come along with the wait
-    const bool lists = s->list_work && s->pinned != nullptr;
+    const bool lists = s->list_work;
     s->list_work = false;
     if (lists)
         WD_CUDA(cudaMemcpyAsync(s->pinned, s->counters, sizeof(unsigned long long) * wd::kNumCounters,
@@ -1133,11 +1191,11 @@ int sync_stream(wd_sim* s) {
     WD_CUDA(cudaStreamSynchronize(s->stream));
     WD_CUDA(cudaGetLastError());
     if (!lists) return WD_OK;
-    if (!s->picard && s->pinned[wd::kCntLaunchFail]) {
+    if (s->pinned[wd::kCntLaunchFail]) {
         // a list build whose device-side graph launch failed did not run
         WD_CUDA(cudaMemset(s->counters + wd::kCntLaunchFail, 0, sizeof(unsigned long long)));
         WD_CUDA(request_list_build(s));
-        return fail(WD_ERR_CUDA, "list build: a device-side graph launch failed; the "
+        return fail(WD_ERR_CUDA, "list build or search: a device-side graph launch failed; the "
                                  "steps since the last synchronisation are invalid");
     }
     if (s->pinned[wd::kCntStageTimeout]) {
@@ -1150,6 +1208,16 @@ int sync_stream(wd_sim* s) {
                                  "complete within its wait limit; the state is invalid");
     }
     return WD_OK;
+}
+
+// Bytes of the device to the host, and the wait for them: small results by way of pinned
+// memory, which a copy reaches without staging.
+int read_small(wd_sim* s, void* dst, const void* src, size_t bytes) {
+    void* via = bytes <= sizeof(unsigned long long) * kPinnedExtra ? s->pinned + wd::kNumCounters : dst;
+    WD_CUDA(cudaMemcpyAsync(via, src, bytes, cudaMemcpyDeviceToHost, s->stream));
+    const int rc = sync_stream(s);
+    if (rc == WD_OK && via != dst) std::memcpy(dst, via, bytes);
+    return rc;
 }
 
 // Skin of the library's own lists for a handle whose configuration has none, or 0 where
@@ -1179,8 +1247,6 @@ cudaError_t alloc_list_buffers(wd_sim* s) {
     if (e == cudaSuccess && !s->list_ctrl) e = dalloc(&s->list_ctrl, wd::kLcWords);
     if (e == cudaSuccess && !s->list_len) e = dalloc(&s->list_len, 1);
     if (e == cudaSuccess && !s->tail_count) e = dalloc(&s->tail_count, 1);
-    if (e == cudaSuccess && !s->pinned)
-        e = cudaMallocHost(reinterpret_cast<void**>(&s->pinned), sizeof(unsigned long long) * wd::kNumCounters);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->list_ctrl, 0, sizeof(uint32_t) * wd::kLcWords, s->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->tail_count, 0, sizeof(unsigned), s->stream);
     if (e == cudaSuccess) e = dalloc(&s->nbr, static_cast<size_t>(n) * wd::kNbrCap);
@@ -1322,6 +1388,8 @@ int alloc_sim(wd_sim* s) {
     WD_CUDA(dalloc(&sb.table, s->num_cells));
     WD_CUDA(cudaMemset(sb.table, 0xFF, sizeof(int2) * s->num_cells));
     WD_CUDA(dalloc(&s->counters, wd::kNumCounters));
+    WD_CUDA(cudaMallocHost(reinterpret_cast<void**>(&s->pinned),
+                           sizeof(unsigned long long) * (wd::kNumCounters + kPinnedExtra)));
     WD_CUDA(cudaMemset(s->counters, 0, sizeof(unsigned long long) * wd::kNumCounters));
     WD_CUDA(dalloc(&s->picard_res, s->picard_iters > 0 ? s->picard_iters : 1));
     WD_CUDA(cudaMemset(s->picard_res, 0, sizeof(uint32_t) * (s->picard_iters > 0 ? s->picard_iters : 1)));
@@ -2100,11 +2168,9 @@ int wd_compute_scene_energies(wd_sim* sim, double* energies) {
     if (rc) return rc;
     wd::launch_energy(sim->P, tab(sim, sim->sceneC), sim->posC, sim->velC, sim->idsC,
                       sim->sb.table, sim->hist[sim->hist_cur], sim->hcnt_slot, sim->sb.src,
-                      segments(sim), sim->grain_vals, sim->partials, sim->scene_sums, sim->stream);
+                      segments(sim), sim->scenes > 1 ? sim->grain_vals : nullptr, sim->partials, sim->scene_sums, sim->stream);
     WD_CUDA(cudaGetLastError());
-    WD_CUDA(cudaMemcpyAsync(energies, sim->scene_sums, sizeof(double) * sim->scenes,
-                            cudaMemcpyDeviceToHost, sim->stream));
-    return sync_stream(sim);
+    return read_small(sim, energies, sim->scene_sums, sizeof(double) * sim->scenes);
 }
 
 int wd_grain_energies(wd_sim* sim, double* energies) {
@@ -2144,9 +2210,7 @@ int wd_compute_scene_momenta(wd_sim* sim, double* momenta) {
     wd::launch_momentum(sim->n, sim->velA, sim->idsA, segments(sim), sim->grain_vals, sim->partials,
                         sim->scene_sums, sim->stream);
     WD_CUDA(cudaGetLastError());
-    WD_CUDA(cudaMemcpyAsync(momenta, sim->scene_sums, 3 * sizeof(double) * sim->scenes,
-                            cudaMemcpyDeviceToHost, sim->stream));
-    return sync_stream(sim);
+    return read_small(sim, momenta, sim->scene_sums, 3 * sizeof(double) * sim->scenes);
 }
 
 int wd_compute_momentum(wd_sim* sim, double* momentum3) {
@@ -2169,9 +2233,7 @@ int wd_is_stable(wd_sim* sim, int32_t* stable) {
                          sim->stream);
     WD_CUDA(cudaGetLastError());
     unsigned long long flag = 0;
-    WD_CUDA(cudaMemcpyAsync(&flag, sim->counters + wd::kCntUnstable, sizeof(flag),
-                            cudaMemcpyDeviceToHost, sim->stream));
-    int rc = sync_stream(sim);
+    const int rc = read_small(sim, &flag, sim->counters + wd::kCntUnstable, sizeof(flag));
     if (rc) return rc;
     *stable = flag ? 0 : 1;
     return WD_OK;
@@ -2183,9 +2245,7 @@ int wd_compute_max_acceleration(wd_sim* sim, float* max_accel) {
     wd::launch_max_accel(sim->n, sim->acc, sim->counters, sim->stream);
     WD_CUDA(cudaGetLastError());
     unsigned long long bits = 0;
-    WD_CUDA(cudaMemcpyAsync(&bits, sim->counters + wd::kCntMaxAccel, sizeof(bits),
-                            cudaMemcpyDeviceToHost, sim->stream));
-    int rc = sync_stream(sim);
+    const int rc = read_small(sim, &bits, sim->counters + wd::kCntMaxAccel, sizeof(bits));
     if (rc) return rc;
     const uint32_t b = static_cast<uint32_t>(bits);
     std::memcpy(max_accel, &b, sizeof(float));
@@ -2194,8 +2254,7 @@ int wd_compute_max_acceleration(wd_sim* sim, float* max_accel) {
 
 static int read_counter(wd_sim* sim, int which, int64_t* out) {
     unsigned long long v = 0;
-    WD_CUDA(cudaMemcpyAsync(&v, sim->counters + which, sizeof(v), cudaMemcpyDeviceToHost, sim->stream));
-    int rc = sync_stream(sim);
+    const int rc = read_small(sim, &v, sim->counters + which, sizeof(v));
     if (rc) return rc;
     *out = static_cast<int64_t>(v);
     return WD_OK;
