@@ -422,10 +422,13 @@ def _roomy(n, seed, mu, history, picard=False):
 
 @pytest.mark.parametrize("n,history,picard", [(31, True, False), (33, False, False), (16383, True, False),
                                               (16385, True, False), (20011, False, False),
-                                              (17001, True, True), (2049, True, True)])
+                                              (17001, True, True), (2049, True, True),
+                                              (6143, True, False), (6145, False, False),
+                                              (24575, False, False), (24577, True, False)])
 def test_contact_parallel_kernel_equals_search(n, history, picard):
     """The contact-parallel kernel on both sides of its lanes-per-grain rule (four lanes
-    below 16,384 grains, one from there), with more contacts in a warp than one round
+    below 16,384 grains, one from there) and of the list build's (32 below 6,144, 8 below
+    24,576), whose reach here takes in outer cells at some faces, with more contacts in a warp than one round
     holds and with grains whose contacts a cell crossing re-ordered, against the searched
     step bit for bit (both are sums in the canonical order, so no tolerance)."""
     cfg, st, rad = _roomy(n, 50, 0.5, history, picard)

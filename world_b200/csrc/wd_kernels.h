@@ -19,11 +19,13 @@ inline int blocks_for(int64_t n, int block = kBlock) {
     return static_cast<int>((n + block - 1) / block);
 }
 
-// Incremental search: at most this many grains may change cell between searches
-// for the mover path (a bitonic sort on one 8-CTA cluster, kMoverThreads per CTA);
-// more falls back to the radix sort.
-constexpr int kMoverCap = 8192;
+// Incremental search: at most mover_cap(n) grains may change cell between searches for the
+// mover path (their keys fit one block's shared memory); more falls back to the radix sort.
+// Ordering m movers takes about m^2 time (16,384: 27 us, 28,672: 70), the radix sort of n
+// grains about 45 us below 2^17 and 135 at 2^20, which is why the cap grows with n.
+constexpr int kMoverCap = 28672;
 constexpr int kMoverThreads = 1024;
+int mover_cap(int n);
 
 // Buffers of one neighbor search (sorted by (cell key, grain id)).
 struct SearchBuffers {
@@ -37,9 +39,12 @@ struct SearchBuffers {
     uint32_t* moved;         // n/32 words: bit set when a slot's key changed
     int* blk_cnt;            // movers per 256-slot block
     int* blk_off;            // exclusive prefix of blk_cnt
-    int* ctrl;               // [0] mover count, [1] 1 = radix path this search
-    unsigned long long* mv_key;  // kMoverCap: (key << 32 | id) of each mover
-    uint32_t* mv_slot;       // kMoverCap: its state slot
+    int* ctrl;               // [0] mover count, [1] 1 = radix path this search, [2] movers so far
+    int mover_cap;
+    unsigned long long* mv_raw;  // mover_cap: (key << 32 | id) of each mover, in any order
+    uint32_t* mv_raw_slot;   // mover_cap: its state slot
+    unsigned long long* mv_key;  // mover_cap: the same in order
+    uint32_t* mv_slot;
     int* src;                // n: state slot of each sorted position
     uint32_t* tile_counts;   // kRadix * num_tiles
     uint32_t* digit_totals;  // kRadix * max_passes
@@ -60,8 +65,8 @@ struct Skip {
 // A search orders the state slots by (cell key, grain id) into keys[out] (sorted
 // keys), vals[out] (grain ids) and src (source slot of each position). It has three
 // parts, split so a CUDA graph can put the radix path under a conditional node:
-//   head  -- keys of every slot, mover bits, and the cluster mover kernel, which
-//            picks the path (ctrl[1]) and sets `cond` when use_cond;
+//   head  -- keys of every slot, mover bits, and the mover kernel, which orders the movers
+//            and picks the path (ctrl[1]) and sets `cond` when use_cond;
 //   radix -- stable LSD radix sort of all keys (runs when ctrl[1]);
 //   merge -- merges the sorted movers into the still-sorted rest (idle when ctrl[1]).
 void launch_search_head(const DevParams& P, SceneTab T, const float4* pos, const int* ids,

@@ -24,6 +24,7 @@
 // within 0.49 skin of the build; if one is not, the step is redone from its start
 // state with the per-iteration search, so the results stay those of the searched step.
 #include <algorithm>
+#include <type_traits>
 
 #include "wd_kernels.h"
 
@@ -231,68 +232,193 @@ __device__ __forceinline__ void list_far_shell(const DevParams& P, const int2* _
     }
 }
 
+// Which of the outer cells (two away along one axis) a grain's list has to look into, as
+// list_far_shell decides it per cell: bits 0-1 x lower / upper, 2-3 y, 4-5 z. Bit 6: the
+// reach covers cells two away along two axes, which only list_far_shell walks.
+__device__ __forceinline__ unsigned list_outer_faces(const DevParams& P, float4 pi, int cx, int cy,
+                                                     int cz) {
+    const float reach = (pi.w + P.rmax) + P.skin;
+    if (!(reach > P.cell_min)) return 0u;
+    const float r2 = (reach * reach) * 1.0001f;
+    const float w = P.cell_min * (1.f - 3.f * fmaxf(P.cell_err[0], fmaxf(P.cell_err[1], P.cell_err[2])) - 1e-4f);
+    if (r2 > 2.f * w * w) return 1u << 6;
+    const float p3[3] = {pi.x, pi.y, pi.z};
+    const int c3[3] = {cx, cy, cz};
+    unsigned faces = 0u;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float f = ((p3[a] - P.lo[a]) * P.inv_len[a]) * static_cast<float>(P.grid[a]) -
+                        static_cast<float>(c3[a]);
+        const float m = 2.f * P.cell_err[a] + 1e-4f;
+        const float lower = fmaxf(0.f, 1.f + f - m) * P.cell_len[a];
+        const float upper = fmaxf(0.f, 2.f - f - m) * P.cell_len[a];
+        if (!(lower * lower > r2)) faces |= 1u << (2 * a);
+        if (!(upper * upper > r2)) faces |= 2u << (2 * a);
+    }
+    return faces;
+}
+
+// Slots of the cells (nx, ny, z0 .. z1), at most five: consecutive, or [0, 0) if empty.
+__device__ __forceinline__ int2 table_row(const DevParams& P, const int2* __restrict__ table, int nx,
+                                          int ny, int z0, int z1) {
+    const bool col = nx >= 0 && nx < P.grid[0] && ny >= 0 && ny < P.grid[1];
+    const int2* t = table + P.cell_base +
+                    (static_cast<uint32_t>(nx) * static_cast<uint32_t>(P.grid[1]) + static_cast<uint32_t>(ny)) *
+                        static_cast<uint32_t>(P.grid[2]);
+    int2 e[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const int z = z0 + k;
+        e[k] = col && z <= z1 && z >= 0 && z < P.grid[2] ? __ldg(&t[z]) : make_int2(-1, -1);
+    }
+    int lo = 0x7fffffff, hi = 0;
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+        if (e[k].x >= 0) {
+            lo = min(lo, e[k].x);
+            hi = max(hi, e[k].y);
+        }
+    return lo < hi ? make_int2(lo, hi) : make_int2(0, 0);
+}
+
 // The list of every grain, from the run table of the build's sorted state: the
-// contact kernel's stencil walk with the skin added to the contact distance. The sorted
-// state is copied back into the step's buffers on the way.
-template <bool BATCH>
+// contact kernel's stencil walk with the skin added to the contact distance, widened by the
+// outer cells in reach. The sorted state is copied back into the step's buffers on the way.
+//
+// The cells to look into form rows along z: the nine of the stencil, longer by a cell where
+// a z face is in reach, and three beyond each x or y face in reach; a lane walks its own
+// outer rows, whichever faces they lie at (cell by cell, each of the 54 outer cells cost the
+// warp its test, table load and loop). With LPG lanes to a grain the rows' slot ranges go
+// to shared memory and the lanes walk the candidates as one sequence, LPG apart and four
+// each at a time; for one lane that costs more than row by row (175 us: 4,700 warp
+// instructions per 32 grains). Bound by issue. 1,000,003 packed grains 126 us (before 175),
+// 2^20 falling 82 (110), 100,003 packed 23 (31), 5,003 packed 10 (23).
+constexpr int kListRows = 21;
+
+template <bool BATCH, int LPG>
 __global__ void __launch_bounds__(kBlock)
 k_list_build(DevParams P0, SceneTab T, const float4* __restrict__ pos,
              const int2* __restrict__ table, int* __restrict__ nbr, int* __restrict__ nbr_cnt,
              float4* __restrict__ xbuild, uint32_t* __restrict__ ctrl, ListCopy cp, Skip skip) {
     if (skipped(skip)) return;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int kPer = kBlock / LPG;
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ int2 rows[LPG > 1 ? kListRows : 1][LPG > 1 ? kPer : 1];
+    const int g = static_cast<int>(threadIdx.x) / LPG, sub = static_cast<int>(threadIdx.x) % LPG;
+    const int s = blockIdx.x * kPer + g;
     const int n = P0.n;
-    if (s >= n) return;
-    const DevParams& P = scene_params<BATCH>(P0, T, s);
-    const float4 pi = pos[s];
-    cp.pos_out[s] = pi;
-    cp.vel_out[s] = cp.vel[s];
-    cp.ids_out[s] = cp.ids[s];
-    if (cp.hcnt) cp.hcnt_out[s] = cp.hcnt[s];
-    if (BATCH) cp.scene_out[s] = cp.scene[s];
-    int cx, cy, cz;
-    cell_coords(P, pi.x, pi.y, pi.z, cx, cy, cz);
-    // the nine rows' slot ranges first (27 independent table loads), then the
-    // candidates two at a time, in the stencil order
-    int lo[9], hi[9];
+    const bool live = s < n;
+    if (LPG == 1 && !live) return;
+    const DevParams& P = BATCH ? T.params[live ? T.scene[s] : 0] : P0;
+    float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
+    int cx = 0, cy = 0, cz = 0;
+    if (live) {
+        pi = pos[s];
+        if (sub == 0) {
+            cp.pos_out[s] = pi;
+            cp.vel_out[s] = cp.vel[s];
+            cp.ids_out[s] = cp.ids[s];
+            if (cp.hcnt) cp.hcnt_out[s] = cp.hcnt[s];
+            if (BATCH) cp.scene_out[s] = cp.scene[s];
+        }
+        cell_coords(P, pi.x, pi.y, pi.z, cx, cy, cz);
+    }
+    const unsigned faces = live ? list_outer_faces(P, pi, cx, cy, cz) : 0u;
+    const int z0 = cz - 1 - ((faces >> 4) & 1), z1 = cz + 1 + ((faces >> 5) & 1);
+    int cnt = 0;
+    auto reach = [&](int j, float4 pj) {
+        float3 d;
+        const float ns = pair_norm_sq(pi, pj, d);
+        const float far = (pi.w + pj.w) + P.skin;
+        return j != s && ns < far * far;
+    };
+    if (LPG == 1) {
+        auto visit = [&](int j, float4 pj) {
+            if (!reach(j, pj)) return;
+            if (cnt < kNbrCap) nbr[static_cast<int64_t>(cnt) * n + s] = j;
+            ++cnt;
+        };
+        auto walk = [&](int2 q) {
+            int j = q.x;
+            for (; q.y - j > 1; j += 2) {
+                const float4 p0 = __ldg(&pos[j]), p1 = __ldg(&pos[j + 1]);
+                visit(j, p0);
+                visit(j + 1, p1);
+            }
+            if (j < q.y) visit(j, __ldg(&pos[j]));
+        };
+        // the nine stencil rows, a column of x at a time, then each lane's own outer rows
+        for (int dx = -1; dx <= 1; ++dx) {
+            int2 q[3];
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        const int nx = cx + r - 1;
-        if (nx >= 0 && nx < P.grid[0]) {
-            row_ranges(P, table, nx, cy, cz, lo + 3 * r, hi + 3 * r);
-        } else {
+            for (int t = 0; t < 3; ++t) q[t] = table_row(P, table, cx + dx, cy + t - 1, z0, z1);
 #pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                lo[3 * r + t] = 0;
-                hi[3 * r + t] = 0;
+            for (int t = 0; t < 3; ++t) walk(q[t]);
+        }
+        for (unsigned more = faces & 15u; more; more &= more - 1u) {
+            const int face = __ffs(static_cast<int>(more)) - 1;
+            const int out = face & 1 ? 2 : -2;
+            int2 q[3];
+#pragma unroll
+            for (int t = 0; t < 3; ++t)
+                q[t] = table_row(P, table, cx + (face < 2 ? out : t - 1), cy + (face < 2 ? t - 1 : out),
+                                 cz - 1, cz + 1);
+#pragma unroll
+            for (int t = 0; t < 3; ++t) walk(q[t]);
+        }
+    } else {
+        for (int q = sub; q < kListRows; q += LPG) {
+            // 3 rows at dx = -2, 5 at each of -1, 0, 1, and 3 at 2
+            const int dx = q < 3 ? -2 : q < 18 ? (q - 3) / 5 - 1 : 2;
+            const int dy = q < 3 ? q - 1 : q < 18 ? (q - 3) % 5 - 2 : q - 19;
+            const bool wanted = live && (dx != -2 || (faces & 1u)) && (dx != 2 || (faces & 2u)) &&
+                                (dy != -2 || (faces & 4u)) && (dy != 2 || (faces & 8u));
+            const bool face = dx == -2 || dx == 2 || dy == -2 || dy == 2;
+            rows[q][g] = wanted ? table_row(P, table, cx + dx, cy + dy, face ? cz - 1 : z0, face ? cz + 1 : z1)
+                                : make_int2(0, 0);
+        }
+        __syncwarp();
+        int r = -1, j = sub, hi = 0;
+        for (;;) {
+            int jj[4];
+            float4 pp[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                while (j >= hi && r < kListRows) {
+                    const int over = j - hi;      // how far into the next row
+                    if (++r < kListRows) {
+                        const int2 q = rows[r][g];
+                        j = q.x + over;
+                        hi = q.y;
+                    }
+                }
+                jj[u] = r < kListRows ? j : -1;
+                j += LPG;
+            }
+            if (!__any_sync(kAll, jj[0] >= 0)) break;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) pp[u] = jj[u] >= 0 ? __ldg(&pos[jj[u]]) : pi;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const bool hit = jj[u] >= 0 && reach(jj[u], pp[u]);
+                // the group's lanes hold consecutive candidates
+                const unsigned shift = (threadIdx.x & 31u) - static_cast<unsigned>(sub);
+                const unsigned mine = (__ballot_sync(kAll, hit) >> shift) & (kAll >> (32 - LPG));
+                const int at = cnt + __popc(mine & ((1u << sub) - 1u));
+                cnt += __popc(mine);
+                if (hit && at < kNbrCap) nbr[static_cast<int64_t>(at) * n + s] = jj[u];
             }
         }
     }
-    int cnt = 0;
-    auto visit = [&](int j, float4 pj) {
-        if (j == s) return;
-        float3 d;
-        const float ns = pair_norm_sq(pi, pj, d);
-        const float reach = (pi.w + pj.w) + P.skin;
-        if (ns < reach * reach) {
-            if (cnt < kNbrCap) nbr[static_cast<int64_t>(cnt) * n + s] = j;
+    if (!live || sub != 0) return;
+    if (faces & (1u << 6)) {
+        auto visit = [&](int q, float4 pq) {
+            if (!reach(q, pq)) return;
+            if (cnt < kNbrCap) nbr[static_cast<int64_t>(cnt) * n + s] = q;
             ++cnt;
-        }
-    };
-#pragma unroll
-    for (int r = 0; r < 9; ++r) {
-        int j = lo[r];
-        const int e = hi[r];
-        // an empty row has lo = INT_MAX, hi = 0: the difference does not overflow
-        for (; e - j > 1; j += 2) {
-            const float4 a = __ldg(&pos[j]);
-            const float4 b = __ldg(&pos[j + 1]);
-            visit(j, a);
-            visit(j + 1, b);
-        }
-        if (j < e) visit(j, __ldg(&pos[j]));
+        };
+        list_far_shell(P, table, pos, pi, cx, cy, cz, visit);
     }
-    if ((pi.w + P.rmax) + P.skin > P.cell_min) list_far_shell(P, table, pos, pi, cx, cy, cz, visit);
     nbr_cnt[s] = cnt;
     xbuild[s] = pi;
     if (cnt > kNbrCap) atomicOr(&ctrl[kLcOverflow], 1u);
@@ -1386,12 +1512,23 @@ void launch_list_build(const DevParams& P, SceneTab T, const float4* pos, const 
                                                                list_ctrl, cp, skip, counters);
         return;
     }
-    if (T.params)
-        k_list_build<true><<<blocks_for(P.n), kBlock, 0, st>>>(P, T, pos, table, nbr, nbr_cnt,
-                                                                xbuild, list_ctrl, cp, skip);
-    else
-        k_list_build<false><<<blocks_for(P.n), kBlock, 0, st>>>(P, T, pos, table, nbr, nbr_cnt,
-                                                                 xbuild, list_ctrl, cp, skip);
+    auto go = [&](auto lanes) {
+        constexpr int L = decltype(lanes)::value;
+        const int nb = blocks_for(P.n, kBlock / L);
+        if (T.params)
+            k_list_build<true, L><<<nb, kBlock, 0, st>>>(P, T, pos, table, nbr, nbr_cnt, xbuild,
+                                                         list_ctrl, cp, skip);
+        else
+            k_list_build<false, L><<<nb, kBlock, 0, st>>>(P, T, pos, table, nbr, nbr_cnt, xbuild,
+                                                          list_ctrl, cp, skip);
+    };
+    // Lanes per grain: as many as the chip has room for while a build is one warp's latency.
+    // Upload, build and one step with 32 / 8 / 1 lanes: 1,000 grains 84 / 87 / 92 us, 5,000
+    // 93.2 / 95.0 / 96.8, 8,000 96.2 / 95.9 / 98.9, 20,000 107.8 / 96.6 / 100.2, 30,000
+    // 121 / 107.6 / 107.5, 50,000 142 / 111 / 106.
+    if (P.n < 6144) go(std::integral_constant<int, 32>());
+    else if (P.n < 24576) go(std::integral_constant<int, 8>());
+    else go(std::integral_constant<int, 1>());
 }
 
 void launch_list_copy(int n, const float4* pos, const float4* vel, const int* ids,

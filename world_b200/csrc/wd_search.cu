@@ -7,18 +7,16 @@
 //   * the key of every grain is the reference's cell mapping; grains are ordered by
 //     (key, grain id): deterministic, no per-cell capacity, nothing dropped;
 //   * between steps few grains change cell, so the search re-sorts only those
-//     ("movers": a bitonic sort on one 8-CTA cluster over distributed shared memory)
-//     and merges them into the still-sorted rest
-//     by binary search; the first search, or one with more than kMoverCap movers,
-//     runs a stable LSD radix sort of all keys instead. The choice is made on the
+//     ("movers", ordered by counting the smaller ones) and merges them into the
+//     still-sorted rest by binary search; the first search, or one with more than
+//     mover_cap(n) movers, runs a stable LSD radix sort of all keys instead. The choice is made on the
 //     device, so both paths sit in the same CUDA graph and the idle one returns at
 //     once. Both produce the same order;
 //   * the run table is a dense [start, end) per cell, but only the cells of the
 //     previous search are cleared (O(n), not the reference's O(cells) memset);
 //   * no candidate list is materialised: the contact kernel walks the sorted runs.
+#include <algorithm>
 #include <cstdio>
-
-#include <cooperative_groups.h>
 
 #include "wd_kernels.h"
 
@@ -48,17 +46,21 @@ __device__ __forceinline__ int movers_before(const uint32_t* __restrict__ bits,
     return c;
 }
 
-// Search pass 1: key of every state slot, mover bits and per-block mover counts;
+// Search pass 1: key of every state slot, mover bits and per-block mover counts, the
+// movers themselves (in any order: they are ranked next) as far as `cap` holds them;
 // clear the runs of the previous search; zero the radix digit totals.
 template <bool BATCH>
 __global__ void __launch_bounds__(kBlock)
-k_keys(DevParams P, SceneTab T, const float4* __restrict__ pos, uint32_t* __restrict__ newkey,
-       uint32_t* __restrict__ moved, int* __restrict__ blk_cnt, int num_blocks,
+k_keys(DevParams P, SceneTab T, const float4* __restrict__ pos, const int* __restrict__ ids,
+       unsigned long long* __restrict__ mv_raw, uint32_t* __restrict__ mv_raw_slot,
+       int* __restrict__ ctrl, int cap, uint32_t* __restrict__ newkey, uint32_t* __restrict__ moved, int* __restrict__ blk_cnt, int num_blocks,
        const uint32_t* __restrict__ slot_keys, const uint32_t* __restrict__ table_keys,
        int2* __restrict__ table, uint32_t* __restrict__ digit_totals, int totals_count,
        uint32_t* __restrict__ zero_res, int zero_res_count, Skip skip) {
     if (skipped(skip)) return;
     __shared__ int warp_movers[kBlock / 32];
+    __shared__ int block_first;
+    uint32_t key = 0u;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < totals_count) digit_totals[s] = 0u;
     if (zero_res != nullptr && s < zero_res_count) zero_res[s] = 0u;
@@ -68,7 +70,7 @@ k_keys(DevParams P, SceneTab T, const float4* __restrict__ pos, uint32_t* __rest
         const float4 p = pos[s];
         int cx, cy, cz;
         cell_coords(Q, p.x, p.y, p.z, cx, cy, cz);
-        const uint32_t key = Q.cell_base + flat_cell(Q, cx, cy, cz);
+        key = Q.cell_base + flat_cell(Q, cx, cy, cz);
         newkey[s] = key;
         mv = key != slot_keys[s];
         const uint32_t kp = table_keys[s];
@@ -86,6 +88,16 @@ k_keys(DevParams P, SceneTab T, const float4* __restrict__ pos, uint32_t* __rest
 #pragma unroll
         for (int w = 0; w < kBlock / 32; ++w) c += warp_movers[w];
         blk_cnt[blockIdx.x] = c;
+        block_first = c > 0 ? atomicAdd(&ctrl[2], c) : 0;
+    }
+    __syncthreads();
+    if (mv) {
+        int at = block_first + __popc(ballot & lanemask_lt());
+        for (int w = 0; w < warp; ++w) at += warp_movers[w];
+        if (at < cap) {
+            mv_raw[at] = (static_cast<unsigned long long>(key) << 32) | static_cast<uint32_t>(ids[s]);
+            mv_raw_slot[at] = static_cast<uint32_t>(s);
+        }
     }
 }
 
@@ -248,150 +260,86 @@ k_sort_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict_
     }
 }
 
-// Search pass 2, one thread-block cluster of kMoverCtas CTAs (one CTA per SM, the
-// cluster's shared memories together holding kMoverCap movers, one per thread): mover
-// offsets per 256-slot block, the mover count and the path. When the movers fit
-// kMoverCap they are compacted from the bit mask (only blocks that have movers are
-// read) into the distributed shared memory and sorted by (key << 32 | id) with a
-// bitonic network whose stages across CTAs use remote shared-memory accesses (DSMEM)
-// and a cluster barrier, the others a CTA barrier; otherwise ctrl[1] selects the radix
-// sort, and when the search runs inside a CUDA graph the radix path's conditional node
-// is switched on. (A single CTA did the same network on one SM, issue-bound at about
-// 100 us for 8192 movers.)
-constexpr int kMoverCtas = 8;
-constexpr int kMoverPer = kMoverCap / kMoverCtas;  // elements per CTA: one per thread
-static_assert(kMoverPer == kMoverThreads, "one mover element per thread");
+// Search pass 2. Block 0: mover offsets per 256-slot block, the mover count and the path
+// (more than `cap` movers: ctrl[1] selects the radix sort, and when the search runs inside a
+// CUDA graph the radix path's conditional node is switched on). The other blocks order the
+// movers: each copies all their (key << 32 | id) into shared memory, and its warps count,
+// for R movers at a time, the smaller ones among them; a mover goes to the place of its
+// count. That is m^2 comparisons, but over the whole chip and without a barrier: at 5,003
+// packed grains 5 to 10 us, where a bitonic network on one 8-CTA cluster took 28 to 50; at
+// 1,000,003, whose 20,000 and more movers went to the radix sort (135), 50 to 69.
+template <int R>
+__device__ __forceinline__ void rank_movers(const unsigned long long* keys, int m, int first, int stride,
+                                            const uint32_t* __restrict__ raw_slot,
+                                            unsigned long long* __restrict__ mv_key,
+                                            uint32_t* __restrict__ mv_slot) {
+    const int lane = threadIdx.x & 31;
+    for (int i = first * R; i < m; i += stride * R) {
+        unsigned long long mine[R];
+        unsigned below[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            mine[r] = i + r < m ? keys[i + r] : 0ull;
+            below[r] = 0u;
+        }
+#pragma unroll 4
+        for (int j = lane; j < m; j += 32) {
+            const unsigned long long k = keys[j];
+#pragma unroll
+            for (int r = 0; r < R; ++r) below[r] += k < mine[r] ? 1u : 0u;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const unsigned place = __reduce_add_sync(0xffffffffu, below[r]);
+            if (lane == r && i + r < m) {
+                mv_key[place] = mine[r];
+                mv_slot[place] = raw_slot[i + r];
+            }
+        }
+    }
+}
 
-__global__ void __cluster_dims__(kMoverCtas, 1, 1) __launch_bounds__(kMoverThreads)
+__global__ void __launch_bounds__(kMoverThreads)
 k_movers(int n, const int* __restrict__ blk_cnt, int* __restrict__ blk_off, int num_blocks,
-         const uint32_t* __restrict__ moved, const uint32_t* __restrict__ newkey,
-         const int* __restrict__ ids, unsigned long long* __restrict__ mv_key,
-         uint32_t* __restrict__ mv_slot, int* __restrict__ ctrl, int use_cond,
-         cudaGraphConditionalHandle cond, unsigned long long* __restrict__ counters, Skip skip) {
-    namespace cg = cooperative_groups;
-    if (skipped(skip)) return;  // the same flag for every CTA of the cluster
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank = static_cast<int>(cluster.block_rank());
-    __shared__ unsigned long long k[kMoverPer];
-    __shared__ uint32_t v[kMoverPer];
-    __shared__ uint32_t cta_total;
-    __shared__ uint32_t s_off, s_m;
+         const unsigned long long* __restrict__ raw, const uint32_t* __restrict__ raw_slot,
+         unsigned long long* __restrict__ mv_key, uint32_t* __restrict__ mv_slot,
+         int* __restrict__ ctrl, int cap, int use_cond, cudaGraphConditionalHandle cond,
+         unsigned long long* __restrict__ counters, Skip skip) {
+    if (skipped(skip)) return;
+    extern __shared__ unsigned long long keys[];   // cap
+    const int m = ctrl[2];                         // counted by the keys kernel
     const int tid = static_cast<int>(threadIdx.x);
-    const int g = rank * kMoverPer + tid;  // the cluster-wide thread, owner of element g
-    const int gthreads = kMoverCtas * kMoverThreads;
-    const int chunk = (num_blocks + gthreads - 1) / gthreads;
-    const int b0 = min(g * chunk, num_blocks);
-    const int b1 = min(b0 + chunk, num_blocks);
-    uint32_t sum = 0u;
-    for (int b = b0; b < b1; ++b) sum += static_cast<uint32_t>(blk_cnt[b]);
-    uint32_t total = 0u;
-    const uint32_t first_local = block_exclusive_scan<kMoverThreads>(sum, &total);
-    if (tid == 0) cta_total = total;
-    cluster.sync();  // every CTA's total visible
-    if (tid == 0) {
-        uint32_t off = 0u, m = 0u;
-        for (int r = 0; r < kMoverCtas; ++r) {
-            const uint32_t t = *cluster.map_shared_rank(&cta_total, r);
-            if (r < rank) off += t;
-            m += t;
+    if (blockIdx.x == 0) {
+        const int chunk = (num_blocks + kMoverThreads - 1) / kMoverThreads;
+        const int b0 = min(tid * chunk, num_blocks);
+        const int b1 = min(b0 + chunk, num_blocks);
+        uint32_t sum = 0u;
+#pragma unroll 4
+        for (int b = b0; b < b1; ++b) sum += static_cast<uint32_t>(blk_cnt[b]);
+        uint32_t run = block_exclusive_scan<kMoverThreads>(sum, nullptr);
+        for (int b = b0; b < b1; ++b) {
+            blk_off[b] = static_cast<int>(run);
+            run += static_cast<uint32_t>(blk_cnt[b]);
         }
-        s_off = off;
-        s_m = m;
-    }
-    cluster.sync();  // remote reads done before any CTA may leave
-    const uint32_t total_all = s_m;
-    uint32_t run = s_off + first_local;
-    for (int b = b0; b < b1; ++b) {
-        blk_off[b] = static_cast<int>(run);
-        run += static_cast<uint32_t>(blk_cnt[b]);
-    }
-    const int m = static_cast<int>(total_all);
-    const int full = total_all > static_cast<uint32_t>(kMoverCap) ? 1 : 0;
-    if (rank == 0 && tid == 0) {
-        blk_off[num_blocks] = m;
-        ctrl[0] = m;
-        ctrl[1] = full;
-        if (use_cond) cudaGraphSetConditional(cond, static_cast<unsigned>(full));
-        if (full) atomicAdd(&counters[kCntRadixSearches], 1ull);
-    }
-    if (full || m == 0) return;  // the same decision in every CTA
-    // compaction in slot order, each mover stored in the CTA that owns its position
-    run = s_off + first_local;
-    for (int b = b0; b < b1; ++b) {
-        if (blk_cnt[b] == 0) continue;
-        const int w0 = b * (kBlock / 32);
-        for (int w = w0; w < w0 + kBlock / 32 && 32 * w < n; ++w) {
-            uint32_t bits = moved[w];
-            while (bits) {
-                const int lane = __ffs(bits) - 1;
-                bits &= bits - 1u;
-                const int slot = 32 * w + lane;
-                const int owner = static_cast<int>(run) / kMoverPer;
-                const int at = static_cast<int>(run) % kMoverPer;
-                *cluster.map_shared_rank(&k[at], owner) =
-                    (static_cast<unsigned long long>(newkey[slot]) << 32) |
-                    static_cast<uint32_t>(ids[slot]);
-                *cluster.map_shared_rank(&v[at], owner) = static_cast<uint32_t>(slot);
-                ++run;
-            }
+        if (tid == 0) {
+            const int full = m > cap ? 1 : 0;
+            blk_off[num_blocks] = m;
+            ctrl[0] = m;
+            ctrl[1] = full;
+            if (use_cond) cudaGraphSetConditional(cond, static_cast<unsigned>(full));
+            if (full) atomicAdd(&counters[kCntRadixSearches], 1ull);
         }
+        return;
     }
-    int p = 1;
-    while (p < m) p <<= 1;
-    if (g >= m && g < p) {
-        k[tid] = ~0ull;
-        v[tid] = 0u;
-    }
-    cluster.sync();  // the compacted movers and the padding visible everywhere
-    for (int size = 2; size <= p; size <<= 1) {
-        int stride = size >> 1;
-        for (; stride >= 32; stride >>= 1) {
-            const int j = g ^ stride;
-            if (g < p && j > g) {
-                const bool up = (g & size) == 0;
-                unsigned long long* kj = cluster.map_shared_rank(&k[j % kMoverPer], j / kMoverPer);
-                uint32_t* vj = cluster.map_shared_rank(&v[j % kMoverPer], j / kMoverPer);
-                const unsigned long long a = k[tid], c = *kj;
-                if ((a > c) == up) {
-                    k[tid] = c;
-                    *kj = a;
-                    const uint32_t t = v[tid];
-                    v[tid] = *vj;
-                    *vj = t;
-                }
-            }
-            // a stage that crosses CTAs, or precedes one, ends at a cluster barrier
-            const bool cross = stride >= kMoverPer;
-            const bool next_cross = (stride >> 1) >= kMoverPer;
-            if (cross || next_cross) cluster.sync();
-            else __syncthreads();
-        }
-        // strides below 32 pair lanes of one warp: exchanged through shuffles, no barrier
-        // (an element at or above p is padding that sorts last; its lane still shuffles)
-        unsigned long long a = k[tid];
-        uint32_t av = v[tid];
-        const bool up = (g & size) == 0;
-        for (; stride > 0; stride >>= 1) {
-            const unsigned long long c = __shfl_xor_sync(0xffffffffu, a, stride);
-            const uint32_t cv = __shfl_xor_sync(0xffffffffu, av, stride);
-            const bool lower = (g & stride) == 0;  // this lane holds the lower index
-            // ascending: the lower index keeps the smaller key; descending: the larger
-            const bool take = lower == up ? c < a : c > a;
-            if (take && g < p) {
-                a = c;
-                av = cv;
-            }
-        }
-        k[tid] = a;
-        v[tid] = av;
-        // the next size starts with a stride >= 32 (or none): across warps, maybe CTAs
-        if ((size << 1) <= p && size >= kMoverPer) cluster.sync();
-        else __syncthreads();
-    }
-    if (g < m) {
-        mv_key[g] = k[tid];
-        mv_slot[g] = v[tid];
-    }
+    if (m > cap || m == 0) return;
+    const int warps = (static_cast<int>(gridDim.x) - 1) * (kMoverThreads / 32);
+    // warps of a block take movers far apart, so that few movers use all blocks
+    const int first = (tid >> 5) * (static_cast<int>(gridDim.x) - 1) + static_cast<int>(blockIdx.x) - 1;
+    if (static_cast<int>(blockIdx.x) - 1 >= m) return;
+    for (int j = tid; j < m; j += kMoverThreads) keys[j] = raw[j];
+    __syncthreads();
+    if (m <= warps) rank_movers<1>(keys, m, first, warps, raw_slot, mv_key, mv_slot);
+    else rank_movers<4>(keys, m, first, warps, raw_slot, mv_key, mv_slot);
 }
 
 // Mover path, merge: final position of every grain. A stayer keeps its rank among
@@ -447,7 +395,7 @@ template <bool SNAP, bool SNAP_FROM_STATE>
 __global__ void __launch_bounds__(kBlock)
 k_gather(int n, int ppc, const uint32_t* __restrict__ skey, const uint32_t* __restrict__ sid,
          const int* __restrict__ src, const int* __restrict__ slot_of_id,
-         const int* __restrict__ ctrl, const float4* __restrict__ posA,
+         int* __restrict__ ctrl, const float4* __restrict__ posA,
          const float4* __restrict__ velA, float4* __restrict__ posB, float4* __restrict__ velB,
          int* __restrict__ idsB, const float4* __restrict__ nposA,
          const float4* __restrict__ nvelA, float4* __restrict__ nposB,
@@ -460,6 +408,7 @@ k_gather(int n, int ppc, const uint32_t* __restrict__ skey, const uint32_t* __re
     if (skipped(skip)) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
+    if (s == 0) ctrl[2] = 0;   // the next search counts its movers from zero
     const uint32_t id = sid[s];
     const int p = ctrl[1] ? slot_of_id[id] : src[s];
     const float4 x = posA[p], v = velA[p];
@@ -614,18 +563,21 @@ void launch_search_head(const DevParams& P, SceneTab T, const float4* pos, const
     const int totals = kRadix * sb.passes;
     const int kb = blocks_for(n > totals ? n : totals);
     if (T.params) {
-        k_keys<true><<<kb, kBlock, 0, st>>>(P, T, pos, sb.newkey, sb.moved, sb.blk_cnt,
+        k_keys<true><<<kb, kBlock, 0, st>>>(P, T, pos, ids, sb.mv_raw, sb.mv_raw_slot, sb.ctrl,
+                                            sb.mover_cap, sb.newkey, sb.moved, sb.blk_cnt,
                                             sb.num_blocks, sb.slot_keys, sb.table_keys, sb.table,
                                             sb.digit_totals, totals, zero_res, zero_res_count, skip);
     } else {
-        k_keys<false><<<kb, kBlock, 0, st>>>(P, T, pos, sb.newkey, sb.moved, sb.blk_cnt,
+        k_keys<false><<<kb, kBlock, 0, st>>>(P, T, pos, ids, sb.mv_raw, sb.mv_raw_slot, sb.ctrl,
+                                             sb.mover_cap, sb.newkey, sb.moved, sb.blk_cnt,
                                              sb.num_blocks, sb.slot_keys, sb.table_keys, sb.table,
                                              sb.digit_totals, totals, zero_res, zero_res_count, skip);
     }
-    k_movers<<<kMoverCtas, kMoverThreads, 0, st>>>(n, sb.blk_cnt, sb.blk_off, sb.num_blocks,
-                                                       sb.moved, sb.newkey, ids, sb.mv_key,
-                                                       sb.mv_slot, sb.ctrl, use_cond ? 1 : 0,
-                                                       cond, counters, skip);
+    // one block per SM, fewer where there cannot be that many movers
+    const int rankers = std::min(147, (std::min(n, sb.mover_cap) + 31) / 32);
+    k_movers<<<1 + rankers, kMoverThreads, sizeof(unsigned long long) * std::min(n, sb.mover_cap), st>>>(
+        n, sb.blk_cnt, sb.blk_off, sb.num_blocks, sb.mv_raw, sb.mv_raw_slot, sb.mv_key, sb.mv_slot,
+        sb.ctrl, sb.mover_cap, use_cond ? 1 : 0, cond, counters, skip);
 }
 
 void launch_search_radix(const DevParams& P, const int* ids, SearchBuffers& sb, Skip skip,
@@ -673,7 +625,12 @@ void launch_search(const DevParams& P, SceneTab T, const float4* pos, const int*
     launch_search_merge(P, ids, sb, skip, st);
 }
 
-cudaError_t search_prepare() { return cudaSuccess; }
+int mover_cap(int n) { return n < (1 << 16) ? 8192 : n < (1 << 19) ? 16384 : kMoverCap; }
+
+cudaError_t search_prepare() {
+    return cudaFuncSetAttribute(k_movers, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(sizeof(unsigned long long)) * kMoverCap);
+}
 
 int radix_output(int passes) { return (passes - 1) & 1; }
 

@@ -389,7 +389,7 @@ void free_sim(wd_sim* s) {
                     s->hcnt_snap[1], s->sb.key_by_id,
                     s->sb.slot_of_id, s->sb.keys[0], s->sb.keys[1], s->sb.vals[0],
                     s->sb.vals[1], s->sb.table_keys, s->sb.slot_keys, s->sb.newkey, s->sb.moved,
-                    s->sb.blk_cnt, s->sb.blk_off, s->sb.ctrl, s->sb.mv_key, s->sb.mv_slot,
+                    s->sb.blk_cnt, s->sb.blk_off, s->sb.ctrl, s->sb.mv_raw, s->sb.mv_raw_slot, s->sb.mv_key, s->sb.mv_slot,
                     s->sb.src, s->sb.tile_counts, s->sb.digit_totals,
                     s->sb.table, s->counters, s->picard_res, s->picard_used, s->partials,
                     s->red_out, s->dep_bounds, s->dep_acc, s->dep_out, s->staging,
@@ -1373,10 +1373,13 @@ int alloc_sim(wd_sim* s) {
     sb.num_blocks = wd::blocks_for(n);
     WD_CUDA(dalloc(&sb.blk_cnt, sb.num_blocks));
     WD_CUDA(dalloc(&sb.blk_off, static_cast<size_t>(sb.num_blocks) + 1));
-    WD_CUDA(dalloc(&sb.ctrl, 2));
-    WD_CUDA(cudaMemset(sb.ctrl, 0, 2 * sizeof(int)));
-    WD_CUDA(dalloc(&sb.mv_key, wd::kMoverCap));
-    WD_CUDA(dalloc(&sb.mv_slot, wd::kMoverCap));
+    WD_CUDA(dalloc(&sb.ctrl, 4));
+    WD_CUDA(cudaMemset(sb.ctrl, 0, 4 * sizeof(int)));
+    sb.mover_cap = wd::mover_cap(n);
+    WD_CUDA(dalloc(&sb.mv_raw, sb.mover_cap));
+    WD_CUDA(dalloc(&sb.mv_raw_slot, sb.mover_cap));
+    WD_CUDA(dalloc(&sb.mv_key, sb.mover_cap));
+    WD_CUDA(dalloc(&sb.mv_slot, sb.mover_cap));
     WD_CUDA(dalloc(&sb.src, n));
     WD_CUDA(wd::search_prepare());
     sb.num_tiles = static_cast<int>((static_cast<int64_t>(n) + wd::kSortTile - 1) / wd::kSortTile);
