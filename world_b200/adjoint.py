@@ -16,8 +16,9 @@ history rows); set them (set_history) before evaluating the same window again.
 """
 from __future__ import annotations
 
-import numpy as np
 import torch
+
+from ._lib import check, lib, ptr
 
 
 class _Window(torch.autograd.Function):
@@ -45,10 +46,13 @@ class _Deposit(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, v, sim):
         ctx.sim = sim
-        sim.compute_density_grid()
-        g = torch.from_numpy(sim.host_density_grid.copy()).to("cuda")
-        return g.reshape(4, sim.density_grid_size_x, sim.density_grid_size_y,
-                         sim.density_grid_size_z)
+        grid = torch.empty(4 * sim.density_grid_nodes(), dtype=torch.float32, device="cuda")
+        torch.cuda.current_stream().synchronize()
+        check(lib.wd_compute_density_grid_device(sim.handle, ptr(grid)))
+        check(lib.wd_synchronize(sim.handle))
+        torch.from_numpy(sim.host_density_grid).copy_(grid)
+        return grid.reshape(4, sim.density_grid_size_x, sim.density_grid_size_y,
+                            sim.density_grid_size_z)
 
     @staticmethod
     def backward(ctx, ggrid):

@@ -20,34 +20,6 @@
 namespace wd {
 namespace {
 
-struct AdjStep {
-    // sorted state of step t (the step's gathered copy) and its run table
-    const float4* pos;
-    const float4* vel;
-    const int* ids;
-    const int2* table;
-    // springs of step t (rows by grain id, counts by sorted slot) and of step t+1
-    // (rows and counts by grain id)
-    const float4* hist_in;
-    const int* hcnt_in;
-    const float4* hist_next;
-    const int* hcnt_next;
-    // the step's pair contacts per sorted slot, in the forward's visiting order
-    const int* clist;
-    const int* ccnt;
-    // adjoints of step t's outputs, by grain id
-    const float4* lx;
-    const float4* lvt;     // lv' + dt lx'
-    const float4* lf;      // dt / m * lvt
-    const float4* lxi;     // rows like hist_next
-    // adjoints of step t's inputs, by grain id
-    float4* lx_out;
-    float4* lv_out;
-    float4* lxi_out;       // rows like hist_in (zeroed before the launch)
-    double* theta;         // [3][n]: d/dmu, d/d ln e, d/dk_n, accumulated
-    int kt_from_kn;
-};
-
 __device__ __forceinline__ float3 f3(float4 a) { return make_float3(a.x, a.y, a.z); }
 
 template <class S>
@@ -85,38 +57,7 @@ __device__ __forceinline__ void vjp_add(const ContactOut<Dual<3>>& o, float3 wf,
 using D3 = Dual<3>;
 
 template <bool HIST>
-__device__ __forceinline__ void pair_blocks(const DevParams& P, const AdjStep& A, float3 d,
-                                            float3 vr, float3 xi, float ri, float rj, float mi,
-                                            float mj, float3 w_rel_f, float3 w_rel_x,
-                                            float3 w_own_f, float3 w_own_x, float ax[3],
-                                            float av[3], float axi[3], double th[3]) {
-    const float dv[3] = {d.x, d.y, d.z}, vv[3] = {vr.x, vr.y, vr.z}, xv[3] = {xi.x, xi.y, xi.z};
-    const Theta<D3> th0 = make_theta<D3>(P, A.kt_from_kn, 0);
-    for (int blk = 0; blk < 4; ++blk) {
-        D3 dd[3], vd[3], xd[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            dd[c] = dseed<3>(dv[c], blk == 0 ? c : -1);
-            vd[c] = dseed<3>(vv[c], blk == 1 ? c : -1);
-            xd[c] = dseed<3>(xv[c], blk == 2 ? c : -1);
-        }
-        const Theta<D3> tt = blk == 3 ? make_theta<D3>(P, A.kt_from_kn, 1) : th0;
-        ContactOut<D3> o;
-        pair_t<D3, HIST>(P, tt, dd, vd, xd, ri, rj, mi, mj, o);
-        if (blk == 0) vjp_add(o, w_rel_f, w_rel_x, ax);
-        else if (blk == 1) vjp_add(o, w_rel_f, w_rel_x, av);
-        else if (blk == 2) vjp_add(o, w_own_f, w_own_x, axi);
-        else {
-            float t[3] = {0.f, 0.f, 0.f};
-            vjp_add(o, w_own_f, w_own_x, t);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) th[c] += t[c];
-        }
-    }
-}
-
-template <bool HIST>
-__device__ __forceinline__ void wall_blocks(const DevParams& P, const AdjStep& A, float3 x,
+__device__ __forceinline__ void wall_blocks(const DevParams& P, const AdjArgs& A, float3 x,
                                             float3 v, float3 xi, float ri, float mi, int a,
                                             bool upper, float3 wf, float3 wx, float ax[3],
                                             float av[3], float axi[3], double th[3]) {
@@ -145,141 +86,179 @@ __device__ __forceinline__ void wall_blocks(const DevParams& P, const AdjStep& A
     }
 }
 
-// lvt = lv' + dt lx' and lF = dt / m lvt, by grain id.
-__global__ void __launch_bounds__(kBlock)
-k_adj_prep(int n, float dt, const float4* __restrict__ vel, const int* __restrict__ ids,
-           const float4* __restrict__ lx, const float4* __restrict__ lv,
-           float4* __restrict__ lvt, float4* __restrict__ lf) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const int id = ids[s];
-    const float m = vel[s].w;
-    const float4 x = lx[id], v = lv[id];
-    const float4 t = make_float4(fmaf(dt, x.x, v.x), fmaf(dt, x.y, v.y), fmaf(dt, x.z, v.z), 0.f);
-    lvt[id] = t;
+// lvt = lv' + dt lx' and lF = dt / m lvt of one grain of mass m.
+__device__ __forceinline__ float3 force_adjoint(float dt, float m, float4 x, float4 v, float3* lvt) {
+    const float3 t = make_float3(fmaf(dt, x.x, v.x), fmaf(dt, x.y, v.y), fmaf(dt, x.z, v.z));
+    if (lvt) *lvt = t;
     const float g = m != 0.f ? dt / m : 0.f;
-    lf[id] = make_float4(g * t.x, g * t.y, g * t.z, 0.f);
+    return make_float3(g * t.x, g * t.y, g * t.z);
 }
 
+// One step back. A warp's contacts are numbered grain by grain and taken 32 at a time: first
+// a lane each looks one up (geometry, springs, adjoints of both grains), then four lanes
+// each evaluate one, a block of three inputs per lane (position, velocity, stored spring,
+// parameters), 8 contacts at a time; last, each grain's lane adds its own in order. (A lane
+// that evaluates its grain's contacts alone runs the four long passes once per contact of
+// the busiest of its 32 grains.) Every entry of the input's spring rows is written: zero, or
+// the contact's. Bound by the latency of the dual arithmetic's chains.
+constexpr int kAdjBlock = 128;
+
+struct AdjWarp {
+    float geo[9][32];        // d, v_rel, stored spring
+    float w[12][32];         // relative and own weights: force, spring, each
+    float rj[32], mj[32];
+    int k_in[32];            // the stored spring's place in the owner's row, or -1
+    int queue[32];           // owner lane << 8 | contact
+    float out[32][13];
+    float ri[32], mi[32], lf[3][32];
+    int id[32], rows[32], walls[32];
+};
+
 template <bool HIST>
-__global__ void __launch_bounds__(kBlock)
-k_adj_step(DevParams P, AdjStep A) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= P.n) return;
-    const float4 pi = A.pos[s];
-    const float4 vi = A.vel[s];
-    const int id = A.ids[s];
-    const float3 pos = f3(pi), vel = f3(vi);
-    const float ri = pi.w, mi = vi.w;
-    const float3 lf_i = f3(A.lf[id]);
-    const float3 zero = make_float3(0.f, 0.f, 0.f);
-    const float4* in_row = HIST ? A.hist_in + static_cast<int64_t>(id) * kHistCap : nullptr;
-    const int in_count = HIST ? A.hcnt_in[s] : 0;
-    int out_count = 0;
+__global__ void __launch_bounds__(kAdjBlock)
+k_adj_step(DevParams P, AdjArgs A) {
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ AdjWarp warps[kAdjBlock / 32];
+    AdjWarp& W = warps[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int s = blockIdx.x * kAdjBlock + static_cast<int>(threadIdx.x);
+    const int s0 = s - lane;                 // the warp's first slot
+    const bool live = s < P.n;
+    float4 pi = make_float4(0.f, 0.f, 0.f, 0.f), vi = pi, lx = pi;
+    float3 lvt = make_float3(0.f, 0.f, 0.f), lf_i = lvt;
+    int id = 0, in_count = 0, nc = 0, out_count = 0;
     float ax[3] = {0.f, 0.f, 0.f}, av[3] = {0.f, 0.f, 0.f};
     double th[3] = {0.0, 0.0, 0.0};
-
-    // walls, in the forward's order: axis 0 lower, upper, axis 1, axis 2
-    const float p3[3] = {pos.x, pos.y, pos.z};
-    for (int a = 0; a < 3; ++a) {
-        for (int up = 0; up < 2; ++up) {
-            const float dl = up ? (P.wall_hi[a] - p3[a]) - ri : (p3[a] - P.wall_lo[a]) - ri;
-            if (!(dl < 0.f)) continue;
-            const int partner = up ? -2 - 2 * a : -1 - 2 * a;
-            float3 xi = zero, lxi_own = zero;
+    if (live) {
+        pi = A.pos[s];
+        vi = A.vel[s];
+        id = A.ids[s];
+        nc = A.ccnt[s];
+        lx = A.lx[id];
+        lf_i = force_adjoint(P.dt, vi.w, lx, A.lv[id], &lvt);
+        const float4* in_row = HIST ? A.hist_in + static_cast<int64_t>(id) * kHistCap : nullptr;
+        if (HIST) {
+            in_count = A.hcnt_in[s];
+            for (int k = 0; k < in_count; ++k)
+                A.lxi_out[static_cast<int64_t>(id) * kHistCap + k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        // walls, in the forward's order: axis 0 lower, upper, axis 1, axis 2
+        const float p3[3] = {pi.x, pi.y, pi.z};
+        for (int a = 0; a < 3; ++a) {
+            for (int up = 0; up < 2; ++up) {
+                const float dl = up ? (P.wall_hi[a] - p3[a]) - pi.w : (p3[a] - P.wall_lo[a]) - pi.w;
+                if (!(dl < 0.f)) continue;
+                const int partner = up ? -2 - 2 * a : -1 - 2 * a;
+                float3 xi = make_float3(0.f, 0.f, 0.f), lxi_own = xi;
+                int k_in = -1;
+                if (HIST) {
+                    k_in = row_find(in_row, in_count, partner);
+                    if (k_in >= 0) xi = f3(in_row[k_in]);
+                    if (out_count < kHistCap)
+                        lxi_own = f3(A.lxi[static_cast<int64_t>(id) * kHistCap + out_count]);
+                    ++out_count;
+                }
+                float axi[3] = {0.f, 0.f, 0.f};
+                wall_blocks<HIST>(P, A, f3(pi), f3(vi), xi, pi.w, vi.w, a, up != 0, lf_i, lxi_own, ax, av, axi, th);
+                if (HIST && k_in >= 0)
+                    A.lxi_out[static_cast<int64_t>(id) * kHistCap + k_in] =
+                        make_float4(axi[0], axi[1], axi[2], 0.f);
+            }
+        }
+    }
+    W.ri[lane] = pi.w;
+    W.mi[lane] = vi.w;
+    W.lf[0][lane] = lf_i.x;
+    W.lf[1][lane] = lf_i.y;
+    W.lf[2][lane] = lf_i.z;
+    W.id[lane] = id;
+    W.rows[lane] = in_count;
+    W.walls[lane] = out_count;
+    int upto = nc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kAll, upto, o);
+        if (lane >= o) upto += y;
+    }
+    const int off = upto - nc;
+    const int total = __shfl_sync(kAll, upto, 31);
+    for (int base = 0; base < total; base += 32) {
+        const int cnt = min(32, total - base);
+        for (int q = max(off, base); q < min(upto, base + 32); ++q) W.queue[q - base] = (lane << 8) | (q - off);
+        __syncwarp();
+        if (lane < cnt) {
+            const int o = W.queue[lane] >> 8, e = W.queue[lane] & 255, so = s0 + o;
+            const int j = A.clist[static_cast<int64_t>(e) * P.n + so];
+            const float4 po = A.pos[so], vo = A.vel[so], pj = A.pos[j], vj = A.vel[j];
+            float3 d;
+            pair_norm_sq(po, pj, d);
+            const int jd = A.ids[j], io = W.id[o];
+            const float3 lf_j = force_adjoint(P.dt, vj.w, A.lx[jd], A.lv[jd], nullptr);
+            float3 xi = make_float3(0.f, 0.f, 0.f), lxi_ij = xi, lxi_ji = xi;
             int k_in = -1;
             if (HIST) {
-                k_in = row_find(in_row, in_count, partner);
-                if (k_in >= 0) xi = f3(in_row[k_in]);
-                if (out_count < kHistCap)
-                    lxi_own = f3(A.lxi[static_cast<int64_t>(id) * kHistCap + out_count]);
-                ++out_count;
+                const float4* row = A.hist_in + static_cast<int64_t>(io) * kHistCap;
+                k_in = row_find(row, W.rows[o], jd);
+                if (k_in >= 0) xi = f3(row[k_in]);
+                const int at = W.walls[o] + e;
+                if (at < kHistCap) lxi_ij = f3(A.lxi[static_cast<int64_t>(io) * kHistCap + at]);
+                const int kj = row_find(A.hist_next + static_cast<int64_t>(jd) * kHistCap, A.hcnt_next[jd], io);
+                if (kj >= 0) lxi_ji = f3(A.lxi[static_cast<int64_t>(jd) * kHistCap + kj]);
             }
-            float axi[3] = {0.f, 0.f, 0.f};
-            wall_blocks<HIST>(P, A, pos, vel, xi, ri, mi, a, up != 0, lf_i, lxi_own, ax, av, axi, th);
-            if (HIST && k_in >= 0)
-                A.lxi_out[static_cast<int64_t>(id) * kHistCap + k_in] =
-                    make_float4(axi[0], axi[1], axi[2], 0.f);
+            const float geo[9] = {d.x, d.y, d.z, vo.x - vj.x, vo.y - vj.y, vo.z - vj.z, xi.x, xi.y, xi.z};
+            const float own[3] = {W.lf[0][o], W.lf[1][o], W.lf[2][o]};
+            const float w[12] = {own[0] - lf_j.x, own[1] - lf_j.y, own[2] - lf_j.z,
+                                 lxi_ij.x - lxi_ji.x, lxi_ij.y - lxi_ji.y, lxi_ij.z - lxi_ji.z,
+                                 own[0], own[1], own[2], lxi_ij.x, lxi_ij.y, lxi_ij.z};
+#pragma unroll
+            for (int k = 0; k < 9; ++k) W.geo[k][lane] = geo[k];
+#pragma unroll
+            for (int k = 0; k < 12; ++k) W.w[k][lane] = w[k];
+            W.rj[lane] = pj.w;
+            W.mj[lane] = vj.w;
+            W.k_in[lane] = k_in;
         }
-    }
-
-    // pairs, in the forward's visiting order (recorded by the replay)
-    const int nc = A.ccnt[s];
-    for (int e = 0; e < nc; ++e) {
-        const int j = A.clist[static_cast<int64_t>(e) * P.n + s];
-        const float4 pj = A.pos[j];
-        float3 d;
-        pair_norm_sq(pi, pj, d);
-        const float4 vj = A.vel[j];
-        const int jd = A.ids[j];
-        const float3 lf_j = f3(A.lf[jd]);
-        float3 xi = zero, lxi_ij = zero, lxi_ji = zero;
-        int k_in = -1;
-        if (HIST) {
-            k_in = row_find(in_row, in_count, jd);
-            if (k_in >= 0) xi = f3(in_row[k_in]);
-            if (out_count < kHistCap)
-                lxi_ij = f3(A.lxi[static_cast<int64_t>(id) * kHistCap + out_count]);
-            ++out_count;
-            const float4* jrow = A.hist_next + static_cast<int64_t>(jd) * kHistCap;
-            const int kj = row_find(jrow, A.hcnt_next[jd], id);
-            if (kj >= 0) lxi_ji = f3(A.lxi[static_cast<int64_t>(jd) * kHistCap + kj]);
+        __syncwarp();
+        const int blk = lane & 3;
+        for (int c = lane >> 2; c < cnt; c += 8) {
+            const int o = W.queue[c] >> 8;
+            D3 dd[3], vd[3], xd[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                dd[k] = dseed<3>(W.geo[k][c], blk == 0 ? k : -1);
+                vd[k] = dseed<3>(W.geo[3 + k][c], blk == 1 ? k : -1);
+                xd[k] = dseed<3>(W.geo[6 + k][c], blk == 2 ? k : -1);
+            }
+            const Theta<D3> tt = make_theta<D3>(P, A.kt_from_kn, blk == 3);
+            ContactOut<D3> r;
+            pair_t<D3, HIST>(P, tt, dd, vd, xd, W.ri[o], W.rj[c], W.mi[o], W.mj[c], r);
+            const int u = blk < 2 ? 0 : 6;     // relative weights for d and v_rel, own for the rest
+            float t[3] = {0.f, 0.f, 0.f};
+            vjp_add(r, make_float3(W.w[u][c], W.w[u + 1][c], W.w[u + 2][c]),
+                    make_float3(W.w[u + 3][c], W.w[u + 4][c], W.w[u + 5][c]), t);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) W.out[c][3 * blk + k] = t[k];
+            if (HIST && blk == 2 && W.k_in[c] >= 0)
+                A.lxi_out[static_cast<int64_t>(W.id[o]) * kHistCap + W.k_in[c]] =
+                    make_float4(t[0], t[1], t[2], 0.f);
         }
-        const float3 w_rel_f = make_float3(lf_i.x - lf_j.x, lf_i.y - lf_j.y, lf_i.z - lf_j.z);
-        const float3 w_rel_x = make_float3(lxi_ij.x - lxi_ji.x, lxi_ij.y - lxi_ji.y,
-                                           lxi_ij.z - lxi_ji.z);
-        const float3 vr = make_float3(vel.x - vj.x, vel.y - vj.y, vel.z - vj.z);
-        float axi[3] = {0.f, 0.f, 0.f};
-        pair_blocks<HIST>(P, A, d, vr, xi, ri, pj.w, mi, vj.w, w_rel_f, w_rel_x, lf_i,
-                          lxi_ij, ax, av, axi, th);
-        if (HIST && k_in >= 0)
-            A.lxi_out[static_cast<int64_t>(id) * kHistCap + k_in] =
-                make_float4(axi[0], axi[1], axi[2], 0.f);
+        __syncwarp();
+        for (int q = max(off, base); q < min(upto, base + 32); ++q) {
+            const float* r = W.out[q - base];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                ax[k] += r[k];
+                av[k] += r[3 + k];
+                th[k] += r[9 + k];
+            }
+        }
+        __syncwarp();                        // the records are free again
     }
-    const float4 lx = A.lx[id], lvt = A.lvt[id];
+    if (!live) return;
     A.lx_out[id] = make_float4(lx.x + ax[0], lx.y + ax[1], lx.z + ax[2], 0.f);
     A.lv_out[id] = make_float4(lvt.x + av[0], lvt.y + av[1], lvt.z + av[2], 0.f);
 #pragma unroll
     for (int c = 0; c < 3; ++c) A.theta[static_cast<int64_t>(c) * P.n + id] += th[c];
-}
-
-// The pair contacts of every sorted slot in the contact kernel's visiting order
-// (run-table stencil walk, the same tests), for the reverse pass.
-__global__ void __launch_bounds__(kBlock)
-k_contact_record(DevParams P, const float4* __restrict__ pos, const int2* __restrict__ table,
-                 int* __restrict__ clist, int* __restrict__ ccnt,
-                 unsigned long long* __restrict__ overflow) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= P.n) return;
-    const float4 pi = pos[s];
-    const float ri = pi.w;
-    const float cut = contact_cutoff_sq(ri, P.rmax);
-    int cx, cy, cz;
-    cell_coords(P, pi.x, pi.y, pi.z, cx, cy, cz);
-    int cnt = 0;
-    for (int dx = -1; dx <= 1; ++dx) {
-        const int nx = cx + dx;
-        if (nx < 0 || nx >= P.grid[0]) continue;
-        int lo[3], hi[3];
-        row_ranges(P, table, nx, cy, cz, lo, hi);
-        for (int t = 0; t < 3; ++t) {
-            for (int j = lo[t]; j < hi[t]; ++j) {
-                const float4 pj = __ldg(&pos[j]);
-                float3 d;
-                const float ns = pair_norm_sq(pi, pj, d);
-                if (ns > cut || j == s) continue;
-                const float dist = pair_dist(sqrtf(ns), ri, pj.w);
-                if (!(dist < 0.f)) continue;
-                if (cnt < kAdjContacts) clist[static_cast<int64_t>(cnt) * P.n + s] = j;
-                ++cnt;
-            }
-        }
-    }
-    if (cnt > kAdjContacts) {
-        atomicAdd(overflow, 1ull);
-        cnt = kAdjContacts;
-    }
-    ccnt[s] = cnt;
 }
 
 // Counts of a spring snapshot by grain id (snapshots keep them by sorted slot).
@@ -352,25 +331,10 @@ k_deposit_vjp(int n, const float4* __restrict__ pos, const float4* __restrict__ 
 
 }  // namespace
 
-void launch_adj_prep(int n, float dt, const float4* vel, const int* ids, const float4* lx,
-                     const float4* lv, float4* lvt, float4* lf, cudaStream_t st) {
-    k_adj_prep<<<blocks_for(n), kBlock, 0, st>>>(n, dt, vel, ids, lx, lv, lvt, lf);
-}
-
-void launch_contact_record(const DevParams& P, const float4* pos, const int2* table, int* clist,
-                           int* ccnt, unsigned long long* overflow, cudaStream_t st) {
-    k_contact_record<<<blocks_for(P.n), kBlock, 0, st>>>(P, pos, table, clist, ccnt, overflow);
-}
-
 void launch_adj_step(const DevParams& P, const AdjArgs& a, cudaStream_t st) {
-    AdjStep A;
-    A.pos = a.pos; A.vel = a.vel; A.ids = a.ids; A.table = a.table;
-    A.hist_in = a.hist_in; A.hcnt_in = a.hcnt_in; A.hist_next = a.hist_next;
-    A.hcnt_next = a.hcnt_next; A.clist = a.clist; A.ccnt = a.ccnt; A.lx = a.lx; A.lvt = a.lvt; A.lf = a.lf; A.lxi = a.lxi;
-    A.lx_out = a.lx_out; A.lv_out = a.lv_out; A.lxi_out = a.lxi_out; A.theta = a.theta;
-    A.kt_from_kn = a.kt_from_kn;
-    if (P.history) k_adj_step<true><<<blocks_for(P.n), kBlock, 0, st>>>(P, A);
-    else k_adj_step<false><<<blocks_for(P.n), kBlock, 0, st>>>(P, A);
+    const int nb = blocks_for(P.n, kAdjBlock);
+    if (P.history) k_adj_step<true><<<nb, kAdjBlock, 0, st>>>(P, a);
+    else k_adj_step<false><<<nb, kAdjBlock, 0, st>>>(P, a);
 }
 
 void launch_counts_by_id(int n, const int* ids, const int* cnt_slot, int* cnt_id, cudaStream_t st) {

@@ -27,7 +27,9 @@ __device__ __forceinline__ bool skipped(const Skip& s) {
 // 5 resident blocks of 256 per SM (<= 51 registers): the candidate loop is
 // latency-bound, so occupancy matters more than the few values the rarely taken
 // contact path may keep in local memory.
-template <bool HIST, bool PICARD, bool BATCH>
+// REC: also note down the contacts, for the reverse pass (a walk of its own cost as much as
+// this one).
+template <bool HIST, bool PICARD, bool BATCH, bool REC = false>
 __global__ void __launch_bounds__(kBlock, 5)
 k_force(DevParams P0, ForceArgs A, Skip skip) {
     if (PICARD && skipped(skip)) return;
@@ -61,6 +63,8 @@ k_force(DevParams P0, ForceArgs A, Skip skip) {
             }
             wall_forces<HIST>(P, pos, vel, ri, mi, f, h, A.counters);
 
+            if (REC && HIST) A.rec_hcnt[id] = h.in_count;
+            int noted = 0;
             const float cut = contact_cutoff_sq(ri, P.rmax);
             int cx, cy, cz;
             cell_coords(P, pi.x, pi.y, pi.z, cx, cy, cz);
@@ -79,6 +83,11 @@ k_force(DevParams P0, ForceArgs A, Skip skip) {
                         const float norm = sqrtf(ns);
                         const float dist = pair_dist(norm, ri, pj.w);
                         if (!(dist < 0.f)) continue;
+                        if (REC) {
+                            if (noted < kAdjContacts)
+                                A.rec_list[static_cast<int64_t>(noted) * P0.n + s] = j;
+                            ++noted;
+                        }
                         const float4 vj = __ldg(&A.vel[j]);
                         const int partner = HIST ? __ldg(&A.ids[j]) : 0;
                         pair_force<HIST>(P, d, norm, dist, vel, mi, vj, partner, f, h, A.counters);
@@ -86,6 +95,10 @@ k_force(DevParams P0, ForceArgs A, Skip skip) {
                 }
             }
             if (HIST) A.hcnt_out[s] = h.out_count;
+            if (REC) {
+                A.rec_cnt[s] = min(noted, kAdjContacts);
+                if (noted > kAdjContacts) atomicAdd(A.rec_over, 1ull);
+            }
 
             const float3 a = make_float3(f.x / mi, f.y / mi, f.z / mi);
             float3 v1, x1;
@@ -335,6 +348,11 @@ void launch_force(const DevParams& P, const ForceArgs& a, bool picard, Skip skip
                   cudaStream_t st, int block) {
     const int nb = blocks_for(P.n, block);
     const bool batch = a.scene_params != nullptr;
+    if (a.rec_list) {
+        if (P.history) k_force<true, false, false, true><<<nb, block, 0, st>>>(P, a, skip);
+        else k_force<false, false, false, true><<<nb, block, 0, st>>>(P, a, skip);
+        return;
+    }
 #define WD_FORCE(H, PI, B) k_force<H, PI, B><<<nb, block, 0, st>>>(P, a, skip)
     if (P.history) {
         if (picard) { if (batch) WD_FORCE(true, true, true); else WD_FORCE(true, true, false); }

@@ -117,7 +117,11 @@ struct ForceArgs {
     const DevParams* scene_params;                         // batched scenes (or NULL)
     const int* scene;                                      // scene of each input slot
     int* scene_out;                                        // scene of each output slot
+    // the reverse pass's replay (single scenes): each slot's pair contacts in visiting order,
+    // their counts, contacts beyond kAdjContacts, and hcnt_in by grain id
+    int* rec_list; int* rec_cnt; unsigned long long* rec_over; int* rec_hcnt;
 };
+constexpr int kAdjContacts = 32;  // pair contacts per grain the reverse pass records
 
 // Scene segments of the sorted order, for per-scene reductions: seg[S+1] grain
 // offsets (scene s holds sorted positions [seg[s], seg[s+1])), chunk_base[S+1] prefix
@@ -284,20 +288,14 @@ int reduction_blocks(int n);
 // id; spring rows are kHistCap entries per grain id.
 struct AdjArgs {
     const float4* pos; const float4* vel; const int* ids;  // sorted state of step t
-    const int2* table;
     const float4* hist_in; const int* hcnt_in;     // springs at t (counts by sorted slot)
     const float4* hist_next; const int* hcnt_next; // springs at t+1 (counts by id)
     const int* clist; const int* ccnt;             // pair contacts per slot (kAdjContacts)
-    const float4* lx; const float4* lvt; const float4* lf; const float4* lxi;
-    float4* lx_out; float4* lv_out; float4* lxi_out;
+    const float4* lx; const float4* lv; const float4* lxi;   // adjoints of step t's outputs
+    float4* lx_out; float4* lv_out; float4* lxi_out;         // of its inputs (whole rows written)
     double* theta;                                  // [3][n], accumulated
     int kt_from_kn;
 };
-constexpr int kAdjContacts = 32;  // pair contacts per grain the reverse pass records
-void launch_contact_record(const DevParams& P, const float4* pos, const int2* table, int* clist,
-                           int* ccnt, unsigned long long* overflow, cudaStream_t st);
-void launch_adj_prep(int n, float dt, const float4* vel, const int* ids, const float4* lx,
-                     const float4* lv, float4* lvt, float4* lf, cudaStream_t st);
 void launch_adj_step(const DevParams& P, const AdjArgs& a, cudaStream_t st);
 void launch_counts_by_id(int n, const int* ids, const int* cnt_slot, int* cnt_id,
                          cudaStream_t st);

@@ -2493,9 +2493,9 @@ cudaError_t adj_replay_body(wd_sim* s, int len, bool capture, cudaStream_t st) {
                           nullptr, nullptr, false, hist ? s->hcnt_slot : nullptr,
                           hist ? T.hcnt : nullptr, nullptr, nullptr, true, s->counters, nullptr,
                           nullptr, none, st);
-        wd::launch_contact_record(P, T.pos, s->sb.table, T.clist, T.ccnt, s->adj_ovf, st);
-        if (hist) wd::launch_counts_by_id(n, T.ids, T.hcnt, T.cnt_id, st);
         wd::ForceArgs fa{};
+        fa.rec_list = T.clist; fa.rec_cnt = T.ccnt; fa.rec_over = s->adj_ovf;
+        fa.rec_hcnt = hist ? T.cnt_id : nullptr;
         fa.pos = T.pos; fa.vel = T.vel; fa.ids = T.ids; fa.table = s->sb.table;
         fa.pos_out = s->posA; fa.vel_out = s->velA; fa.ids_out = s->idsA;
         fa.acc_out = s->acc;
@@ -2521,20 +2521,14 @@ cudaError_t adj_back_body(wd_sim* s, int len, int cur, cudaStream_t st) {
     for (int t = len - 1; t >= 0; --t) {
         const wd_sim::TapeStep& T = s->adj_tape[static_cast<size_t>(t)];
         const wd_sim::TapeStep& T1 = s->adj_tape[static_cast<size_t>(t) + 1];
-        if (hist) {
-            cudaError_t e = cudaMemsetAsync(s->adj_lxi[cur ^ 1], 0, rows * sizeof(float4), st);
-            if (e != cudaSuccess) return e;
-        }
-        wd::launch_adj_prep(n, P.dt, T.vel, T.ids, s->adj_lx[cur], s->adj_lv[cur], s->adj_lvt,
-                            s->adj_lf, st);
         wd::AdjArgs a{};
-        a.pos = T.pos; a.vel = T.vel; a.ids = T.ids; a.table = nullptr;
+        a.pos = T.pos; a.vel = T.vel; a.ids = T.ids;
         a.hist_in = hist ? T.hist : nullptr;
         a.hcnt_in = hist ? T.hcnt : nullptr;
         a.hist_next = hist ? T1.hist : nullptr;
         a.hcnt_next = hist ? T1.cnt_id : nullptr;
         a.clist = T.clist; a.ccnt = T.ccnt;
-        a.lx = s->adj_lx[cur]; a.lvt = s->adj_lvt; a.lf = s->adj_lf;
+        a.lx = s->adj_lx[cur]; a.lv = s->adj_lv[cur];
         a.lxi = hist ? s->adj_lxi[cur] : nullptr;
         a.lx_out = s->adj_lx[cur ^ 1]; a.lv_out = s->adj_lv[cur ^ 1];
         a.lxi_out = hist ? s->adj_lxi[cur ^ 1] : nullptr;
