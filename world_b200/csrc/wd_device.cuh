@@ -30,7 +30,10 @@ enum Counter : int {
     kCntStageTimeout = 9,   // bulk-staged contact kernel: stages that never completed
     kCntListResort = 10,    // list contact kernels: grains whose contacts were re-ordered
     kCntLaunchFail = 11,    // device-side launches of a list build's graphs that failed
-    kNumCounters = 12,
+    kCntAutoSteps = 12,     // steps on the library's own lists (neighbor_skin 0)
+    kCntAutoBuilds = 13,    // builds that such steps decided
+    kCntAutoCrowded = 14,   // a build found a cell that could overfill
+    kNumCounters = 15,
 };
 
 // Everything a step kernel needs, passed by value (baked into the captured graph).

@@ -133,9 +133,7 @@ struct Segments {
     int total_chunks;
 };
 
-// block: threads per block (a multiple of 32, at most kBlock; the autotuner's choice)
-void launch_force(const DevParams& P, const ForceArgs& a, bool picard, Skip skip,
-                  cudaStream_t st, int block = kBlock);
+void launch_force(const DevParams& P, const ForceArgs& a, bool picard, Skip skip, cudaStream_t st);
 
 // Verlet lists (simulation.neighbor_skin > 0). list_ctrl words:
 // [0] max |x - x_build|^2 over the last step's output (float bits; measured only when
@@ -152,9 +150,8 @@ void launch_force(const DevParams& P, const ForceArgs& a, bool picard, Skip skip
 // tests). Picard builds earlier, at kPicardBuildAt, so that its iterates rarely leave.
 constexpr float kListValid = 0.49f;
 constexpr float kPicardBuildAt = 0.30f;
-// kLcCrowded / kLcSteps / kLcBuilds: the library's own lists under neighbor_skin 0 (a cell
-// may hold more than particles_per_cell grains before the next build; list steps and their
-// builds so far).
+// kLcCrowded: the library's own lists under neighbor_skin 0, a cell may hold more than
+// particles_per_cell grains before the next build.
 // kLcStallTest / kLcWaitUs: the bulk-staged contact kernel's wait test. A nonzero
 // kLcStallTest makes each warp's first stage expect 16 bytes that no copy delivers (no
 // copy is issued for it), so its bounded wait runs out; kLcWaitUs is that wait's limit
@@ -162,7 +159,7 @@ constexpr float kPicardBuildAt = 0.30f;
 enum ListCtrl {
     kLcDisp = 0, kLcOverflow = 1, kLcForce = 2, kLcDecision = 3, kLcViol = 4, kLcRedo = 5,
     kLcStep = 6, kLcExact = 7, kLcBound = 8, kLcStallTest = 10, kLcWaitUs = 11, kLcCrowded = 12,
-    kLcSteps = 13, kLcBuilds = 14, kLcWords = 16
+    kLcWords = 16
 };
 struct ListArgs {
     const float4* pos; const float4* vel; const int* ids;  // state of the step
@@ -184,8 +181,8 @@ struct ListArgs {
     // semi-implicit Euler: the build decision for the next step, made by the kernel's
     // last block (threshold on max |x - x_build|, block ticket, the build's IF node)
     float thr; unsigned* tail_count; int use_cond; cudaGraphConditionalHandle cond;
-    // the library's own lists: counters of the last build's gather, host-visible words
-    unsigned long long* pend; uint32_t* host_word;
+    // the library's own lists: counters of the last build's gather
+    unsigned long long* pend;
 };
 // Device-side launches of the list build's graphs (wd_launch.cu, the one translation
 // unit built with relocatable device code for the device runtime): one thread

@@ -51,10 +51,10 @@ __device__ __forceinline__ bool skipped(const Skip& s) {
 // A build counts them of the state it sorts into pend; they are due when the next step
 // starts from that state, here at its end (`step`). Between builds there are none unless the
 // build found a cell that could fill up (kLcCrowded): then every step builds, and
-// host_word[2] tells the host to search instead.
+// kCntAutoCrowded tells the host to search instead.
 __device__ bool list_decide_core(uint32_t* ctrl_, float thr, int always_exact,
                                  unsigned long long* counters, unsigned long long* pend,
-                                 uint32_t* host_word, bool at_step) {
+                                 bool at_step) {
     volatile uint32_t* ctrl = ctrl_;
     volatile double* bound = reinterpret_cast<volatile double*>(ctrl_ + kLcBound);
     const double grow = 1.0 + 1.0 / 65536.0;
@@ -67,15 +67,10 @@ __device__ bool list_decide_core(uint32_t* ctrl_, float thr, int always_exact,
         const bool crowded = ctrl[kLcCrowded] != 0u;
         if (at_step) {
             counters[kCntGridOverflow] += pend[kCntGridOverflow];
-            ctrl[kLcSteps] = ctrl[kLcSteps] + 1u;
             build |= crowded;
-            if (build) {
-                ctrl[kLcBuilds] = ctrl[kLcBuilds] + 1u;
-                volatile uint32_t* w = host_word;
-                w[0] = ctrl[kLcSteps];
-                w[1] = ctrl[kLcBuilds];
-                if (crowded) w[2] = 1u;
-            }
+            counters[kCntAutoSteps] += 1ull;
+            if (build) counters[kCntAutoBuilds] += 1ull;
+            if (crowded) counters[kCntAutoCrowded] = 1ull;
         }
         if (build) {
             pend[kCntGridOverflow] = 0ull;
@@ -103,7 +98,7 @@ __global__ void k_list_decide(uint32_t* __restrict__ ctrl, float thr, int always
                               unsigned long long* __restrict__ pend, int use_cond,
                               cudaGraphConditionalHandle cond) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const bool build = list_decide_core(ctrl, thr, always_exact, counters, pend, nullptr, false);
+    const bool build = list_decide_core(ctrl, thr, always_exact, counters, pend, false);
     if (use_cond) cudaGraphSetConditional(cond, build ? 1u : 0u);
 }
 
@@ -157,7 +152,7 @@ __device__ __forceinline__ void list_tail_decide(const ListArgs& A) {
         if (ticket == gridDim.x - 1) {
             __threadfence();
             const bool build =
-                list_decide_core(A.list_ctrl, A.thr, 0, A.counters, A.pend, A.host_word, true);
+                list_decide_core(A.list_ctrl, A.thr, 0, A.counters, A.pend, true);
             *reinterpret_cast<volatile unsigned*>(A.tail_count) = 0u;
             if (A.use_cond) cudaGraphSetConditional(A.cond, build ? 1u : 0u);
         }

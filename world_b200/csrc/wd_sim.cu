@@ -33,8 +33,6 @@ namespace {
 
 using wd::DevParams;
 
-constexpr int kPinnedExtra = 64;   // 8-byte words for small results (see read_small)
-
 constexpr const char* kVersion = "world_b200 0.1.0 (sm_100a)";
 
 int fail(int code, const std::string& msg) {
@@ -165,14 +163,12 @@ struct wd_sim {
     bool auto_ok = false;                    // this handle may use them
     unsigned long long* auto_pend = nullptr; // counters that a build's gather adds to
     uint32_t* auto_load = nullptr;           // per cell: grains that can be in it before the next build
-    uint32_t* auto_word = nullptr;           // pinned: list steps, builds, a crowded cell seen
-    uint32_t* auto_word_dev = nullptr;
     int64_t run_steps = 0, last_run = 0;     // steps since the last upload, and between the two before
     int64_t auto_off = 0, auto_backoff = 512;// steps to search before lists are tried again
-    uint32_t auto_seen[2] = {0, 0};
+    int64_t auto_look = 0;                   // list step of the run that reads the device's counts next
+    unsigned long long auto_seen[2] = {0, 0};// list steps and builds at the last look
     bool list_work = false;                  // list steps or builds since the last synchronise
-    // host copies read after a synchronise: the counters, then kPinnedExtra words for results
-    unsigned long long* pinned = nullptr;
+    unsigned long long seen[wd::kNumCounters] = {};  // the counters as of the last synchronise
 
     // reverse pass: snapshots of the step state (checkpoints of a recorded window and
     // the states of the segment being replayed) and the adjoint buffers
@@ -401,8 +397,6 @@ void free_sim(wd_sim* s) {
                     s->tail_count, s->auto_pend, s->auto_load, s->xpos, s->xvel, s->xids, s->xscene, s->rhs_vel, s->rhs_ids};
     for (void* b : bufs)
         if (b) cudaFree(b);
-    if (s->auto_word) cudaFreeHost(s->auto_word);
-    if (s->pinned) cudaFreeHost(s->pinned);
     for (cudaEvent_t e : s->ev_pool) cudaEventDestroy(e);
     for (cudaEvent_t e : s->ev_pending) cudaEventDestroy(e);
     free_tape(s);
@@ -572,7 +566,7 @@ void enqueue_step_tail(wd_sim* s, int parity, cudaStream_t st, cudaEvent_t mid) 
     if (mid) cudaEventRecord(mid, st);
     wd::ForceArgs fa = step_force_args(s, parity);
     fa.hcnt_in = s->hcnt_g;
-    wd::launch_force(P, fa, false, none, st, s->force_block);
+    wd::launch_force(P, fa, false, none, st);
 }
 
 cudaError_t enqueue_step(wd_sim* s, int parity, cudaStream_t st, bool capture,
@@ -623,7 +617,7 @@ cudaError_t enqueue_step(wd_sim* s, int parity, cudaStream_t st, bool capture,
         fa.res_slot = s->picard_res + k;
         fa.picard_used = s->picard_used;
         fa.iter = k;
-        wd::launch_force(P, fa, true, skip, st, s->force_block);
+        wd::launch_force(P, fa, true, skip, st);
     }
     return cudaGetLastError();
 }
@@ -955,7 +949,6 @@ cudaError_t enqueue_step_list(wd_sim* s, int parity, cudaStream_t st, bool captu
     a.thr = wd::kListValid * P.skin;
     a.tail_count = s->tail_count;
     a.pend = s->auto_ok ? s->auto_pend : nullptr;
-    a.host_word = s->auto_word_dev;
     a.use_cond = capture && !device_build ? 1 : 0;
     a.cond = cond;
     a.pos = s->posA; a.vel = s->velA; a.ids = s->idsA; a.table = s->sb.table;
@@ -1186,19 +1179,18 @@ int sync_stream(wd_sim* s) {
     const bool lists = s->list_work;
     s->list_work = false;
     if (lists)
-        WD_CUDA(cudaMemcpyAsync(s->pinned, s->counters, sizeof(unsigned long long) * wd::kNumCounters,
-                                cudaMemcpyDeviceToHost, s->stream));
+        WD_CUDA(cudaMemcpyAsync(s->seen, s->counters, sizeof(s->seen), cudaMemcpyDeviceToHost, s->stream));
     WD_CUDA(cudaStreamSynchronize(s->stream));
     WD_CUDA(cudaGetLastError());
     if (!lists) return WD_OK;
-    if (s->pinned[wd::kCntLaunchFail]) {
+    if (s->seen[wd::kCntLaunchFail]) {
         // a list build whose device-side graph launch failed did not run
         WD_CUDA(cudaMemset(s->counters + wd::kCntLaunchFail, 0, sizeof(unsigned long long)));
         WD_CUDA(request_list_build(s));
         return fail(WD_ERR_CUDA, "list build or search: a device-side graph launch failed; the "
                                  "steps since the last synchronisation are invalid");
     }
-    if (s->pinned[wd::kCntStageTimeout]) {
+    if (s->seen[wd::kCntStageTimeout]) {
         // reported once: the handle stays usable. The step stopped part-way, so even
         // its slot order may be mixed (the first step after a build rewrites the
         // ids); the next state upload starts from a fresh slot order.
@@ -1210,14 +1202,10 @@ int sync_stream(wd_sim* s) {
     return WD_OK;
 }
 
-// Bytes of the device to the host, and the wait for them: small results by way of pinned
-// memory, which a copy reaches without staging.
+// Bytes of the device to the host, and the wait for them.
 int read_small(wd_sim* s, void* dst, const void* src, size_t bytes) {
-    void* via = bytes <= sizeof(unsigned long long) * kPinnedExtra ? s->pinned + wd::kNumCounters : dst;
-    WD_CUDA(cudaMemcpyAsync(via, src, bytes, cudaMemcpyDeviceToHost, s->stream));
-    const int rc = sync_stream(s);
-    if (rc == WD_OK && via != dst) std::memcpy(dst, via, bytes);
-    return rc;
+    WD_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s->stream));
+    return sync_stream(s);
 }
 
 // Skin of the library's own lists for a handle whose configuration has none, or 0 where
@@ -1266,12 +1254,6 @@ void auto_prepare(wd_sim* s) {
         if (e == cudaSuccess && !s->auto_load) e = dalloc(&s->auto_load, s->num_cells);
         if (e == cudaSuccess)
             e = cudaMemsetAsync(s->auto_load, 0, sizeof(uint32_t) * s->num_cells, s->stream);
-        if (e == cudaSuccess)
-            e = cudaHostAlloc(reinterpret_cast<void**>(&s->auto_word), 3 * sizeof(uint32_t), cudaHostAllocMapped);
-        if (e == cudaSuccess) {
-            std::memset(s->auto_word, 0, 3 * sizeof(uint32_t));
-            e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->auto_word_dev), s->auto_word, 0);
-        }
         // the build positions are read before a first build has written them: any in-range
         // cells are cleared then
         if (e == cudaSuccess) e = cudaMemsetAsync(s->xbuild, 0, sizeof(float4) * s->n, s->stream);
@@ -1298,10 +1280,19 @@ constexpr int64_t kAutoRun = 3;
 
 cudaError_t auto_mode(wd_sim* s, int64_t ahead) {
     if (s->auto_off > 0) --s->auto_off;
-    if (s->lists && (s->run_steps & 15) == 0 && s->auto_word) {
-        const volatile uint32_t* w = s->auto_word;
-        const uint32_t steps = w[0] - s->auto_seen[0], builds = w[1] - s->auto_seen[1];
-        if (w[2]) {
+    if (s->lists) {
+        // the device's counts come with every synchronise; without one for long, they are
+        // read after 32 list steps and then every 256
+        if (s->run_steps >= s->auto_look) {
+            s->auto_look = s->run_steps + 256;
+            cudaError_t e = cudaMemcpyAsync(s->seen, s->counters, sizeof(s->seen), cudaMemcpyDeviceToHost,
+                                            s->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+            if (e != cudaSuccess) return e;
+        }
+        const unsigned long long steps = s->seen[wd::kCntAutoSteps] - s->auto_seen[0];
+        const unsigned long long builds = s->seen[wd::kCntAutoBuilds] - s->auto_seen[1];
+        if (s->seen[wd::kCntAutoCrowded]) {
             // a cell may hold more than particles_per_cell grains: every step has to be
             // searched to count that
             s->auto_ok = false;
@@ -1322,6 +1313,7 @@ cudaError_t auto_mode(wd_sim* s, int64_t ahead) {
     }
     const bool lists = s->auto_off == 0 && (s->run_steps + ahead >= kAutoRun || s->last_run >= kAutoRun);
     const bool enter = lists && !s->lists;
+    if (enter) s->auto_look = s->run_steps + 32;
     s->lists = lists;
     return enter ? request_list_build(s) : cudaSuccess;
 }
@@ -1330,6 +1322,7 @@ cudaError_t auto_mode(wd_sim* s, int64_t ahead) {
 void note_upload(wd_sim* s) {
     if (s->run_steps > 0) s->last_run = s->run_steps;
     s->run_steps = 0;
+    s->auto_look = 32;
 }
 
 int alloc_sim(wd_sim* s) {
@@ -1376,10 +1369,11 @@ int alloc_sim(wd_sim* s) {
     WD_CUDA(dalloc(&sb.ctrl, 4));
     WD_CUDA(cudaMemset(sb.ctrl, 0, 4 * sizeof(int)));
     sb.mover_cap = wd::mover_cap(n);
-    WD_CUDA(dalloc(&sb.mv_raw, sb.mover_cap));
-    WD_CUDA(dalloc(&sb.mv_raw_slot, sb.mover_cap));
-    WD_CUDA(dalloc(&sb.mv_key, sb.mover_cap));
-    WD_CUDA(dalloc(&sb.mv_slot, sb.mover_cap));
+    const int movers = std::min(n, sb.mover_cap);
+    WD_CUDA(dalloc(&sb.mv_raw, movers));
+    WD_CUDA(dalloc(&sb.mv_raw_slot, movers));
+    WD_CUDA(dalloc(&sb.mv_key, movers));
+    WD_CUDA(dalloc(&sb.mv_slot, movers));
     WD_CUDA(dalloc(&sb.src, n));
     WD_CUDA(wd::search_prepare());
     sb.num_tiles = static_cast<int>((static_cast<int64_t>(n) + wd::kSortTile - 1) / wd::kSortTile);
@@ -1391,8 +1385,6 @@ int alloc_sim(wd_sim* s) {
     WD_CUDA(dalloc(&sb.table, s->num_cells));
     WD_CUDA(cudaMemset(sb.table, 0xFF, sizeof(int2) * s->num_cells));
     WD_CUDA(dalloc(&s->counters, wd::kNumCounters));
-    WD_CUDA(cudaMallocHost(reinterpret_cast<void**>(&s->pinned),
-                           sizeof(unsigned long long) * (wd::kNumCounters + kPinnedExtra)));
     WD_CUDA(cudaMemset(s->counters, 0, sizeof(unsigned long long) * wd::kNumCounters));
     WD_CUDA(dalloc(&s->picard_res, s->picard_iters > 0 ? s->picard_iters : 1));
     WD_CUDA(cudaMemset(s->picard_res, 0, sizeof(uint32_t) * (s->picard_iters > 0 ? s->picard_iters : 1)));
@@ -2504,7 +2496,7 @@ cudaError_t adj_replay_body(wd_sim* s, int len, bool capture, cudaStream_t st) {
         fa.hist_out = hist ? T1.hist : nullptr;
         fa.hcnt_out = hist ? s->hcnt_slot : nullptr;
         fa.counters = s->counters;
-        wd::launch_force(P, fa, false, none, st, s->force_block);
+        wd::launch_force(P, fa, false, none, st);
     }
     if (hist)
         wd::launch_counts_by_id(n, s->idsA, s->hcnt_slot,
