@@ -470,3 +470,39 @@ def test_contact_parallel_kernel_many_contacts_on_one_grain(small):
     ref, lst = _pair(cfg, state, radius, 40, 0.5e-3)
     _same(ref, lst)
     assert lst.tuning()["contact_variant"] == "warp-cooperative"
+
+
+@pytest.mark.parametrize("own", [False, True])
+@pytest.mark.parametrize("history", [False, True])
+@pytest.mark.parametrize("speed", [0.2, 3.0, 12.0])
+def test_chains_of_steps_equal_search(history, speed, own):
+    """Long advances run eight steps a graph: a build that one of them decides runs before
+    the rest, whichever step it was. Runs of many lengths (chains, single steps, both
+    parities), with builds rare to several a chain, on an explicit skin and on the
+    library's own lists."""
+    cfg, st, rad = packed_poly(n=2500, seed=55, history=history)
+    cfg.kernel_timing = False
+    st = st.copy()
+    st[:, 3:] = np.random.default_rng(56).normal(0, speed, (2500, 3))
+    ref = ParticleDynamics(cfg, state=st, radius=rad)
+    ref.set_neighbor_skin(0.0)
+    c = cfg.copy()
+    c.neighbor_skin = 0.0 if own else 0.5e-3
+    lst = ParticleDynamics(c, state=st, radius=rad)
+    for run in (129, 8, 16, 7, 64, 1, 9, 40, 3, 23, 100):
+        ref.advance(run)
+        lst.advance(run)
+        _same(ref, lst)
+        assert lst.time == ref.time
+    state = ref.get_state()
+    for sim in (ref, lst):
+        sim.dt = 0.4e-5
+        sim.set_state(state)
+        sim.advance(31)
+    _same(ref, lst)
+    if not own:
+        for kernel in ((256, 1), (128, 48), (256, 0)):
+            lst.set_contact_kernel(*kernel)
+            lst.advance(17)
+            ref.advance(17)
+            _same(ref, lst)

@@ -150,6 +150,8 @@ void launch_force(const DevParams& P, const ForceArgs& a, bool picard, Skip skip
 // tests). Picard builds earlier, at kPicardBuildAt, so that its iterates rarely leave.
 constexpr float kListValid = 0.49f;
 constexpr float kPicardBuildAt = 0.30f;
+// kLcPending / kLcLeft: a step of a chain decided a build that has not run yet; the chain's
+// steps after it.
 // kLcCrowded: the library's own lists under neighbor_skin 0, a cell may hold more than
 // particles_per_cell grains before the next build.
 // kLcStallTest / kLcWaitUs: the bulk-staged contact kernel's wait test. A nonzero
@@ -159,7 +161,7 @@ constexpr float kPicardBuildAt = 0.30f;
 enum ListCtrl {
     kLcDisp = 0, kLcOverflow = 1, kLcForce = 2, kLcDecision = 3, kLcViol = 4, kLcRedo = 5,
     kLcStep = 6, kLcExact = 7, kLcBound = 8, kLcStallTest = 10, kLcWaitUs = 11, kLcCrowded = 12,
-    kLcWords = 16
+    kLcPending = 13, kLcLeft = 14, kLcWords = 16
 };
 struct ListArgs {
     const float4* pos; const float4* vel; const int* ids;  // state of the step
@@ -181,6 +183,8 @@ struct ListArgs {
     // semi-implicit Euler: the build decision for the next step, made by the kernel's
     // last block (threshold on max |x - x_build|, block ticket, the build's IF node)
     float thr; unsigned* tail_count; int use_cond; cudaGraphConditionalHandle cond;
+    // steps of the chain from this one on (0: not in a chain)
+    int left;
     // the library's own lists: counters of the last build's gather
     unsigned long long* pend;
 };
@@ -192,6 +196,14 @@ struct ListArgs {
 // failed launch counts in counters[kCntLaunchFail].
 void launch_graph_if(const uint32_t* flag, cudaGraphExec_t graph, unsigned long long* counters,
                      cudaStream_t st);
+// The end of a chain of `steps` list steps: tail-launches the build that one of them decided,
+// if any, by whether that was an even or an odd one (from 0).
+void launch_graph_chain(const uint32_t* list_ctrl, int steps, cudaGraphExec_t even,
+                        cudaGraphExec_t odd, unsigned long long* counters, cudaStream_t st);
+// The end of a build: tail-launches the graph of the chain's steps left over, by_left[kLcLeft]
+// (device memory), if there are any, and clears kLcPending and kLcLeft.
+void launch_graph_resume(uint32_t* list_ctrl, const cudaGraphExec_t* by_left,
+                         unsigned long long* counters, cudaStream_t st);
 void launch_graph_pick(const int* flag, cudaGraphExec_t on_zero, cudaGraphExec_t on_one,
                        unsigned long long* counters, cudaStream_t st);
 void launch_list_decide(uint32_t* list_ctrl, float thr, bool always_exact,

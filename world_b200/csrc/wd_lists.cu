@@ -54,7 +54,7 @@ __device__ __forceinline__ bool skipped(const Skip& s) {
 // kCntAutoCrowded tells the host to search instead.
 __device__ bool list_decide_core(uint32_t* ctrl_, float thr, int always_exact,
                                  unsigned long long* counters, unsigned long long* pend,
-                                 bool at_step) {
+                                 bool at_step, int left) {
     volatile uint32_t* ctrl = ctrl_;
     volatile double* bound = reinterpret_cast<volatile double*>(ctrl_ + kLcBound);
     const double grow = 1.0 + 1.0 / 65536.0;
@@ -78,6 +78,9 @@ __device__ bool list_decide_core(uint32_t* ctrl_, float thr, int always_exact,
         }
     }
     ctrl[kLcDecision] = build ? __float_as_uint(1.f) : 0u;
+    // in a chain of steps (left: with this one), the rest waits for the build
+    ctrl[kLcPending] = build && left > 0 ? 1u : 0u;
+    ctrl[kLcLeft] = build && left > 0 ? static_cast<uint32_t>(left - 1) : 0u;
     if (build) {
         b = 0.0;
         ctrl[kLcOverflow] = 0u;
@@ -98,7 +101,7 @@ __global__ void k_list_decide(uint32_t* __restrict__ ctrl, float thr, int always
                               unsigned long long* __restrict__ pend, int use_cond,
                               cudaGraphConditionalHandle cond) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const bool build = list_decide_core(ctrl, thr, always_exact, counters, pend, false);
+    const bool build = list_decide_core(ctrl, thr, always_exact, counters, pend, false, 0);
     if (use_cond) cudaGraphSetConditional(cond, build ? 1u : 0u);
 }
 
@@ -152,11 +155,17 @@ __device__ __forceinline__ void list_tail_decide(const ListArgs& A) {
         if (ticket == gridDim.x - 1) {
             __threadfence();
             const bool build =
-                list_decide_core(A.list_ctrl, A.thr, 0, A.counters, A.pend, true);
+                list_decide_core(A.list_ctrl, A.thr, 0, A.counters, A.pend, true, A.left);
             *reinterpret_cast<volatile unsigned*>(A.tail_count) = 0u;
             if (A.use_cond) cudaGraphSetConditional(A.cond, build ? 1u : 0u);
         }
     }
+}
+
+// A step of a chain whose predecessor decided a build: it runs after the build instead, from
+// the graph that the build launches for the steps left over.
+__device__ __forceinline__ bool list_step_waits(const ListArgs& A) {
+    return A.left > 0 && A.list_ctrl[kLcPending] != 0u;
 }
 
 // Grains in cells two apart along an axis are more than a cell width apart, so the 27
@@ -748,7 +757,7 @@ __device__ __forceinline__ void list_grain(const DevParams& P0, const ListArgs& 
 template <bool HIST, bool BATCH, int MINB, bool PICARD>
 __global__ void __launch_bounds__(kBlock, MINB)
 k_force_list(DevParams P0, ListArgs A) {
-    if (PICARD && skipped(A.skip)) return;
+    if (PICARD ? skipped(A.skip) : list_step_waits(A)) return;
     const int n = P0.n;
     uint32_t disp_bits = 0u, step_bits = 0u;
     uint32_t res_bits = 0u;
@@ -881,6 +890,7 @@ __device__ __forceinline__ void stage_issue(const ListArgs& A, int tile, bool ex
 template <bool HIST, bool BATCH, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB)
 k_force_list_staged(DevParams P0, ListArgs A) {
+    if (list_step_waits(A)) return;
     __shared__ SlotStage stage[kStageWarps][2];
     __shared__ uint64_t bars[kStageWarps][2];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1223,6 +1233,34 @@ __device__ __forceinline__ void coop_stage(const ListArgs& A, CoopStage& S, int 
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
+// The contacts of one grain on its own lane: a list that overflowed (this step built the
+// lists, so the run table is fresh), or more contacts than one round holds. (Out of line it
+// cost the packed step 7%: the call's saved registers.)
+struct AloneResult {
+    float3 f;
+    int out_count;
+};
+template <bool HIST>
+__device__ __forceinline__ AloneResult coop_alone(const DevParams& P, const ListArgs& A, float4 pi, float4 vi,
+                                               int id, int hcnt_in, int s, int n, int cnt,
+                                               unsigned long long hits, float3 f, int out_count) {
+    HistRow h;
+    if (HIST) {
+        h.in = A.hist_in + static_cast<int64_t>(id) * kHistCap;
+        h.in_count = hcnt_in;
+        h.out = A.hist_out + static_cast<int64_t>(id) * kHistCap;
+    }
+    h.out_count = out_count;
+    const float3 vel = make_float3(vi.x, vi.y, vi.z);
+    int cx, cy, cz;
+    cell_coords(P, pi.x, pi.y, pi.z, cx, cy, cz);
+    if (cnt > kNbrCap)
+        list_contacts_table<HIST>(P, A, s, pi, vel, vi.w, contact_cutoff_sq(pi.w, P.rmax), cx, cy, cz, f, h);
+    else
+        list_contacts_sorted_mask<HIST>(P, A, s, n, hits, pi, vel, vi.w, cx, cy, cz, f, h);
+    return {f, h.out_count};
+}
+
 // One slot per group of LPG lanes (all lanes of the warp together; s may be >= n).
 template <bool HIST, bool BATCH, bool PICARD, int LPG>
 __device__ __forceinline__ void coop_slot(const DevParams& P0, const ListArgs& A, CoopWarp& W,
@@ -1232,50 +1270,42 @@ __device__ __forceinline__ void coop_slot(const DevParams& P0, const ListArgs& A
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31, sub = lane % LPG, g = lane / LPG;
     const bool live = s < n;
-    int scene = 0, id = 0, cnt = 0, hcnt_in = 0;
-    float4 pi = make_float4(0.f, 0.f, 0.f, 0.f), vi = pi;
-    if (live) {
-        scene = BATCH ? S.scene[g] : 0;
-        pi = S.pos[g];
-        vi = S.vel[g];
-        id = S.id[g];
-        cnt = S.cnt[g];
-        hcnt_in = HIST ? S.hcnt[g] : 0;
-    }
+    const int scene = BATCH && live ? S.scene[g] : 0;
     const DevParams& P = BATCH ? A.scene_params[scene] : P0;
     const bool frozen = BATCH && live && P.frozen;
     const bool own = live && sub == 0;      // the lane that carries the grain
+    const bool work = own && !frozen;
+    int cnt = live && !frozen ? S.cnt[g] : 0;
+    float3 f = make_float3(0.f, 0.f, 0.f);
+    int out_walls = 0, out_count = 0;
     if (PICARD && own) {
         // the rhs of a Picard step pairs the last iterate's velocity with its forces
-        A.rhs_vel[s] = vi;
-        A.rhs_ids[s] = id;
+        A.rhs_vel[s] = S.vel[g];
+        A.rhs_ids[s] = S.id[g];
         if (A.iter > 0) {
-            const float4 xb = A.xbuild[s];
-            const float ex = pi.x - xb.x, ey = pi.y - xb.y, ez = pi.z - xb.z;
+            const float4 xb = A.xbuild[s], x = S.pos[g];
+            const float ex = x.x - xb.x, ey = x.y - xb.y, ez = x.z - xb.z;
             viol |= !(ex * ex + ey * ey + ez * ez < A.viol_thr);
         }
     }
-    const float3 vel = make_float3(vi.x, vi.y, vi.z);
-    const float ri = pi.w, mi = vi.w;
-    float3 f = make_float3(0.f, 0.f, 0.f);
-    int out_walls = 0, out_count = 0;
-    const bool work = own && !frozen;
     if (work) {
+        const float4 x = S.pos[g], v = S.vel[g];
         HistRow h;
         if (HIST) {
-            h.in = A.hist_in + static_cast<int64_t>(id) * kHistCap;
-            h.in_count = hcnt_in;
-            h.out = A.hist_out + static_cast<int64_t>(id) * kHistCap;
+            h.in = A.hist_in + static_cast<int64_t>(S.id[g]) * kHistCap;
+            h.in_count = S.hcnt[g];
+            h.out = A.hist_out + static_cast<int64_t>(S.id[g]) * kHistCap;
             h.out_count = 0;
         }
-        wall_forces<HIST>(P, make_float3(pi.x, pi.y, pi.z), vel, ri, mi, f, h, A.counters);
+        wall_forces<HIST>(P, make_float3(x.x, x.y, x.z), make_float3(v.x, v.y, v.z), x.w, v.w, f, h,
+                          A.counters);
         if (HIST) out_walls = out_count = h.out_count;
     }
-    if (frozen) cnt = 0;
     if (__any_sync(kAll, cnt != 0)) {
         // scan: this lane's entries, four entries' loads in flight at a time
         unsigned long long hits = 0ull;
         const int scan = cnt <= kNbrCap ? cnt : 0;
+        const float4 pi = S.pos[g];
         for (int e0 = sub; e0 < scan; e0 += 4 * LPG) {
             int jj[4];
             float4 pp[4];
@@ -1295,24 +1325,11 @@ __device__ __forceinline__ void coop_slot(const DevParams& P0, const ListArgs& A
 #pragma unroll
         for (int o = 1; o < LPG; o <<= 1) hits |= __shfl_xor_sync(kAll, hits, o);
         if (cnt > kNbrCap || __popcll(hits) > 32) {
-            // a list that overflowed (this step built the lists, so the run table is fresh),
-            // or more contacts than one round holds: the grain's own lane takes them all
             if (work) {
-                HistRow h;
-                if (HIST) {
-                    h.in = A.hist_in + static_cast<int64_t>(id) * kHistCap;
-                    h.in_count = hcnt_in;
-                    h.out = A.hist_out + static_cast<int64_t>(id) * kHistCap;
-                }
-                h.out_count = out_count;
-                int cx, cy, cz;
-                cell_coords(P, pi.x, pi.y, pi.z, cx, cy, cz);
-                if (cnt > kNbrCap)
-                    list_contacts_table<HIST>(P, A, s, pi, vel, mi, contact_cutoff_sq(ri, P.rmax), cx,
-                                              cy, cz, f, h);
-                else
-                    list_contacts_sorted_mask<HIST>(P, A, s, n, hits, pi, vel, mi, cx, cy, cz, f, h);
-                out_count = h.out_count;
+                const AloneResult r = coop_alone<HIST>(P, A, S.pos[g], S.vel[g], S.id[g],
+                                                       HIST ? S.hcnt[g] : 0, s, n, cnt, hits, f, out_count);
+                f = r.f;
+                out_count = r.out_count;
             }
             hits = 0ull;
         }
@@ -1437,7 +1454,7 @@ __device__ __forceinline__ void coop_slot(const DevParams& P0, const ListArgs& A
                                             out_count, xb, exact, order_out, disp_bits,
                                             step_bits, res_bits);
     } else if (own) {
-        list_copy_frozen<HIST>(A, s, scene, pi, vi, id, order_out);
+        list_copy_frozen<HIST>(A, s, scene, S.pos[g], S.vel[g], S.id[g], order_out);
     }
 }
 
@@ -1445,8 +1462,8 @@ __device__ __forceinline__ void coop_slot(const DevParams& P0, const ListArgs& A
 // build decision waits once per resident block.
 template <bool HIST, bool BATCH, bool PICARD, int LPG>
 __global__ void __launch_bounds__(kCoopBlock, PICARD ? 6 : 8)
-k_force_list_coop(DevParams P0, ListArgs A) {
-    if (PICARD && skipped(A.skip)) return;
+k_force_list_coop(const __grid_constant__ DevParams P0, const __grid_constant__ ListArgs A) {
+    if (PICARD ? skipped(A.skip) : list_step_waits(A)) return;
     __shared__ CoopWarp warps[kCoopWarps];
     CoopWarp& W = warps[threadIdx.x >> 5];
     const int n = P0.n;
