@@ -80,7 +80,7 @@ __device__ __forceinline__ void force_walk(const DevParams& P, const ForceArgs& 
 template <bool HIST, bool PICARD, bool BATCH, bool REC, int LPG>
 __global__ void __launch_bounds__(kForceBlock, 8)
 k_force(DevParams P0, ForceArgs A, Skip skip) {
-    if (PICARD && skipped(skip)) return;
+    if (skipped(skip)) return;
     using Warp = ForceWarp<LPG>;
     constexpr unsigned kAll = 0xffffffffu;
     __shared__ Warp warps[kForceBlock / 32];

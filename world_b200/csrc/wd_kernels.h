@@ -39,7 +39,9 @@ struct SearchBuffers {
     uint32_t* moved;         // n/32 words: bit set when a slot's key changed
     int* blk_cnt;            // movers per 256-slot block
     int* blk_off;            // exclusive prefix of blk_cnt
-    int* ctrl;               // [0] mover count, [1] 1 = radix path this search, [2] movers so far
+    // [0] mover count, [1] 1 = radix path this search, [2] movers so far, [3] float: 1 where the
+    // mover path runs (what follows the search on that path is gated by it), else 0
+    int* ctrl;
     int mover_cap;
     unsigned long long* mv_raw;  // mover_cap: (key << 32 | id) of each mover, in any order
     uint32_t* mv_raw_slot;   // mover_cap: its state slot
@@ -201,11 +203,11 @@ void launch_graph_if(const uint32_t* flag, cudaGraphExec_t graph, unsigned long 
 void launch_graph_chain(const uint32_t* list_ctrl, int steps, cudaGraphExec_t even,
                         cudaGraphExec_t odd, unsigned long long* counters, cudaStream_t st);
 // The end of a build: tail-launches the graph of the chain's steps left over, by_left[kLcLeft]
-// (device memory), if there are any, and clears kLcPending and kLcLeft.
-void launch_graph_resume(uint32_t* list_ctrl, const cudaGraphExec_t* by_left,
-                         unsigned long long* counters, cudaStream_t st);
-void launch_graph_pick(const int* flag, cudaGraphExec_t on_zero, cudaGraphExec_t on_one,
-                       unsigned long long* counters, cudaStream_t st);
+// (device memory), if there are any, and clears kLcPending and kLcLeft; where the search
+// wants the radix path (radix_flag nonzero; NULL on that path itself), the graph that builds
+// that way instead. by_left NULL: no chain waits for this build.
+void launch_build_end(uint32_t* list_ctrl, const cudaGraphExec_t* by_left, const int* radix_flag,
+                      cudaGraphExec_t radix, unsigned long long* counters, cudaStream_t st);
 void launch_list_decide(uint32_t* list_ctrl, float thr, bool always_exact,
                         unsigned long long* counters, unsigned long long* pend, bool use_cond, cudaGraphConditionalHandle cond, cudaStream_t st);
 // The library's own lists under neighbor_skin 0: counts, per collision cell, the grains of

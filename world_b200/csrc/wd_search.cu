@@ -326,6 +326,7 @@ k_movers(int n, const int* __restrict__ blk_cnt, int* __restrict__ blk_off, int 
             blk_off[num_blocks] = m;
             ctrl[0] = m;
             ctrl[1] = full;
+            ctrl[3] = __float_as_int(full ? 0.f : 1.f);
             if (use_cond) cudaGraphSetConditional(cond, static_cast<unsigned>(full));
             if (full) atomicAdd(&counters[kCntRadixSearches], 1ull);
         }

@@ -230,19 +230,18 @@ struct wd_sim {
     // Step graphs, captured when first needed, by what their nodes' pointers depend on: the
     // mode (searched or on lists), which buffers are A (lpar) and the spring parity
     // (hist_cur). Each keeps the device-launchable graphs that its kernels tail-launch:
-    //   on lists (semi-implicit Euler): the list build -- the search head (keys, mover
-    //     sort), then the mover path (merge) or the radix path, each followed by the
-    //     gather and the listing; the contact kernel's successor launches the head when a
-    //     build was decided, the mover kernel's the rest;
-    //   searched: the rest of the step after the search head, the mover path or the radix
-    //     path, each followed by the gather and the contact kernel.
+    //   on lists (semi-implicit Euler): the list build (head), which the contact kernel's
+    //     successor launches when one was decided: the search's mover path, the gather and
+    //     the listing, and in a graph of its own (radix) the same by way of the radix path;
+    //   searched: the rest of the step by way of the radix path (radix), which the step's
+    //     last kernel launches when the mover kernel asked for it.
     struct StepGraph {
         cudaGraphExec_t step = nullptr;
         cudaGraphExec_t build_if = nullptr;   // on lists: the launcher of the build alone
-        cudaGraphExec_t head = nullptr, mover = nullptr, radix = nullptr;
+        cudaGraphExec_t head = nullptr, radix = nullptr;
         // on lists: the build of the state in A, launched from the host (graphs of its own:
         // one that the device may yet launch is not launched from the host)
-        cudaGraphExec_t now_head = nullptr, now_mover = nullptr, now_radix = nullptr;
+        cudaGraphExec_t now_head = nullptr, now_radix = nullptr;
     };
     StepGraph graphs[8];
     bool built_now = false;   // a host-requested build has run before
@@ -256,7 +255,7 @@ struct wd_sim {
     int64_t list_steps = 0;
     // the on-demand search (energy, probes) per buffer parity
     struct SearchGraph {
-        cudaGraphExec_t head = nullptr, mover = nullptr, radix = nullptr;
+        cudaGraphExec_t head = nullptr, radix = nullptr;
         bool seen = false, failed = false;
     };
     SearchGraph search_graph[2];
@@ -278,7 +277,7 @@ void clear_adj_graphs(wd_sim* s) {
 }
 
 void drop_search_graph(wd_sim::SearchGraph& g) {
-    for (cudaGraphExec_t x : {g.head, g.mover, g.radix})
+    for (cudaGraphExec_t x : {g.head, g.radix})
         if (x) cudaGraphExecDestroy(x);
     g = wd_sim::SearchGraph{};
 }
@@ -288,8 +287,7 @@ void destroy_graphs(wd_sim* s) {
     if (s->stream) cudaStreamSynchronize(s->stream);
     clear_adj_graphs(s);
     for (auto& g : s->graphs) {
-        for (cudaGraphExec_t x : {g.step, g.build_if, g.head, g.mover, g.radix, g.now_head, g.now_mover,
-                                  g.now_radix})
+        for (cudaGraphExec_t x : {g.step, g.build_if, g.head, g.radix, g.now_head, g.now_radix})
             if (x) cudaGraphExecDestroy(x);
         g = wd_sim::StepGraph{};
     }
@@ -568,21 +566,26 @@ wd::ForceArgs step_force_args(wd_sim* s, int parity) {
     return fa;
 }
 
+// Gate of what follows a search on its mover path: closed when the search wants the radix
+// sort, whose graph then does it all.
+wd::Skip mover_gate(const wd_sim* s) {
+    return wd::Skip{reinterpret_cast<const uint32_t*>(s->sb.ctrl + 3), 0.5f};
+}
+
 // A searched semi-implicit Euler step after its search: gather into the new order (B),
 // then the contact kernel (B -> A).
-void enqueue_step_tail(wd_sim* s, int parity, cudaStream_t st, cudaEvent_t mid) {
+void enqueue_step_tail(wd_sim* s, int parity, cudaStream_t st, cudaEvent_t mid, wd::Skip gate) {
     const DevParams& P = s->P;
     const bool hist = P.history != 0, batch = s->scenes > 1;
-    const wd::Skip none{nullptr, 0.f};
     wd::launch_gather(P, s->sb, s->posA, s->velA, s->posB, s->velB, s->idsB, nullptr, nullptr,
                       nullptr, nullptr, false, hist ? s->hcnt_slot : nullptr,
                       hist ? s->hcnt_g : nullptr, batch ? s->sceneA : nullptr,
                       batch ? s->sceneB : nullptr, true, s->counters, s->scene_overflow,
-                      s->d_scene_P, none, st);
+                      s->d_scene_P, gate, st);
     if (mid) cudaEventRecord(mid, st);
     wd::ForceArgs fa = step_force_args(s, parity);
     fa.hcnt_in = s->hcnt_g;
-    wd::launch_force(P, fa, false, none, st);
+    wd::launch_force(P, fa, false, gate, st);
 }
 
 cudaError_t enqueue_step(wd_sim* s, int parity, cudaStream_t st, bool capture,
@@ -602,17 +605,19 @@ cudaError_t enqueue_step(wd_sim* s, int parity, cudaStream_t st, bool capture,
     fa.scene_out = s->sceneA;
     const wd::Skip none{nullptr, 0.f};
     if (!s->picard) {
-        if (capture && s->graph_now().mover != nullptr) {
-            // the search head here, the rest of the step tail-launched from the device
+        if (capture && s->graph_now().radix != nullptr) {
+            // the mover path here, gated; the radix path tail-launched from the device
             wd::launch_search_head(P, tab(s, s->sceneA), s->posA, s->idsA, s->sb, none, nullptr,
                                    0, false, 0, s->counters, st);
-            wd::launch_graph_pick(s->sb.ctrl + 1, s->graph_now().mover, s->graph_now().radix,
-                                  s->counters, st);
+            wd::launch_search_merge(P, s->idsA, s->sb, none, st);
+            enqueue_step_tail(s, parity, st, nullptr, mover_gate(s));
+            wd::launch_graph_if(reinterpret_cast<const uint32_t*>(s->sb.ctrl + 1),
+                                s->graph_now().radix, s->counters, st);
             return cudaGetLastError();
         }
         cudaError_t e = enqueue_search(s, none, nullptr, 0, capture, st);
         if (e != cudaSuccess) return e;
-        enqueue_step_tail(s, parity, st, mid);
+        enqueue_step_tail(s, parity, st, mid, none);
         return cudaGetLastError();
     }
     for (int k = 0; k < s->picard_iters; ++k) {
@@ -878,37 +883,33 @@ cudaError_t capture_device_graph(wd_sim* s, cudaGraphExec_t* out, Body body) {
 }
 
 void drop_device_graphs(wd_sim::StepGraph& g) {
-    for (cudaGraphExec_t* x : {&g.build_if, &g.head, &g.mover, &g.radix}) {
+    for (cudaGraphExec_t* x : {&g.build_if, &g.head, &g.radix}) {
         if (*x) cudaGraphExecDestroy(*x);
         *x = nullptr;
     }
     cudaGetLastError();
 }
 
-// The list build of the state in A as three device graphs: the head, which launches one of
-// the other two.
+// The list build of the state in A as two device graphs: the head, with the search's mover
+// path, and the same by way of the radix path, which the head launches when it has to.
 // resume: device table of the graphs that take up a chain's steps after the build, or NULL.
-cudaError_t capture_build(wd_sim* s, cudaGraphExec_t* head, cudaGraphExec_t* mover,
-                          cudaGraphExec_t* radix, const cudaGraphExec_t* resume) {
+cudaError_t capture_build(wd_sim* s, cudaGraphExec_t* head, cudaGraphExec_t* radix,
+                          const cudaGraphExec_t* resume) {
     const DevParams& P = s->P;
     const wd::Skip none{nullptr, 0.f};
-    cudaError_t e = capture_device_graph(s, mover, [&](cudaStream_t st) {
-        wd::launch_search_merge(P, s->idsA, s->sb, none, st);
+    cudaError_t e = capture_device_graph(s, radix, [&](cudaStream_t st) {
+        wd::launch_search_radix(P, s->idsA, s->sb, none, st);
         enqueue_list_build_tail(s, none, st);
-        if (resume) wd::launch_graph_resume(s->list_ctrl, resume, s->counters, st);
+        if (resume)
+            wd::launch_build_end(s->list_ctrl, resume, nullptr, nullptr, s->counters, st);
     });
-    if (e == cudaSuccess)
-        e = capture_device_graph(s, radix, [&](cudaStream_t st) {
-            wd::launch_search_radix(P, s->idsA, s->sb, none, st);
-            enqueue_list_build_tail(s, none, st);
-            if (resume) wd::launch_graph_resume(s->list_ctrl, resume, s->counters, st);
-        });
     if (e == cudaSuccess)
         e = capture_device_graph(s, head, [&](cudaStream_t st) {
             wd::launch_search_head(P, tab(s, s->sceneA), s->posA, s->idsA, s->sb, none, nullptr,
                                    0, false, 0, s->counters, st);
-            // the path the mover kernel picked (ctrl[1]: the radix sort)
-            wd::launch_graph_pick(s->sb.ctrl + 1, *mover, *radix, s->counters, st);
+            wd::launch_search_merge(P, s->idsA, s->sb, none, st);
+            enqueue_list_build_tail(s, mover_gate(s), st);
+            wd::launch_build_end(s->list_ctrl, resume, s->sb.ctrl + 1, *radix, s->counters, st);
         });
     return e;
 }
@@ -925,7 +926,7 @@ cudaError_t capture_device_builds(wd_sim* s) {
         e = dalloc(&s->chain_table, 4 * 8);
         if (e == cudaSuccess) e = cudaMemset(s->chain_table, 0, 4 * 8 * sizeof(cudaGraphExec_t));
     }
-    if (e == cudaSuccess) e = capture_build(s, &g.head, &g.mover, &g.radix, s->chain_table + 8 * next);
+    if (e == cudaSuccess) e = capture_build(s, &g.head, &g.radix, s->chain_table + 8 * next);
     if (e == cudaSuccess)
         e = capture_device_graph(s, &g.build_if, [&](cudaStream_t st) {
             wd::launch_graph_if(s->list_ctrl + wd::kLcDecision, g.head, s->counters, st);
@@ -935,21 +936,16 @@ cudaError_t capture_device_builds(wd_sim* s) {
     return e;
 }
 
-// The rest of a searched step from the current buffers as device graphs. On failure none
-// is kept and the step graph holds the radix path in a conditional node.
+// The rest of a searched step from the current buffers on the radix path as a device graph.
+// On failure it is not kept and the step graph holds the radix path in a conditional node.
 cudaError_t capture_device_search_steps(wd_sim* s, int parity) {
     const DevParams& P = s->P;
     const wd::Skip none{nullptr, 0.f};
     wd_sim::StepGraph& g = s->graph_now();
-    cudaError_t e = capture_device_graph(s, &g.mover, [&](cudaStream_t st) {
-        wd::launch_search_merge(P, s->idsA, s->sb, none, st);
-        enqueue_step_tail(s, parity, st, nullptr);
+    cudaError_t e = capture_device_graph(s, &g.radix, [&](cudaStream_t st) {
+        wd::launch_search_radix(P, s->idsA, s->sb, none, st);
+        enqueue_step_tail(s, parity, st, nullptr, none);
     });
-    if (e == cudaSuccess)
-        e = capture_device_graph(s, &g.radix, [&](cudaStream_t st) {
-            wd::launch_search_radix(P, s->idsA, s->sb, none, st);
-            enqueue_step_tail(s, parity, st, nullptr);
-        });
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux_stream);
     if (e != cudaSuccess) drop_device_graphs(g);
     return e;
@@ -1023,10 +1019,10 @@ cudaError_t enqueue_pending_build(wd_sim* s, cudaStream_t st) {
     // graphs (directly, gated: about 18 launches, most of them idle; 2^20 grains 0.05 ms).
     if (s->built_now && !s->graph_dirty && s->graphs[4 + 2 * s->lpar].now_head == nullptr) {
         wd_sim::StepGraph& g = s->graphs[4 + 2 * s->lpar];
-        cudaError_t e = capture_build(s, &g.now_head, &g.now_mover, &g.now_radix, nullptr);
+        cudaError_t e = capture_build(s, &g.now_head, &g.now_radix, nullptr);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux_stream);
         if (e != cudaSuccess) {
-            for (cudaGraphExec_t* x : {&g.now_head, &g.now_mover, &g.now_radix}) {
+            for (cudaGraphExec_t* x : {&g.now_head, &g.now_radix}) {
                 if (*x) cudaGraphExecDestroy(*x);
                 *x = nullptr;
             }
@@ -1058,7 +1054,7 @@ int ensure_graph(wd_sim* s, bool launcher_only = false) {
     const int parity = s->P.history ? s->hist_cur : 0;
     // semi-implicit Euler: the build, or the rest of a searched step, as device-launched
     // graphs (kept only when they instantiate; otherwise the step graph holds an IF node)
-    if (!s->picard && !sg.head && !sg.mover) {
+    if (!s->picard && !sg.head && !sg.radix) {
         if (s->lists) capture_device_builds(s);
         else capture_device_search_steps(s, parity);
     }
@@ -1255,17 +1251,17 @@ cudaError_t alloc_c_buffers(wd_sim* s) {
     return e;
 }
 
-void enqueue_gather_c(wd_sim* s, cudaStream_t st) {
+void enqueue_gather_c(wd_sim* s, cudaStream_t st, wd::Skip gate) {
     const bool batch = s->scenes > 1;
     wd::launch_gather(s->P, s->sb, s->posA, s->velA, s->posC, s->velC, s->idsC, nullptr, nullptr,
                       nullptr, nullptr, false, nullptr, nullptr, batch ? s->sceneA : nullptr,
                       batch ? s->sceneC : nullptr, false, s->counters, s->scene_overflow,
-                      s->d_scene_P, wd::Skip{nullptr, 0.f}, st);
+                      s->d_scene_P, gate, st);
 }
 
 // Search on the current state into the C buffers (energy, probes). From the second on (per
-// buffer parity) it is one launch of device graphs: the head, which launches the mover or
-// the radix path with the gather; directly it is 8 to 17 launches, the idle path's among
+// buffer parity) it is one launch of a device graph, which launches another for
+// the radix path when it has to; directly it is 8 to 17 launches, the idle path's among
 // them.
 int ondemand_search(wd_sim* s) {
     WD_CUDA(alloc_c_buffers(s));
@@ -1276,20 +1272,19 @@ int ondemand_search(wd_sim* s) {
     }
     wd_sim::SearchGraph& g = s->search_graph[s->lpar];
     if (g.seen && !g.head && !g.failed) {
-        cudaError_t e = capture_device_graph(s, &g.mover, [&](cudaStream_t st) {
-            wd::launch_search_merge(s->P, s->idsA, s->sb, none, st);
-            enqueue_gather_c(s, st);
+        const wd::Skip gate = mover_gate(s);
+        cudaError_t e = capture_device_graph(s, &g.radix, [&](cudaStream_t st) {
+            wd::launch_search_radix(s->P, s->idsA, s->sb, none, st);
+            enqueue_gather_c(s, st, none);
         });
-        if (e == cudaSuccess)
-            e = capture_device_graph(s, &g.radix, [&](cudaStream_t st) {
-                wd::launch_search_radix(s->P, s->idsA, s->sb, none, st);
-                enqueue_gather_c(s, st);
-            });
         if (e == cudaSuccess)
             e = capture_device_graph(s, &g.head, [&](cudaStream_t st) {
                 wd::launch_search_head(s->P, tab(s, s->sceneA), s->posA, s->idsA, s->sb, none, nullptr,
                                        0, false, 0, s->counters, st);
-                wd::launch_graph_pick(s->sb.ctrl + 1, g.mover, g.radix, s->counters, st);
+                wd::launch_search_merge(s->P, s->idsA, s->sb, none, st);
+                enqueue_gather_c(s, st, gate);
+                wd::launch_graph_if(reinterpret_cast<const uint32_t*>(s->sb.ctrl + 1), g.radix,
+                                    s->counters, st);
             });
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux_stream);
         if (e != cudaSuccess) {
@@ -1306,7 +1301,7 @@ int ondemand_search(wd_sim* s) {
     }
     wd::launch_search(s->P, tab(s, s->sceneA), s->posA, s->idsA, s->sb, none, nullptr, 0,
                       s->counters, s->stream);
-    enqueue_gather_c(s, s->stream);
+    enqueue_gather_c(s, s->stream, none);
     WD_CUDA(cudaGetLastError());
     return WD_OK;
 }
@@ -2438,7 +2433,7 @@ int wd_set_kernel_timing(wd_sim* sim, int32_t enabled) {
 // Whether the step graphs of the current mode hand work to device-launched graphs.
 static bool device_graphs(const wd_sim* sim) {
     for (int k = 0; k < 4; ++k)
-        if (sim->graphs[(sim->lists ? 4 : 0) + k].mover != nullptr) return true;
+        if (sim->graphs[(sim->lists ? 4 : 0) + k].radix != nullptr) return true;
     return false;
 }
 
