@@ -44,32 +44,37 @@ __device__ __forceinline__ bool skipped(const Skip& s) {
 // next kernel measures exactly when B is within two last-step displacements of the
 // threshold, so a build is triggered by the bound only when the exact value is close.
 // A NaN or infinite displacement makes B infinite: the step builds.
-// One thread. Volatile accesses: the fused form runs in the last block of a contact
-// kernel whose other blocks updated these words with atomics.
+// One thread. The fused form runs in the last block of a contact kernel whose other blocks
+// updated these words with atomics: all of them are read from L2, at once, before anything is
+// decided (read one after another as they were needed, they held every step up by five round
+// trips: 12.3 against 11.1 us a step for 32768 grains).
 // pend: non-null for the library's own lists under neighbor_skin 0, whose searched steps
 // count a (cell, search) incident whenever a cell holds more than particles_per_cell grains.
 // A build counts them of the state it sorts into pend; they are due when the next step
 // starts from that state, here at its end (`step`). Between builds there are none unless the
 // build found a cell that could fill up (kLcCrowded): then every step builds, and
 // kCntAutoCrowded tells the host to search instead.
-__device__ bool list_decide_core(uint32_t* ctrl_, float thr, int always_exact,
+__device__ bool list_decide_core(uint32_t* ctrl, float thr, int always_exact,
                                  unsigned long long* counters, unsigned long long* pend,
                                  bool at_step, int left) {
-    volatile uint32_t* ctrl = ctrl_;
-    volatile double* bound = reinterpret_cast<volatile double*>(ctrl_ + kLcBound);
+    static_assert(kLcDisp == 0 && kLcOverflow == 1 && kLcForce == 2 && kLcStep == 6 &&
+                      kLcExact == 7 && kLcBound == 8 && kLcCrowded == 12, "read as vectors");
+    const uint4 w0 = __ldcg(reinterpret_cast<const uint4*>(ctrl));
+    const uint4 w1 = __ldcg(reinterpret_cast<const uint4*>(ctrl + 4));
+    const double bound = __ldcg(reinterpret_cast<const double*>(ctrl + kLcBound));
+    const bool crowded = pend != nullptr && __ldcg(ctrl + kLcCrowded) != 0u;
+    const unsigned long long overflow = pend != nullptr && at_step ? __ldcg(pend + kCntGridOverflow) : 0ull;
     const double grow = 1.0 + 1.0 / 65536.0;
-    const double step = sqrt(static_cast<double>(__uint_as_float(ctrl[kLcStep]))) * grow;
-    double b = ctrl[kLcExact] != 0u
-                   ? sqrt(static_cast<double>(__uint_as_float(ctrl[kLcDisp]))) * grow
-                   : *bound + step;
-    bool build = ctrl[kLcForce] != 0u || ctrl[kLcOverflow] != 0u || !(b < thr);
+    const double step = sqrt(static_cast<double>(__uint_as_float(w1.z))) * grow;
+    const double disp = sqrt(static_cast<double>(__uint_as_float(w0.x))) * grow;
+    double b = w1.w != 0u ? disp : bound + step;
+    bool build = w0.z != 0u || w0.y != 0u || !(b < thr);
     if (pend != nullptr) {
-        const bool crowded = ctrl[kLcCrowded] != 0u;
         if (at_step) {
-            counters[kCntGridOverflow] += pend[kCntGridOverflow];
             build |= crowded;
-            counters[kCntAutoSteps] += 1ull;
-            if (build) counters[kCntAutoBuilds] += 1ull;
+            if (overflow) atomicAdd(&counters[kCntGridOverflow], overflow);
+            atomicAdd(&counters[kCntAutoSteps], 1ull);
+            if (build) atomicAdd(&counters[kCntAutoBuilds], 1ull);
             if (crowded) counters[kCntAutoCrowded] = 1ull;
         }
         if (build) {
@@ -85,14 +90,14 @@ __device__ bool list_decide_core(uint32_t* ctrl_, float thr, int always_exact,
         b = 0.0;
         ctrl[kLcOverflow] = 0u;
         ctrl[kLcForce] = 0u;
-        if (pend == nullptr) counters[kCntListBuilds] += 1ull;
+        if (pend == nullptr) atomicAdd(&counters[kCntListBuilds], 1ull);
     }
-    *bound = b;
+    *reinterpret_cast<double*>(ctrl + kLcBound) = b;
     ctrl[kLcDisp] = 0u;
     ctrl[kLcStep] = 0u;
     const bool exact = always_exact || (!build && !(b + 2.0 * step < thr));
     ctrl[kLcExact] = exact ? 1u : 0u;
-    if (exact && pend == nullptr) counters[kCntListExact] += 1ull;
+    if (exact && pend == nullptr) atomicAdd(&counters[kCntListExact], 1ull);
     return build;
 }
 
@@ -145,18 +150,33 @@ k_cell_load(DevParams P, const float4* __restrict__ pos, uint32_t* __restrict__ 
 // rebuilt before the next step: it switches the build's conditional node where the step
 // graph holds one, or leaves the decision word to the kernel that launches the build's
 // graphs from the device (wd_launch.cu). All threads
-// of every block call it. The barrier orders the block's atomics before thread 0's
-// fence and ticket (the grid-barrier pattern: one fence per block, not per thread).
-__device__ __forceinline__ void list_tail_decide(const ListArgs& A) {
+// of every block call it, with their displacement maxima. The block's maxima meet in shared
+// memory first (one atomic a block and word instead of one a warp: 4736 at one address), and
+// thread 0's fence orders its atomics before its ticket.
+__device__ __forceinline__ void list_tail_decide(const ListArgs& A, bool exact, uint32_t disp_bits,
+                                                 uint32_t step_bits) {
+    __shared__ uint32_t top[kBlock / 32][2];
+    disp_bits = exact ? __reduce_max_sync(0xffffffffu, disp_bits) : 0u;
+    step_bits = __reduce_max_sync(0xffffffffu, step_bits);
+    if ((threadIdx.x & 31) == 0) {
+        top[threadIdx.x >> 5][0] = disp_bits;
+        top[threadIdx.x >> 5][1] = step_bits;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
+        for (int w = 1; w < static_cast<int>(blockDim.x) / 32; ++w) {
+            disp_bits = max(disp_bits, top[w][0]);
+            step_bits = max(step_bits, top[w][1]);
+        }
+        if (disp_bits != 0u) atomicMax(&A.list_ctrl[kLcDisp], disp_bits);
+        if (step_bits != 0u) atomicMax(&A.list_ctrl[kLcStep], step_bits);
         __threadfence();
         const unsigned ticket = atomicAdd(A.tail_count, 1u);
         if (ticket == gridDim.x - 1) {
             __threadfence();
             const bool build =
                 list_decide_core(A.list_ctrl, A.thr, 0, A.counters, A.pend, true, A.left);
-            *reinterpret_cast<volatile unsigned*>(A.tail_count) = 0u;
+            *A.tail_count = 0u;
             if (A.use_cond) cudaGraphSetConditional(A.cond, build ? 1u : 0u);
         }
     }
@@ -466,23 +486,10 @@ __device__ __forceinline__ uint32_t disp_sq_bits(float3 x1, float4 x0) {
     return disp_sq_bits(x1, make_float3(x0.x, x0.y, x0.z));
 }
 
-// Warp maxima of the displacement measures into list_ctrl (the exact one only on the
-// steps that measure it; the per-step one for semi-implicit Euler).
-template <bool PICARD>
-__device__ __forceinline__ void list_disp_report(uint32_t* ctrl, bool exact, uint32_t disp_bits,
-                                                 uint32_t step_bits) {
-    if (exact) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            disp_bits = max(disp_bits, __shfl_xor_sync(0xffffffffu, disp_bits, o));
-        if ((threadIdx.x & 31) == 0 && disp_bits != 0u) atomicMax(&ctrl[kLcDisp], disp_bits);
-    }
-    if (!PICARD) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            step_bits = max(step_bits, __shfl_xor_sync(0xffffffffu, step_bits, o));
-        if ((threadIdx.x & 31) == 0 && step_bits != 0u) atomicMax(&ctrl[kLcStep], step_bits);
-    }
+// Warp maxima of a Picard iteration's displacements from the build into list_ctrl.
+__device__ __forceinline__ void list_disp_report(uint32_t* ctrl, uint32_t disp_bits) {
+    disp_bits = __reduce_max_sync(0xffffffffu, disp_bits);
+    if ((threadIdx.x & 31) == 0 && disp_bits != 0u) atomicMax(&ctrl[kLcDisp], disp_bits);
 }
 
 // Asks L1 for the line holding p; nothing is read into registers, so a later __ldg of
@@ -791,9 +798,12 @@ k_force_list(DevParams P0, ListArgs A) {
                 P0, A, s, n, scene, pi, vi, id, cnt, xb, hcnt_in, exact, order_out, warp_listed,
                 disp_bits, step_bits, res_bits, viol);
     }
-    list_disp_report<PICARD>(A.list_ctrl, exact, disp_bits, step_bits);
-    if (!PICARD) list_tail_decide(A);
-    if (PICARD) list_picard_report(A, res_bits, viol);
+    if (PICARD) {
+        list_disp_report(A.list_ctrl, disp_bits);
+        list_picard_report(A, res_bits, viol);
+    } else {
+        list_tail_decide(A, exact, disp_bits, step_bits);
+    }
 }
 
 // ---- bulk-staged list kernel -------------------------------------------------------
@@ -977,10 +987,9 @@ k_force_list_staged(DevParams P0, ListArgs A) {
             if (cur < whole) mbar_wait(&bar[it & 1], (it >> 1) & 1, limit_ns);
             if (nxt < whole) mbar_wait(&bar[(it + 1) & 1], ((it + 1) >> 1) & 1, limit_ns);
         }
-    } else {
-        list_disp_report<false>(A.list_ctrl, exact, disp_bits, step_bits);
+        disp_bits = step_bits = 0u;   // and its displacements unreported
     }
-    list_tail_decide(A);
+    list_tail_decide(A, exact, disp_bits, step_bits);
 }
 
 // ---- list build with the tile's neighbour window staged in shared memory ----------
@@ -1463,10 +1472,11 @@ __device__ __forceinline__ void coop_slot(const DevParams& P0, const ListArgs& A
 template <bool HIST, bool BATCH, bool PICARD, int LPG>
 __global__ void __launch_bounds__(kCoopBlock, PICARD ? 6 : 8)
 k_force_list_coop(const __grid_constant__ DevParams P0, const __grid_constant__ ListArgs A) {
-    if (PICARD ? skipped(A.skip) : list_step_waits(A)) return;
+    if (PICARD && skipped(A.skip)) return;
     __shared__ CoopWarp warps[kCoopWarps];
     CoopWarp& W = warps[threadIdx.x >> 5];
     const int n = P0.n;
+    const bool waits = !PICARD && list_step_waits(A);
     const bool exact = PICARD || A.list_ctrl[kLcExact] != 0u;
     const bool order_out = PICARD || A.list_ctrl[kLcDecision] != 0u;  // first step after a build
     uint32_t disp_bits = 0u, step_bits = 0u, res_bits = 0u;
@@ -1476,6 +1486,11 @@ k_force_list_coop(const __grid_constant__ DevParams P0, const __grid_constant__ 
     const int stride = gridDim.x * per;
     int s = blockIdx.x * per + static_cast<int>(threadIdx.x) / LPG;
     coop_stage<HIST, BATCH, LPG>(A, W.stage[0], s, n);
+    if (waits) {
+        // (asked after the first copies are issued: one round trip less before the work)
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        return;
+    }
     int st = 0;
     for (int base = blockIdx.x * per; base < n; base += stride, s += stride, st ^= 1) {
         __syncwarp();                       // the other stage has been read
@@ -1486,9 +1501,12 @@ k_force_list_coop(const __grid_constant__ DevParams P0, const __grid_constant__ 
                                             step_bits, res_bits, viol);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    list_disp_report<PICARD>(A.list_ctrl, exact, disp_bits, step_bits);
-    if (PICARD) list_picard_report(A, res_bits, viol);
-    else list_tail_decide(A);
+    if (PICARD) {
+        list_disp_report(A.list_ctrl, disp_bits);
+        list_picard_report(A, res_bits, viol);
+    } else {
+        list_tail_decide(A, exact, disp_bits, step_bits);
+    }
 }
 
 __global__ void __launch_bounds__(kBlock)
