@@ -1200,7 +1200,10 @@ __global__ void k_list_picard_check(uint32_t* __restrict__ ctrl,
 // for the busiest: a few hundred such grains in a million set the kernel's time.)
 //
 // The slots' own values come through shared memory by asynchronous copies issued one
-// group ahead, which hides their latency without holding registers.
+// group ahead, which hides their latency without holding registers. What the stages take of
+// the SM's 256 KB L1 loses: with 16.6 KB a block (the 164 KB carve-out) the steps of large
+// scenes took 1% longer than with 15.6 KB (132 KB), with 20.7 KB (list entries staged too,
+// 196 KB) 5% longer. Only batches stage the scene.
 //
 // Bound by load latency and issue. Measured at 64 registers, 8 blocks per SM (80 and 6 for
 // Picard, whose grid is not one wave of equal work): 2^20 falling grains 41.3 us a step
@@ -1209,12 +1212,21 @@ __global__ void k_list_picard_check(uint32_t* __restrict__ ctrl,
 constexpr int kCoopBlock = 128;
 constexpr int kCoopWarps = kCoopBlock / 32;
 
+template <bool BATCH>
 struct __align__(16) CoopStage {
     float4 pos[32], vel[32];
-    int id[32], cnt[32], hcnt[32], scene[32];
+    int id[32], cnt[32], hcnt[32];
+    int scene[BATCH ? 32 : 1];
 };
+template <>
+struct __align__(16) CoopStage<false> {
+    float4 pos[32], vel[32];
+    int id[32], cnt[32], hcnt[32];
+    static constexpr int* scene = nullptr;
+};
+template <bool BATCH>
 struct __align__(16) CoopWarp {
-    CoopStage stage[2];
+    CoopStage<BATCH> stage[2];
     float4 term[32][2];            // (nrm, fp), (t, cvn)
     unsigned short queue[32];      // owner lane << 6 | list entry
 };
@@ -1229,7 +1241,7 @@ __device__ __forceinline__ void async_copy4(void* dst, const void* src) {
 // This lane's share of the copies of one slot group into S: the lane that carries grain s
 // copies its values. One copy group per call, possibly empty.
 template <bool HIST, bool BATCH, int LPG>
-__device__ __forceinline__ void coop_stage(const ListArgs& A, CoopStage& S, int s, int n) {
+__device__ __forceinline__ void coop_stage(const ListArgs& A, CoopStage<BATCH>& S, int s, int n) {
     const int lane = threadIdx.x & 31, g = lane / LPG;
     if (lane % LPG == 0 && s < n) {
         async_copy16(&S.pos[g], &A.pos[s]);
@@ -1272,8 +1284,8 @@ __device__ __forceinline__ AloneResult coop_alone(const DevParams& P, const List
 
 // One slot per group of LPG lanes (all lanes of the warp together; s may be >= n).
 template <bool HIST, bool BATCH, bool PICARD, int LPG>
-__device__ __forceinline__ void coop_slot(const DevParams& P0, const ListArgs& A, CoopWarp& W,
-                                          const CoopStage& S, int s, int n, bool exact,
+__device__ __forceinline__ void coop_slot(const DevParams& P0, const ListArgs& A, CoopWarp<BATCH>& W,
+                                          const CoopStage<BATCH>& S, int s, int n, bool exact,
                                           bool order_out, uint32_t& disp_bits, uint32_t& step_bits,
                                           uint32_t& res_bits, bool& viol) {
     constexpr unsigned kAll = 0xffffffffu;
@@ -1473,8 +1485,8 @@ template <bool HIST, bool BATCH, bool PICARD, int LPG>
 __global__ void __launch_bounds__(kCoopBlock, PICARD ? 6 : 8)
 k_force_list_coop(const __grid_constant__ DevParams P0, const __grid_constant__ ListArgs A) {
     if (PICARD && skipped(A.skip)) return;
-    __shared__ CoopWarp warps[kCoopWarps];
-    CoopWarp& W = warps[threadIdx.x >> 5];
+    __shared__ CoopWarp<BATCH> warps[kCoopWarps];
+    CoopWarp<BATCH>& W = warps[threadIdx.x >> 5];
     const int n = P0.n;
     const bool waits = !PICARD && list_step_waits(A);
     const bool exact = PICARD || A.list_ctrl[kLcExact] != 0u;
