@@ -506,3 +506,16 @@ def test_chains_of_steps_equal_search(history, speed, own):
             lst.advance(17)
             ref.advance(17)
             _same(ref, lst)
+
+
+@pytest.mark.parametrize("n", [16383, 16384, 75776, 75777])
+def test_chains_launched_early_equal_search(n):
+    """A chain's steps are launched while the step before still runs where two grids of the
+    contact kernel fit the chip at once (75,776 grains on 148 SMs), else after it: both sides
+    of that line and of the lanes-per-grain rule, with builds inside chains."""
+    cfg, st, rad = _roomy(n, 57, 0.5, True)
+    st = st.copy()
+    st[:, 3:] *= 5
+    ref, lst = _pair(cfg, st, rad, 200, 0.5e-3)
+    _same(ref, lst)
+    assert lst.list_stats()[0] > 2

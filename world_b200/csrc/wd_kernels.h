@@ -185,8 +185,9 @@ struct ListArgs {
     // semi-implicit Euler: the build decision for the next step, made by the kernel's
     // last block (threshold on max |x - x_build|, block ticket, the build's IF node)
     float thr; unsigned* tail_count; int use_cond; cudaGraphConditionalHandle cond;
-    // steps of the chain from this one on (0: not in a chain)
-    int left;
+    // steps of the chain from this one on (0: not in a chain); early: its blocks may start
+    // while the step before ends (contact-parallel kernel only)
+    int left, early;
     // the library's own lists: counters of the last build's gather
     unsigned long long* pend;
 };

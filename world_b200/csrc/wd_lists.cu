@@ -1485,6 +1485,11 @@ template <bool HIST, bool BATCH, bool PICARD, int LPG>
 __global__ void __launch_bounds__(kCoopBlock, PICARD ? 6 : 8)
 k_force_list_coop(const __grid_constant__ DevParams P0, const __grid_constant__ ListArgs A) {
     if (PICARD && skipped(A.skip)) return;
+    if (!PICARD) {
+        // an early launch: nothing of the step before is touched until it has ended
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     __shared__ CoopWarp<BATCH> warps[kCoopWarps];
     CoopWarp<BATCH>& W = warps[threadIdx.x >> 5];
     const int n = P0.n;
@@ -1633,9 +1638,23 @@ void force_list_variant(const DevParams& P, const ListArgs& a, cudaStream_t st, 
 template <bool HIST, bool BATCH, bool PICARD, int LPG>
 void force_list_coop_launch(const DevParams& P, const ListArgs& a, cudaStream_t st) {
     const int per = kCoopBlock / LPG;
-    const int nb = std::min((P.n + per - 1) / per,
-                            one_wave<k_force_list_coop<HIST, BATCH, PICARD, LPG>>(kCoopBlock));
-    k_force_list_coop<HIST, BATCH, PICARD, LPG><<<nb, kCoopBlock, 0, st>>>(P, a);
+    const int wave = one_wave<k_force_list_coop<HIST, BATCH, PICARD, LPG>>(kCoopBlock);
+    const int nb = std::min((P.n + per - 1) / per, wave);
+    // An early launch hides the next step's launch where both grids are resident at once (up to
+    // 75776 grains): 32768 falling grains 11.1 -> 10.7 us a step, 5120 in 24-step runs 776 ->
+    // 760 us. Blocks that wait for room gain nothing (2^20 grains 0.5%) or cost (24 scenes,
+    // 600 thousand grains, -1.7%).
+    const bool overlap = !PICARD && a.early != 0 && 2 * nb <= wave;
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nb);
+    cfg.blockDim = dim3(kCoopBlock);
+    cfg.stream = st;
+    cfg.attrs = &early;
+    cfg.numAttrs = overlap ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k_force_list_coop<HIST, BATCH, PICARD, LPG>, P, a);
 }
 
 template <bool PICARD, int LPG>

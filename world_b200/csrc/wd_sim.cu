@@ -955,9 +955,10 @@ cudaError_t capture_device_search_steps(wd_sim* s, int parity) {
 // `launcher`: outside a capture, the graph that launches a decided build from the device
 // (NULL: the build's kernels directly, gated by the decision).
 // `left`: in a chain, its steps from this one on; the chain's end launches the builds.
+// `early`: the contact kernel may be launched while the step before ends.
 cudaError_t enqueue_step_list(wd_sim* s, int parity, cudaStream_t st, bool capture,
                               cudaEvent_t mid = nullptr, cudaGraphExec_t launcher = nullptr,
-                              int left = 0) {
+                              int left = 0, bool early = false) {
     if (s->picard) return enqueue_step_list_picard(s, parity, st, capture, mid);
     const DevParams& P = s->P;
     const bool hist = P.history != 0, batch = s->scenes > 1;
@@ -974,6 +975,7 @@ cudaError_t enqueue_step_list(wd_sim* s, int parity, cudaStream_t st, bool captu
     a.tail_count = s->tail_count;
     a.pend = s->auto_ok ? s->auto_pend : nullptr;
     a.left = left;
+    a.early = early ? 1 : 0;
     a.use_cond = capture && !device_build && left == 0 ? 1 : 0;
     a.cond = cond;
     a.pos = s->posA; a.vel = s->velA; a.ids = s->idsA; a.table = s->sb.table;
@@ -1095,7 +1097,8 @@ cudaError_t enqueue_chain(wd_sim* s, int m, cudaStream_t st) {
     const bool hist = s->P.history != 0;
     for (int k = 0; k < m; ++k) {
         if (e == cudaSuccess)
-            e = enqueue_step_list(s, hist ? s->hist_cur : 0, st, true, nullptr, nullptr, m - k);
+            e = enqueue_step_list(s, hist ? s->hist_cur : 0, st, true, nullptr, nullptr, m - k,
+                                  m == kChain && k > 0);
         swap_state(s);
         if (hist) s->hist_cur ^= 1;
     }
