@@ -193,8 +193,8 @@ struct ListArgs {
 };
 // Device-side launches of the list build's graphs (wd_launch.cu, the one translation
 // unit built with relocatable device code for the device runtime): one thread
-// tail-launches `graph` when *flag is nonzero (the step's build decision), or `on_zero`
-// / `on_one` by *flag (the search's path). The launched graph runs once the graph that
+// tail-launches `graph` when *flag is nonzero (the step's build decision, or the search
+// asking for its radix path). The launched graph runs once the graph that
 // holds the launching kernel has completed; later work of the stream waits for it. A
 // failed launch counts in counters[kCntLaunchFail].
 void launch_graph_if(const uint32_t* flag, cudaGraphExec_t graph, unsigned long long* counters,

@@ -1205,10 +1205,15 @@ __global__ void k_list_picard_check(uint32_t* __restrict__ ctrl,
 // scenes took 1% longer than with 15.6 KB (132 KB), with 20.7 KB (list entries staged too,
 // 196 KB) 5% longer. Only batches stage the scene.
 //
-// Bound by load latency and issue. Measured at 64 registers, 8 blocks per SM (80 and 6 for
-// Picard, whose grid is not one wave of equal work): 2^20 falling grains 41.3 us a step
-// (per-lane 42.3; without the copies 46); 1,000,003 packed grains (8 list entries, 0.4
-// springs each) 134 against 176; 200,003 packed, 8 Picard iterations 230 against 492.
+// Bound by load latency and issue (1,475 warp instructions per 32 packed grains, 328 per 32
+// falling ones; half the chip's warps, an instruction every second cycle). Measured at 64
+// registers, 8 blocks per SM (80 and 6 for Picard, whose grid is not one wave of equal work)
+// against the per-lane kernel, single step graphs: 2^20 falling grains 41.3 us a step against
+// 42.3; 1,000,003 packed grains (8 list entries, 0.4 springs each) 134 against 176; 200,003
+// packed, 8 Picard iterations 230 against 492. In chains, with the build, now 36.0, 119 and
+// 225. A settled 2^20-grain layer (1.5 entries, a floor spring each) takes 108, the per-lane
+// kernel at 64 registers 96: there the tuner takes that one; 32,768 settled grains 14.9
+// against 15.9.
 constexpr int kCoopBlock = 128;
 constexpr int kCoopWarps = kCoopBlock / 32;
 

@@ -9,8 +9,9 @@
 //   * between steps few grains change cell, so the search re-sorts only those
 //     ("movers", ordered by counting the smaller ones) and merges them into the
 //     still-sorted rest by binary search; the first search, or one with more than
-//     mover_cap(n) movers, runs a stable LSD radix sort of all keys instead. The choice is made on the
-//     device, so both paths sit in the same CUDA graph and the idle one returns at
+//     mover_cap(n) movers, runs a stable LSD radix sort of all keys instead. The choice is
+//     made on the device: where the search stands in a graph that can launch another, that
+//     one holds the radix path; elsewhere the idle path sits in an IF node or returns at
 //     once. Both produce the same order;
 //   * the run table is a dense [start, end) per cell, but only the cells of the
 //     previous search are cleared (O(n), not the reference's O(cells) memset);

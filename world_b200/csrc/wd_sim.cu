@@ -206,7 +206,6 @@ struct wd_sim {
     float4* adj_lxi[2] = {nullptr, nullptr};
     float4* adj_lvt = nullptr;
     float4* adj_lf = nullptr;
-    int* adj_cnt_next = nullptr;
     double* adj_theta = nullptr;
 
     unsigned long long* counters = nullptr;
@@ -425,7 +424,7 @@ void free_sim(wd_sim* s) {
     if (s->io_up) cudaStreamDestroy(s->io_up);
     if (s->io_down) cudaStreamDestroy(s->io_down);
     void* adj[] = {s->adj_lx[0], s->adj_lx[1], s->adj_lv[0], s->adj_lv[1], s->adj_lxi[0],
-                   s->adj_lxi[1], s->adj_lvt, s->adj_lf, s->adj_cnt_next, s->adj_theta};
+                   s->adj_lxi[1], s->adj_lvt, s->adj_lf, s->adj_theta};
     for (void* p : adj) cudaFree(p);
     if (s->own_stream) cudaStreamDestroy(s->own_stream);
     if (s->aux_stream) cudaStreamDestroy(s->aux_stream);
@@ -1084,9 +1083,10 @@ int ensure_graph(wd_sim* s, bool launcher_only = false) {
 // return at once (list_step_waits), the launcher starts the build, and the build's end
 // launches a graph of the steps left over, with a launcher of its own. The host never has
 // to know. Captured once a handle has run kChainAfter list steps: about 16 graphs.
-// Measured (50 steps with the upload, a build every 10, 5,003 packed grains) 1,070 -> 806 us;
-// 100 steps of 32,768 falling grains with their stored fields 1,830 -> 1,226; 50 of 2^20
-// falling 2,120 -> 1,945.
+// Measured against single step graphs (50 steps with the upload, a build every 10, 5,003
+// packed grains) 1,070 -> 806 us; 100 steps of 32,768 falling grains with their stored fields
+// 1,830 -> 1,226; 50 of 2^20 falling 2,120 -> 1,945. (With the decision's words read at once
+// and early launches the second is 1,086.)
 constexpr int kChain = 8;
 constexpr int64_t kChainAfter = 128;
 
@@ -2656,8 +2656,6 @@ cudaError_t adj_replay_body(wd_sim* s, int len, bool capture, cudaStream_t st) {
 cudaError_t adj_back_body(wd_sim* s, int len, int cur, cudaStream_t st) {
     const DevParams& P = s->P;
     const bool hist = P.history != 0;
-    const int n = s->n;
-    const size_t rows = static_cast<size_t>(n) * wd::kHistCap;
     for (int t = len - 1; t >= 0; --t) {
         const wd_sim::TapeStep& T = s->adj_tape[static_cast<size_t>(t)];
         const wd_sim::TapeStep& T1 = s->adj_tape[static_cast<size_t>(t) + 1];
@@ -2948,7 +2946,6 @@ int wd_adjoint_backward(wd_sim* sim, const float* d_gx, const float* d_gv, float
         }
         WD_CUDA(dalloc(&sim->adj_lvt, n));
         WD_CUDA(dalloc(&sim->adj_lf, n));
-        WD_CUDA(dalloc(&sim->adj_cnt_next, n));
         WD_CUDA(dalloc(&sim->adj_theta, static_cast<size_t>(3) * n));
     }
     const int every = sim->adj_every;
@@ -2970,8 +2967,6 @@ int wd_adjoint_backward(wd_sim* sim, const float* d_gx, const float* d_gv, float
     if (hist)
         WD_CUDA(cudaMemsetAsync(sim->adj_lxi[0], 0, sizeof(float4) * n * wd::kHistCap, st));
     WD_CUDA(cudaMemsetAsync(sim->adj_theta, 0, sizeof(double) * 3 * n, st));
-    const DevParams& P = sim->P;
-    const wd::Skip none{nullptr, 0.f};
     const size_t rows = static_cast<size_t>(n) * wd::kHistCap;
     const int64_t nseg = static_cast<int64_t>(sim->adj_ckpt.size() == 0 ? 0 :
                                               (sim->adj_steps + every - 1) / every);
@@ -3026,7 +3021,6 @@ int wd_deposit_vjp(wd_sim* sim, const float* d_ggrid, float* d_gx, float* d_gv) 
         }
         WD_CUDA(dalloc(&sim->adj_lvt, n));
         WD_CUDA(dalloc(&sim->adj_lf, n));
-        WD_CUDA(dalloc(&sim->adj_cnt_next, n));
         WD_CUDA(dalloc(&sim->adj_theta, static_cast<size_t>(3) * n));
         if (sim->P.history)
             for (int b = 0; b < 2; ++b)
