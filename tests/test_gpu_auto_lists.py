@@ -153,3 +153,17 @@ def test_windows_of_odd_length_give_the_searched_gradient(steps, every):
             out.append((sim.get_state(), gx.cpu().numpy(), gv.cpu().numpy(), th))
         for a, b in zip(*out):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("first,kernels", [(36, 6), (37, 2)])
+def test_a_new_handle_searches_until_lists_pay(first, kernels):
+    """2,744 grains: a call of 36 steps on a new handle is searched, one of 37 is not (40 x
+    32768 / (32768 + n) steps, rounded up), and the searched ones count towards the line."""
+    cfg, st, rad = _touching(65, True)
+    cfg.kernel_timing = False
+    own, searched = _both(cfg, st, rad)
+    for run, expect in ((first, kernels), (1, 2), (3, 2)):
+        for sim in (own, searched):
+            sim.advance(run)
+        assert own.kernels_per_step() == expect
+        _equal(own, searched)

@@ -164,6 +164,7 @@ struct wd_sim {
     unsigned long long* auto_pend = nullptr; // counters that a build's gather adds to
     uint32_t* auto_load = nullptr;           // per cell: grains that can be in it before the next build
     int64_t run_steps = 0, last_run = 0;     // steps since the last upload, and between the two before
+    int64_t auto_wait = 0;                   // steps a new handle searches unless it has as many to come
     int64_t auto_off = 0, auto_backoff = 512;// steps to search before lists are tried again
     int64_t auto_look = 0;                   // list step of the run that reads the device's counts next
     unsigned long long auto_seen[2] = {0, 0};// list steps and builds at the last look
@@ -1377,6 +1378,13 @@ cudaError_t alloc_list_buffers(wd_sim* s) {
     return e;
 }
 
+// A new handle's first list steps capture the graphs of their builds, 0.4 to 0.7 ms, and a list
+// step saves 10 us of a searched one at 10^3 grains, 20 at 3 10^4, 80 at 10^5: lists pay once
+// a handle has stepped, or has in hand, 40 steps, 20 and 10. Measured (a new handle's upload and
+// 10 steps; lists at once against searched): the default cube 1361 and 667 us, 20,011 packed
+// grains 1361 and 796, 32,768 falling 1267 and 866; 100 steps of 5,003 packed 2979 and 3539.
+constexpr int64_t kAutoNew = 40;
+
 // The buffers of the library's own lists, at creation (allocated between two steps they cost
 // 5 to 500 ms at 2^20 grains); not where they would take more than a quarter of the free
 // memory: such a handle searches.
@@ -1402,6 +1410,8 @@ void auto_prepare(wd_sim* s) {
     }
     if (!ok) cudaGetLastError();
     s->auto_ok = ok;
+    const int64_t per = 32768 + static_cast<int64_t>(s->n);
+    s->auto_wait = (kAutoNew * 32768 + per - 1) / per;
 }
 
 // The mode of the next step of a handle that may use the library's own lists, with
@@ -1409,7 +1419,8 @@ void auto_prepare(wd_sim* s) {
 // bit; what they cost is a build after every upload and one whenever a grain has moved
 // half a skin. So they are used for runs of kAutoRun steps and more between uploads (this
 // call's, or as long as the last such run), and not while more than one step in four
-// would build; the wait before they are tried again then doubles. Measured, upload and k
+// would build; the wait before they are tried again then doubles; a new handle waits until
+// they pay (kAutoNew). Measured, upload and k
 // steps, searched against lists: 2^20 falling grains 75 + 157 k and 260 + 37 k us,
 // 100,003 packed 30 + 113 k and 100 + 31 k, the default cube 68 + 98 k and 175 + 10 k.
 constexpr int64_t kAutoRun = 3;
@@ -1447,7 +1458,9 @@ cudaError_t auto_mode(wd_sim* s, int64_t ahead) {
             }
         }
     }
-    const bool lists = s->auto_off == 0 && (s->run_steps + ahead >= kAutoRun || s->last_run >= kAutoRun);
+    const bool lists = s->auto_off == 0 && ahead >= s->auto_wait &&
+                       (s->run_steps + ahead >= kAutoRun || s->last_run >= kAutoRun);
+    s->auto_wait = lists ? 0 : std::max<int64_t>(0, s->auto_wait - 1);
     const bool enter = lists && !s->lists;
     if (enter) s->auto_look = s->run_steps + 32;
     s->lists = lists;
