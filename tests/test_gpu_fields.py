@@ -58,3 +58,23 @@ def test_deposit_is_the_rounded_sum(n, scale):
     e = [sim.compute_total_energy() for _ in range(3)]   # direct, then as device graphs
     assert e[0] == e[1] == e[2] == pytest.approx(sim.grain_energies().sum(), rel=1e-12)
     sim.close()
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+@pytest.mark.parametrize("n", [1, 33, 257])
+def test_states_on_any_float_alignment(n, offset):
+    """States in and out of CUDA tensors that start on 4, 8 or 16 bytes, after a step has
+    re-ordered the slots: copies, so equal to the bit, with nothing written beside them."""
+    import torch
+    cfg, st, rad = packed_poly(n=n, seed=68)
+    sim = ParticleDynamics(cfg, state=st, radius=rad)
+    sim.advance(1)
+    want = np.random.default_rng(69).uniform(-0.01, 0.01, 6 * n).astype(np.float32)
+    buf = torch.zeros(6 * n + 8, device="cuda")
+    buf[offset:offset + 6 * n] = torch.from_numpy(want).cuda()
+    sim.set_state_tensor(buf[offset:offset + 6 * n])
+    out = torch.full((6 * n + 8,), 7.0, device="cuda")
+    sim.state_tensor(out[offset:offset + 6 * n])
+    got = out.cpu().numpy()
+    assert np.array_equal(got[offset:offset + 6 * n], want)
+    assert np.all(got[:offset] == 7.0) and np.all(got[offset + 6 * n:] == 7.0)

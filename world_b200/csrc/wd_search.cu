@@ -504,6 +504,10 @@ k_cand_fill(DevParams P0, SceneTab T, const float4* __restrict__ pos, const int*
     }
 }
 
+// The caller's states by grain id. Bound by the sector transactions of the scattered 24-byte
+// records. PAIRS: the caller's array starts on 8 bytes, so a record is three 8-byte accesses
+// (else six of 4): an upload and a download of 2^20 grains together 17 to 19 us less.
+template <bool PAIRS>
 __global__ void k_state_to_aos(int n, const float4* __restrict__ pos,
                                const float4* __restrict__ vel, const int* __restrict__ ids,
                                float* __restrict__ out) {
@@ -511,7 +515,14 @@ __global__ void k_state_to_aos(int n, const float4* __restrict__ pos,
     if (s >= n) return;
     const float4 x = pos[s], v = vel[s];
     float* o = out + 6 * static_cast<int64_t>(ids[s]);
-    o[0] = x.x; o[1] = x.y; o[2] = x.z; o[3] = v.x; o[4] = v.y; o[5] = v.z;
+    if (PAIRS) {
+        float2* o2 = reinterpret_cast<float2*>(o);
+        o2[0] = make_float2(x.x, x.y);
+        o2[1] = make_float2(x.z, v.x);
+        o2[2] = make_float2(v.y, v.z);
+    } else {
+        o[0] = x.x; o[1] = x.y; o[2] = x.z; o[3] = v.x; o[4] = v.y; o[5] = v.z;
+    }
 }
 
 __global__ void k_positions_to_aos(int n, const float4* __restrict__ pos,
@@ -533,14 +544,24 @@ __global__ void k_rhs_to_aos(int n, const float4* __restrict__ vel,
     o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = a.x; o[4] = a.y; o[5] = a.z;
 }
 
+template <bool PAIRS>
 __global__ void k_state_from_aos(int n, const float* __restrict__ in, float4* __restrict__ pos,
                                  float4* __restrict__ vel, const int* __restrict__ ids) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const float* q = in + 6 * static_cast<int64_t>(ids[s]);
-    pos[s] = make_float4(q[0], q[1], q[2], pos[s].w);
-    vel[s] = make_float4(q[3], q[4], q[5], vel[s].w);
+    if (PAIRS) {
+        const float2* q2 = reinterpret_cast<const float2*>(q);
+        const float2 a = q2[0], b = q2[1], c = q2[2];
+        pos[s] = make_float4(a.x, a.y, b.x, pos[s].w);
+        vel[s] = make_float4(b.y, c.x, c.y, vel[s].w);
+    } else {
+        pos[s] = make_float4(q[0], q[1], q[2], pos[s].w);
+        vel[s] = make_float4(q[3], q[4], q[5], vel[s].w);
+    }
 }
+
+bool on_pairs(const float* p) { return reinterpret_cast<uintptr_t>(p) % sizeof(float2) == 0; }
 
 // Cell key of every grain within its own scene's grid, by grain id.
 template <bool BATCH>
@@ -684,7 +705,8 @@ void launch_candidate_fill(const DevParams& P, SceneTab T, const float4* pos, co
 
 void launch_state_to_aos(int n, const float4* pos, const float4* vel, const int* ids,
                          float* out6, cudaStream_t st) {
-    k_state_to_aos<<<blocks_for(n), kBlock, 0, st>>>(n, pos, vel, ids, out6);
+    if (on_pairs(out6)) k_state_to_aos<true><<<blocks_for(n), kBlock, 0, st>>>(n, pos, vel, ids, out6);
+    else k_state_to_aos<false><<<blocks_for(n), kBlock, 0, st>>>(n, pos, vel, ids, out6);
 }
 
 void launch_positions_to_aos(int n, const float4* pos, const int* ids, float* out3,
@@ -699,7 +721,8 @@ void launch_rhs_to_aos(int n, const float4* vel_used, const float4* acc, const i
 
 void launch_state_from_aos(int n, const float* in6, float4* pos, float4* vel, const int* ids,
                            cudaStream_t st) {
-    k_state_from_aos<<<blocks_for(n), kBlock, 0, st>>>(n, in6, pos, vel, ids);
+    if (on_pairs(in6)) k_state_from_aos<true><<<blocks_for(n), kBlock, 0, st>>>(n, in6, pos, vel, ids);
+    else k_state_from_aos<false><<<blocks_for(n), kBlock, 0, st>>>(n, in6, pos, vel, ids);
 }
 
 void launch_cell_keys_by_id(const DevParams& P, SceneTab T, const float4* pos, const int* ids,
