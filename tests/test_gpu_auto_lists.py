@@ -167,3 +167,24 @@ def test_a_new_handle_searches_until_lists_pay(first, kernels):
             sim.advance(run)
         assert own.kernels_per_step() == expect
         _equal(own, searched)
+
+
+def test_chains_captured_for_both_pairs_of_buffers():
+    """A list step swaps the state buffers and the spring rows, a searched one the rows only,
+    so a searched step between two long runs changes which of them go together: chains exist
+    for both pairings, and the ones captured first still finish their steps after the others
+    have been captured. Builds come about every eight steps, most inside chains."""
+    cfg, st, rad = _touching(67, True)
+    cfg.kernel_timing = False
+    st = st.copy()
+    st[:, 3:] = np.random.default_rng(68).normal(0, 1.0, (2744, 3))
+    own, searched = _both(cfg, st, rad)
+    for run in (200,) + (1, 1, 100) * 5:
+        for sim in (own, searched):
+            sim.advance(run)
+        _equal(own, searched)
+        assert own.time == searched.time
+        state = own.get_state()
+        for sim in (own, searched):
+            sim.set_state(state)
+    assert own.kernels_per_step() == 2          # the long runs were on lists

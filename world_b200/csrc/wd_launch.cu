@@ -46,7 +46,11 @@ __global__ void k_build_end(uint32_t* __restrict__ ctrl, const cudaGraphExec_t* 
         const uint32_t left = ctrl[kLcLeft];
         ctrl[kLcPending] = 0u;
         ctrl[kLcLeft] = 0u;
-        if (left > 0u) next = by_left[left];
+        if (left > 0u) {
+            next = by_left[left];
+            // steps that nothing takes up are an error, not steps left out
+            if (next == nullptr) atomicAdd(&counters[kCntLaunchFail], 1ull);
+        }
     }
     if (next != nullptr && cudaGraphLaunch(next, cudaStreamGraphTailLaunch) != cudaSuccess)
         atomicAdd(&counters[kCntLaunchFail], 1ull);

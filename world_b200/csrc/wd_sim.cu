@@ -1109,7 +1109,6 @@ cudaError_t enqueue_chain(wd_sim* s, int m, cudaStream_t st) {
 cudaError_t capture_chains(wd_sim* s) {
     const bool hist = s->P.history != 0;
     cudaError_t e = cudaSuccess;
-    cudaGraphExec_t handles[4][8] = {};
     for (int side = 0; side < 2; ++side) {
         // both sides' builds first: the launchers hold their handles
         wd_sim::StepGraph& g = s->graph_now();
@@ -1136,7 +1135,6 @@ cudaError_t capture_chains(wd_sim* s) {
             cudaError_t be = cudaSuccess;
             e = capture_device_graph(s, &s->chain_rest[at][m], [&](cudaStream_t st) { be = body(m, st); });
             if (be != cudaSuccess) e = be;
-            handles[at][m] = s->chain_rest[at][m];
         }
         if (e == cudaSuccess) {
             cudaGraph_t g = nullptr;
@@ -1153,11 +1151,14 @@ cudaError_t capture_chains(wd_sim* s) {
         if (hist) s->hist_cur ^= 1;
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux_stream);
-    // on the step stream: builds in flight may still read the table (all zero before)
+    // On the step stream: builds in flight may still read the table. All of it: the other
+    // pair of parities keeps its chains and so the rows of their remainders.
+    static_assert(sizeof(s->chain_rest) == 4 * 8 * sizeof(cudaGraphExec_t), "the table's layout");
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(s->chain_table, handles, sizeof(handles), cudaMemcpyHostToDevice, s->stream);
+        e = cudaMemcpyAsync(s->chain_table, s->chain_rest, sizeof(s->chain_rest), cudaMemcpyHostToDevice, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) {
+        cudaStreamSynchronize(s->stream);   // the other pair's may be in flight
         for (int k = 0; k < 4; ++k) {
             if (s->chain[k]) cudaGraphExecDestroy(s->chain[k]);
             s->chain[k] = nullptr;
