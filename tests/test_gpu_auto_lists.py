@@ -188,3 +188,20 @@ def test_chains_captured_for_both_pairs_of_buffers():
         for sim in (own, searched):
             sim.set_state(state)
     assert own.kernels_per_step() == 2          # the long runs were on lists
+
+
+def test_the_stage_wait_hook_needs_lists_that_the_caller_asked_for():
+    from world_b200 import WorldError
+    from world_b200._lib import check, lib
+    cfg, st, rad = _touching(69, False)
+    cfg.kernel_timing = False
+    sim = ParticleDynamics(cfg, state=st, radius=rad)
+    for _ in range(2):
+        with pytest.raises(WorldError, match="no Verlet lists"):
+            check(lib.wd_debug_stage_wait(sim.handle, 0, 0))
+        sim.advance(40)
+    sim.set_neighbor_skin(0.0)
+    with pytest.raises(WorldError, match="no Verlet lists"):
+        check(lib.wd_debug_stage_wait(sim.handle, 0, 0))
+    sim.set_neighbor_skin(0.5e-3)
+    check(lib.wd_debug_stage_wait(sim.handle, 0, 0))

@@ -137,6 +137,7 @@ struct wd_sim {
     int io_i = 0, io_o = 0;
 
     bool lists = false;
+    bool skin_asked = false;        // the caller has had lists, by a skin above 0
     int lpar = 0;
     int force_block = wd::kBlock;   // threads per block of the contact kernel
     int force_minb = 0;             // list contact kernel variant (0: contact-parallel)
@@ -1702,7 +1703,7 @@ int create_scenes(const wd::Config* const* cfgs, int S, const int64_t* counts,
     s->dt = c0.dt;
     s->picard = c0.time_integrator != "semi_implicit_euler";
     s->picard_iters = s->picard ? c0.picard_iterations : 1;
-    s->lists = c0.neighbor_skin > 0.f;
+    s->lists = s->skin_asked = c0.neighbor_skin > 0.f;
     s->num_cells = cells;
     s->scene_off.assign(1, 0);
     s->scene_nodes_off.assign(1, 0);
@@ -2544,6 +2545,7 @@ static int apply_skin(wd_sim* s, float skin) {
     const bool lists = skin > 0.f;
     s->auto_ok = false;   // the caller's choice, 0 included
     if (lists) WD_CUDA(alloc_list_buffers(s));
+    s->skin_asked |= lists;
     if (lists && s->picard && !s->xpos) {
         const int n = s->n;
         WD_CUDA(dalloc(&s->xpos, n));
@@ -2753,7 +2755,7 @@ int wd_set_contact_kernel(wd_sim* sim, int32_t block, int32_t variant) {
 
 int wd_debug_stage_wait(wd_sim* sim, int32_t stall, int32_t wait_us) {
     if (!sim) return fail(WD_ERR_INVALID, "wd_debug_stage_wait: NULL handle");
-    if (!sim->list_ctrl)
+    if (!sim->skin_asked)
         return fail(WD_ERR_INVALID, "wd_debug_stage_wait: the handle has no Verlet lists");
     if (wait_us < 0) return fail(WD_ERR_INVALID, "wd_debug_stage_wait: wait_us must be >= 0");
     int rc = sync_stream(sim);
