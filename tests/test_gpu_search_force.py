@@ -68,3 +68,30 @@ def test_many_contacts_on_one_grain(n, touching, oracle_for):
     radius = np.full(n, 1.2e-3, np.float32)
     radius[0] = 10e-3
     _check(cfg, state, radius, oracle_for, 12)
+
+
+@pytest.mark.parametrize("history", [True, False])
+@pytest.mark.parametrize("skin,kernel", [(0.0, None), (0.5e-3, (256, 0)), (0.5e-3, (128, 64)), (0.5e-3, (256, 1))])
+def test_grains_with_one_nan_coordinate(skin, kernel, history, oracle_for):
+    """Grains clear of every wall but for one coordinate that is NaN: that axis' two wall
+    forces are the clamp (max(0, min(F, NaN)) = F) added and taken away again, which is NaN
+    where there is no clamp and a rounding where there is one. Contacts of the others as ever."""
+    for clamp in (0.0, 250.0):                  # 0: no clamp
+        cfg, st, rad = _roomy(1500, 83, 0.5, history)
+        cfg.physics.max_force = clamp
+        cfg.neighbor_skin = skin
+        st = st.copy()
+        for k, axis in ((100, 0), (700, 1), (1300, 2)):
+            st[k, :3] = 1e-3 * (axis - 1)
+            st[k, axis] = np.nan
+        sim = ParticleDynamics(cfg, state=st, radius=rad)
+        if kernel:
+            sim.set_contact_kernel(*kernel)
+        else:
+            sim.set_neighbor_skin(0.0)
+        orc = oracle_for(cfg, st, radius=rad)
+        sim.advance(3)
+        orc.step(3)
+        np.testing.assert_array_equal(sim.get_state(), orc.state)
+        np.testing.assert_array_equal(sim.get_rhs(), orc.rhs)
+        sim.close()

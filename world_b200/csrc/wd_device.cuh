@@ -237,12 +237,12 @@ __device__ __forceinline__ void wall_forces(const DevParams& P, float3 pos, floa
     auto c_wall = [&]() { return damping(P, mi); };
     f.z = fmaf(-mi, P.gravity, f.z);
     // A grain clear of all six walls adds six zeros (of either sign, to sums that such a
-    // zero leaves as they are): skipped. NaN takes the long way.
-    const float clear = fminf(
-        fminf(fminf((pos.x - P.wall_lo[0]) - ri, (P.wall_hi[0] - pos.x) - ri),
-              fminf((pos.y - P.wall_lo[1]) - ri, (P.wall_hi[1] - pos.y) - ri)),
-        fminf((pos.z - P.wall_lo[2]) - ri, (P.wall_hi[2] - pos.z) - ri));
-    if (clear > 0.f) return;
+    // zero leaves as they are): skipped. One NaN distance fails its comparison and so takes
+    // the long way, where the clamp turns it into a force (a minimum of the six would drop it).
+    const bool clear = ((pos.x - P.wall_lo[0]) - ri > 0.f) & ((P.wall_hi[0] - pos.x) - ri > 0.f) &
+                       ((pos.y - P.wall_lo[1]) - ri > 0.f) & ((P.wall_hi[1] - pos.y) - ri > 0.f) &
+                       ((pos.z - P.wall_lo[2]) - ri > 0.f) & ((P.wall_hi[2] - pos.z) - ri > 0.f);
+    if (clear) return;
     const float p3[3] = {pos.x, pos.y, pos.z};
     const float v3[3] = {vel.x, vel.y, vel.z};
 #pragma unroll
