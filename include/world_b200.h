@@ -313,6 +313,9 @@ int wd_set_build_kernel(wd_sim* sim, int32_t tiled);
  * and no stored springs; wd_set_history restores those). No copy is ever left in
  * flight. Handles with Verlet lists only. */
 int wd_debug_stage_wait(wd_sim* sim, int32_t stall, int32_t wait_us);
+/* CUDA graphs the handle has captured so far (no counterpart in the reference): a test's
+ * view of what a parameter change or a tuning run costs beside its steps. */
+int wd_debug_graph_captures(wd_sim* sim, int64_t* captures);
 /* Verlet lists: steps so far whose contact kernel measured the exact displacement
  * since the build (reading the build positions). The other steps decide on a bound:
  * the last exact value plus the largest per-step displacement of each step since. */

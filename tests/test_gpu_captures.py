@@ -1,0 +1,53 @@
+"""What a parameter change and a tuning run capture beside their steps (wd_debug_graph_captures).
+
+Steps are CUDA graphs, captured when first needed and dropped when dt, a contact parameter,
+the skin or the contact kernel changes. On lists each of the two buffer parities has a step
+graph with three launchers of builds, and two graphs for a build that the host asks for; runs
+that are long enough add the chains, 14 remainders and 2 chains of eight steps."""
+from __future__ import annotations
+
+import ctypes
+
+import pytest
+
+from test_gpu_auto_lists import _touching
+from test_gpu_lists import _same
+from world_b200 import ParticleDynamics
+from world_b200._lib import check, lib
+from world_b200.scenes import column_collapse
+
+pytestmark = pytest.mark.gpu
+
+
+def _captures(sim):
+    got = ctypes.c_int64()
+    check(lib.wd_debug_graph_captures(sim.handle, ctypes.byref(got)))
+    return got.value
+
+
+@pytest.mark.parametrize("skin", [0.0, 0.5e-3])
+def test_a_changed_parameter_costs_step_graphs_only(skin):
+    cfg, st, rad = _touching(71, True)
+    cfg.kernel_timing = False
+    cfg.neighbor_skin = skin
+    sim = ParticleDynamics(cfg, state=st, radius=rad)
+    ref = ParticleDynamics(cfg, state=st, radius=rad)
+    ref.set_neighbor_skin(0.0)
+    for s in (sim, ref):
+        s.advance(300)
+    assert _captures(sim) >= 16                 # chains among them
+    for k in range(4):
+        before = _captures(sim)
+        for s in (sim, ref):
+            if k % 2:
+                s.dt = 1e-5 * (1 - 1e-3 * k)
+            else:
+                s.set_contact_params(0.5 - 0.01 * (k + 1), 0.5, 1e5)
+            s.advance(40)
+        assert _captures(sim) - before <= 12
+        _same(ref, sim)
+    before = _captures(sim)
+    for s in (sim, ref):
+        s.advance(300)
+    assert _captures(sim) - before >= 16        # long runs at one setting have chains again
+    _same(ref, sim)

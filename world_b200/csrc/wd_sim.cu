@@ -253,13 +253,14 @@ struct wd_sim {
     cudaGraphExec_t chain_rest[4][8] = {};
     cudaGraphExec_t* chain_table = nullptr;   // [4][8]
     bool chain_failed = false;
-    int64_t list_steps = 0;
+    int64_t list_steps = 0;                   // list steps one by one since the graphs were dropped
     // the on-demand search (energy, probes) per buffer parity
     struct SearchGraph {
         cudaGraphExec_t head = nullptr, radix = nullptr;
         bool seen = false, failed = false;
     };
     SearchGraph search_graph[2];
+    int64_t captures = 0;   // graphs captured over the handle's lifetime
     StepGraph& graph_now() { return graphs[(lists ? 4 : 0) + 2 * lpar + hist_cur]; }
     bool graph_dirty = true;
 
@@ -301,6 +302,7 @@ void destroy_graphs(wd_sim* s) {
             x = nullptr;
         }
     }
+    s->list_steps = 0;   // new chains have to pay for their capture again
     s->graph_dirty = true;
 }
 
@@ -880,6 +882,7 @@ cudaError_t capture_device_graph(wd_sim* s, cudaGraphExec_t* out, Body body) {
         *out = nullptr;
         return e;
     }
+    ++s->captures;
     return cudaGraphUpload(*out, s->aux_stream);
 }
 
@@ -1074,6 +1077,7 @@ int ensure_graph(wd_sim* s, bool launcher_only = false) {
     const cudaError_t e = cudaGraphInstantiate(&sg.step, g, 0);
     cudaGraphDestroy(g);
     WD_CUDA(e);
+    ++s->captures;
     return WD_OK;
 }
 
@@ -1084,7 +1088,8 @@ int ensure_graph(wd_sim* s, bool launcher_only = false) {
 // build that a step decides has to run before the next: the chain's later kernels then
 // return at once (list_step_waits), the launcher starts the build, and the build's end
 // launches a graph of the steps left over, with a launcher of its own. The host never has
-// to know. Captured once a handle has run kChainAfter list steps: about 16 graphs.
+// to know. Captured (16 graphs, 2 to 3 ms) once a handle has run kChainAfter list steps since
+// its graphs were last dropped: a changed dt or contact parameter drops them.
 // Measured against single step graphs (50 steps with the upload, a build every 10, 5,003
 // packed grains) 1,070 -> 806 us; 100 steps of 32,768 falling grains with their stored fields
 // 1,830 -> 1,226; 50 of 2^20 falling 2,120 -> 1,945. (With the decision's words read at once
@@ -1147,6 +1152,7 @@ cudaError_t capture_chains(wd_sim* s) {
             }
             if (e == cudaSuccess) e = cudaGraphInstantiate(&s->chain[at], g, 0);
             if (g) cudaGraphDestroy(g);
+            ++s->captures;
         }
         swap_state(s);
         if (hist) s->hist_cur ^= 1;
@@ -1175,9 +1181,9 @@ cudaError_t capture_chains(wd_sim* s) {
 
 // The chain graph that starts from the current parities, or NULL where steps go one by one.
 cudaGraphExec_t chain_now(wd_sim* s) {
-    if (s->picard || s->chain_failed || s->list_steps < kChainAfter) return nullptr;
     if (s->graph_dirty) destroy_graphs(s);
     s->graph_dirty = false;
+    if (s->picard || s->chain_failed || s->list_steps < kChainAfter) return nullptr;
     const int at = 2 * s->lpar + s->hist_cur;
     if (!s->chain[at]) {
         const int lpar = s->lpar, cur = s->hist_cur;
@@ -2715,6 +2721,7 @@ cudaError_t run_adj_graph(wd_sim* s, int len, int parity) {
         e = cudaGraphInstantiate(&exec, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return e;
+        ++s->captures;
         it = s->adj_graphs.emplace(key, exec).first;
     }
     return cudaGraphLaunch(it->second, s->stream);
@@ -2763,6 +2770,12 @@ int wd_debug_stage_wait(wd_sim* sim, int32_t stall, int32_t wait_us) {
     const uint32_t words[2] = {stall ? 1u : 0u, static_cast<uint32_t>(wait_us)};
     WD_CUDA(cudaMemcpy(sim->list_ctrl + wd::kLcStallTest, words, sizeof(words),
                        cudaMemcpyHostToDevice));
+    return WD_OK;
+}
+
+int wd_debug_graph_captures(wd_sim* sim, int64_t* captures) {
+    if (!sim || !captures) return fail(WD_ERR_INVALID, "wd_debug_graph_captures: NULL argument");
+    *captures = sim->captures;
     return WD_OK;
 }
 
