@@ -51,3 +51,20 @@ def test_a_changed_parameter_costs_step_graphs_only(skin):
         s.advance(300)
     assert _captures(sim) - before >= 16        # long runs at one setting have chains again
     _same(ref, sim)
+
+
+@pytest.mark.parametrize("steps", [20, 150])
+def test_autotune_captures_no_chains(steps):
+    """The tuner times every candidate stepping one by one: its captures are the candidates'
+    step graphs and builds, made by the untimed steps before (36 list candidates of at most
+    12 graphs, the searched step and the first ones), and no chains of steps, which a timed
+    run would capture between its two events."""
+    sc = column_collapse(4096, diameters="uniform", mu=0.5, cic=32)
+    sc.cfg.kernel_timing = False
+    ref = ParticleDynamics(sc.cfg, state=sc.state, radius=sc.radius)
+    sim = ParticleDynamics(sc.cfg, state=sc.state, radius=sc.radius)
+    sim.autotune(steps=steps)
+    assert _captures(sim) <= 43 * 12
+    for s in (ref, sim):
+        s.advance(300)
+    _same(ref, sim)

@@ -253,6 +253,7 @@ struct wd_sim {
     cudaGraphExec_t chain_rest[4][8] = {};
     cudaGraphExec_t* chain_table = nullptr;   // [4][8]
     bool chain_failed = false;
+    bool no_chains = false;                   // the tuner's steps go one by one
     int64_t list_steps = 0;                   // list steps one by one since the graphs were dropped
     // the on-demand search (energy, probes) per buffer parity
     struct SearchGraph {
@@ -1183,7 +1184,7 @@ cudaError_t capture_chains(wd_sim* s) {
 cudaGraphExec_t chain_now(wd_sim* s) {
     if (s->graph_dirty) destroy_graphs(s);
     s->graph_dirty = false;
-    if (s->picard || s->chain_failed || s->list_steps < kChainAfter) return nullptr;
+    if (s->picard || s->chain_failed || s->no_chains || s->list_steps < kChainAfter) return nullptr;
     const int at = 2 * s->lpar + s->hist_cur;
     if (!s->chain[at]) {
         const int lpar = s->lpar, cur = s->hist_cur;
@@ -2837,6 +2838,9 @@ int wd_autotune(wd_sim* sim, int32_t steps, const char* cache_path, float* skin_
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
         float best_ms = INFINITY;
+        // every candidate steps one by one: a chain's capture (2 to 3 ms) would fall between
+        // the events of whichever candidate came to it
+        sim->no_chains = true;
         for (float sk : skins) {
             for (int cand = 0; cand < ncands && rc == WD_OK; ++cand) {
                 const int bl = cands[cand][0];
@@ -2870,6 +2874,7 @@ int wd_autotune(wd_sim* sim, int32_t steps, const char* cache_path, float* skin_
             }
             if (rc != WD_OK) break;
         }
+        sim->no_chains = false;
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         if (rc == WD_OK) {
