@@ -278,11 +278,12 @@ int wd_grid_overflow_count(wd_sim* sim, int64_t* count);
  * buffers of at most a quarter of the free device memory); calling this (or the
  * autotuner) ends that. */
 int wd_set_neighbor_skin(wd_sim* sim, float skin);
-/* Autotuner (extension): times `steps` steps for each neighbor skin in {0, 0.05,
- * 0.1, 0.15, 0.2, 0.3, 0.4} mean diameters, contact-kernel block size in {128, 256} and, with
- * lists, its variant (per-lane with 48 or 64 registers, warp-cooperative, bulk-staged)
- * from the same saved state, keeps
- * the fastest and restores the state (results do not depend on the choice). With
+/* Autotuner (extension): times `steps` steps, one by one, from the same saved state with a
+ * search every step and, for each neighbor skin in {0.05, 0.1, 0.15, 0.2, 0.3, 0.4} mean
+ * diameters, with each list contact kernel (per-lane with 48 or 64 registers and 128 or 256
+ * threads a block, warp-cooperative, bulk-staged), keeps the fastest and restores the state
+ * (results do not depend on the choice). The block size is the per-lane kernel's; with any
+ * other, the searched step's included, 256 is reported. With
  * cache_path, a line "key skin block variant" keyed by grain count,
  * scenes, grid, SM count, history, integrator and launch mode is reused or appended.
  * skin_out / block_out (may be NULL) receive the choice. */

@@ -68,3 +68,16 @@ def test_autotune_captures_no_chains(steps):
     for s in (ref, sim):
         s.advance(300)
     _same(ref, sim)
+
+
+def test_autotune_has_one_searched_candidate():
+    """Grains that cross half of any skin within a step or two: searching wins. Its kernel has
+    a block of its own, so the block reported beside it is always the same."""
+    cfg, st, rad = _touching(72, False)
+    cfg.kernel_timing = False
+    st = st.copy()
+    st[:, 3] += 150.0
+    sim = ParticleDynamics(cfg, state=st, radius=rad)
+    for _ in range(6):
+        assert sim.autotune(steps=10) == (0.0, 256)
+    assert sim.tuning()["contact_variant"] == "warp-cooperative"    # lists, if switched on later

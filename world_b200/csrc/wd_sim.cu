@@ -2845,7 +2845,8 @@ int wd_autotune(wd_sim* sim, int32_t steps, const char* cache_path, float* skin_
             for (int cand = 0; cand < ncands && rc == WD_OK; ++cand) {
                 const int bl = cands[cand][0];
                 const int mb = cands[cand][1];
-                if (sk == 0.f && mb != 5) continue;  // the searched kernel has one variant
+                // the searched kernel has one form: once, with the default list kernel beside it
+                if (sk == 0.f && mb != 0) continue;
                 if (sim->picard && (mb == 1 || mb == 2)) continue;  // no bulk-staged Picard form
                 rc = apply_skin(sim, sk);
                 if (rc == WD_OK) {

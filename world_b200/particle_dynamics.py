@@ -340,8 +340,9 @@ class ParticleDynamics:
         check(lib.wd_set_neighbor_skin(self._h, ctypes.c_float(skin)))
 
     def autotune(self, steps: int = 50, cache: Optional[str] = None) -> tuple[float, int]:
-        """Pick the neighbor skin and contact-kernel block size by timing (the state is
-        restored afterwards; results do not depend on the choice). Returns them."""
+        """Pick the neighbor skin and the list contact kernel by timing (the state is restored
+        afterwards; results do not depend on the choice). Returns the skin and the block
+        size, which is the per-lane kernel's (256 with any other)."""
         sk = ctypes.c_float()
         bl = ctypes.c_int32()
         check(lib.wd_autotune(self._h, int(steps), None if cache is None else str(cache).encode(),
