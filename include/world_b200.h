@@ -317,6 +317,10 @@ int wd_debug_stage_wait(wd_sim* sim, int32_t stall, int32_t wait_us);
 /* CUDA graphs the handle has captured so far (no counterpart in the reference): a test's
  * view of what a parameter change or a tuning run costs beside its steps. */
 int wd_debug_graph_captures(wd_sim* sim, int64_t* captures);
+/* Test hook (no counterpart in the reference): as if a device-side launch, of a list build
+ * or of a search's radix path, had failed. The next synchronizing call reports it once, as
+ * WD_ERR_CUDA; nothing else changes. */
+int wd_debug_launch_failure(wd_sim* sim);
 /* Verlet lists: steps so far whose contact kernel measured the exact displacement
  * since the build (reading the build positions). The other steps decide on a bound:
  * the last exact value plus the largest per-step displacement of each step since. */

@@ -84,6 +84,7 @@ SIGNATURES = {
     "wd_set_build_kernel": ([_p, c_int32], c_int),
     "wd_debug_stage_wait": ([_p, c_int32, c_int32], c_int),
     "wd_debug_graph_captures": ([_p, _i64], c_int),
+    "wd_debug_launch_failure": ([_p], c_int),
     "wd_set_state_async": ([_p, _p], c_int),
     "wd_get_positions_async": ([_p, _p], c_int),
     "wd_io_join": ([_p], c_int),

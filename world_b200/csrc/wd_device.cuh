@@ -29,11 +29,10 @@ enum Counter : int {
     kCntListExact = 8,      // list steps whose contact kernel read the build positions
     kCntStageTimeout = 9,   // bulk-staged contact kernel: stages that never completed
     kCntListResort = 10,    // list contact kernels: grains whose contacts were re-ordered
-    kCntLaunchFail = 11,    // device-side launches of a list build's graphs that failed
-    kCntAutoSteps = 12,     // steps on the library's own lists (neighbor_skin 0)
-    kCntAutoBuilds = 13,    // builds that such steps decided
-    kCntAutoCrowded = 14,   // a build found a cell that could overfill
-    kNumCounters = 15,
+    kCntAutoSteps = 11,     // steps on the library's own lists (neighbor_skin 0)
+    kCntAutoBuilds = 12,    // builds that such steps decided
+    kCntAutoCrowded = 13,   // a build found a cell that could overfill
+    kNumCounters = 14,
 };
 
 // Everything a step kernel needs, passed by value (baked into the captured graph).

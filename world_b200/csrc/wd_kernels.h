@@ -196,19 +196,19 @@ struct ListArgs {
 // tail-launches `graph` when *flag is nonzero (the step's build decision, or the search
 // asking for its radix path). The launched graph runs once the graph that
 // holds the launching kernel has completed; later work of the stream waits for it. A
-// failed launch counts in counters[kCntLaunchFail].
-void launch_graph_if(const uint32_t* flag, cudaGraphExec_t graph, unsigned long long* counters,
+// failed launch sets *failed, a word in pinned host memory.
+void launch_graph_if(const uint32_t* flag, cudaGraphExec_t graph, volatile uint32_t* failed,
                      cudaStream_t st);
 // The end of a chain of `steps` list steps: tail-launches the build that one of them decided,
 // if any, by whether that was an even or an odd one (from 0).
 void launch_graph_chain(const uint32_t* list_ctrl, int steps, cudaGraphExec_t even,
-                        cudaGraphExec_t odd, unsigned long long* counters, cudaStream_t st);
+                        cudaGraphExec_t odd, volatile uint32_t* failed, cudaStream_t st);
 // The end of a build: tail-launches the graph of the chain's steps left over, by_left[kLcLeft]
 // (device memory), if there are any, and clears kLcPending and kLcLeft; where the search
 // wants the radix path (radix_flag nonzero; NULL on that path itself), the graph that builds
 // that way instead. by_left NULL: no chain waits for this build.
 void launch_build_end(uint32_t* list_ctrl, const cudaGraphExec_t* by_left, const int* radix_flag,
-                      cudaGraphExec_t radix, unsigned long long* counters, cudaStream_t st);
+                      cudaGraphExec_t radix, volatile uint32_t* failed, cudaStream_t st);
 void launch_list_decide(uint32_t* list_ctrl, float thr, bool always_exact,
                         unsigned long long* counters, unsigned long long* pend, bool use_cond, cudaGraphConditionalHandle cond, cudaStream_t st);
 // The library's own lists under neighbor_skin 0: counts, per collision cell, the grains of

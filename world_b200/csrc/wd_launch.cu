@@ -20,24 +20,24 @@ namespace wd {
 namespace {
 
 __global__ void k_graph_if(const uint32_t* __restrict__ flag, cudaGraphExec_t graph,
-                           unsigned long long* __restrict__ counters) {
+                           volatile uint32_t* __restrict__ failed) {
     if (threadIdx.x != 0 || *flag == 0u) return;
     if (cudaGraphLaunch(graph, cudaStreamGraphTailLaunch) != cudaSuccess)
-        atomicAdd(&counters[kCntLaunchFail], 1ull);
+        *failed = 1u;
 }
 
 __global__ void k_graph_chain(const uint32_t* __restrict__ ctrl, int steps, cudaGraphExec_t even,
-                              cudaGraphExec_t odd, unsigned long long* __restrict__ counters) {
+                              cudaGraphExec_t odd, volatile uint32_t* __restrict__ failed) {
     if (threadIdx.x != 0 || ctrl[kLcDecision] == 0u) return;
     // the step that decided: the chain's steps before it are done, kLcLeft wait
     const int step = steps - 1 - static_cast<int>(ctrl[kLcLeft]);
     if (cudaGraphLaunch(step & 1 ? odd : even, cudaStreamGraphTailLaunch) != cudaSuccess)
-        atomicAdd(&counters[kCntLaunchFail], 1ull);
+        *failed = 1u;
 }
 
 __global__ void k_build_end(uint32_t* __restrict__ ctrl, const cudaGraphExec_t* __restrict__ by_left,
                             const int* __restrict__ radix_flag, cudaGraphExec_t radix,
-                            unsigned long long* __restrict__ counters) {
+                            volatile uint32_t* __restrict__ failed) {
     if (threadIdx.x != 0) return;
     cudaGraphExec_t next = nullptr;
     if (radix_flag != nullptr && *radix_flag != 0) {
@@ -49,28 +49,28 @@ __global__ void k_build_end(uint32_t* __restrict__ ctrl, const cudaGraphExec_t* 
         if (left > 0u) {
             next = by_left[left];
             // steps that nothing takes up are an error, not steps left out
-            if (next == nullptr) atomicAdd(&counters[kCntLaunchFail], 1ull);
+            if (next == nullptr) *failed = 1u;
         }
     }
     if (next != nullptr && cudaGraphLaunch(next, cudaStreamGraphTailLaunch) != cudaSuccess)
-        atomicAdd(&counters[kCntLaunchFail], 1ull);
+        *failed = 1u;
 }
 
 }  // namespace
 
 void launch_graph_chain(const uint32_t* list_ctrl, int steps, cudaGraphExec_t even,
-                        cudaGraphExec_t odd, unsigned long long* counters, cudaStream_t st) {
-    k_graph_chain<<<1, 32, 0, st>>>(list_ctrl, steps, even, odd, counters);
+                        cudaGraphExec_t odd, volatile uint32_t* failed, cudaStream_t st) {
+    k_graph_chain<<<1, 32, 0, st>>>(list_ctrl, steps, even, odd, failed);
 }
 
 void launch_build_end(uint32_t* list_ctrl, const cudaGraphExec_t* by_left, const int* radix_flag,
-                      cudaGraphExec_t radix, unsigned long long* counters, cudaStream_t st) {
-    k_build_end<<<1, 32, 0, st>>>(list_ctrl, by_left, radix_flag, radix, counters);
+                      cudaGraphExec_t radix, volatile uint32_t* failed, cudaStream_t st) {
+    k_build_end<<<1, 32, 0, st>>>(list_ctrl, by_left, radix_flag, radix, failed);
 }
 
-void launch_graph_if(const uint32_t* flag, cudaGraphExec_t graph, unsigned long long* counters,
+void launch_graph_if(const uint32_t* flag, cudaGraphExec_t graph, volatile uint32_t* failed,
                      cudaStream_t st) {
-    k_graph_if<<<1, 32, 0, st>>>(flag, graph, counters);
+    k_graph_if<<<1, 32, 0, st>>>(flag, graph, failed);
 }
 
 }  // namespace wd

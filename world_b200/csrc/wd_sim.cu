@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -64,6 +65,45 @@ int key_bits(uint64_t cells) {
         v >>= 1;
     }
     return b;
+}
+
+// A handle's words in page-locked host memory: the device writes them, the host reads them
+// without a copy (a copy with every wait cost a searched step 29 -> 42 us of a call and its
+// wait). Pages of 64 outlive the handles, which take one each and give it back: locking a page
+// for every handle would cost its creation milliseconds.
+struct alignas(64) HostWords {
+    volatile uint32_t launch_failed;   // a device-side graph launch failed: its work is missing
+};
+constexpr size_t kWordsPage = 4096;
+std::mutex words_lock;
+std::vector<HostWords*> words_free;
+
+HostWords* take_words() {
+    std::lock_guard<std::mutex> lock(words_lock);
+    if (words_free.empty()) {
+        void* page = std::aligned_alloc(kWordsPage, kWordsPage);
+        if (!page) return nullptr;
+        for (size_t at = kWordsPage; at > 0; at -= sizeof(HostWords))
+            words_free.push_back(reinterpret_cast<HostWords*>(static_cast<char*>(page) + at - sizeof(HostWords)));
+    }
+    HostWords* w = words_free.back();
+    // a new page, or one that a cudaDeviceReset has unlocked
+    cudaPointerAttributes is{};
+    if (cudaPointerGetAttributes(&is, w) != cudaSuccess || is.type != cudaMemoryTypeHost) {
+        cudaGetLastError();
+        void* page = reinterpret_cast<void*>(reinterpret_cast<uintptr_t>(w) & ~(kWordsPage - 1));
+        if (cudaHostRegister(page, kWordsPage, cudaHostRegisterPortable | cudaHostRegisterMapped) != cudaSuccess)
+            return nullptr;
+    }
+    words_free.pop_back();
+    std::memset(static_cast<void*>(w), 0, sizeof(*w));
+    return w;
+}
+
+void give_words(HostWords* w) {
+    if (!w) return;
+    std::lock_guard<std::mutex> lock(words_lock);
+    words_free.push_back(w);
 }
 
 }  // namespace
@@ -169,7 +209,7 @@ struct wd_sim {
     int64_t auto_off = 0, auto_backoff = 512;// steps to search before lists are tried again
     int64_t auto_look = 0;                   // list step of the run that reads the device's counts next
     unsigned long long auto_seen[2] = {0, 0};// list steps and builds at the last look
-    bool list_work = false;                  // list steps or builds since the last synchronise
+    bool list_work = false;                  // list steps since the last synchronise
     unsigned long long seen[wd::kNumCounters] = {};  // the counters as of the last synchronise
 
     // reverse pass: snapshots of the step state (checkpoints of a recorded window and
@@ -211,6 +251,8 @@ struct wd_sim {
     double* adj_theta = nullptr;
 
     unsigned long long* counters = nullptr;
+    HostWords* words = nullptr;           // what the device leaves for the host to find,
+    HostWords* d_words = nullptr;         // and its address on the device
     uint32_t* picard_res = nullptr;
     int* picard_used = nullptr;
     double* partials = nullptr;
@@ -431,6 +473,7 @@ void free_sim(wd_sim* s) {
     void* adj[] = {s->adj_lx[0], s->adj_lx[1], s->adj_lv[0], s->adj_lv[1], s->adj_lxi[0],
                    s->adj_lxi[1], s->adj_lvt, s->adj_lf, s->adj_theta};
     for (void* p : adj) cudaFree(p);
+    give_words(s->words);
     if (s->own_stream) cudaStreamDestroy(s->own_stream);
     if (s->aux_stream) cudaStreamDestroy(s->aux_stream);
     delete s;
@@ -616,7 +659,7 @@ cudaError_t enqueue_step(wd_sim* s, int parity, cudaStream_t st, bool capture,
             wd::launch_search_merge(P, s->idsA, s->sb, none, st);
             enqueue_step_tail(s, parity, st, nullptr, mover_gate(s));
             wd::launch_graph_if(reinterpret_cast<const uint32_t*>(s->sb.ctrl + 1),
-                                s->graph_now().radix, s->counters, st);
+                                s->graph_now().radix, &s->d_words->launch_failed, st);
             return cudaGetLastError();
         }
         cudaError_t e = enqueue_search(s, none, nullptr, 0, capture, st);
@@ -906,7 +949,7 @@ cudaError_t capture_build(wd_sim* s, cudaGraphExec_t* head, cudaGraphExec_t* rad
         wd::launch_search_radix(P, s->idsA, s->sb, none, st);
         enqueue_list_build_tail(s, none, st);
         if (resume)
-            wd::launch_build_end(s->list_ctrl, resume, nullptr, nullptr, s->counters, st);
+            wd::launch_build_end(s->list_ctrl, resume, nullptr, nullptr, &s->d_words->launch_failed, st);
     });
     if (e == cudaSuccess)
         e = capture_device_graph(s, head, [&](cudaStream_t st) {
@@ -914,7 +957,7 @@ cudaError_t capture_build(wd_sim* s, cudaGraphExec_t* head, cudaGraphExec_t* rad
                                    0, false, 0, s->counters, st);
             wd::launch_search_merge(P, s->idsA, s->sb, none, st);
             enqueue_list_build_tail(s, mover_gate(s), st);
-            wd::launch_build_end(s->list_ctrl, resume, s->sb.ctrl + 1, *radix, s->counters, st);
+            wd::launch_build_end(s->list_ctrl, resume, s->sb.ctrl + 1, *radix, &s->d_words->launch_failed, st);
         });
     return e;
 }
@@ -934,7 +977,7 @@ cudaError_t capture_device_builds(wd_sim* s) {
     if (e == cudaSuccess) e = capture_build(s, &g.head, &g.radix, s->chain_table + 8 * next);
     if (e == cudaSuccess)
         e = capture_device_graph(s, &g.build_if, [&](cudaStream_t st) {
-            wd::launch_graph_if(s->list_ctrl + wd::kLcDecision, g.head, s->counters, st);
+            wd::launch_graph_if(s->list_ctrl + wd::kLcDecision, g.head, &s->d_words->launch_failed, st);
         });
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux_stream);
     if (e != cudaSuccess) drop_device_graphs(g);
@@ -1000,7 +1043,7 @@ cudaError_t enqueue_step_list(wd_sim* s, int parity, cudaStream_t st, bool captu
     if (!capture && launcher) return cudaGraphLaunch(launcher, st);
     if (device_build) {
         // the build the kernel's last block decided on (kLcDecision), from the device
-        wd::launch_graph_if(s->list_ctrl + wd::kLcDecision, s->graph_now().head, s->counters, st);
+        wd::launch_graph_if(s->list_ctrl + wd::kLcDecision, s->graph_now().head, &s->d_words->launch_failed, st);
         return cudaGetLastError();
     }
     // the build the kernel's last block decided on, of the new state in B
@@ -1135,7 +1178,7 @@ cudaError_t capture_chains(wd_sim* s) {
                 swap_state(s);
                 if (hist) s->hist_cur ^= 1;
             }
-            wd::launch_graph_chain(s->list_ctrl, m, own, other, s->counters, st);
+            wd::launch_graph_chain(s->list_ctrl, m, own, other, &s->d_words->launch_failed, st);
             return be;
         };
         for (int m = 1; m < kChain && e == cudaSuccess; ++m) {
@@ -1297,7 +1340,7 @@ int ondemand_search(wd_sim* s) {
                 wd::launch_search_merge(s->P, s->idsA, s->sb, none, st);
                 enqueue_gather_c(s, st, gate);
                 wd::launch_graph_if(reinterpret_cast<const uint32_t*>(s->sb.ctrl + 1), g.radix,
-                                    s->counters, st);
+                                    &s->d_words->launch_failed, st);
             });
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux_stream);
         if (e != cudaSuccess) {
@@ -1308,7 +1351,6 @@ int ondemand_search(wd_sim* s) {
     }
     g.seen = true;
     if (g.head) {
-        s->list_work = true;   // a launch that fails on the device is looked for at the next wait
         WD_CUDA(cudaGraphLaunch(g.head, s->stream));
         return WD_OK;
     }
@@ -1320,22 +1362,22 @@ int ondemand_search(wd_sim* s) {
 }
 
 int sync_stream(wd_sim* s) {
-    // list builds that did not launch, and stages of the bulk-staged contact kernel that
-    // never arrived, are counted on the device: the counters come along with the wait
+    // stages of the bulk-staged contact kernel that never arrived are counted on the device, as
+    // are the builds of the library's own lists: the counters come along with the wait
     const bool lists = s->list_work;
     s->list_work = false;
     if (lists)
         WD_CUDA(cudaMemcpyAsync(s->seen, s->counters, sizeof(s->seen), cudaMemcpyDeviceToHost, s->stream));
     WD_CUDA(cudaStreamSynchronize(s->stream));
     WD_CUDA(cudaGetLastError());
-    if (!lists) return WD_OK;
-    if (s->seen[wd::kCntLaunchFail]) {
-        // a list build whose device-side graph launch failed did not run
-        WD_CUDA(cudaMemset(s->counters + wd::kCntLaunchFail, 0, sizeof(unsigned long long)));
+    if (s->words->launch_failed) {
+        // a list build, or a searched step's radix path, whose launch failed did not run
+        s->words->launch_failed = 0u;
         WD_CUDA(request_list_build(s));
         return fail(WD_ERR_CUDA, "list build or search: a device-side graph launch failed; the "
                                  "steps since the last synchronisation are invalid");
     }
+    if (!lists) return WD_OK;
     if (s->seen[wd::kCntStageTimeout]) {
         // reported once: the handle stays usable. The step stopped part-way, so even
         // its slot order may be mixed (the first step after a build rewrites the
@@ -1488,6 +1530,11 @@ int alloc_sim(wd_sim* s) {
     WD_CUDA(cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking));
     WD_CUDA(cudaStreamCreateWithFlags(&s->aux_stream, cudaStreamNonBlocking));
     s->stream = s->own_stream;
+    s->words = take_words();
+    if (!s->words) return fail(WD_ERR_OOM, "wd_create: no page-locked host memory");
+    void* words = nullptr;
+    WD_CUDA(cudaHostGetDevicePointer(&words, s->words, 0));
+    s->d_words = static_cast<HostWords*>(words);
     WD_CUDA(dalloc(&s->posA, n)); WD_CUDA(dalloc(&s->velA, n)); WD_CUDA(dalloc(&s->idsA, n));
     WD_CUDA(dalloc(&s->posB, n)); WD_CUDA(dalloc(&s->velB, n)); WD_CUDA(dalloc(&s->idsB, n));
     WD_CUDA(dalloc(&s->acc, n));
@@ -2777,6 +2824,12 @@ int wd_debug_stage_wait(wd_sim* sim, int32_t stall, int32_t wait_us) {
 int wd_debug_graph_captures(wd_sim* sim, int64_t* captures) {
     if (!sim || !captures) return fail(WD_ERR_INVALID, "wd_debug_graph_captures: NULL argument");
     *captures = sim->captures;
+    return WD_OK;
+}
+
+int wd_debug_launch_failure(wd_sim* sim) {
+    if (!sim) return fail(WD_ERR_INVALID, "wd_debug_launch_failure: NULL handle");
+    sim->words->launch_failed = 1u;
     return WD_OK;
 }
 
