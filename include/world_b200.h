@@ -140,7 +140,9 @@ int wd_chaos_metrics(wd_sim* sim, int32_t reference_scene, double* metrics3);
 
 /* ---- stepping: take_step() (src/particle_dynamics.cu:264-281) -------------------- */
 
-/* nsteps x take_step(), launched asynchronously on the handle's stream. */
+/* nsteps x take_step(), launched asynchronously on the handle's stream. (On lists of the
+ * library's own choice, see wd_set_neighbor_skin, a caller 256 steps ahead of the device's
+ * last known counts waits for newer ones.) */
 int wd_step(wd_sim* sim, int64_t nsteps);
 
 /* dt is re-read at every step, as the reference re-applies sim.dt

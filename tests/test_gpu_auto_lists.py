@@ -205,3 +205,43 @@ def test_the_stage_wait_hook_needs_lists_that_the_caller_asked_for():
         check(lib.wd_debug_stage_wait(sim.handle, 0, 0))
     sim.set_neighbor_skin(0.5e-3)
     check(lib.wd_debug_stage_wait(sim.handle, 0, 0))
+
+
+def test_a_rollout_is_queued_without_waiting():
+    """A hundred steps are queued behind half a second of other work on the handle's stream:
+    the call returns while that work still runs."""
+    torch = pytest.importorskip("torch")
+    cfg, st, rad = _touching(93, True)
+    cfg.kernel_timing = False
+    own, searched = _both(cfg, st, rad)
+    state = torch.from_numpy(st).cuda()
+    stream = torch.cuda.ExternalStream(own.stream_ptr())
+    for k in range(4):
+        if k == 3:                              # graphs and chains exist by now
+            own.synchronize()
+            with torch.cuda.stream(stream):
+                torch.cuda._sleep(1_000_000_000)
+            busy = torch.cuda.Event()
+            busy.record(stream)
+        for sim in (own, searched) if k < 3 else (own,):
+            sim.set_state_tensor(state)
+            sim.advance(100)
+    assert not busy.query()
+    searched.set_state_tensor(state)
+    searched.advance(100)
+    assert own.kernels_per_step() == 2
+    _equal(own, searched)
+
+
+def test_lists_that_do_not_pay_are_left_within_one_call():
+    """One call of 500 steps, nothing read meanwhile: the handle tries lists, learns that
+    nearly every step builds, and searches by the end of it."""
+    cfg, st, rad = packed_poly(n=2500, seed=63, history=False)
+    cfg.kernel_timing = False
+    st = st.copy()
+    st[:, 3] += 60.0
+    own, searched = _both(cfg, st, rad)
+    own.advance(500)
+    assert own.kernels_per_step() == 6
+    searched.advance(500)
+    _equal(own, searched)

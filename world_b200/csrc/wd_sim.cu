@@ -73,6 +73,7 @@ int key_bits(uint64_t cells) {
 // for every handle would cost its creation milliseconds.
 struct alignas(64) HostWords {
     volatile uint32_t launch_failed;   // a device-side graph launch failed: its work is missing
+    unsigned long long looked[3];      // kCntAutoSteps, Builds, Crowded, as of ev_look
 };
 constexpr size_t kWordsPage = 4096;
 std::mutex words_lock;
@@ -207,7 +208,10 @@ struct wd_sim {
     int64_t run_steps = 0, last_run = 0;     // steps since the last upload, and between the two before
     int64_t auto_wait = 0;                   // steps a new handle searches unless it has as many to come
     int64_t auto_off = 0, auto_backoff = 512;// steps to search before lists are tried again
-    int64_t auto_look = 0;                   // list step of the run that reads the device's counts next
+    int64_t auto_look = 0;                   // list step of the run that asks for the device's counts next
+    int64_t auto_steps = 0;                  // steps of the handle's life, searched or not
+    int64_t auto_asked = -1;                 // auto_steps when the counts on their way were asked for, or -1
+    cudaEvent_t ev_look = nullptr;           // they have arrived
     unsigned long long auto_seen[2] = {0, 0};// list steps and builds at the last look
     bool list_work = false;                  // list steps since the last synchronise
     unsigned long long seen[wd::kNumCounters] = {};  // the counters as of the last synchronise
@@ -468,6 +472,7 @@ void free_sim(wd_sim* s) {
             if (e) cudaEventDestroy(e);
     }
     if (s->ev_join) cudaEventDestroy(s->ev_join);
+    if (s->ev_look) cudaEventDestroy(s->ev_look);
     if (s->io_up) cudaStreamDestroy(s->io_up);
     if (s->io_down) cudaStreamDestroy(s->io_down);
     void* adj[] = {s->adj_lx[0], s->adj_lx[1], s->adj_lv[0], s->adj_lv[1], s->adj_lxi[0],
@@ -1366,8 +1371,10 @@ int sync_stream(wd_sim* s) {
     // are the builds of the library's own lists: the counters come along with the wait
     const bool lists = s->list_work;
     s->list_work = false;
-    if (lists)
+    if (lists) {
+        s->auto_asked = -1;   // what is on its way is older
         WD_CUDA(cudaMemcpyAsync(s->seen, s->counters, sizeof(s->seen), cudaMemcpyDeviceToHost, s->stream));
+    }
     WD_CUDA(cudaStreamSynchronize(s->stream));
     WD_CUDA(cudaGetLastError());
     if (s->words->launch_failed) {
@@ -1457,6 +1464,7 @@ void auto_prepare(wd_sim* s) {
         if (e == cudaSuccess)
             e = cudaMemsetAsync(pend, 0, sizeof(unsigned long long) * wd::kNumCounters, s->stream);
         s->auto_pend = pend;
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev_look, cudaEventDisableTiming);
         ok = e == cudaSuccess;
     }
     if (!ok) cudaGetLastError();
@@ -1475,18 +1483,36 @@ void auto_prepare(wd_sim* s) {
 // steps, searched against lists: 2^20 falling grains 75 + 157 k and 260 + 37 k us,
 // 100,003 packed 30 + 113 k and 100 + 31 k, the default cube 68 + 98 k and 175 + 10 k.
 constexpr int64_t kAutoRun = 3;
+constexpr int64_t kAutoAhead = 256;
 
 cudaError_t auto_mode(wd_sim* s, int64_t ahead) {
     if (s->auto_off > 0) --s->auto_off;
     if (s->lists) {
-        // the device's counts come with every synchronise; without one for long, they are
-        // read after 32 list steps and then every 256
-        if (s->run_steps >= s->auto_look) {
+        // The device's counts come with every synchronise; without one for long, they are asked
+        // for after 32 list steps and then every 256, and looked at once they are there. A host
+        // that has gone another kAutoAhead steps by then waits for them, so that lists which do
+        // not pay are left after a bounded number of steps.
+        static_assert(wd::kCntAutoBuilds == wd::kCntAutoSteps + 1 && wd::kCntAutoCrowded == wd::kCntAutoSteps + 2,
+                      "copied together");
+        if (s->auto_asked >= 0) {
+            const bool wait = s->auto_steps - s->auto_asked >= kAutoAhead;
+            const cudaError_t e = wait ? cudaEventSynchronize(s->ev_look) : cudaEventQuery(s->ev_look);
+            if (e == cudaSuccess) {
+                std::memcpy(s->seen + wd::kCntAutoSteps, s->words->looked, sizeof(s->words->looked));
+                s->auto_asked = -1;
+            } else if (e == cudaErrorNotReady) {
+                cudaGetLastError();
+            } else {
+                return e;
+            }
+        }
+        if (s->auto_asked < 0 && s->run_steps >= s->auto_look) {
             s->auto_look = s->run_steps + 256;
-            cudaError_t e = cudaMemcpyAsync(s->seen, s->counters, sizeof(s->seen), cudaMemcpyDeviceToHost,
-                                            s->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+            cudaError_t e = cudaMemcpyAsync(s->words->looked, s->counters + wd::kCntAutoSteps,
+                                            sizeof(s->words->looked), cudaMemcpyDeviceToHost, s->stream);
+            if (e == cudaSuccess) e = cudaEventRecord(s->ev_look, s->stream);
             if (e != cudaSuccess) return e;
+            s->auto_asked = s->auto_steps;
         }
         const unsigned long long steps = s->seen[wd::kCntAutoSteps] - s->auto_seen[0];
         const unsigned long long builds = s->seen[wd::kCntAutoBuilds] - s->auto_seen[1];
@@ -1991,6 +2017,7 @@ int wd_step(wd_sim* sim, int64_t nsteps) {
                     WD_CUDA(cudaGraphLaunch(chain, sim->stream));
                     for (int i = 0; i < kChain; ++i) sim->time += sim->dt;
                     sim->run_steps += kChain;
+                    sim->auto_steps += kChain;
                     k += kChain;
                     continue;
                 }
@@ -1998,6 +2025,7 @@ int wd_step(wd_sim* sim, int64_t nsteps) {
             ++sim->list_steps;
         }
         ++sim->run_steps;
+        ++sim->auto_steps;
         ++k;
         if (sim->cfg.kernel_timing) {
             const int rc = timed_step(sim, parity);
