@@ -45,6 +45,7 @@ int fail(int code, const std::string& msg) {
     do {                                                                                \
         const cudaError_t e_ = (call);                                                  \
         if (e_ != cudaSuccess) {                                                        \
+            cudaGetLastError(); /* reported here, not once more by a later call */      \
             return fail(e_ == cudaErrorMemoryAllocation ? WD_ERR_OOM : WD_ERR_CUDA,     \
                         std::string(#call) + ": " + cudaGetErrorString(e_));            \
         }                                                                               \
