@@ -58,6 +58,27 @@ cudaError_t dalloc(T** p, size_t count) {
     return cudaMalloc(reinterpret_cast<void**>(p), count * sizeof(T));
 }
 
+// The same unless it is there: sets of buffers whose allocation failed part-way are completed
+// when they are next needed.
+template <typename T>
+cudaError_t dalloc_missing(T** p, size_t count) {
+    return *p ? cudaSuccess : dalloc(p, count);
+}
+
+// Streams and events likewise. (A failed creation may leave a handle behind.)
+cudaError_t create_missing(cudaStream_t* p) {
+    if (*p) return cudaSuccess;
+    const cudaError_t e = cudaStreamCreateWithFlags(p, cudaStreamNonBlocking);
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+cudaError_t create_missing(cudaEvent_t* p) {
+    if (*p) return cudaSuccess;
+    const cudaError_t e = cudaEventCreateWithFlags(p, cudaEventDisableTiming);
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+
 int key_bits(uint64_t cells) {
     int b = 0;
     uint64_t v = cells > 0 ? cells - 1 : 0;
@@ -251,8 +272,8 @@ struct wd_sim {
     float4* adj_lx[2] = {nullptr, nullptr};
     float4* adj_lv[2] = {nullptr, nullptr};
     float4* adj_lxi[2] = {nullptr, nullptr};
-    float4* adj_lvt = nullptr;
-    float4* adj_lf = nullptr;
+    float4* vjp_x = nullptr;   // the deposit's pullback by grain id
+    float4* vjp_v = nullptr;
     double* adj_theta = nullptr;
 
     unsigned long long* counters = nullptr;
@@ -382,25 +403,25 @@ void free_tape(wd_sim* s) {
 
 cudaError_t alloc_tape_step(wd_sim* s, wd_sim::TapeStep& t) {
     const size_t n = static_cast<size_t>(s->n);
-    cudaError_t e = dalloc(&t.pos, n);
-    if (e == cudaSuccess) e = dalloc(&t.vel, n);
-    if (e == cudaSuccess) e = dalloc(&t.ids, n);
-    if (e == cudaSuccess) e = dalloc(&t.clist, n * wd::kAdjContacts);
-    if (e == cudaSuccess) e = dalloc(&t.ccnt, n);
-    if (e == cudaSuccess && s->P.history) e = dalloc(&t.hcnt, n);
-    if (e == cudaSuccess && s->P.history) e = dalloc(&t.hist, n * wd::kHistCap);
-    if (e == cudaSuccess && s->P.history) e = dalloc(&t.cnt_id, n);
+    cudaError_t e = dalloc_missing(&t.pos, n);
+    if (e == cudaSuccess) e = dalloc_missing(&t.vel, n);
+    if (e == cudaSuccess) e = dalloc_missing(&t.ids, n);
+    if (e == cudaSuccess) e = dalloc_missing(&t.clist, n * wd::kAdjContacts);
+    if (e == cudaSuccess) e = dalloc_missing(&t.ccnt, n);
+    if (e == cudaSuccess && s->P.history) e = dalloc_missing(&t.hcnt, n);
+    if (e == cudaSuccess && s->P.history) e = dalloc_missing(&t.hist, n * wd::kHistCap);
+    if (e == cudaSuccess && s->P.history) e = dalloc_missing(&t.cnt_id, n);
     return e;
 }
 
 cudaError_t alloc_snap(wd_sim* s, wd_sim::Snap& q) {
     const size_t n = static_cast<size_t>(s->n);
-    cudaError_t e = dalloc(&q.pos, n);
-    if (e == cudaSuccess) e = dalloc(&q.vel, n);
-    if (e == cudaSuccess) e = dalloc(&q.ids, n);
-    if (e == cudaSuccess) e = dalloc(&q.keys, n);
-    if (e == cudaSuccess && s->P.history) e = dalloc(&q.hcnt, n);
-    if (e == cudaSuccess && s->P.history) e = dalloc(&q.hist, n * wd::kHistCap);
+    cudaError_t e = dalloc_missing(&q.pos, n);
+    if (e == cudaSuccess) e = dalloc_missing(&q.vel, n);
+    if (e == cudaSuccess) e = dalloc_missing(&q.ids, n);
+    if (e == cudaSuccess) e = dalloc_missing(&q.keys, n);
+    if (e == cudaSuccess && s->P.history) e = dalloc_missing(&q.hcnt, n);
+    if (e == cudaSuccess && s->P.history) e = dalloc_missing(&q.hist, n * wd::kHistCap);
     return e;
 }
 
@@ -477,7 +498,7 @@ void free_sim(wd_sim* s) {
     if (s->io_up) cudaStreamDestroy(s->io_up);
     if (s->io_down) cudaStreamDestroy(s->io_down);
     void* adj[] = {s->adj_lx[0], s->adj_lx[1], s->adj_lv[0], s->adj_lv[1], s->adj_lxi[0],
-                   s->adj_lxi[1], s->adj_lvt, s->adj_lf, s->adj_theta};
+                   s->adj_lxi[1], s->vjp_x, s->vjp_v, s->adj_theta};
     for (void* p : adj) cudaFree(p);
     give_words(s->words);
     if (s->own_stream) cudaStreamDestroy(s->own_stream);
@@ -1465,7 +1486,7 @@ void auto_prepare(wd_sim* s) {
         if (e == cudaSuccess)
             e = cudaMemsetAsync(pend, 0, sizeof(unsigned long long) * wd::kNumCounters, s->stream);
         s->auto_pend = pend;
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev_look, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = create_missing(&s->ev_look);
         ok = e == cudaSuccess;
     }
     if (!ok) cudaGetLastError();
@@ -2232,18 +2253,18 @@ int wd_synchronize(wd_sim* sim) {
 }
 
 static int io_setup(wd_sim* s) {
-    if (s->io_up) return WD_OK;
+    if (s->ev_join) return WD_OK;   // the last of it
     const size_t n = static_cast<size_t>(s->n);
-    WD_CUDA(cudaStreamCreateWithFlags(&s->io_up, cudaStreamNonBlocking));
-    WD_CUDA(cudaStreamCreateWithFlags(&s->io_down, cudaStreamNonBlocking));
+    WD_CUDA(create_missing(&s->io_up));
+    WD_CUDA(create_missing(&s->io_down));
     for (int b = 0; b < 2; ++b) {
-        WD_CUDA(dalloc(&s->io_in[b], 6 * n));
-        WD_CUDA(dalloc(&s->io_out[b], 3 * n));
+        WD_CUDA(dalloc_missing(&s->io_in[b], 6 * n));
+        WD_CUDA(dalloc_missing(&s->io_out[b], 3 * n));
         cudaEvent_t* evs[] = {&s->ev_in_ready[b], &s->ev_in_free[b], &s->ev_out_ready[b],
                               &s->ev_out_free[b]};
-        for (cudaEvent_t* e : evs) WD_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        for (cudaEvent_t* e : evs) WD_CUDA(create_missing(e));
     }
-    WD_CUDA(cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming));
+    WD_CUDA(create_missing(&s->ev_join));
     return WD_OK;
 }
 
@@ -2365,7 +2386,7 @@ int wd_density_grid_nodes(const wd_sim* sim, int64_t* nodes) {
 int wd_compute_density_grid_device(wd_sim* sim, float* d_grid) {
     if (!sim || !d_grid) return fail(WD_ERR_INVALID, "wd_compute_density_grid_device: NULL argument");
     if (!sim->dep_acc) {
-        WD_CUDA(dalloc(&sim->dep_bounds, static_cast<size_t>(4) * sim->scenes));
+        WD_CUDA(dalloc_missing(&sim->dep_bounds, static_cast<size_t>(4) * sim->scenes));
         WD_CUDA(dalloc(&sim->dep_acc, static_cast<size_t>(4) * sim->dep_nodes));
     }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -2584,9 +2605,9 @@ int wd_debug_candidates(wd_sim* sim, int64_t* offsets, int32_t* cand, uint8_t* c
     int rc = ondemand_search(sim);
     if (rc) return rc;
     const int n = sim->n;
-    if (!sim->cand_count) {
-        WD_CUDA(dalloc(&sim->cand_count, n));
-        WD_CUDA(dalloc(&sim->cand_offsets, static_cast<size_t>(n) + 1));
+    if (!sim->cand_offsets) {
+        WD_CUDA(dalloc_missing(&sim->cand_count, n));
+        WD_CUDA(dalloc_missing(&sim->cand_offsets, static_cast<size_t>(n) + 1));
     }
     wd::launch_candidate_count(sim->P, tab(sim, sim->sceneC), sim->posC, sim->idsC, sim->sb.table,
                                sim->cand_count, sim->stream);
@@ -2629,17 +2650,20 @@ static int apply_skin(wd_sim* s, float skin) {
     s->auto_ok = false;   // the caller's choice, 0 included
     if (lists) WD_CUDA(alloc_list_buffers(s));
     s->skin_asked |= lists;
-    if (lists && s->picard && !s->xpos) {
+    if (lists && s->picard) {
         const int n = s->n;
-        WD_CUDA(dalloc(&s->xpos, n));
-        WD_CUDA(dalloc(&s->xvel, n));
-        WD_CUDA(dalloc(&s->xids, n));
-        WD_CUDA(dalloc(&s->rhs_vel, n));
-        WD_CUDA(dalloc(&s->rhs_ids, n));
-        // the rhs getter reads these in list mode: start them at the current rhs source
-        WD_CUDA(cudaMemcpyAsync(s->rhs_vel, s->velB, sizeof(float4) * n, cudaMemcpyDeviceToDevice, s->stream));
-        WD_CUDA(cudaMemcpyAsync(s->rhs_ids, s->idsB, sizeof(int) * n, cudaMemcpyDeviceToDevice, s->stream));
-        if (s->scenes > 1) WD_CUDA(dalloc(&s->xscene, n));
+        const bool fresh = !s->rhs_ids;   // the last of them
+        WD_CUDA(dalloc_missing(&s->xpos, n));
+        WD_CUDA(dalloc_missing(&s->xvel, n));
+        WD_CUDA(dalloc_missing(&s->xids, n));
+        if (s->scenes > 1) WD_CUDA(dalloc_missing(&s->xscene, n));
+        WD_CUDA(dalloc_missing(&s->rhs_vel, n));
+        WD_CUDA(dalloc_missing(&s->rhs_ids, n));
+        if (fresh) {
+            // the rhs getter reads these in list mode: start them at the current rhs source
+            WD_CUDA(cudaMemcpyAsync(s->rhs_vel, s->velB, sizeof(float4) * n, cudaMemcpyDeviceToDevice, s->stream));
+            WD_CUDA(cudaMemcpyAsync(s->rhs_ids, s->idsB, sizeof(int) * n, cudaMemcpyDeviceToDevice, s->stream));
+        }
     }
     s->lists = lists;
     s->cfg.neighbor_skin = skin;
@@ -3022,11 +3046,11 @@ int wd_adjoint_record(wd_sim* sim, int64_t steps, int32_t checkpoint_every) {
     // snapshots are kept between windows and grown when a window needs more
     const size_t nck = static_cast<size_t>((steps + checkpoint_every - 1) / checkpoint_every);
     sim->adj_steps = 0;
-    for (size_t k = sim->adj_ckpt.size(); k < nck; ++k) {
-        sim->adj_ckpt.emplace_back();
-        WD_CUDA(alloc_snap(sim, sim->adj_ckpt.back()));
+    for (size_t k = 0; k < nck; ++k) {
+        if (k == sim->adj_ckpt.size()) sim->adj_ckpt.emplace_back();
+        WD_CUDA(alloc_snap(sim, sim->adj_ckpt[k]));
     }
-    if (!sim->adj_end.pos) WD_CUDA(alloc_snap(sim, sim->adj_end));
+    WD_CUDA(alloc_snap(sim, sim->adj_end));
     sim->last_run = std::max(sim->last_run, steps);   // the run's length is known
     int64_t hist_over0 = 0;
     rc = read_counter(sim, wd::kCntHistOverflow, &hist_over0);
@@ -3055,21 +3079,17 @@ int wd_adjoint_backward(wd_sim* sim, const float* d_gx, const float* d_gv, float
     const int n = sim->n;
     cudaStream_t st = sim->stream;
     const bool hist = sim->P.history != 0;
-    if (!sim->adj_lvt) {
-        for (int b = 0; b < 2; ++b) {
-            WD_CUDA(dalloc(&sim->adj_lx[b], n));
-            WD_CUDA(dalloc(&sim->adj_lv[b], n));
-            if (hist) WD_CUDA(dalloc(&sim->adj_lxi[b], static_cast<size_t>(n) * wd::kHistCap));
-        }
-        WD_CUDA(dalloc(&sim->adj_lvt, n));
-        WD_CUDA(dalloc(&sim->adj_lf, n));
-        WD_CUDA(dalloc(&sim->adj_theta, static_cast<size_t>(3) * n));
+    for (int b = 0; b < 2; ++b) {
+        WD_CUDA(dalloc_missing(&sim->adj_lx[b], n));
+        WD_CUDA(dalloc_missing(&sim->adj_lv[b], n));
+        if (hist) WD_CUDA(dalloc_missing(&sim->adj_lxi[b], static_cast<size_t>(n) * wd::kHistCap));
     }
+    WD_CUDA(dalloc_missing(&sim->adj_theta, static_cast<size_t>(3) * n));
     const int every = sim->adj_every;
     if (sim->adj_tape.size() < static_cast<size_t>(every) + 1) clear_adj_graphs(sim);
-    for (size_t k = sim->adj_tape.size(); k < static_cast<size_t>(every) + 1; ++k) {
-        sim->adj_tape.emplace_back();
-        WD_CUDA(alloc_tape_step(sim, sim->adj_tape.back()));
+    for (size_t k = 0; k < static_cast<size_t>(every) + 1; ++k) {
+        if (k == sim->adj_tape.size()) sim->adj_tape.emplace_back();
+        WD_CUDA(alloc_tape_step(sim, sim->adj_tape[k]));
     }
     if (!sim->adj_ovf) WD_CUDA(dalloc(&sim->adj_ovf, 1));
     WD_CUDA(cudaMemsetAsync(sim->adj_ovf, 0, sizeof(unsigned long long), st));
@@ -3131,22 +3151,12 @@ int wd_deposit_vjp(wd_sim* sim, const float* d_ggrid, float* d_gx, float* d_gv) 
     if (!sim || !d_ggrid) return fail(WD_ERR_INVALID, "wd_deposit_vjp: NULL argument");
     if (sim->scenes != 1) return fail(WD_ERR_INVALID, "wd_deposit_vjp: not for a batch of scenes");
     const int n = sim->n;
-    if (!sim->adj_lvt) {
-        for (int b = 0; b < 2; ++b) {
-            WD_CUDA(dalloc(&sim->adj_lx[b], n));
-            WD_CUDA(dalloc(&sim->adj_lv[b], n));
-        }
-        WD_CUDA(dalloc(&sim->adj_lvt, n));
-        WD_CUDA(dalloc(&sim->adj_lf, n));
-        WD_CUDA(dalloc(&sim->adj_theta, static_cast<size_t>(3) * n));
-        if (sim->P.history)
-            for (int b = 0; b < 2; ++b)
-                WD_CUDA(dalloc(&sim->adj_lxi[b], static_cast<size_t>(n) * wd::kHistCap));
-    }
+    WD_CUDA(dalloc_missing(&sim->vjp_x, n));
+    WD_CUDA(dalloc_missing(&sim->vjp_v, n));
     wd::launch_deposit_vjp(n, sim->posA, sim->velA, sim->idsA, sim->cfg.dom_lo, sim->cfg.dom_hi,
-                           sim->cfg.dgrid, d_ggrid, sim->adj_lvt, sim->adj_lf, sim->stream);
-    if (d_gx) wd::launch_f4_to_aos3(n, sim->adj_lvt, d_gx, sim->stream);
-    if (d_gv) wd::launch_f4_to_aos3(n, sim->adj_lf, d_gv, sim->stream);
+                           sim->cfg.dgrid, d_ggrid, sim->vjp_x, sim->vjp_v, sim->stream);
+    if (d_gx) wd::launch_f4_to_aos3(n, sim->vjp_x, d_gx, sim->stream);
+    if (d_gv) wd::launch_f4_to_aos3(n, sim->vjp_v, d_gv, sim->stream);
     WD_CUDA(cudaGetLastError());
     return sync_stream(sim);
 }
@@ -3208,22 +3218,22 @@ int wd_chaos_metrics(wd_sim* sim, int32_t reference_scene, double* metrics3) {
                                         "count and density grid");
     }
     const int total_nodes = static_cast<int>(sim->dep_nodes);
-    if (!sim->d_node_seg) {
+    if (!sim->chaos_grid) {
         std::vector<int> seg(S + 1), chunk(S + 1);
         chunk[0] = 0;
         for (int k = 0; k <= S; ++k) seg[k] = static_cast<int>(sim->scene_nodes_off[k]);
         for (int k = 0; k < S; ++k)
             chunk[k + 1] = chunk[k] + static_cast<int>((seg[k + 1] - seg[k] + wd::kBlock - 1) / wd::kBlock);
         sim->node_chunks = chunk[S];
-        WD_CUDA(dalloc(&sim->d_node_seg, S + 1));
-        WD_CUDA(dalloc(&sim->d_node_chunk, S + 1));
+        WD_CUDA(dalloc_missing(&sim->d_node_seg, S + 1));
+        WD_CUDA(dalloc_missing(&sim->d_node_chunk, S + 1));
         WD_CUDA(cudaMemcpy(sim->d_node_seg, seg.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice));
         WD_CUDA(cudaMemcpy(sim->d_node_chunk, chunk.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice));
-        WD_CUDA(dalloc(&sim->node_vals, static_cast<size_t>(6) * total_nodes));
-        WD_CUDA(dalloc(&sim->chaos_partials, static_cast<size_t>(6) * sim->node_chunks));
-        WD_CUDA(dalloc(&sim->chaos_sums, static_cast<size_t>(6) * S));
-        WD_CUDA(dalloc(&sim->grain_sums, S));
-        WD_CUDA(dalloc(&sim->chaos_grid, static_cast<size_t>(4) * total_nodes));
+        WD_CUDA(dalloc_missing(&sim->node_vals, static_cast<size_t>(6) * total_nodes));
+        WD_CUDA(dalloc_missing(&sim->chaos_partials, static_cast<size_t>(6) * sim->node_chunks));
+        WD_CUDA(dalloc_missing(&sim->chaos_sums, static_cast<size_t>(6) * S));
+        WD_CUDA(dalloc_missing(&sim->grain_sums, S));
+        WD_CUDA(dalloc_missing(&sim->chaos_grid, static_cast<size_t>(4) * total_nodes));
     }
     int rc = wd_compute_density_grid_device(sim, sim->chaos_grid);
     if (rc) return rc;
