@@ -601,6 +601,8 @@ def run_ours(args) -> int:
                               "grains": sim.n, "springs_per_grain": float(cnt.sum()) / sim.n}))
             sim.close()
             return 0
+    if args.skin == 0.0:
+        sim.set_neighbor_skin(0.0)   # a configuration without a skin may step on the library's lists
     sim.set_kernel_timing(args.direct)
     tuned = None
     if args.skin < 0:
