@@ -277,8 +277,9 @@ int wd_grid_overflow_count(wd_sim* sim, int64_t* count);
  * never switched uses lists of the library's own where a run of three steps or more
  * between state uploads pays for them: the same states, springs and counts to the bit
  * (single scenes, semi-implicit Euler, cells at least one largest diameter wide, list
- * buffers of at most a quarter of the free device memory); calling this (or the
- * autotuner) ends that. */
+ * buffers, 248 bytes a grain and 4 a cell, of at most a quarter of the free device memory at
+ * creation, given back when another call of the handle finds too little); calling this (or
+ * the autotuner) ends that. */
 int wd_set_neighbor_skin(wd_sim* sim, float skin);
 /* Autotuner (extension): times `steps` steps, one by one, from the same saved state with a
  * search every step and, for each neighbor skin in {0.05, 0.1, 0.15, 0.2, 0.3, 0.4} mean

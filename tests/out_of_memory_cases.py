@@ -17,6 +17,7 @@ pytestmark = pytest.mark.gpu
 
 def test_a_failed_allocation_is_reported_once():
     sc = column_collapse(1 << 16, diameters="uniform", mu=0.5, cic=16)
+    sc.cfg.neighbor_skin = 0.5e-3              # lists that do not give way
     sc.cfg.kernel_timing = False
     sim = ParticleDynamics(sc.cfg, state=sc.state, radius=sc.radius)
     sim.advance(1)
@@ -40,6 +41,7 @@ def test_a_failed_allocation_is_reported_once():
 def test_a_window_survives_a_failed_allocation(left):
     n, steps, every = 1 << 15, 8, 8
     sc = column_collapse(n, diameters="uniform", mu=0.5, cic=16)
+    sc.cfg.neighbor_skin = 0.5e-3              # lists that do not give way
     sc.cfg.kernel_timing = False
     g = torch.from_numpy(np.random.default_rng(94).normal(size=(n, 3)).astype(np.float32)).cuda()
     grid = torch.ones(4 * 16 ** 3, device="cuda")
@@ -94,6 +96,7 @@ def test_lists_for_picard_survive_a_failed_allocation(left):
 @pytest.mark.parametrize("left", [3 << 20, 5 << 20])
 def test_asynchronous_copies_survive_a_failed_allocation(left):
     sc = column_collapse(1 << 16, diameters="uniform", mu=0.5, cic=16)
+    sc.cfg.neighbor_skin = 0.5e-3              # lists that do not give way
     sc.cfg.kernel_timing = False
     sim = ParticleDynamics(sc.cfg, state=sc.state, radius=sc.radius)
     host = torch.from_numpy(sc.state.copy()).pin_memory()
@@ -107,3 +110,32 @@ def test_asynchronous_copies_survive_a_failed_allocation(left):
     sim.synchronize()
     np.testing.assert_array_equal(sim.get_state(), sc.state.reshape(sim.get_state().shape))
     sim.close()
+
+
+@pytest.mark.parametrize("first", [1, 200])
+def test_the_librarys_own_lists_give_way(first):
+    """2^18 grains without springs: a checkpoint takes 10 MB, a deposit's accumulators 64, the
+    lists that the handle holds for itself 65. Four megabytes are left."""
+    n = 1 << 18
+    sc = column_collapse(n, diameters="uniform", mu=0.0, cic=64)
+    sc.cfg.history = False
+    sc.cfg.kernel_timing = False
+    out = []
+    for short in (False, True):
+        sim = ParticleDynamics(sc.cfg, state=sc.state, radius=sc.radius)
+        sim.advance(first)
+        sim.advance(first)
+        fill = short and torch.empty(torch.cuda.mem_get_info()[0] - (4 << 20), dtype=torch.uint8, device="cuda")
+        sim.adjoint_record(4, 2)
+        sim.advance(40)
+        if short:
+            assert sim.kernels_per_step() == 6
+        del fill
+        torch.cuda.empty_cache()
+        sim.advance(10)
+        sim.set_neighbor_skin(0.5e-3)
+        sim.advance(10)
+        out.append((sim.get_state(), sim.get_rhs(), sim.compute_momentum(), sim.grid_overflow_count()))
+        sim.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)

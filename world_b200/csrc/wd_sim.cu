@@ -58,14 +58,7 @@ cudaError_t dalloc(T** p, size_t count) {
     return cudaMalloc(reinterpret_cast<void**>(p), count * sizeof(T));
 }
 
-// The same unless it is there: sets of buffers whose allocation failed part-way are completed
-// when they are next needed.
-template <typename T>
-cudaError_t dalloc_missing(T** p, size_t count) {
-    return *p ? cudaSuccess : dalloc(p, count);
-}
-
-// Streams and events likewise. (A failed creation may leave a handle behind.)
+// A stream or event unless it is there. (A failed creation may leave a handle behind.)
 cudaError_t create_missing(cudaStream_t* p) {
     if (*p) return cudaSuccess;
     const cudaError_t e = cudaStreamCreateWithFlags(p, cudaStreamNonBlocking);
@@ -401,27 +394,57 @@ void free_tape(wd_sim* s) {
     s->adj_every = 0;
 }
 
+// The memory of the library's own lists back to the device: the handle searches from then on.
+bool drop_own_lists(wd_sim* s) {
+    if (!s->nbr || s->cfg.neighbor_skin > 0.f) return false;
+    destroy_graphs(s);   // and waits for the steps that use them
+    s->auto_ok = s->lists = s->need_build = false;
+    void* bufs[] = {s->nbr, s->nbr_cnt, s->xbuild, s->list_ctrl, s->list_len, s->tail_count,
+                    s->auto_pend, s->auto_load};
+    for (void* b : bufs) cudaFree(b);
+    s->nbr = s->nbr_cnt = nullptr;
+    s->xbuild = nullptr;
+    s->list_ctrl = s->auto_load = nullptr;
+    s->list_len = s->auto_pend = nullptr;
+    s->tail_count = nullptr;
+    return true;
+}
+
+// A buffer that a handle allocates on demand, unless it is there: sets of them whose allocation
+// failed part-way are completed when they are next needed. A call is not refused for memory that
+// the handle's own lists hold.
+template <typename T>
+cudaError_t dalloc_missing(wd_sim* s, T** p, size_t count) {
+    if (*p) return cudaSuccess;
+    cudaError_t e = dalloc(p, count);
+    if (e == cudaErrorMemoryAllocation && drop_own_lists(s)) {
+        cudaGetLastError();
+        e = dalloc(p, count);
+    }
+    return e;
+}
+
 cudaError_t alloc_tape_step(wd_sim* s, wd_sim::TapeStep& t) {
     const size_t n = static_cast<size_t>(s->n);
-    cudaError_t e = dalloc_missing(&t.pos, n);
-    if (e == cudaSuccess) e = dalloc_missing(&t.vel, n);
-    if (e == cudaSuccess) e = dalloc_missing(&t.ids, n);
-    if (e == cudaSuccess) e = dalloc_missing(&t.clist, n * wd::kAdjContacts);
-    if (e == cudaSuccess) e = dalloc_missing(&t.ccnt, n);
-    if (e == cudaSuccess && s->P.history) e = dalloc_missing(&t.hcnt, n);
-    if (e == cudaSuccess && s->P.history) e = dalloc_missing(&t.hist, n * wd::kHistCap);
-    if (e == cudaSuccess && s->P.history) e = dalloc_missing(&t.cnt_id, n);
+    cudaError_t e = dalloc_missing(s, &t.pos, n);
+    if (e == cudaSuccess) e = dalloc_missing(s, &t.vel, n);
+    if (e == cudaSuccess) e = dalloc_missing(s, &t.ids, n);
+    if (e == cudaSuccess) e = dalloc_missing(s, &t.clist, n * wd::kAdjContacts);
+    if (e == cudaSuccess) e = dalloc_missing(s, &t.ccnt, n);
+    if (e == cudaSuccess && s->P.history) e = dalloc_missing(s, &t.hcnt, n);
+    if (e == cudaSuccess && s->P.history) e = dalloc_missing(s, &t.hist, n * wd::kHistCap);
+    if (e == cudaSuccess && s->P.history) e = dalloc_missing(s, &t.cnt_id, n);
     return e;
 }
 
 cudaError_t alloc_snap(wd_sim* s, wd_sim::Snap& q) {
     const size_t n = static_cast<size_t>(s->n);
-    cudaError_t e = dalloc_missing(&q.pos, n);
-    if (e == cudaSuccess) e = dalloc_missing(&q.vel, n);
-    if (e == cudaSuccess) e = dalloc_missing(&q.ids, n);
-    if (e == cudaSuccess) e = dalloc_missing(&q.keys, n);
-    if (e == cudaSuccess && s->P.history) e = dalloc_missing(&q.hcnt, n);
-    if (e == cudaSuccess && s->P.history) e = dalloc_missing(&q.hist, n * wd::kHistCap);
+    cudaError_t e = dalloc_missing(s, &q.pos, n);
+    if (e == cudaSuccess) e = dalloc_missing(s, &q.vel, n);
+    if (e == cudaSuccess) e = dalloc_missing(s, &q.ids, n);
+    if (e == cudaSuccess) e = dalloc_missing(s, &q.keys, n);
+    if (e == cudaSuccess && s->P.history) e = dalloc_missing(s, &q.hcnt, n);
+    if (e == cudaSuccess && s->P.history) e = dalloc_missing(s, &q.hist, n * wd::kHistCap);
     return e;
 }
 
@@ -2258,8 +2281,8 @@ static int io_setup(wd_sim* s) {
     WD_CUDA(create_missing(&s->io_up));
     WD_CUDA(create_missing(&s->io_down));
     for (int b = 0; b < 2; ++b) {
-        WD_CUDA(dalloc_missing(&s->io_in[b], 6 * n));
-        WD_CUDA(dalloc_missing(&s->io_out[b], 3 * n));
+        WD_CUDA(dalloc_missing(s, &s->io_in[b], 6 * n));
+        WD_CUDA(dalloc_missing(s, &s->io_out[b], 3 * n));
         cudaEvent_t* evs[] = {&s->ev_in_ready[b], &s->ev_in_free[b], &s->ev_out_ready[b],
                               &s->ev_out_free[b]};
         for (cudaEvent_t* e : evs) WD_CUDA(create_missing(e));
@@ -2386,8 +2409,8 @@ int wd_density_grid_nodes(const wd_sim* sim, int64_t* nodes) {
 int wd_compute_density_grid_device(wd_sim* sim, float* d_grid) {
     if (!sim || !d_grid) return fail(WD_ERR_INVALID, "wd_compute_density_grid_device: NULL argument");
     if (!sim->dep_acc) {
-        WD_CUDA(dalloc_missing(&sim->dep_bounds, static_cast<size_t>(4) * sim->scenes));
-        WD_CUDA(dalloc(&sim->dep_acc, static_cast<size_t>(4) * sim->dep_nodes));
+        WD_CUDA(dalloc_missing(sim, &sim->dep_bounds, static_cast<size_t>(4) * sim->scenes));
+        WD_CUDA(dalloc_missing(sim, &sim->dep_acc, static_cast<size_t>(4) * sim->dep_nodes));
     }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (sim->cfg.kernel_timing) {
@@ -2416,7 +2439,7 @@ int wd_compute_density_grid_device(wd_sim* sim, float* d_grid) {
 
 int wd_compute_density_grid(wd_sim* sim, float* grid) {
     if (!sim || !grid) return fail(WD_ERR_INVALID, "wd_compute_density_grid: NULL argument");
-    if (!sim->dep_out) WD_CUDA(dalloc(&sim->dep_out, static_cast<size_t>(4) * sim->dep_nodes));
+    WD_CUDA(dalloc_missing(sim, &sim->dep_out, static_cast<size_t>(4) * sim->dep_nodes));
     int rc = wd_compute_density_grid_device(sim, sim->dep_out);
     if (rc) return rc;
     WD_CUDA(cudaMemcpyAsync(grid, sim->dep_out, sizeof(float) * 4 * static_cast<size_t>(sim->dep_nodes),
@@ -2606,8 +2629,8 @@ int wd_debug_candidates(wd_sim* sim, int64_t* offsets, int32_t* cand, uint8_t* c
     if (rc) return rc;
     const int n = sim->n;
     if (!sim->cand_offsets) {
-        WD_CUDA(dalloc_missing(&sim->cand_count, n));
-        WD_CUDA(dalloc_missing(&sim->cand_offsets, static_cast<size_t>(n) + 1));
+        WD_CUDA(dalloc_missing(sim, &sim->cand_count, n));
+        WD_CUDA(dalloc_missing(sim, &sim->cand_offsets, static_cast<size_t>(n) + 1));
     }
     wd::launch_candidate_count(sim->P, tab(sim, sim->sceneC), sim->posC, sim->idsC, sim->sb.table,
                                sim->cand_count, sim->stream);
@@ -2653,12 +2676,12 @@ static int apply_skin(wd_sim* s, float skin) {
     if (lists && s->picard) {
         const int n = s->n;
         const bool fresh = !s->rhs_ids;   // the last of them
-        WD_CUDA(dalloc_missing(&s->xpos, n));
-        WD_CUDA(dalloc_missing(&s->xvel, n));
-        WD_CUDA(dalloc_missing(&s->xids, n));
-        if (s->scenes > 1) WD_CUDA(dalloc_missing(&s->xscene, n));
-        WD_CUDA(dalloc_missing(&s->rhs_vel, n));
-        WD_CUDA(dalloc_missing(&s->rhs_ids, n));
+        WD_CUDA(dalloc_missing(s, &s->xpos, n));
+        WD_CUDA(dalloc_missing(s, &s->xvel, n));
+        WD_CUDA(dalloc_missing(s, &s->xids, n));
+        if (s->scenes > 1) WD_CUDA(dalloc_missing(s, &s->xscene, n));
+        WD_CUDA(dalloc_missing(s, &s->rhs_vel, n));
+        WD_CUDA(dalloc_missing(s, &s->rhs_ids, n));
         if (fresh) {
             // the rhs getter reads these in list mode: start them at the current rhs source
             WD_CUDA(cudaMemcpyAsync(s->rhs_vel, s->velB, sizeof(float4) * n, cudaMemcpyDeviceToDevice, s->stream));
@@ -2863,7 +2886,7 @@ int wd_set_contact_kernel(wd_sim* sim, int32_t block, int32_t variant) {
 
 int wd_debug_stage_wait(wd_sim* sim, int32_t stall, int32_t wait_us) {
     if (!sim) return fail(WD_ERR_INVALID, "wd_debug_stage_wait: NULL handle");
-    if (!sim->skin_asked)
+    if (!sim->skin_asked || !sim->list_ctrl)
         return fail(WD_ERR_INVALID, "wd_debug_stage_wait: the handle has no Verlet lists");
     if (wait_us < 0) return fail(WD_ERR_INVALID, "wd_debug_stage_wait: wait_us must be >= 0");
     int rc = sync_stream(sim);
@@ -3080,18 +3103,18 @@ int wd_adjoint_backward(wd_sim* sim, const float* d_gx, const float* d_gv, float
     cudaStream_t st = sim->stream;
     const bool hist = sim->P.history != 0;
     for (int b = 0; b < 2; ++b) {
-        WD_CUDA(dalloc_missing(&sim->adj_lx[b], n));
-        WD_CUDA(dalloc_missing(&sim->adj_lv[b], n));
-        if (hist) WD_CUDA(dalloc_missing(&sim->adj_lxi[b], static_cast<size_t>(n) * wd::kHistCap));
+        WD_CUDA(dalloc_missing(sim, &sim->adj_lx[b], n));
+        WD_CUDA(dalloc_missing(sim, &sim->adj_lv[b], n));
+        if (hist) WD_CUDA(dalloc_missing(sim, &sim->adj_lxi[b], static_cast<size_t>(n) * wd::kHistCap));
     }
-    WD_CUDA(dalloc_missing(&sim->adj_theta, static_cast<size_t>(3) * n));
+    WD_CUDA(dalloc_missing(sim, &sim->adj_theta, static_cast<size_t>(3) * n));
     const int every = sim->adj_every;
     if (sim->adj_tape.size() < static_cast<size_t>(every) + 1) clear_adj_graphs(sim);
     for (size_t k = 0; k < static_cast<size_t>(every) + 1; ++k) {
         if (k == sim->adj_tape.size()) sim->adj_tape.emplace_back();
         WD_CUDA(alloc_tape_step(sim, sim->adj_tape[k]));
     }
-    if (!sim->adj_ovf) WD_CUDA(dalloc(&sim->adj_ovf, 1));
+    WD_CUDA(dalloc_missing(sim, &sim->adj_ovf, 1));
     WD_CUDA(cudaMemsetAsync(sim->adj_ovf, 0, sizeof(unsigned long long), st));
     unsigned long long saved[wd::kNumCounters];
     WD_CUDA(cudaMemcpyAsync(saved, sim->counters, sizeof(saved), cudaMemcpyDeviceToHost, st));
@@ -3151,8 +3174,8 @@ int wd_deposit_vjp(wd_sim* sim, const float* d_ggrid, float* d_gx, float* d_gv) 
     if (!sim || !d_ggrid) return fail(WD_ERR_INVALID, "wd_deposit_vjp: NULL argument");
     if (sim->scenes != 1) return fail(WD_ERR_INVALID, "wd_deposit_vjp: not for a batch of scenes");
     const int n = sim->n;
-    WD_CUDA(dalloc_missing(&sim->vjp_x, n));
-    WD_CUDA(dalloc_missing(&sim->vjp_v, n));
+    WD_CUDA(dalloc_missing(sim, &sim->vjp_x, n));
+    WD_CUDA(dalloc_missing(sim, &sim->vjp_v, n));
     wd::launch_deposit_vjp(n, sim->posA, sim->velA, sim->idsA, sim->cfg.dom_lo, sim->cfg.dom_hi,
                            sim->cfg.dgrid, d_ggrid, sim->vjp_x, sim->vjp_v, sim->stream);
     if (d_gx) wd::launch_f4_to_aos3(n, sim->vjp_x, d_gx, sim->stream);
@@ -3225,15 +3248,15 @@ int wd_chaos_metrics(wd_sim* sim, int32_t reference_scene, double* metrics3) {
         for (int k = 0; k < S; ++k)
             chunk[k + 1] = chunk[k] + static_cast<int>((seg[k + 1] - seg[k] + wd::kBlock - 1) / wd::kBlock);
         sim->node_chunks = chunk[S];
-        WD_CUDA(dalloc_missing(&sim->d_node_seg, S + 1));
-        WD_CUDA(dalloc_missing(&sim->d_node_chunk, S + 1));
+        WD_CUDA(dalloc_missing(sim, &sim->d_node_seg, S + 1));
+        WD_CUDA(dalloc_missing(sim, &sim->d_node_chunk, S + 1));
         WD_CUDA(cudaMemcpy(sim->d_node_seg, seg.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice));
         WD_CUDA(cudaMemcpy(sim->d_node_chunk, chunk.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice));
-        WD_CUDA(dalloc_missing(&sim->node_vals, static_cast<size_t>(6) * total_nodes));
-        WD_CUDA(dalloc_missing(&sim->chaos_partials, static_cast<size_t>(6) * sim->node_chunks));
-        WD_CUDA(dalloc_missing(&sim->chaos_sums, static_cast<size_t>(6) * S));
-        WD_CUDA(dalloc_missing(&sim->grain_sums, S));
-        WD_CUDA(dalloc_missing(&sim->chaos_grid, static_cast<size_t>(4) * total_nodes));
+        WD_CUDA(dalloc_missing(sim, &sim->node_vals, static_cast<size_t>(6) * total_nodes));
+        WD_CUDA(dalloc_missing(sim, &sim->chaos_partials, static_cast<size_t>(6) * sim->node_chunks));
+        WD_CUDA(dalloc_missing(sim, &sim->chaos_sums, static_cast<size_t>(6) * S));
+        WD_CUDA(dalloc_missing(sim, &sim->grain_sums, S));
+        WD_CUDA(dalloc_missing(sim, &sim->chaos_grid, static_cast<size_t>(4) * total_nodes));
     }
     int rc = wd_compute_density_grid_device(sim, sim->chaos_grid);
     if (rc) return rc;
