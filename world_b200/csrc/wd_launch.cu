@@ -19,11 +19,17 @@
 namespace wd {
 namespace {
 
+// Launches a graph behind the one that runs, and notes why it could not.
+__device__ void tail_launch(cudaGraphExec_t graph, volatile uint32_t* failed) {
+    const cudaError_t e =
+        graph == nullptr ? cudaErrorInvalidResourceHandle : cudaGraphLaunch(graph, cudaStreamGraphTailLaunch);
+    if (e != cudaSuccess) *failed = static_cast<uint32_t>(e);
+}
+
 __global__ void k_graph_if(const uint32_t* __restrict__ flag, cudaGraphExec_t graph,
                            volatile uint32_t* __restrict__ failed) {
     if (threadIdx.x != 0 || *flag == 0u) return;
-    if (cudaGraphLaunch(graph, cudaStreamGraphTailLaunch) != cudaSuccess)
-        *failed = 1u;
+    tail_launch(graph, failed);
 }
 
 __global__ void k_graph_chain(const uint32_t* __restrict__ ctrl, int steps, cudaGraphExec_t even,
@@ -31,29 +37,22 @@ __global__ void k_graph_chain(const uint32_t* __restrict__ ctrl, int steps, cuda
     if (threadIdx.x != 0 || ctrl[kLcDecision] == 0u) return;
     // the step that decided: the chain's steps before it are done, kLcLeft wait
     const int step = steps - 1 - static_cast<int>(ctrl[kLcLeft]);
-    if (cudaGraphLaunch(step & 1 ? odd : even, cudaStreamGraphTailLaunch) != cudaSuccess)
-        *failed = 1u;
+    tail_launch(step & 1 ? odd : even, failed);
 }
 
 __global__ void k_build_end(uint32_t* __restrict__ ctrl, const cudaGraphExec_t* __restrict__ by_left,
                             const int* __restrict__ radix_flag, cudaGraphExec_t radix,
                             volatile uint32_t* __restrict__ failed) {
     if (threadIdx.x != 0) return;
-    cudaGraphExec_t next = nullptr;
     if (radix_flag != nullptr && *radix_flag != 0) {
-        next = radix;
+        tail_launch(radix, failed);
     } else if (by_left != nullptr) {
         const uint32_t left = ctrl[kLcLeft];
         ctrl[kLcPending] = 0u;
         ctrl[kLcLeft] = 0u;
-        if (left > 0u) {
-            next = by_left[left];
-            // steps that nothing takes up are an error, not steps left out
-            if (next == nullptr) *failed = 1u;
-        }
+        // steps that nothing takes up (no handle) are an error, not steps left out
+        if (left > 0u) tail_launch(by_left[left], failed);
     }
-    if (next != nullptr && cudaGraphLaunch(next, cudaStreamGraphTailLaunch) != cudaSuccess)
-        *failed = 1u;
 }
 
 }  // namespace

@@ -87,7 +87,7 @@ int key_bits(uint64_t cells) {
 // wait). Pages of 64 outlive the handles, which take one each and give it back: locking a page
 // for every handle would cost its creation milliseconds.
 struct alignas(64) HostWords {
-    volatile uint32_t launch_failed;   // a device-side graph launch failed: its work is missing
+    volatile uint32_t launch_failed;   // why a device-side graph launch failed (its work is missing), or 0
     unsigned long long looked[3];      // kCntAutoSteps, Builds, Crowded, as of ev_look
 };
 constexpr size_t kWordsPage = 4096;
@@ -1422,12 +1422,13 @@ int sync_stream(wd_sim* s) {
     }
     WD_CUDA(cudaStreamSynchronize(s->stream));
     WD_CUDA(cudaGetLastError());
-    if (s->words->launch_failed) {
+    if (const uint32_t why = s->words->launch_failed) {
         // a list build, or a searched step's radix path, whose launch failed did not run
         s->words->launch_failed = 0u;
         WD_CUDA(request_list_build(s));
-        return fail(WD_ERR_CUDA, "list build or search: a device-side graph launch failed; the "
-                                 "steps since the last synchronisation are invalid");
+        return fail(WD_ERR_CUDA, std::string("list build or search: a device-side graph launch failed (") +
+                                     cudaGetErrorName(static_cast<cudaError_t>(why)) +
+                                     "); the steps since the last synchronisation are invalid");
     }
     if (!lists) return WD_OK;
     if (s->seen[wd::kCntStageTimeout]) {
@@ -2905,7 +2906,7 @@ int wd_debug_graph_captures(wd_sim* sim, int64_t* captures) {
 
 int wd_debug_launch_failure(wd_sim* sim) {
     if (!sim) return fail(WD_ERR_INVALID, "wd_debug_launch_failure: NULL handle");
-    sim->words->launch_failed = 1u;
+    sim->words->launch_failed = cudaErrorUnknown;
     return WD_OK;
 }
 
