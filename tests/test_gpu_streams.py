@@ -1,0 +1,61 @@
+"""Other work on the device, on the default stream, while a handle is set up and steps: nothing
+of the handle's waits behind it and lands later, on top of what its own stream has done since."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from test_gpu_auto_lists import _touching
+from test_gpu_lists import _same
+from world_b200 import ParticleDynamics
+
+pytestmark = pytest.mark.gpu
+
+HALF_A_SECOND = 1_000_000_000      # clock cycles
+
+
+@pytest.mark.parametrize("history", [False, True])
+@pytest.mark.parametrize("skin", [0.0, 0.2e-3])
+def test_steps_beside_a_busy_default_stream(skin, history):
+    """Grains that cross half the skin every few steps, so that most builds fall inside chains."""
+    cfg, st, rad = _touching(95, history)
+    cfg.kernel_timing = False
+    st = st.copy()
+    st[:, 3:] = np.random.default_rng(96).normal(0, 1.0, (2744, 3))
+    ref = ParticleDynamics(cfg, state=st, radius=rad)
+    ref.set_neighbor_skin(0.0)
+    cfg.neighbor_skin = skin
+    # the kernels' first use loads them, which waits for the device
+    with ParticleDynamics(cfg, state=st, radius=rad) as warm:
+        warm.advance(200)
+    sim = ParticleDynamics(cfg, state=st, radius=rad)
+    torch.cuda._sleep(HALF_A_SECOND)
+    busy = torch.cuda.Event()
+    busy.record()
+    sim.advance(200)
+    sim.synchronize()
+    assert not busy.query()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        sim.advance(200)
+    ref.advance(800)
+    _same(ref, sim)
+    assert sim.time == ref.time
+
+
+def test_a_handle_is_whole_when_it_is_there():
+    """Nothing of a handle's creation is still to come when the call returns."""
+    cfg, st, rad = _touching(97, True)
+    cfg.kernel_timing = False
+    ref = ParticleDynamics(cfg, state=st, radius=rad)
+    ref.advance(3)
+    torch.cuda._sleep(HALF_A_SECOND)
+    busy = torch.cuda.Event()
+    busy.record()
+    sim = ParticleDynamics(cfg, state=st, radius=rad)
+    sim.advance(3)
+    sim.synchronize()
+    assert not busy.query()
+    torch.cuda.synchronize()
+    _same(ref, sim)

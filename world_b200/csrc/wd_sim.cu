@@ -1022,7 +1022,9 @@ cudaError_t capture_device_builds(wd_sim* s) {
     cudaError_t e = cudaSuccess;
     if (!s->chain_table) {
         e = dalloc(&s->chain_table, 4 * 8);
-        if (e == cudaSuccess) e = cudaMemset(s->chain_table, 0, 4 * 8 * sizeof(cudaGraphExec_t));
+        // in the step stream's order, as the table's other writes
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(s->chain_table, 0, 4 * 8 * sizeof(cudaGraphExec_t), s->stream);
     }
     if (e == cudaSuccess) e = capture_build(s, &g.head, &g.radix, s->chain_table + 8 * next);
     if (e == cudaSuccess)
@@ -1435,7 +1437,7 @@ int sync_stream(wd_sim* s) {
         // reported once: the handle stays usable. The step stopped part-way, so even
         // its slot order may be mixed (the first step after a build rewrites the
         // ids); the next state upload starts from a fresh slot order.
-        WD_CUDA(cudaMemset(s->counters + wd::kCntStageTimeout, 0, sizeof(unsigned long long)));
+        WD_CUDA(cudaMemsetAsync(s->counters + wd::kCntStageTimeout, 0, sizeof(unsigned long long), s->stream));
         s->slots_invalid = true;
         return fail(WD_ERR_CUDA, "contact kernel: a bulk copy into shared memory did not "
                                  "complete within its wait limit; the state is invalid");
@@ -1597,6 +1599,9 @@ void note_upload(wd_sim* s) {
     s->auto_look = 32;
 }
 
+// Everything that a handle clears or copies to the device goes down its own stream, which does
+// not wait for the default one: work there, another handle's too, may hold such a copy back until
+// after steps that read or write the same memory.
 int alloc_sim(wd_sim* s) {
     const int n = s->n;
     WD_CUDA(cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking));
@@ -1620,7 +1625,7 @@ int alloc_sim(wd_sim* s) {
         for (int b = 0; b < 2; ++b)
             WD_CUDA(dalloc(&s->hist[b], static_cast<size_t>(n) * wd::kHistCap));
         WD_CUDA(dalloc(&s->hcnt_slot, n));
-        WD_CUDA(cudaMemset(s->hcnt_slot, 0, sizeof(int) * static_cast<size_t>(n)));
+        WD_CUDA(cudaMemsetAsync(s->hcnt_slot, 0, sizeof(int) * static_cast<size_t>(n), s->stream));
         WD_CUDA(dalloc(&s->hcnt_g, n));
         if (s->picard) {
             WD_CUDA(dalloc(&s->hcnt_snap[0], n));
@@ -1635,16 +1640,16 @@ int alloc_sim(wd_sim* s) {
         WD_CUDA(dalloc(&sb.vals[b], n));
     }
     WD_CUDA(dalloc(&sb.table_keys, n));
-    WD_CUDA(cudaMemset(sb.table_keys, 0xFF, sizeof(uint32_t) * static_cast<size_t>(n)));
+    WD_CUDA(cudaMemsetAsync(sb.table_keys, 0xFF, sizeof(uint32_t) * static_cast<size_t>(n), s->stream));
     WD_CUDA(dalloc(&sb.slot_keys, n));
-    WD_CUDA(cudaMemset(sb.slot_keys, 0xFF, sizeof(uint32_t) * static_cast<size_t>(n)));
+    WD_CUDA(cudaMemsetAsync(sb.slot_keys, 0xFF, sizeof(uint32_t) * static_cast<size_t>(n), s->stream));
     WD_CUDA(dalloc(&sb.newkey, n));
     WD_CUDA(dalloc(&sb.moved, (static_cast<size_t>(n) + 31) / 32));
     sb.num_blocks = wd::blocks_for(n);
     WD_CUDA(dalloc(&sb.blk_cnt, sb.num_blocks));
     WD_CUDA(dalloc(&sb.blk_off, static_cast<size_t>(sb.num_blocks) + 1));
     WD_CUDA(dalloc(&sb.ctrl, 4));
-    WD_CUDA(cudaMemset(sb.ctrl, 0, 4 * sizeof(int)));
+    WD_CUDA(cudaMemsetAsync(sb.ctrl, 0, 4 * sizeof(int), s->stream));
     sb.mover_cap = wd::mover_cap(n);
     const int movers = std::min(n, sb.mover_cap);
     WD_CUDA(dalloc(&sb.mv_raw, movers));
@@ -1660,13 +1665,13 @@ int alloc_sim(wd_sim* s) {
     WD_CUDA(dalloc(&sb.tile_counts, static_cast<size_t>(wd::kRadix) * sb.num_tiles));
     WD_CUDA(dalloc(&sb.digit_totals, static_cast<size_t>(wd::kRadix) * sb.passes));
     WD_CUDA(dalloc(&sb.table, s->num_cells));
-    WD_CUDA(cudaMemset(sb.table, 0xFF, sizeof(int2) * s->num_cells));
+    WD_CUDA(cudaMemsetAsync(sb.table, 0xFF, sizeof(int2) * s->num_cells, s->stream));
     WD_CUDA(dalloc(&s->counters, wd::kNumCounters));
-    WD_CUDA(cudaMemset(s->counters, 0, sizeof(unsigned long long) * wd::kNumCounters));
+    WD_CUDA(cudaMemsetAsync(s->counters, 0, sizeof(unsigned long long) * wd::kNumCounters, s->stream));
     WD_CUDA(dalloc(&s->picard_res, s->picard_iters > 0 ? s->picard_iters : 1));
-    WD_CUDA(cudaMemset(s->picard_res, 0, sizeof(uint32_t) * (s->picard_iters > 0 ? s->picard_iters : 1)));
+    WD_CUDA(cudaMemsetAsync(s->picard_res, 0, sizeof(uint32_t) * (s->picard_iters > 0 ? s->picard_iters : 1), s->stream));
     WD_CUDA(dalloc(&s->picard_used, 1));
-    WD_CUDA(cudaMemset(s->picard_used, 0, sizeof(int)));
+    WD_CUDA(cudaMemsetAsync(s->picard_used, 0, sizeof(int), s->stream));
     WD_CUDA(dalloc(&s->red_out, 4));
     WD_CUDA(dalloc(&s->staging, static_cast<size_t>(6) * n));
     s->dep_nodes = s->scene_nodes_off.back();
@@ -1680,18 +1685,18 @@ int alloc_sim(wd_sim* s) {
     s->total_chunks = chunk[S];
     WD_CUDA(dalloc(&s->d_seg, S + 1));
     WD_CUDA(dalloc(&s->d_chunk_base, S + 1));
-    WD_CUDA(cudaMemcpy(s->d_seg, seg.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice));
-    WD_CUDA(cudaMemcpy(s->d_chunk_base, chunk.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice));
+    WD_CUDA(cudaMemcpyAsync(s->d_seg, seg.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice, s->stream));
+    WD_CUDA(cudaMemcpyAsync(s->d_chunk_base, chunk.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice, s->stream));
     WD_CUDA(dalloc(&s->partials, static_cast<size_t>(3) * s->total_chunks));
     WD_CUDA(dalloc(&s->scene_sums, static_cast<size_t>(3) * S));
     WD_CUDA(dalloc(&s->grain_vals, static_cast<size_t>(4) * n));
     if (S > 1) {
         WD_CUDA(dalloc(&s->d_scene_P, S));
-        WD_CUDA(cudaMemcpy(s->d_scene_P, s->scene_P.data(), sizeof(DevParams) * S, cudaMemcpyHostToDevice));
+        WD_CUDA(cudaMemcpyAsync(s->d_scene_P, s->scene_P.data(), sizeof(DevParams) * S, cudaMemcpyHostToDevice, s->stream));
         WD_CUDA(dalloc(&s->sceneA, n));
         WD_CUDA(dalloc(&s->sceneB, n));
         WD_CUDA(dalloc(&s->scene_overflow, S));
-        WD_CUDA(cudaMemset(s->scene_overflow, 0, sizeof(unsigned long long) * S));
+        WD_CUDA(cudaMemsetAsync(s->scene_overflow, 0, sizeof(unsigned long long) * S, s->stream));
         WD_CUDA(dalloc(&s->scene_unstable, S));
     }
     if (s->lists) {
@@ -1699,7 +1704,7 @@ int alloc_sim(wd_sim* s) {
         WD_CUDA(cudaStreamSynchronize(s->stream));
         uint32_t init[wd::kLcWords] = {};
         init[wd::kLcForce] = 1u;  // the first step builds
-        WD_CUDA(cudaMemcpy(s->list_ctrl, init, sizeof(init), cudaMemcpyHostToDevice));
+        WD_CUDA(cudaMemcpyAsync(s->list_ctrl, init, sizeof(init), cudaMemcpyHostToDevice, s->stream));
         s->need_build = true;
         if (s->picard) {
             WD_CUDA(dalloc(&s->xpos, n));
@@ -1723,25 +1728,26 @@ int upload_initial(wd_sim* s, const float* state) {
         vel[i] = make_float4(q[3], q[4], q[5], s->mass[i]);
         ids[i] = i;
     }
-    WD_CUDA(cudaMemcpy(s->posA, pos.data(), sizeof(float4) * n, cudaMemcpyHostToDevice));
-    WD_CUDA(cudaMemcpy(s->velA, vel.data(), sizeof(float4) * n, cudaMemcpyHostToDevice));
-    WD_CUDA(cudaMemcpy(s->idsA, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+    WD_CUDA(cudaMemcpyAsync(s->posA, pos.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s->stream));
+    WD_CUDA(cudaMemcpyAsync(s->velA, vel.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s->stream));
+    WD_CUDA(cudaMemcpyAsync(s->idsA, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s->stream));
     // B mirrors A until the first step, so get_rhs before a step reads defined data.
-    WD_CUDA(cudaMemcpy(s->posB, s->posA, sizeof(float4) * n, cudaMemcpyDeviceToDevice));
-    WD_CUDA(cudaMemcpy(s->velB, s->velA, sizeof(float4) * n, cudaMemcpyDeviceToDevice));
-    WD_CUDA(cudaMemcpy(s->idsB, s->idsA, sizeof(int) * n, cudaMemcpyDeviceToDevice));
+    WD_CUDA(cudaMemcpyAsync(s->posB, s->posA, sizeof(float4) * n, cudaMemcpyDeviceToDevice, s->stream));
+    WD_CUDA(cudaMemcpyAsync(s->velB, s->velA, sizeof(float4) * n, cudaMemcpyDeviceToDevice, s->stream));
+    WD_CUDA(cudaMemcpyAsync(s->idsB, s->idsA, sizeof(int) * n, cudaMemcpyDeviceToDevice, s->stream));
     if (s->rhs_vel) {
-        WD_CUDA(cudaMemcpy(s->rhs_vel, s->velA, sizeof(float4) * n, cudaMemcpyDeviceToDevice));
-        WD_CUDA(cudaMemcpy(s->rhs_ids, s->idsA, sizeof(int) * n, cudaMemcpyDeviceToDevice));
+        WD_CUDA(cudaMemcpyAsync(s->rhs_vel, s->velA, sizeof(float4) * n, cudaMemcpyDeviceToDevice, s->stream));
+        WD_CUDA(cudaMemcpyAsync(s->rhs_ids, s->idsA, sizeof(int) * n, cudaMemcpyDeviceToDevice, s->stream));
     }
-    WD_CUDA(cudaMemset(s->acc, 0, sizeof(float4) * n));
+    WD_CUDA(cudaMemsetAsync(s->acc, 0, sizeof(float4) * n, s->stream));
     if (s->scenes > 1) {
         std::vector<int> sc(n);
         for (int k = 0; k < s->scenes; ++k)
             for (int64_t i = s->scene_off[k]; i < s->scene_off[k + 1]; ++i) sc[i] = k;
-        WD_CUDA(cudaMemcpy(s->sceneA, sc.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-        WD_CUDA(cudaMemcpy(s->sceneB, sc.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+        WD_CUDA(cudaMemcpyAsync(s->sceneA, sc.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s->stream));
+        WD_CUDA(cudaMemcpyAsync(s->sceneB, sc.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s->stream));
     }
+    WD_CUDA(cudaStreamSynchronize(s->stream));
     return WD_OK;
 }
 
@@ -2165,21 +2171,22 @@ static int reset_slot_order(wd_sim* s) {
         ids[i] = i;
     }
     WD_CUDA(cudaStreamSynchronize(s->stream));
-    WD_CUDA(cudaMemcpy(s->posA, pos.data(), sizeof(float4) * n, cudaMemcpyHostToDevice));
-    WD_CUDA(cudaMemcpy(s->velA, vel.data(), sizeof(float4) * n, cudaMemcpyHostToDevice));
-    WD_CUDA(cudaMemcpy(s->idsA, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    WD_CUDA(cudaMemcpy(s->idsB, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+    WD_CUDA(cudaMemcpyAsync(s->posA, pos.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s->stream));
+    WD_CUDA(cudaMemcpyAsync(s->velA, vel.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s->stream));
+    WD_CUDA(cudaMemcpyAsync(s->idsA, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s->stream));
+    WD_CUDA(cudaMemcpyAsync(s->idsB, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s->stream));
     if (s->scenes > 1) {
         std::vector<int> sc(n);
         for (int k = 0; k < s->scenes; ++k)
             for (int64_t i = s->scene_off[k]; i < s->scene_off[k + 1]; ++i) sc[i] = k;
-        WD_CUDA(cudaMemcpy(s->sceneA, sc.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-        WD_CUDA(cudaMemcpy(s->sceneB, sc.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+        WD_CUDA(cudaMemcpyAsync(s->sceneA, sc.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s->stream));
+        WD_CUDA(cudaMemcpyAsync(s->sceneB, sc.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s->stream));
     }
     if (s->P.history) {
-        WD_CUDA(cudaMemset(s->hcnt_slot, 0, sizeof(int) * n));
-        WD_CUDA(cudaMemset(s->hcnt_g, 0, sizeof(int) * n));
+        WD_CUDA(cudaMemsetAsync(s->hcnt_slot, 0, sizeof(int) * n, s->stream));
+        WD_CUDA(cudaMemsetAsync(s->hcnt_g, 0, sizeof(int) * n, s->stream));
     }
+    WD_CUDA(cudaStreamSynchronize(s->stream));
     s->slots_invalid = false;
     return WD_OK;
 }
@@ -2395,10 +2402,10 @@ int wd_set_history(wd_sim* sim, const int32_t* count, const int32_t* partner, co
     std::vector<int32_t> slot_count(n), slot_id(n);
     WD_CUDA(cudaMemcpy(slot_id.data(), sim->idsA, n * sizeof(int32_t), cudaMemcpyDeviceToHost));
     for (size_t k = 0; k < n; ++k) slot_count[k] = count[slot_id[k]];
-    WD_CUDA(cudaMemcpy(sim->hcnt_slot, slot_count.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
-    WD_CUDA(cudaMemcpy(sim->hist[sim->hist_cur], rows.data(), rows.size() * sizeof(float4),
-                       cudaMemcpyHostToDevice));
-    return WD_OK;
+    WD_CUDA(cudaMemcpyAsync(sim->hcnt_slot, slot_count.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, sim->stream));
+    WD_CUDA(cudaMemcpyAsync(sim->hist[sim->hist_cur], rows.data(), rows.size() * sizeof(float4),
+                            cudaMemcpyHostToDevice, sim->stream));
+    return sync_stream(sim);
 }
 
 int wd_density_grid_nodes(const wd_sim* sim, int64_t* nodes) {
@@ -2893,9 +2900,9 @@ int wd_debug_stage_wait(wd_sim* sim, int32_t stall, int32_t wait_us) {
     int rc = sync_stream(sim);
     if (rc) return rc;
     const uint32_t words[2] = {stall ? 1u : 0u, static_cast<uint32_t>(wait_us)};
-    WD_CUDA(cudaMemcpy(sim->list_ctrl + wd::kLcStallTest, words, sizeof(words),
-                       cudaMemcpyHostToDevice));
-    return WD_OK;
+    WD_CUDA(cudaMemcpyAsync(sim->list_ctrl + wd::kLcStallTest, words, sizeof(words),
+                            cudaMemcpyHostToDevice, sim->stream));
+    return sync_stream(sim);
 }
 
 int wd_debug_graph_captures(wd_sim* sim, int64_t* captures) {
@@ -3251,8 +3258,9 @@ int wd_chaos_metrics(wd_sim* sim, int32_t reference_scene, double* metrics3) {
         sim->node_chunks = chunk[S];
         WD_CUDA(dalloc_missing(sim, &sim->d_node_seg, S + 1));
         WD_CUDA(dalloc_missing(sim, &sim->d_node_chunk, S + 1));
-        WD_CUDA(cudaMemcpy(sim->d_node_seg, seg.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice));
-        WD_CUDA(cudaMemcpy(sim->d_node_chunk, chunk.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice));
+        WD_CUDA(cudaMemcpyAsync(sim->d_node_seg, seg.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice, sim->stream));
+        WD_CUDA(cudaMemcpyAsync(sim->d_node_chunk, chunk.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice, sim->stream));
+        WD_CUDA(cudaStreamSynchronize(sim->stream));
         WD_CUDA(dalloc_missing(sim, &sim->node_vals, static_cast<size_t>(6) * total_nodes));
         WD_CUDA(dalloc_missing(sim, &sim->chaos_partials, static_cast<size_t>(6) * sim->node_chunks));
         WD_CUDA(dalloc_missing(sim, &sim->chaos_sums, static_cast<size_t>(6) * S));
