@@ -265,6 +265,7 @@ struct wd_sim {
     float4* adj_lx[2] = {nullptr, nullptr};
     float4* adj_lv[2] = {nullptr, nullptr};
     float4* adj_lxi[2] = {nullptr, nullptr};
+    float4* adj_acc = nullptr; // accelerations of replayed steps
     float4* vjp_x = nullptr;   // the deposit's pullback by grain id
     float4* vjp_v = nullptr;
     double* adj_theta = nullptr;
@@ -521,7 +522,7 @@ void free_sim(wd_sim* s) {
     if (s->io_up) cudaStreamDestroy(s->io_up);
     if (s->io_down) cudaStreamDestroy(s->io_down);
     void* adj[] = {s->adj_lx[0], s->adj_lx[1], s->adj_lv[0], s->adj_lv[1], s->adj_lxi[0],
-                   s->adj_lxi[1], s->vjp_x, s->vjp_v, s->adj_theta};
+                   s->adj_lxi[1], s->vjp_x, s->vjp_v, s->adj_theta, s->adj_acc};
     for (void* p : adj) cudaFree(p);
     give_words(s->words);
     if (s->own_stream) cudaStreamDestroy(s->own_stream);
@@ -2792,7 +2793,7 @@ cudaError_t adj_replay_body(wd_sim* s, int len, bool capture, cudaStream_t st) {
         fa.rec_hcnt = hist ? T.cnt_id : nullptr;
         fa.pos = T.pos; fa.vel = T.vel; fa.ids = T.ids; fa.table = s->sb.table;
         fa.pos_out = s->posA; fa.vel_out = s->velA; fa.ids_out = s->idsA;
-        fa.acc_out = s->acc;
+        fa.acc_out = s->adj_acc;   // the handle's are those of its last step
         fa.hist_in = hist ? T.hist : nullptr;
         fa.hcnt_in = hist ? T.hcnt : nullptr;
         fa.hist_out = hist ? T1.hist : nullptr;
@@ -3116,6 +3117,7 @@ int wd_adjoint_backward(wd_sim* sim, const float* d_gx, const float* d_gv, float
         if (hist) WD_CUDA(dalloc_missing(sim, &sim->adj_lxi[b], static_cast<size_t>(n) * wd::kHistCap));
     }
     WD_CUDA(dalloc_missing(sim, &sim->adj_theta, static_cast<size_t>(3) * n));
+    WD_CUDA(dalloc_missing(sim, &sim->adj_acc, n));
     const int every = sim->adj_every;
     if (sim->adj_tape.size() < static_cast<size_t>(every) + 1) clear_adj_graphs(sim);
     for (size_t k = 0; k < static_cast<size_t>(every) + 1; ++k) {
