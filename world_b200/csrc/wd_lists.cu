@@ -737,7 +737,14 @@ __device__ __forceinline__ void list_grain(const DevParams& P0, const ListArgs& 
                     // a cell crossing re-ordered this grain's contacts: redo them in
                     // canonical order
                     f = f_walls;
-                    if (HIST) h.out_count = out_walls;
+                    if (HIST) {
+                        // springs without a slot so far are counted again below
+                        const int seen = __popcll(all_hits) - __popcll(hits) - 1;
+                        const int over = out_walls + seen - kHistCap;
+                        if (over > 0)
+                            atomicAdd(&A.counters[kCntHistOverflow], 0ull - static_cast<unsigned long long>(over));
+                        h.out_count = out_walls;
+                    }
                     atomicAdd(&A.counters[kCntListResort], 1ull);
                     list_contacts_sorted_mask<HIST>(P, A, s, n, all_hits, pi, vel, mi, cx, cy, cz,
                                                     f, h);
