@@ -396,7 +396,7 @@ k_merge(int n, const uint32_t* __restrict__ newkey, const uint32_t* __restrict__
 template <bool SNAP, bool SNAP_FROM_STATE>
 __global__ void __launch_bounds__(kBlock)
 k_gather(int n, int ppc, const uint32_t* __restrict__ skey, const uint32_t* __restrict__ sid,
-         const int* __restrict__ src, const int* __restrict__ slot_of_id,
+         int* __restrict__ src, const int* __restrict__ slot_of_id,
          int* __restrict__ ctrl, const float4* __restrict__ posA,
          const float4* __restrict__ velA, float4* __restrict__ posB, float4* __restrict__ velB,
          int* __restrict__ idsB, const float4* __restrict__ nposA,
@@ -412,7 +412,9 @@ k_gather(int n, int ppc, const uint32_t* __restrict__ skey, const uint32_t* __re
     if (s >= n) return;
     if (s == 0) ctrl[2] = 0;   // the next search counts its movers from zero
     const uint32_t id = sid[s];
-    const int p = ctrl[1] ? slot_of_id[id] : src[s];
+    const bool radix = ctrl[1] != 0;
+    const int p = radix ? slot_of_id[id] : src[s];
+    if (radix) src[s] = p;   // the merge's else: who reads it later need not know the path
     const float4 x = posA[p], v = velA[p];
     posB[s] = x;
     velB[s] = v;
