@@ -2684,18 +2684,19 @@ static int apply_skin(wd_sim* s, float skin) {
     s->skin_asked |= lists;
     if (lists && s->picard) {
         const int n = s->n;
-        const bool fresh = !s->rhs_ids;   // the last of them
         WD_CUDA(dalloc_missing(s, &s->xpos, n));
         WD_CUDA(dalloc_missing(s, &s->xvel, n));
         WD_CUDA(dalloc_missing(s, &s->xids, n));
         if (s->scenes > 1) WD_CUDA(dalloc_missing(s, &s->xscene, n));
         WD_CUDA(dalloc_missing(s, &s->rhs_vel, n));
         WD_CUDA(dalloc_missing(s, &s->rhs_ids, n));
-        if (fresh) {
-            // the rhs getter reads these in list mode: start them at the current rhs source
-            WD_CUDA(cudaMemcpyAsync(s->rhs_vel, s->velB, sizeof(float4) * n, cudaMemcpyDeviceToDevice, s->stream));
-            WD_CUDA(cudaMemcpyAsync(s->rhs_ids, s->idsB, sizeof(int) * n, cudaMemcpyDeviceToDevice, s->stream));
-        }
+    }
+    if (s->picard && lists != s->lists) {
+        // the rhs getter reads the last iterate's velocities here on lists, in B otherwise
+        float4* vel[2] = {s->velB, s->rhs_vel};
+        int* ids[2] = {s->idsB, s->rhs_ids};
+        WD_CUDA(cudaMemcpyAsync(vel[lists], vel[!lists], sizeof(float4) * s->n, cudaMemcpyDeviceToDevice, s->stream));
+        WD_CUDA(cudaMemcpyAsync(ids[lists], ids[!lists], sizeof(int) * s->n, cudaMemcpyDeviceToDevice, s->stream));
     }
     s->lists = lists;
     s->cfg.neighbor_skin = skin;
