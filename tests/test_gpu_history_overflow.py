@@ -1,5 +1,6 @@
 """The count of contacts that found no free history slot, on lists: a grain whose contacts a cell
-crossing re-ordered is taken up once more, its dropped springs are not."""
+crossing re-ordered is taken up once more, and a Picard step whose iterates left the lists is
+redone; the dropped springs of what they replace are not counted."""
 from __future__ import annotations
 
 import numpy as np
@@ -54,4 +55,23 @@ def test_dropped_springs_are_counted_once(kernel):
             s.advance(20)
         assert sim.history_overflow_count() == ref.history_overflow_count()
     assert ref.history_overflow_count() > 1000 and sim.list_resort_count() > 10
+    _same(ref, sim)
+
+
+@pytest.mark.parametrize("timing", [False, True])
+@pytest.mark.parametrize("kernel", [(128, 64), (256, 48), (256, 0)])
+def test_redone_picard_steps_count_once(kernel, timing):
+    cfg, st, rad = _crowded()
+    cfg.kernel_timing = timing
+    cfg.time_integrator = "backward_euler_picard"
+    cfg.picard_iterations = 3
+    ref = ParticleDynamics(cfg, state=st, radius=rad)
+    cfg.neighbor_skin = 1e-5
+    sim = ParticleDynamics(cfg, state=st, radius=rad)
+    sim.set_contact_kernel(*kernel)
+    for _ in range(4):
+        for s in (ref, sim):
+            s.advance(5)
+        assert sim.history_overflow_count() == ref.history_overflow_count()
+    assert ref.history_overflow_count() > 1000 and sim.picard_counts()[1] > 0
     _same(ref, sim)

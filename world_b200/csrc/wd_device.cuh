@@ -32,7 +32,8 @@ enum Counter : int {
     kCntAutoSteps = 11,     // steps on the library's own lists (neighbor_skin 0)
     kCntAutoBuilds = 12,    // builds that such steps decided
     kCntAutoCrowded = 13,   // a build found a cell that could overfill
-    kNumCounters = 14,
+    kCntHistBefore = 14,    // kCntHistOverflow when a Picard step on lists began
+    kNumCounters = 15,
 };
 
 // Everything a step kernel needs, passed by value (baked into the captured graph).

@@ -107,6 +107,7 @@ __global__ void k_list_decide(uint32_t* __restrict__ ctrl, float thr, int always
                               cudaGraphConditionalHandle cond) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const bool build = list_decide_core(ctrl, thr, always_exact, counters, pend, false, 0);
+    if (always_exact) counters[kCntHistBefore] = counters[kCntHistOverflow];  // a Picard step begins
     if (use_cond) cudaGraphSetConditional(cond, build ? 1u : 0u);
 }
 
@@ -1184,6 +1185,7 @@ __global__ void k_list_picard_check(uint32_t* __restrict__ ctrl,
     if (redo) {
         ctrl[kLcForce] = 1u;  // the redo re-sorts the state: build next step
         counters[kCntPicardRedos] += 1ull;
+        counters[kCntHistOverflow] = counters[kCntHistBefore];  // the redo counts its own
     }
     if (use_cond) cudaGraphSetConditional(cond, redo ? 1u : 0u);
 }
