@@ -659,6 +659,8 @@ __device__ __forceinline__ void list_grain(const DevParams& P0, const ListArgs& 
         if (A.iter > 0) {
             const float ex = pi.x - xb.x, ey = pi.y - xb.y, ez = pi.z - xb.z;
             viol |= !(ex * ex + ey * ey + ez * ez < A.viol_thr);
+            // an overflowed list's grain walks the run table, which is that of the step's start
+            viol |= cnt > kNbrCap;
         }
     }
     if (BATCH && P.frozen) {
@@ -1320,7 +1322,7 @@ __device__ __forceinline__ void coop_slot(const DevParams& P0, const ListArgs& A
         if (A.iter > 0) {
             const float4 xb = A.xbuild[s], x = S.pos[g];
             const float ex = x.x - xb.x, ey = x.y - xb.y, ez = x.z - xb.z;
-            viol |= !(ex * ex + ey * ey + ez * ez < A.viol_thr);
+            viol |= !(ex * ex + ey * ey + ez * ez < A.viol_thr) || cnt > kNbrCap;
         }
     }
     if (work) {
