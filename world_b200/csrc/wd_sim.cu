@@ -2926,6 +2926,36 @@ int wd_set_neighbor_skin(wd_sim* sim, float skin) {
     return apply_skin(sim, skin);
 }
 
+// What the tuner puts back: the state, and in `rhs` the accelerations (pos) of the last step with
+// the velocities and ids that go with them.
+static cudaError_t tuner_take(wd_sim* s, wd_sim::Snap& snap, wd_sim::Snap& rhs) {
+    const size_t n = static_cast<size_t>(s->n);
+    const bool kept = s->lists && s->picard;
+    cudaError_t e = alloc_snap(s, snap);
+    if (e == cudaSuccess) e = dalloc_missing(s, &rhs.pos, n);
+    if (e == cudaSuccess) e = dalloc_missing(s, &rhs.vel, n);
+    if (e == cudaSuccess) e = dalloc_missing(s, &rhs.ids, n);
+    if (e == cudaSuccess) e = take_snap(s, snap);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(rhs.pos, s->acc, n * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(rhs.vel, kept ? s->rhs_vel : s->velB, n * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(rhs.ids, kept ? s->rhs_ids : s->idsB, n * sizeof(int), cudaMemcpyDeviceToDevice, s->stream);
+    return e;
+}
+
+static cudaError_t tuner_put_rhs(wd_sim* s, const wd_sim::Snap& rhs) {
+    if (!rhs.ids) return cudaSuccess;   // nothing was stepped
+    const size_t n = static_cast<size_t>(s->n);
+    const bool kept = s->lists && s->picard;
+    cudaError_t e = cudaMemcpyAsync(s->acc, rhs.pos, n * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(kept ? s->rhs_vel : s->velB, rhs.vel, n * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(kept ? s->rhs_ids : s->idsB, rhs.ids, n * sizeof(int), cudaMemcpyDeviceToDevice, s->stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(s->stream);
+}
+
 int wd_autotune(wd_sim* sim, int32_t steps, const char* cache_path, float* skin_out,
                 int32_t* block_out) {
     if (!sim || steps < 1) return fail(WD_ERR_INVALID, "wd_autotune: bad argument");
@@ -2933,6 +2963,9 @@ int wd_autotune(wd_sim* sim, int32_t steps, const char* cache_path, float* skin_
     float best_skin = sim->cfg.neighbor_skin;
     int best_block = sim->force_block;
     int best_minb = sim->force_minb;
+    const float skin0 = best_skin;
+    const int block0 = best_block, minb0 = best_minb;
+    wd_sim::Snap rhs;
     bool cached = false;
     if (cache_path) {
         if (std::FILE* f = std::fopen(cache_path, "r")) {
@@ -2968,9 +3001,14 @@ int wd_autotune(wd_sim* sim, int32_t steps, const char* cache_path, float* skin_
         const int cands[][2] = {{128, 5}, {256, 5}, {128, 4}, {256, 4}, {256, 0}, {256, 1},
                                 {256, 2}};
         const int ncands = static_cast<int>(sizeof(cands) / sizeof(cands[0]));
+        // (the state, and the last step's right-hand side, which a state does not hold)
         wd_sim::Snap snap;
-        WD_CUDA(alloc_snap(sim, snap));
-        WD_CUDA(take_snap(sim, snap));
+        const cudaError_t taken = tuner_take(sim, snap, rhs);
+        if (taken != cudaSuccess) {
+            free_snap(snap);
+            free_snap(rhs);
+            WD_CUDA(taken);
+        }
         unsigned long long saved[wd::kNumCounters];
         WD_CUDA(cudaMemcpyAsync(saved, sim->counters, sizeof(saved), cudaMemcpyDeviceToHost, sim->stream));
         cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -3017,16 +3055,21 @@ int wd_autotune(wd_sim* sim, int32_t steps, const char* cache_path, float* skin_
         sim->no_chains = false;
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        if (rc == WD_OK) {
-            const cudaError_t e = put_snap(sim, snap);
-            if (e != cudaSuccess) rc = fail(WD_ERR_CUDA, cudaGetErrorString(e));
-        }
-        if (rc == WD_OK) {
-            cudaMemcpyAsync(sim->counters, saved, sizeof(saved), cudaMemcpyHostToDevice, sim->stream);
-            rc = sync_stream(sim);
-        }
+        // as it was, whatever became of the candidates
+        const cudaError_t e = put_snap(sim, snap);
+        if (e != cudaSuccess && rc == WD_OK) rc = fail(WD_ERR_CUDA, cudaGetErrorString(e));
+        cudaMemcpyAsync(sim->counters, saved, sizeof(saved), cudaMemcpyHostToDevice, sim->stream);
+        const int waited = sync_stream(sim);
+        if (rc == WD_OK) rc = waited;
         free_snap(snap);
-        if (rc) return rc;
+        if (rc) {
+            const std::string why = wd::last_error_cstr();
+            sim->force_block = block0;
+            sim->force_minb = minb0;
+            if (apply_skin(sim, skin0) == WD_OK) tuner_put_rhs(sim, rhs);
+            free_snap(rhs);
+            return fail(rc, why);
+        }
         if (cache_path) {
             if (std::FILE* f = std::fopen(cache_path, "a")) {
                 std::fprintf(f, "%s %.9g %d %d\n", key.c_str(), static_cast<double>(best_skin),
@@ -3036,7 +3079,10 @@ int wd_autotune(wd_sim* sim, int32_t steps, const char* cache_path, float* skin_
         }
     }
     rc = apply_skin(sim, best_skin);
+    const cudaError_t put = rc == WD_OK ? tuner_put_rhs(sim, rhs) : cudaSuccess;
+    free_snap(rhs);
     if (rc) return rc;
+    WD_CUDA(put);
     sim->force_block = best_block;
     sim->force_minb = best_minb;
     sim->graph_dirty = true;
