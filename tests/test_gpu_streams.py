@@ -59,3 +59,36 @@ def test_a_handle_is_whole_when_it_is_there():
     assert not busy.query()
     torch.cuda.synchronize()
     _same(ref, sim)
+
+
+def test_an_uploaded_tensor_is_read_before_its_memory_is_reused():
+    """The upload is queued behind other work on the handle's stream, and the tensor (here also
+    the contiguous copy that the call makes) is gone when the call returns."""
+    cfg, st, rad = _touching(98, False)
+    cfg.kernel_timing = False
+    sim = ParticleDynamics(cfg, state=st, radius=rad)
+    sim.set_state(-st)
+    stream = torch.cuda.ExternalStream(sim.stream_ptr())
+    by_column = torch.from_numpy(st).cuda().t().contiguous().t()
+    assert not by_column.is_contiguous()
+
+    def reuse():
+        out = [torch.full_like(by_column, 7.0, memory_format=torch.contiguous_format) for _ in range(4)]
+        torch.cuda.current_stream().synchronize()
+        return out
+
+    reuse()                                    # the kernels' first use loads them, which waits
+    sim.set_state_tensor(by_column * 1.0)
+    sim.set_state(-st)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(HALF_A_SECOND)
+    busy = torch.cuda.Event()
+    busy.record(stream)
+    sim.set_state_tensor(by_column)
+    sim.set_state_tensor(by_column * 1.0)
+    others = reuse()
+    assert not busy.query()
+    sim.synchronize()
+    del others
+    np.testing.assert_array_equal(sim.get_state().reshape(-1, 6), st)

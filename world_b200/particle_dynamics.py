@@ -56,6 +56,7 @@ class ParticleDynamics:
 
     def _attach(self, h: ctypes.c_void_p) -> None:
         self._h = h
+        self._torch_stream = None
         n64 = ctypes.c_int64()
         check(lib.wd_get_n(h, ctypes.byref(n64)))
         self.n = int(n64.value)
@@ -186,8 +187,15 @@ class ParticleDynamics:
 
     def set_state_tensor(self, t) -> None:
         import torch
+        t = t.contiguous()
         torch.cuda.current_stream().synchronize()
-        check(lib.wd_set_state_device(self._h, ptr(t.contiguous())))
+        check(lib.wd_set_state_device(self._h, ptr(t)))
+        # the copy is queued: the memory is not given to another tensor before it has been read
+        if t.is_cuda:
+            stream = self.stream_ptr()
+            if self._torch_stream is None or self._torch_stream.cuda_stream != stream:
+                self._torch_stream = torch.cuda.ExternalStream(stream)
+            t.record_stream(self._torch_stream)
 
     # -- reverse pass (CUDA tensors, AoS3 by grain id) ---------------------------------
     def set_contact_params(self, mu: float, restitution: float, k_n: float) -> None:
