@@ -92,3 +92,28 @@ def test_an_uploaded_tensor_is_read_before_its_memory_is_reused():
     sim.synchronize()
     del others
     np.testing.assert_array_equal(sim.get_state().reshape(-1, 6), st)
+
+
+@pytest.mark.parametrize("own", [False, True])
+def test_a_read_waits_for_work_queued_on_its_memory(own):
+    """The tensor that takes the state, the caller's or a new one, has memory that torch still
+    writes to or reads from."""
+    cfg, st, rad = _touching(99, False)
+    cfg.kernel_timing = False
+    sim = ParticleDynamics(cfg, state=st, radius=rad)
+    sim.synchronize()
+    out = torch.zeros(6 * sim.n, device="cuda")
+    seen = torch.empty_like(out)
+    seen.copy_(out)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(HALF_A_SECOND)
+    if own:
+        out.fill_(7.0)
+        got = sim.state_tensor(out)
+    else:
+        seen.copy_(out)
+        del out
+        got = sim.state_tensor()
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(got.cpu().numpy().reshape(-1, 6), st)
+    assert own or not seen.any()

@@ -181,6 +181,8 @@ class ParticleDynamics:
         import torch
         if out is None:
             out = torch.empty(6 * self.n, dtype=torch.float32, device="cuda")
+        # work that torch has queued on this memory, or on a tensor that had it before
+        torch.cuda.current_stream().synchronize()
         check(lib.wd_get_state_device(self._h, ptr(out)))
         check(lib.wd_synchronize(self._h))
         return out
