@@ -334,8 +334,8 @@ int wd_list_exact_count(wd_sim* sim, int64_t* steps);
 int wd_list_resort_count(wd_sim* sim, int64_t* grains);
 /* Backward Euler / Picard: iterations executed so far (iterations that a converged
  * step skipped are not counted), and, on Verlet lists, the steps whose iterate went
- * beyond the lists' validity bound and that were redone with the per-iteration search
- * (their iterations count twice). */
+ * beyond the lists' validity bound, or whose lists overflowed, and that were redone with the
+ * per-iteration search (their iterations count twice). */
 int wd_picard_counts(wd_sim* sim, int64_t* iterations, int64_t* redos);
 /* Verlet lists (simulation.neighbor_skin > 0): builds so far, kernels one build
  * launches, and the mean list length of the last build (0 without lists). */

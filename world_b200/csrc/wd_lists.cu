@@ -21,8 +21,9 @@
 //
 // Picard iterates every force evaluation of a step on the same lists. Builds start at
 // 0.30 skin instead of 0.49, and each iteration checks that its input iterate is still
-// within 0.49 skin of the build; if one is not, the step is redone from its start
-// state with the per-iteration search, so the results stay those of the searched step.
+// within 0.49 skin of the build; if one is not, or if a list overflowed, the step is redone
+// from its start state with the per-iteration search, so the results stay those of the
+// searched step.
 #include <algorithm>
 #include <type_traits>
 
