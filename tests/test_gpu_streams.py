@@ -117,3 +117,20 @@ def test_a_read_waits_for_work_queued_on_its_memory(own):
     torch.cuda.synchronize()
     np.testing.assert_array_equal(got.cpu().numpy().reshape(-1, 6), st)
     assert own or not seen.any()
+
+
+@pytest.mark.parametrize("wait", [False, True])
+def test_an_uploaded_tensor_may_outlive_the_handle(wait):
+    cfg, st, rad = _touching(99, False)
+    cfg.kernel_timing = False
+    kept = torch.from_numpy(st).cuda()
+    for _ in range(3):
+        sim = ParticleDynamics(cfg, state=st, radius=rad)
+        sim.set_state_tensor(kept)
+        sim.set_state_tensor(kept * 1.0)
+        if wait:
+            sim.synchronize()
+        sim.close()
+    del kept
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()

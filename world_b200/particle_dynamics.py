@@ -14,6 +14,7 @@ access, and the parity probes (cell keys, sorted order, candidate lists).
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 from typing import Optional
 
@@ -57,6 +58,7 @@ class ParticleDynamics:
     def _attach(self, h: ctypes.c_void_p) -> None:
         self._h = h
         self._torch_stream = None
+        self._uploads = collections.deque()   # (event, tensor) of uploads that may be queued
         n64 = ctypes.c_int64()
         check(lib.wd_get_n(h, ctypes.byref(n64)))
         self.n = int(n64.value)
@@ -99,8 +101,9 @@ class ParticleDynamics:
     # -- lifetime --------------------------------------------------------------------
     def close(self) -> None:
         if getattr(self, "_h", None) is not None and self._h.value:
-            lib.wd_destroy(self._h)
+            lib.wd_destroy(self._h)           # waits for the stream
             self._h = None
+            self._uploads.clear()
 
     def __del__(self):
         try:
@@ -143,6 +146,7 @@ class ParticleDynamics:
 
     def synchronize(self) -> None:
         check(lib.wd_synchronize(self._h))
+        self._uploads.clear()
 
     def picard_stats(self) -> tuple[int, float]:
         it = ctypes.c_int32()
@@ -184,7 +188,7 @@ class ParticleDynamics:
         # work that torch has queued on this memory, or on a tensor that had it before
         torch.cuda.current_stream().synchronize()
         check(lib.wd_get_state_device(self._h, ptr(out)))
-        check(lib.wd_synchronize(self._h))
+        self.synchronize()
         return out
 
     def set_state_tensor(self, t) -> None:
@@ -192,12 +196,15 @@ class ParticleDynamics:
         t = t.contiguous()
         torch.cuda.current_stream().synchronize()
         check(lib.wd_set_state_device(self._h, ptr(t)))
-        # the copy is queued: the memory is not given to another tensor before it has been read
-        if t.is_cuda:
-            stream = self.stream_ptr()
-            if self._torch_stream is None or self._torch_stream.cuda_stream != stream:
-                self._torch_stream = torch.cuda.ExternalStream(stream)
-            t.record_stream(self._torch_stream)
+        # the copy is queued: the tensor is kept until it has been read
+        stream = self.stream_ptr()
+        if self._torch_stream is None or self._torch_stream.cuda_stream != stream:
+            self._torch_stream = torch.cuda.ExternalStream(stream)
+        while self._uploads and self._uploads[0][0].query():
+            self._uploads.popleft()
+        read = torch.cuda.Event()
+        read.record(self._torch_stream)
+        self._uploads.append((read, t))
 
     # -- reverse pass (CUDA tensors, AoS3 by grain id) ---------------------------------
     def set_contact_params(self, mu: float, restitution: float, k_n: float) -> None:
