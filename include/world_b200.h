@@ -322,7 +322,8 @@ int wd_debug_stage_wait(wd_sim* sim, int32_t stall, int32_t wait_us);
 int wd_debug_graph_captures(wd_sim* sim, int64_t* captures);
 /* Test hook (no counterpart in the reference): as if a device-side launch, of a list build
  * or of a search's radix path, had failed. The next synchronizing call reports it once, as
- * WD_ERR_CUDA; nothing else changes. */
+ * WD_ERR_CUDA. The state is then invalid, slot order included: restore one as after
+ * wd_debug_stage_wait. (No step is in fact left out.) */
 int wd_debug_launch_failure(wd_sim* sim);
 /* Verlet lists: steps so far whose contact kernel measured the exact displacement
  * since the build (reading the build positions). The other steps decide on a bound:

@@ -7,8 +7,9 @@ import numpy as np
 import pytest
 
 from test_gpu_auto_lists import _touching
+from test_gpu_lists import _same
 from world_b200 import ParticleDynamics, SceneBatch, WorldError
-from world_b200._lib import check, lib
+from world_b200._lib import check, lib, ptr
 from world_b200.scenes import column_collapse
 
 pytestmark = pytest.mark.gpu
@@ -57,3 +58,30 @@ def test_reads_report_a_failed_launch_of_a_searched_step():
         with pytest.raises(WorldError, match="device-side graph launch failed"):
             read()
         read()
+
+
+@pytest.mark.parametrize("asynchronous", [False, True])
+@pytest.mark.parametrize("skin", [0.0, 0.5e-3])
+def test_a_handle_recovers_with_an_upload(skin, asynchronous):
+    """Steps after a lost one leave nothing to rely on: an upload starts from the order of the
+    grain ids and without springs, as a new handle does."""
+    cfg, st, rad = _touching(93, True)
+    cfg.kernel_timing = False
+    cfg.neighbor_skin = skin
+    sim = ParticleDynamics(cfg, state=st, radius=rad)
+    sim.set_neighbor_skin(skin)
+    sim.advance(200)
+    assert sim.get_history()[0].sum() > 0
+    check(lib.wd_debug_launch_failure(sim.handle))
+    with pytest.raises(WorldError, match="device-side graph launch failed"):
+        sim.synchronize()
+    if asynchronous:
+        check(lib.wd_set_state_async(sim.handle, ptr(st)))
+        sim.synchronize()
+    else:
+        sim.set_state(st)
+    assert sim.get_history()[0].sum() == 0
+    fresh = ParticleDynamics(cfg, state=st, radius=rad)
+    for s in (sim, fresh):
+        s.advance(60)
+    _same(fresh, sim)

@@ -1427,7 +1427,10 @@ int sync_stream(wd_sim* s) {
     WD_CUDA(cudaGetLastError());
     if (const uint32_t why = s->words->launch_failed) {
         // a list build, or a searched step's radix path, whose launch failed did not run
+        // (steps after it may have, so the slots' order, lists and springs need not belong
+        // together: the next state upload starts from a fresh slot order)
         s->words->launch_failed = 0u;
+        s->slots_invalid = true;
         WD_CUDA(request_list_build(s));
         return fail(WD_ERR_CUDA, std::string("list build or search: a device-side graph launch failed (") +
                                      cudaGetErrorName(static_cast<cudaError_t>(why)) +
@@ -2304,6 +2307,10 @@ int wd_set_state_async(wd_sim* sim, const float* state) {
     if (!sim || !state) return fail(WD_ERR_INVALID, "wd_set_state_async: NULL argument");
     int rc = io_setup(sim);
     if (rc) return rc;
+    if (sim->slots_invalid) {
+        rc = reset_slot_order(sim);
+        if (rc) return rc;
+    }
     const int i = sim->io_i;
     sim->io_i ^= 1;
     const size_t bytes = sizeof(float) * 6 * static_cast<size_t>(sim->n);
